@@ -47,6 +47,13 @@ struct xf_ctx {
 // Device workspace of at least `bytes` (nullptr when it cannot grow).
 void* xf_ctx_work(xf_ctx* ctx, size_t bytes);
 
+// Split of a grid's interior into the bricks of the resident CG (xf_cgc.cu):
+// state 0 not looked at, 1 valid, -1 the grid does not fit.
+struct xf_coop_plan {
+  int state, bi, bj, bk, mi, mj, mk, threads;
+  size_t smem;
+};
+
 struct xf_grid {
   xf_ctx* ctx;
   int n1, n2, n3;
@@ -71,6 +78,7 @@ struct xf_grid {
   double* diag;              // device, per cell: diagonal of the Laplace Actual row (fast FP64)
   int uniform;               // every separation of each axis is equal: coefficients are per-axis constants
   double ucx, ucy, ucz;      // then 1/h^2 per axis (== c?m[i] == c?p[i] for every interior index)
+  xf_coop_plan coop[2];      // FP64, mixed
   int lap_status, vardiv_status;
   int64_t lap_bad, vardiv_bad;
 };

@@ -47,6 +47,10 @@ void xf_cg_poly_first_launch(const xf_op* op, const float* r, float* w, const fl
 void xf_cg_poly_second_launch(const xf_op* op, const float* w, const float* r, float* z, const float coeffs[3]);
 void xf_cg_pq32_variant(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int variant);
 bool xf_cg_pqt_supported(const xf_grid* g);
+bool xf_cg_coop_supported(const xf_op* op, bool mixed);
+size_t xf_cg_coop_slots();
+int xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
+                      int maxit, int every);
 int xf_op_ready(const xf_op* op);
 int xf_op_jacobi(const xf_op* op, const double** dinv);
 
@@ -512,6 +516,49 @@ static int true_residual(const xf_op* op, const double* x, const double* b, doub
 }
 
 // ---------------------------------------------------------------------------
+// The whole CG solve as one resident kernel (xf_cgc.cu), for the grids that
+// fit the chip.  The kernel's own last residual is the true one except where
+// the solve broke off between two of them.
+static int solve_cg_coop(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec* bv, xf_solve_stats* st) {
+  xf_ctx* ctx = op->g->ctx;
+  DevScratch* S = ctx->scratch;
+  const int64_t n = op->g->ncell;
+  const bool mixed = o.precision == XF_PREC_MIXED;
+  double* x = (double*)xv->data;
+  const double* b = (const double*)bv->data;
+  Bufs B(ctx);
+  const int64_t words = mixed ? (n + 1) / 2 : n;
+  void* ex[2] = {B.get<double>(words, false), B.get<double>(words, false)};
+  double* slots = B.get<double>((int64_t)xf_cg_coop_slots(), false);
+  if (!ex[0] || !ex[1] || !slots) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate CG vectors");
+  k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit, o.replace_every, mixed ? 1 : 0);
+  int rc = xf_cg_coop_launch(op, x, b, ex, slots, mixed, o.rtol, o.maxit, o.replace_every);
+  if (rc) return rc;
+  long long I[16];
+  double D[32];
+  XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, S->iscalars, sizeof(I), cudaMemcpyDeviceToHost, ctx->stream));
+  XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars + 16, S->scalars + 32, sizeof(D), cudaMemcpyDeviceToHost, ctx->stream));
+  XF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  memcpy(I, ctx->host_scalars, sizeof(I));
+  memcpy(D, ctx->host_scalars + 16, sizeof(D));
+  if (I[I_ERR]) return xf_fail(ctx, XF_ERR_CUDA, "xf_solve: a wait of the resident CG ran out");
+  const double bb = D[D_BB - 32], rr = D[D_RR64 - 32];
+  double rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
+  st->status = (int)I[I_STATUS];
+  if (st->status == XF_NAN || st->status == XF_BREAKDOWN) {
+    double* tmp = B.get<double>(n, false);
+    if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate residual");
+    if ((rc = true_residual(op, x, b, tmp, &rel, nullptr))) return rc;
+  }
+  if (st->status == XF_OK && rel > o.rtol) st->status = I[I_IT] >= o.maxit ? XF_MAXIT : XF_STALL;
+  st->iterations = (int)I[I_IT];
+  st->replacements = (int)I[I_REPL];
+  st->reserved[0] = 2;
+  st->rel_resid = rel;
+  st->abs_resid = rel;
+  return XF_OK;
+}
+
 static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec* bv, xf_solve_stats* st) {
   xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
@@ -520,6 +567,10 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
   const bool mixed = o.precision == XF_PREC_MIXED;
   double* x = (double*)xv->data;
   const double* b = (const double*)bv->data;
+  // XF_PQ_FUSE and XF_PQT name kernels of the launch chain
+  if (o.precond != XF_PRECOND_CHEB && x != b && !getenv("XF_PQ_FUSE") && !getenv("XF_PQT") &&
+      xf_cg_coop_supported(op, mixed))
+    return solve_cg_coop(op, o, xv, bv, st);
   Bufs B(ctx);
   const int rb = red_blocks(ctx, n), eb = grid_blocks(ctx, n, 256);
   const int xb32 = xr_blocks<float>(ctx, n), xb64 = xr_blocks<double>(ctx, n);
