@@ -255,8 +255,8 @@ typedef struct {
   double atol;           /* absolute tolerance of the reference-semantics methods; */
                          /* <= 0 means the reference's hard-coded value            */
   int replace_every;     /* mixed: true-residual replacement period (50)           */
-  int check_every;       /* host polls the device convergence flag every this     */
-                         /* many iterations (16)                                   */
+  int check_every;       /* accepted, without effect: the host watches a word that  */
+                         /* the device writes at the end of every iteration (16)   */
   int exact;             /* reference-semantics methods: use XF_EXACT matvecs      */
   int reserved[7];
 } xf_solve_opts;

@@ -30,6 +30,7 @@ struct DevScratch {
   unsigned int tickets[NUM_SLOTS];
   double scalars[256];
   long long iscalars[64];
+  volatile long long* progress;   // pinned host word: ends of iterations seen, bit 62 once the solve is done
 };
 
 struct xf_ctx {
@@ -111,6 +112,10 @@ struct xf_op {
   // the exact form)
   mutable double* adc64 = nullptr;
   mutable int adc_valid = 0;
+  // per cell, with the table: the neighbours its row reads (bits 0..5, x- to
+  // z+), AD_ROW for a row, AD_OBLIQUE for one that is not of seven points
+  mutable uint8_t* adk = nullptr;
+  mutable int adv32_valid = 0;   // the FP32 copies are made on first use
   // and the inverse row diagonals (0 off the active set), for the Jacobi
   // preconditioner of BiCGStab, refreshed with the table
   mutable double* adj64 = nullptr;
@@ -259,9 +264,40 @@ __device__ inline double block_sum(double v, double* sh) {
   return v;
 }
 
+// Sums of NV values a thread over a block of at most RED_THREADS threads,
+// valid in thread 0: the threads' values go through shared memory and a warp a
+// value adds them.  With every warp adding its own lanes by shuffles, the FP64
+// pipe (16 cycles an instruction here) spent as much on a block's sums as on
+// half a row a thread: 45 additions a value and block instead of 12.
+template <int NV>
+__device__ inline void block_sums(const double (&v)[NV], double (&out)[NV]) {
+  __shared__ double buf[NV * RED_THREADS];
+  const int n = blockDim.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = n >> 5;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; q++) buf[q * RED_THREADS + threadIdx.x] = v[q];
+  __syncthreads();
+  for (int q = w; q < NV; q += nw) {
+    double a = 0.0, b = 0.0;
+    for (int t = lane; t < n; t += 64) {
+      a += buf[q * RED_THREADS + t];
+      if (t + 32 < n) b += buf[q * RED_THREADS + t + 32];
+    }
+    a = warp_sum(a + b);
+    __syncwarp();
+    if (lane == 0) buf[q * RED_THREADS] = a;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; q++) out[q] = buf[q * RED_THREADS];
+}
+
 template <>
-__device__ inline double block_sum_acc<double>(const DotAcc<double>& acc, double* sh) {
-  return block_sum(acc.value(), sh);
+__device__ inline double block_sum_acc<double>(const DotAcc<double>& acc, double*) {
+  const double v[1] = {acc.value()};
+  double s[1];
+  block_sums<1>(v, s);
+  return s[0];
 }
 
 // Publishes one accumulator into partials[slot] under tickets[ticket]; true in
@@ -282,13 +318,12 @@ __device__ inline bool publish_acc(DevScratch* S, int slot, int ticket, const Do
 // Publishes this block's partial of `nval` sums into slot partials and returns
 // true in the last block to arrive (all partials visible).  `flag` is shared.
 template <int NV>
-__device__ inline bool publish_partials(DevScratch* S, int slot0, const double (&v)[NV], double* sh, bool* flag) {
-#pragma unroll
-  for (int q = 0; q < NV; q++) {
-    double s = block_sum(v[q], sh);
-    if (threadIdx.x == 0) S->partials[slot0 + q][lin_block()] = s;
-  }
+__device__ inline bool publish_partials(DevScratch* S, int slot0, const double (&v)[NV], double*, bool* flag) {
+  double s[NV];
+  block_sums<NV>(v, s);
   if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; q++) S->partials[slot0 + q][lin_block()] = s[q];
     __threadfence();
     unsigned int t = atomicAdd(&S->tickets[slot0], 1u);
     *flag = (t == (unsigned)num_blocks() - 1);

@@ -23,13 +23,16 @@ enum {
 // I_PBUF: which of the two direction buffers holds the current p (fused FP32
 // iteration).  I_ERR: a bounded wait in a staged kernel ran out.  I_PFIRST:
 // the preconditioned CG's next (r, z) starts the direction (beta = 0).
-enum { I_DONE = 0, I_STATUS, I_IT, I_REPL, I_NEEDREP, I_MAXIT, I_REPEVERY, I_MIXED, I_PAUSE, I_PBUF, I_ERR, I_PFIRST };
+// I_NOTE: tell the host (DevScratch::progress) how many iterations have ended,
+// I_ENDS, and when the solve is done.
+enum { I_DONE = 0, I_STATUS, I_IT, I_REPL, I_NEEDREP, I_MAXIT, I_REPEVERY, I_MIXED, I_PAUSE, I_PBUF, I_ERR, I_PFIRST,
+       I_NOTE, I_ENDS };
 
 enum {
   CTL_NONE = 0,
   CTL_CG_INIT, CTL_CG_ALPHA, CTL_CG_BETA, CTL_MIXED_REPL, CTL_CG_BETA_FLIP, CTL_CG_ALPHA_FLIP,
   CTL_RCG_INIT, CTL_RCG_TAU0, CTL_RCG_RES0, CTL_RCG_TAU, CTL_RCG_RES,
-  CTL_BCGS_NORM0, CTL_BCGS_PN1, CTL_BCGS_AN, CTL_BCGS_WN, CTL_BCGS_END,
+  CTL_BCGS_NORM0, CTL_BCGS_AN, CTL_BCGS_WN, CTL_BCGS_END,
   CTL_MR_INIT, CTL_MR_ALFA, CTL_MR_RES,
   CTL_BICG_INIT, CTL_BICG_ALPHA, CTL_BICG_BETA,
   CTL_PCG_BETA, CTL_PCG_ALPHA_FLIP, CTL_PCG_RR, CTL_PCG_REPL, CTL_PCG_RR_BETA
@@ -54,6 +57,20 @@ struct MvReq {
 __device__ inline void finish(DevScratch* S, long long status) {
   S->iscalars[I_DONE] = 1;
   S->iscalars[I_STATUS] = status;
+}
+
+// The scalars of BiCGStab's next iteration (XSLAE.cpp:718-722): Pn1 = (sRn, Rn) from SL_A, bn.
+__device__ inline void bcgs_next(DevScratch* S) {
+  double* d = S->scalars;
+  const double pn1 = d[SL_A];
+  S->iscalars[I_IT] += 1;
+  d[D_PN1] = pn1;
+  d[D_BN] = (pn1 / d[D_PN]) * (d[D_AN] / d[D_WN]);
+}
+
+// Whether a control step is the last of an iteration.
+__device__ inline bool ends_iteration(int ctl) {
+  return ctl == CTL_CG_BETA || ctl == CTL_RCG_RES || ctl == CTL_BCGS_END || ctl == CTL_MR_RES || ctl == CTL_BICG_BETA;
 }
 
 // Reliable updates of the preconditioned mixed CG: the FP32 recursion pauses
@@ -220,18 +237,12 @@ __device__ inline void control_step(DevScratch* S, int ctl) {
       break;
     }
     // ---- TSLAE::SolveByBiConjugateGradientsStab (XSLAE.cpp:667-768) --------
-    case CTL_BCGS_NORM0: {  // SL_D: absmax(Rn)
+    case CTL_BCGS_NORM0: {  // SL_D: absmax(Rn), SL_A: (sRn, Rn)
       d[D_PN] = 1; d[D_AN] = 1; d[D_BN] = 1; d[D_WN] = 1;
       d[D_NORM] = d[SL_D];
       I[I_IT] = 0; I[I_DONE] = 0; I[I_STATUS] = XF_OK;
       if (!(d[D_NORM] > d[D_EPS])) finish(S, isnan(d[D_NORM]) ? XF_NAN : XF_OK);
-      break;
-    }
-    case CTL_BCGS_PN1: {  // SL_A: (sRn, Rn)
-      double pn1 = d[SL_A];
-      I[I_IT] += 1;
-      d[D_PN1] = pn1;
-      d[D_BN] = (pn1 / d[D_PN]) * (d[D_AN] / d[D_WN]);
+      else bcgs_next(S);
       break;
     }
     case CTL_BCGS_AN: {  // SL_A: (sRn, Vn)
@@ -242,12 +253,13 @@ __device__ inline void control_step(DevScratch* S, int ctl) {
       d[D_WN] = d[SL_A] / d[SL_A + 1];
       break;
     }
-    case CTL_BCGS_END: {  // SL_D: absmax(Rn)
+    case CTL_BCGS_END: {  // SL_D: absmax(Rn), SL_A: (sRn, Rn)
       d[D_PN] = d[D_PN1];
       d[D_NORM] = d[SL_D];
       if (isnan(d[D_NORM])) finish(S, XF_NAN);
       else if (!(d[D_NORM] > d[D_EPS])) finish(S, XF_OK);
       else if (I[I_IT] >= I[I_MAXIT]) finish(S, XF_MAXIT);
+      else bcgs_next(S);
       break;
     }
     // ---- TSLAE::SolveByMinimalResiduals (XSLAE.cpp:350-414) ----------------
@@ -300,6 +312,10 @@ __device__ inline void control_step(DevScratch* S, int ctl) {
       break;
     }
     default: break;
+  }
+  if (I[I_NOTE] && ctl != CTL_NONE) {
+    if (ends_iteration(ctl)) I[I_ENDS] += 1;
+    *S->progress = I[I_ENDS] | (I[I_DONE] ? 1ll << 62 : 0);
   }
 }
 

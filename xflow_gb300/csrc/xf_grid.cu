@@ -62,6 +62,8 @@ extern "C" int xf_create(int device, xf_ctx** out) {
   if (cudaMalloc(&ctx->scratch, sizeof(DevScratch)) != cudaSuccess) { delete ctx; return XF_ERR_NOMEM; }
   cudaMemsetAsync(ctx->scratch, 0, sizeof(DevScratch), ctx->stream);
   if (cudaMallocHost(&ctx->host_scalars, 256 * sizeof(double)) != cudaSuccess) { delete ctx; return XF_ERR_NOMEM; }
+  volatile long long* progress = (volatile long long*)(ctx->host_scalars + 255);
+  cudaMemcpyAsync((void*)&ctx->scratch->progress, &progress, sizeof(progress), cudaMemcpyHostToDevice, ctx->stream);
   cudaEventCreate(&ctx->ev0);
   cudaEventCreate(&ctx->ev1);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { delete ctx; return XF_ERR_CUDA; }

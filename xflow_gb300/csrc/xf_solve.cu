@@ -52,6 +52,7 @@ size_t xf_cg_coop_slots();
 int xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
                       int maxit, int every);
 int xf_op_ready(const xf_op* op);
+void xf_op_ready32(const xf_op* op);
 int xf_op_jacobi(const xf_op* op, const double** dinv);
 
 #define GUARD_DONE(S) \
@@ -258,39 +259,53 @@ __global__ void k_bcgs_s(double* __restrict__ Sn, const double* __restrict__ Rn,
   }
 }
 
-__device__ __forceinline__ double max_nan_skip(double a, double b) { return b > a ? b : a; }
-__device__ double block_max(double v, double* sh) {
+// max |r| as an integer maximum of the bits (NaN never wins, XSpace.cpp:
+// 3455-3463): a double comparison would cost the FP64 pipe as much as an FMA.
+__device__ __forceinline__ unsigned long long absmax_bits(unsigned long long best, double r) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+  return b > best && b <= 0x7ff0000000000000ull ? b : best;
+}
+__device__ unsigned long long block_max_bits(unsigned long long v, unsigned long long* sh) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max_nan_skip(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
+    v = u > v ? u : v;
+  }
   __syncthreads();
   if (lane == 0) sh[w] = v;
   __syncthreads();
   const int nw = (blockDim.x + 31) >> 5;
-  v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
+  v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0ull;
   if (w == 0)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max_nan_skip(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
+      v = u > v ? u : v;
+    }
   return v;
 }
 
-// XSLAE.cpp:738-749: Un += an*Pn1 + wn*Sn; Rn = Sn - wn*Tn; Pn = Pn1 (no
-// copy when Pn is null: the caller alternates the two direction buffers);
-// then ||Rn||_inf (NaN never wins, XSpace.cpp:3455-3463) with control `ctl`.
-// With a Jacobi preconditioner Un moves along the preconditioned vectors:
-// Un += an*Ph + wn*Sh (Xp, Xs; otherwise Pn1 and Sn).
+// XSLAE.cpp:738-749: Un += an*Pn1 + wn*Sn; Rn = Sn - wn*Tn (the caller
+// alternates the two direction buffers, so there is no Pn = Pn1 copy); then
+// ||Rn||_inf -> SL_D and the next iteration's (sRn, Rn) -> SL_A with control
+// `ctl`.  With a Jacobi preconditioner Un moves along the preconditioned
+// vectors: Un += an*Ph + wn*Sh (Xp, Xs; otherwise Pn1 and Sn).
 template <bool EXACT>
 __global__ void __launch_bounds__(RED_THREADS) k_bcgs_end(double* __restrict__ Un, double* __restrict__ Rn,
-                                                          double* __restrict__ Pn, const double* __restrict__ Pn1,
+                                                          const double* __restrict__ Pn1,
                                                           const double* __restrict__ Sn, const double* __restrict__ Tn,
+                                                          const double* __restrict__ sRn,
                                                           const uint8_t* __restrict__ m, int64_t n, DevScratch* S,
                                                           int update, int ctl, const double* __restrict__ Xp = nullptr,
                                                           const double* __restrict__ Xs = nullptr) {
   __shared__ double sh[32];
+  __shared__ unsigned long long shm[32];
   __shared__ bool last;
   if (update) GUARD_DONE(S);
   const double an = S->scalars[D_AN], wn = S->scalars[D_WN];
-  double best = 0.0;
+  unsigned long long best = 0;
+  DotAcc<double> dot;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (!m[i]) continue;
     double r;
@@ -301,33 +316,27 @@ __global__ void __launch_bounds__(RED_THREADS) k_bcgs_end(double* __restrict__ U
       double t = wn * Tn[i];
       r = Sn[i] - t;
       Rn[i] = r;
-      if (Pn) Pn[i] = Pn1[i];
     } else if (update) {
       const double sn = Sn[i];
-      Un[i] = Un[i] + fma(an, Xp ? Xp[i] : Pn1[i], wn * (Xs ? Xs[i] : sn));
+      Un[i] = fma(an, Xp ? Xp[i] : Pn1[i], fma(wn, Xs ? Xs[i] : sn, Un[i]));
       r = fma(-wn, Tn[i], sn);
       Rn[i] = r;
-      if (Pn) Pn[i] = Pn1[i];
     } else {
       r = Rn[i];
     }
-    best = max_nan_skip(best, fabs(r));
+    best = absmax_bits(best, r);
+    dot.add(sRn[i], r);
   }
-  double bm = block_max(best, sh);
+  best = block_max_bits(best, shm);
+  if (threadIdx.x == 0) S->partials[SL_D][blockIdx.x] = __longlong_as_double((long long)best);
+  if (!publish_acc<double>(S, SL_A, SL_D, dot, sh, &last)) return;
+  const double t = finish_partials(S, SL_A, sh);
+  best = 0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) best = absmax_bits(best, __ldcg(&S->partials[SL_D][b]));
+  best = block_max_bits(best, shm);
   if (threadIdx.x == 0) {
-    S->partials[SL_D][blockIdx.x] = bm;
-    __threadfence();
-    unsigned int t = atomicAdd(&S->tickets[SL_D], 1u);
-    last = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double q = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) q = max_nan_skip(q, __ldcg(&S->partials[SL_D][b]));
-  q = block_max(q, sh);
-  if (threadIdx.x == 0) {
-    S->scalars[SL_D] = q;
+    S->scalars[SL_A] = t;
+    S->scalars[SL_D] = __longlong_as_double((long long)best);
     S->tickets[SL_D] = 0;
     control_step(S, ctl);
   }
@@ -403,8 +412,10 @@ __global__ void k_bicg_p(double* __restrict__ pk, double* __restrict__ pt, const
     }
 }
 
-__global__ void k_reset_state(DevScratch* S, double rtol2, double eps, long long maxit, long long repevery, long long mixed) {
+__global__ void k_reset_state(DevScratch* S, double rtol2, double eps, long long maxit, long long repevery, long long mixed,
+                              int note = 0) {
   for (int q = 0; q < 16; q++) S->iscalars[q] = 0;
+  S->iscalars[I_NOTE] = note;
   S->iscalars[I_STATUS] = XF_OK;
   S->iscalars[I_MAXIT] = maxit;
   S->iscalars[I_REPEVERY] = repevery;
@@ -494,10 +505,53 @@ static int run_loop(xf_ctx* ctx, const std::function<void(int)>& iter, int chunk
   return rs;
 }
 
-static double read_scalar(xf_ctx* ctx, int idx) {
-  cudaMemcpyAsync(ctx->host_scalars, &ctx->scratch->scalars[idx], 8, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaStreamSynchronize(ctx->stream);
-  return ctx->host_scalars[0];
+// Runs `iter` (which enqueues one iteration of `launches` kernels) until the
+// device says done.  The iterations go straight to the stream, at most
+// `ahead` of them before the device has ended them: the control step of an
+// iteration's last kernel writes to a pinned host word, which this thread
+// watches.  So no graph is captured and instantiated for a solve of a few
+// iterations, and past the last one only `ahead` iterations' kernels are left
+// to find the solve done (a graph of 16 iterations, two of them in flight, ran
+// 20 iterations too many of the 12 of a momentum solve).
+static int run_stream(xf_ctx* ctx, const std::function<void(int)>& iter, int launches, int ahead, long long maxit,
+                      HostState* hs) {
+  volatile long long* progress = (volatile long long*)(ctx->host_scalars + 255);
+  const long long done = 1ll << 62;
+  long long queued = 0;
+  cudaError_t ce;
+  while (queued < maxit + ahead) {
+    auto wait = [&]() {
+      const long long p = *progress;
+      return !(p & done) && queued - p >= ahead;
+    };
+    for (unsigned spin = 1; wait(); spin++) {
+      if (spin & 0xfff) continue;
+      // an error ends the solve, and so does a stream that has run all that was queued and still waits
+      ce = cudaStreamQuery(ctx->stream);
+      if (ce == cudaErrorNotReady) continue;
+      if (ce == cudaSuccess && !wait()) break;
+      if (ce == cudaSuccess) ce = cudaGetLastError();
+      return xf_fail(ctx, XF_ERR_CUDA, "solver iteration: %s", ce == cudaSuccess ? "no progress" : cudaGetErrorString(ce));
+    }
+    if (*progress & done) break;
+    iter((int)(queued & 1));
+    queued++;
+  }
+  XF_CUDA(ctx, cudaGetLastError());
+  const long long kernels = hs->kernels + queued * launches;
+  const int rs = read_state(ctx, hs);
+  hs->kernels = kernels;
+  return rs;
+}
+// Before the first launch of a solve that run_stream drives.
+static void reset_progress(xf_ctx* ctx) { *(volatile long long*)(ctx->host_scalars + 255) = 0; }
+constexpr int STREAM_AHEAD = 3;
+
+static int read_scalars(xf_ctx* ctx) {   // all of them, into the pinned buffer
+  XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, ctx->scratch->scalars, 128 * sizeof(double), cudaMemcpyDeviceToHost,
+                               ctx->stream));
+  XF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return XF_OK;
 }
 
 // True relative residual ||b - A x||_2 / ||b||_2 in FP64 (fast rows).
@@ -509,7 +563,9 @@ static int true_residual(const xf_op* op, const double* x, const double* b, doub
   q.x = x; q.y = tmp; q.s = b; q.sign = -1; q.neg = 1; q.zero_inactive = 1; q.dot_self = 1; q.slot = SL_C;
   xf_mv64(op, q);
   XF_CUDA(ctx, cudaGetLastError());
-  double bb = read_scalar(ctx, SL_B), rr = read_scalar(ctx, SL_C + 1);
+  int rc = read_scalars(ctx);
+  if (rc) return rc;
+  const double bb = ctx->host_scalars[SL_B], rr = ctx->host_scalars[SL_C + 1];
   *rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
   if (bbout) *bbout = bb;
   return XF_OK;
@@ -605,10 +661,12 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
   double* tmp = B.get<double>(n, false);
   if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate residual");
   for (int attempt = 0; attempt < 3; attempt++) {
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit - total_it, o.replace_every, mixed ? 1 : 0);
+    reset_progress(ctx);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit - total_it, o.replace_every, mixed ? 1 : 0,
+                                            mixed ? 0 : 1);
     k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(b, b, g->smask, n, S, SL_B, CTL_NONE, 0);
     std::function<void(int)> iter;
-    int chunk = o.check_every > 0 ? o.check_every : 16;
+    int chunk = o.replace_every;
     const bool lap = op->kind == XF_OP_LAPLACE;
     if (!mixed) {
       MvReq<double> m0;
@@ -642,7 +700,6 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
       // quadratic factor of p: w = p_m(A) r (fused with K2 as above), m - 2
       // passes w <- p_k(A) w, and z = p_1(A) w with (r, z).  XF_POLYR=0 runs
       // K2 and K0 as separate launches.
-      chunk = o.replace_every;
       float *e = e32, *r = r32, *pa = p32, *q = q32, *z = z32;
       float *pb = p32b, *rb = r32b, *w = w32, *wb = w32b;
       const bool fused = !(getenv("XF_POLYR") && getenv("XF_POLYR")[0] == '0');
@@ -707,7 +764,6 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
       // chunk = `replace_every` iterations; its last iteration folds the FP32
       // correction into x and replaces r by the true FP64 residual, whose
       // beta the next K1 uses.
-      chunk = o.replace_every;
       float *e = e32, *r = r32, *pa = p32, *q = q32;
       float* pb = p32b;
       XF_CUDA(ctx, cudaMemsetAsync(e, 0, n * 4, ctx->stream));
@@ -726,7 +782,6 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
     } else {
       // One graph chunk = `replace_every` iterations; its last iteration folds
       // the FP32 correction into x and replaces r by the true FP64 residual.
-      chunk = o.replace_every;
       float *e = e32, *r = r32, *p = p32, *q = q32;
       XF_CUDA(ctx, cudaMemsetAsync(e, 0, n * 4, ctx->stream));
       MvReq<double> m0;
@@ -758,8 +813,10 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
         k_cg_p<float><<<eb, 256, 0, ctx->stream>>>(p, r, n, S, c == last ? 1 : 0);
       };
     }
+    if (mixed) xf_op_ready32(op);   // not inside the captured iterations
     XF_CUDA(ctx, cudaGetLastError());
-    int rc = run_loop(ctx, iter, chunk, o.maxit - total_it, &hs);
+    int rc = mixed ? run_loop(ctx, iter, chunk, o.maxit - total_it, &hs)
+                   : run_stream(ctx, iter, 3, STREAM_AHEAD, o.maxit - total_it, &hs);
     if (rc) return rc;
     total_it += (int)hs.it;
     total_repl += (int)hs.repl;
@@ -796,12 +853,13 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
   Bufs B(ctx);
   const int rb = red_blocks(ctx, n), eb = grid_blocks(ctx, n, 256);
   std::function<void(int)> iter;
-  bool even_chunks = false;   // the iteration alternates buffers by parity
+  int launches = 0;   // kernels an iteration
+  reset_progress(ctx);
   HostState hs = {0, 0, 0, 0, 0};
   double eps = o.atol;
   if (o.method == XF_CG_REFERENCE) {
     if (eps <= 0) eps = 1e-5;   // XSLAE.cpp:64
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0, 1);
     // xk_1 = copy(x) (whole box); rk_1 = A(xk_1) - b; (rk_1, rk_1)
     double* xk_1 = B.get<double>(n, false);
     double* rk = B.get<double>(n);
@@ -820,6 +878,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     MvReq<double> q2;
     q2.x = x; q2.y = rk; q2.s = b; q2.sign = -1; q2.dot_self = 1; q2.exact = exact; q2.slot = SL_A; q2.ctl = CTL_RCG_RES0;
     xf_mv64(op, q2);
+    launches = 3;
     iter = [=](int) {
       MvReq<double> a;
       a.x = rk; a.w = rk; a.exact = exact; a.slot = SL_A; a.ctl = CTL_RCG_TAU;
@@ -831,7 +890,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     };
   } else if (o.method == XF_BICGSTAB) {
     if (eps <= 0) eps = 1e-5;   // XSLAE.cpp:669
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0, 1);
     double *Rn = B.get<double>(n), *sRn = B.get<double>(n), *Pn = B.get<double>(n), *Pn1 = B.get<double>(n);
     double *Vn = B.get<double>(n), *Sn = B.get<double>(n), *Tn = B.get<double>(n);
     if (!Rn || !sRn || !Pn || !Pn1 || !Vn || !Sn || !Tn) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
@@ -840,7 +899,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     q0.x = x; q0.y = Rn; q0.s = b; q0.sign = -1; q0.neg = 1; q0.exact = exact;
     xf_mv64(op, q0);
     XF_CUDA(ctx, cudaMemcpyAsync(sRn, Rn, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_bcgs_end<true><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, Pn, Pn1, Sn, Tn, m, n, S, 0, CTL_BCGS_NORM0);
+    k_bcgs_end<true><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, Pn1, Sn, Tn, sRn, m, n, S, 0, CTL_BCGS_NORM0);
     // Jacobi (XF_PRECOND_JACOBI; Laplace and advection-diffusion operators): right
     // preconditioning by the inverse row diagonals, so A sees dinv p and
     // dinv s, x moves along them, and the residual stays b - A x.  It evens
@@ -858,12 +917,11 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
       return xf_fail(ctx, XF_ERR_UNSUPPORTED, "xf_solve: BiCGStab takes XF_PRECOND_JACOBI or none");
     }
     // the previous direction and the new one alternate between Pn and Pn1 with
-    // the iteration's parity (chunks of an even number of iterations)
-    even_chunks = true;
+    // the iteration's parity
+    launches = 5;
     iter = [=](int it) {
       double* Pold = (it & 1) ? Pn1 : Pn;
       double* Pnew = (it & 1) ? Pn : Pn1;
-      k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(sRn, Rn, m, n, S, SL_A, CTL_BCGS_PN1, 1);
       if (exact) k_bcgs_p<true><<<eb, 256, 0, ctx->stream>>>(Pnew, Rn, Pold, Vn, m, n, S, dinv, Ph);
       else k_bcgs_p<false><<<eb, 256, 0, ctx->stream>>>(Pnew, Rn, Pold, Vn, m, n, S, dinv, Ph);
       MvReq<double> a;
@@ -874,19 +932,20 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
       MvReq<double> c;
       c.x = dinv ? Sh : Sn; c.y = Tn; c.w = Sn; c.dot_self = 1; c.exact = exact; c.slot = SL_A; c.ctl = CTL_BCGS_WN;
       xf_mv64(op, c);
-      if (exact) k_bcgs_end<true><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, nullptr, Pnew, Sn, Tn, m, n, S, 1,
+      if (exact) k_bcgs_end<true><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, Pnew, Sn, Tn, sRn, m, n, S, 1,
                                                                         CTL_BCGS_END, Ph, Sh);
-      else k_bcgs_end<false><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, nullptr, Pnew, Sn, Tn, m, n, S, 1,
-                                                                  CTL_BCGS_END, Ph, Sh);
+      else k_bcgs_end<false><<<rb, RED_THREADS, 0, ctx->stream>>>(x, Rn, Pnew, Sn, Tn, sRn, m, n, S, 1, CTL_BCGS_END,
+                                                                  Ph, Sh);
     };
   } else if (o.method == XF_MINRES) {
     if (eps <= 0) eps = 1e-7;   // XSLAE.cpp:358
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0, 1);
     double *rk = B.get<double>(n), *Ark = B.get<double>(n);
     if (!rk || !Ark) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
     MvReq<double> q0;
     q0.x = x; q0.y = rk; q0.s = b; q0.sign = -1; q0.dot_self = 1; q0.exact = exact; q0.slot = SL_A; q0.ctl = CTL_MR_INIT;
     xf_mv64(op, q0);
+    launches = 3;
     iter = [=](int) {
       MvReq<double> a;
       a.x = rk; a.y = Ark; a.w = rk; a.dot_self = 1; a.exact = exact; a.slot = SL_A; a.ctl = CTL_MR_ALFA;
@@ -902,12 +961,13 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     if (op->kind != XF_OP_PACK)
       return xf_fail(ctx, XF_ERR_UNSUPPORTED, "xf_solve: BiCG needs a packed operator (xf_pack_create) for A^T");
     if (eps <= 0) eps = 1e-8;   // XSLAE.cpp:166
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0, 1);
     double *rk = B.get<double>(n), *rt = B.get<double>(n), *pk = B.get<double>(n), *pt = B.get<double>(n);
     double *Ap = B.get<double>(n), *Atp = B.get<double>(n);
     if (!rk || !rt || !pk || !pt || !Ap || !Atp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
     k_bicg_init<<<eb, 256, 0, ctx->stream>>>(x, rk, rt, pk, pt, b, m, n);
     k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(rk, rk, m, n, S, SL_D, CTL_BICG_INIT, 0);
+    launches = 5;
     iter = [=](int) {
       k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(rk, rt, m, n, S, SL_B, CTL_NONE, 1);
       MvReq<double> a;
@@ -923,16 +983,14 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     return xf_fail(ctx, XF_ERR_UNSUPPORTED, "xf_solve: method %d not available", o.method);
   }
   XF_CUDA(ctx, cudaGetLastError());
-  int chunk = o.check_every > 0 ? o.check_every : 16;
-  if (even_chunks) chunk += chunk & 1;
-  int rc = run_loop(ctx, iter, chunk, o.maxit, &hs);
+  int rc = run_stream(ctx, iter, launches, STREAM_AHEAD, o.maxit, &hs);
   if (rc) return rc;
   double* tmp = B.get<double>(n, false);
   if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
-  double own = o.method == XF_BICGSTAB ? read_scalar(ctx, D_NORM) : read_scalar(ctx, D_EPSCUR);
   double rel = 0;
-  int r2 = true_residual(op, x, b, tmp, &rel, nullptr);
+  int r2 = true_residual(op, x, b, tmp, &rel, nullptr);   // leaves the scalars in the pinned buffer
   if (r2) return r2;
+  const double own = ctx->host_scalars[o.method == XF_BICGSTAB ? D_NORM : D_EPSCUR];
   st->status = (int)hs.status;
   st->iterations = (int)hs.it;
   st->rel_resid = rel;

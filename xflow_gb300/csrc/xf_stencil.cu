@@ -52,6 +52,7 @@ struct MatvecArgs {
   const double* __restrict__ diag;
   int sign, neg, zero_inactive, dot_w, dot_self;
   int slot_w, ctl, gate, chunk;
+  const uint8_t* __restrict__ use;   // k_ad_fast: xf_op::adk
   DevScratch* S;
 };
 
@@ -171,44 +172,66 @@ static void set_ad_fields(StencilGrid<T>& s, const xf_op* op) {
   s.adc_n = op->g->ncell;
 }
 
-// Per-axis factors of the fast coefficients, 5 per node m of each axis (the
-// halves folded in): 0.5/hx2, 0.5/h, 0.5 h/hxhxh, 0.5 hx2/hxhxh, 0.5 h_1/hxhxh
-// with h_1 = h[m-1], h = h[m], hx2 = h_1 + h, hxhxh = h_1 h hx2 / 2 (the exact
-// rows' quantities; nodes 0 and n-1, which carry no Actual row, get 0).
-__global__ void k_ad_axis(const double* __restrict__ h, int n, double* __restrict__ t) {
+// Per-axis factors of the fast coefficients, 5 arrays over the nodes m of an
+// axis (the halves and the two flags folded in): conv 0.5/hx2, conv 0.5/h,
+// diff 0.5 h/hxhxh, diff 0.5 hx2/hxhxh, diff 0.5 h_1/hxhxh with h_1 = h[m-1],
+// h = h[m], hx2 = h_1 + h, hxhxh = h_1 h hx2 / 2 (the exact rows' quantities;
+// nodes 0 and n-1, which carry no Actual row, get 0).
+__global__ void k_ad_axis(const double* __restrict__ h, int n, double conv, double diff, double* __restrict__ t) {
   for (int m = threadIdx.x; m < n; m += blockDim.x) {
     double r2 = 0, rh = 0, dA = 0, dB = 0, dC = 0;
     if (m >= 1 && m <= n - 2) {
       const double h_1 = h[m - 1], hh = h[m], hx2 = h_1 + hh, hxhxh = h_1 * hh * hx2 / 2;
-      r2 = 0.5 / hx2;
-      rh = 0.5 / hh;
-      dA = 0.5 * hh / hxhxh;
-      dB = 0.5 * hx2 / hxhxh;
-      dC = 0.5 * h_1 / hxhxh;
+      r2 = conv * (0.5 / hx2);
+      rh = conv * (0.5 / hh);
+      dA = diff * (0.5 * hh / hxhxh);
+      dB = diff * (0.5 * hx2 / hxhxh);
+      dC = diff * (0.5 * h_1 / hxhxh);
     }
-    t[5 * m] = r2; t[5 * m + 1] = rh; t[5 * m + 2] = dA; t[5 * m + 3] = dB; t[5 * m + 4] = dC;
+    t[m] = r2; t[n + m] = rh; t[2 * n + m] = dA; t[3 * n + m] = dB; t[4 * n + m] = dC;
   }
 }
 
-// A, B, C of one direction from the axis factors (central or upwind), as the
-// exact rows define them but with products for the divisions.
-__device__ __forceinline__ void ad_coef_fast(const double* __restrict__ t, double vd, double D, double conv,
-                                             double diff, bool upwind, double& A, double& B, double& C) {
-  const double dA = diff * (-D * t[2]), dB = diff * (D * t[3]), dC = diff * (-D * t[4]);
-  if (!upwind) {
-    A = conv * (-vd * t[0]) + dA;
-    B = dB;
-    C = conv * (vd * t[0]) + dC;
+struct AdAxis { double r2, rh, dA, dB, dC; };
+__device__ __forceinline__ AdAxis ad_axis(const double* __restrict__ t, int n, int m) {
+  return {__ldg(t + m), __ldg(t + n + m), __ldg(t + 2 * n + m), __ldg(t + 3 * n + m), __ldg(t + 4 * n + m)};
+}
+
+// A and C of one direction from the axis factors (central or upwind), as the
+// exact rows define them but with products for the divisions; B is added to
+// the centre.  5 FP64 operations a direction (7 upwind): the FP64 pipe bounds
+// the table's kernel.
+template <bool UP>
+__device__ __forceinline__ void ad_coef_fast(const AdAxis& t, double vd, double D, double& A, double& C, double& centre) {
+  A = -D * t.dA;
+  C = -D * t.dC;
+  centre = fma(D, t.dB, centre);
+  if (!UP) {
+    A = fma(-vd, t.r2, A);
+    C = fma(vd, t.r2, C);
   } else if (vd < 0) {
-    A = dA;
-    B = conv * (-vd * t[1]) + dB;
-    C = conv * (vd * t[1]) + dC;
+    centre = fma(-vd, t.rh, centre);
+    C = fma(vd, t.rh, C);
   } else {
-    A = conv * (-vd * t[1]) + dA;
-    B = conv * (vd * t[1]) + dB;
-    C = dC;
+    A = fma(-vd, t.rh, A);
+    centre = fma(vd, t.rh, centre);
   }
 }
+
+// 1/d by two Newton-Raphson steps y <- y + y (1 - d y) from the hardware's
+// approximation (2^-23 of it): 4 operations on the FP64 pipe where a division
+// takes three times as many.  Within a rounding of 1/d, for the
+// preconditioner; divided where the steps could leave the normal range.
+__device__ __forceinline__ double ad_reciprocal(double d) {
+  const int e = (__double2hiint(d) >> 20) & 0x7ff;
+  if (e < 64 || e > 1982) return d != 0 ? 1.0 / d : 0.0;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
+enum { AD_ROW = 64, AD_OBLIQUE = 128 };
 
 // The border rows in the same seven-coefficient form (centre, x-, x+, y-,
 // y+, z-, z+): a semi-sum row takes 1/2 of itself and of its neighbour
@@ -251,34 +274,72 @@ __device__ void ad_border_coeffs(const StencilGrid<double>& g, int64_t c, int ro
   }
 }
 
+// A unit probe at the row's own cell: a border row evaluated on it is the
+// row's diagonal coefficient.
+struct UnitProbe {
+  __device__ __forceinline__ double operator()(int a, int b, int d) const { return (a | b | d) == 0 ? 1.0 : 0.0; }
+};
+
+// A border row's part of the table: its coefficients, the neighbours it reads and its inverse diagonal.
+__device__ __noinline__ void ad_border_cell(const StencilGrid<double>& g, int64_t n, int64_t c, int row, int i, int j,
+                                            int k, double* __restrict__ out, uint8_t* __restrict__ use,
+                                            double* __restrict__ dinv) {
+  double q[7];
+  ad_border_coeffs(g, c, row, q);
+  uint8_t u = AD_ROW;
+  if (q[0] != q[0]) u |= AD_OBLIQUE;
+  for (int t = 0; t < 7; t++) {
+    out[t * n + c] = q[t];
+    if (t > 0 && q[t] != 0) u |= 1 << (t - 1);
+  }
+  use[c] = u;
+  const double d = boundary_row_acc<double, false>(g, UnitProbe{}, i, j, k, (int)c, row);
+  dinv[c] = d != 0 ? 1.0 / d : 0.0;
+}
+
 // The FP64 coefficient table of the fast rows: for Actual rows a centre
 // coefficient 1/tau + B_x + B_y + B_z and the six neighbour coefficients;
-// border rows as ad_border_coeffs.
-__global__ void k_ad_coeffs(StencilGrid<double> g, int64_t n, const double* __restrict__ tx,
-                            const double* __restrict__ ty, const double* __restrict__ tz, double* __restrict__ out) {
-  const bool up = g.ad_upwind != 0;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+// border rows as ad_border_coeffs; with it the bytes of the neighbours a row
+// reads and the inverse row diagonals (0 off the active set and where a
+// diagonal is 0; border rows: the row on a unit probe).  A thread owns a
+// (j, k) column and marches a chunk of planes with its y and z factors in
+// registers.
+constexpr int ADC_THREADS = 256, ADC_CHUNK = 8;
+template <bool UP>
+__global__ void __launch_bounds__(ADC_THREADS) k_ad_coeffs(StencilGrid<double> g, int64_t n,
+                                                           const double* __restrict__ tx, const double* __restrict__ ty,
+                                                           const double* __restrict__ tz, double* __restrict__ out,
+                                                           uint8_t* __restrict__ use, double* __restrict__ dinv) {
+  const int P = g.s1, p = blockIdx.x * ADC_THREADS + threadIdx.x;
+  if (p >= P) return;
+  const int j = p / g.n3, k = p - j * g.n3;
+  const AdAxis fy = ad_axis(ty, g.n2, j), fz = ad_axis(tz, g.n3, k);
+  const int i0 = blockIdx.y * ADC_CHUNK, i1 = min(g.n1, i0 + ADC_CHUNK);
+  for (int i = i0; i < i1; i++) {
+    const int64_t c = (int64_t)i * P + p;
     const int row = row_of(g.kind[c]);
-    if (row == ROW_NONE) continue;
-    if (row != ROW_ACTUAL) {
-      double q[7];
-      ad_border_coeffs(g, c, row, q);
-      for (int t = 0; t < 7; t++) out[t * n + c] = q[t];
+    if (row == ROW_NONE) {
+      use[c] = 0;
+      dinv[c] = 0.0;
       continue;
     }
-    const int i = (int)(c / g.s1), j = (int)((c - (int64_t)i * g.s1) / g.s2), k = (int)(c % g.s2);
+    if (row != ROW_ACTUAL) {
+      ad_border_cell(g, n, c, row, i, j, k, out, use, dinv);
+      continue;
+    }
     const double D = g.adDf ? g.adDf[c] : g.ad_D;
-    double Ax, Bx, Cx, Ay, By, Cy, Az, Bz, Cz;
-    ad_coef_fast(tx + 5 * i, g.adv0[c], D, g.ad_conv, g.ad_diff, up, Ax, Bx, Cx);
-    ad_coef_fast(ty + 5 * j, g.adv1[c], D, g.ad_conv, g.ad_diff, up, Ay, By, Cy);
-    ad_coef_fast(tz + 5 * k, g.adv2[c], D, g.ad_conv, g.ad_diff, up, Az, Bz, Cz);
-    out[c] = g.ad_itau + Bx + By + Bz;
-    out[n + c] = Ax;
-    out[2 * n + c] = Cx;
-    out[3 * n + c] = Ay;
-    out[4 * n + c] = Cy;
-    out[5 * n + c] = Az;
-    out[6 * n + c] = Cz;
+    double A[3], C[3], q0 = g.ad_itau;
+    ad_coef_fast<UP>(ad_axis(tx, g.n1, i), g.adv0[c], D, A[0], C[0], q0);
+    ad_coef_fast<UP>(fy, g.adv1[c], D, A[1], C[1], q0);
+    ad_coef_fast<UP>(fz, g.adv2[c], D, A[2], C[2], q0);
+    out[c] = q0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      out[(1 + 2 * d) * n + c] = A[d];
+      out[(2 + 2 * d) * n + c] = C[d];
+    }
+    use[c] = AD_ROW | 63;
+    dinv[c] = ad_reciprocal(q0);
   }
 }
 
@@ -286,10 +347,15 @@ __global__ void k_ad_coeffs(StencilGrid<double> g, int64_t n, const double* __re
 // thread takes cell after cell (the row reads its seven coefficients and its
 // neighbours directly, so the plane march buys nothing), at full occupancy.
 // Border rows read the table too (their semi-sums and axis-aligned normal
-// differences are seven-point rows), so a warp that holds a face cell does
-// not wait on the general border row; only oblique normal differences take
-// it.  Same dots and control step as k_matvec.
-constexpr int AD_THREADS = 256;
+// differences are seven-point rows), by the same instructions: the cell's byte
+// says which neighbours its row reads, and the others are not read but taken
+// as 0 with the coefficient 0.  (A branch for border rows ran both sides in a
+// quarter of the warps, a k-row ending every 130 cells: 15 FP64 instructions a
+// cell on average, where the row takes 7 and its dots 1 or 2.)  Only oblique
+// normal differences take the general row.  Same dots and control step as
+// k_matvec.  What bounds it: FP64 issue and, a little behind, the 81 bytes a
+// cell.
+constexpr int AD_THREADS = 256, AD_RESIDENT = 4;   // four blocks an SM, one wave
 // The border rows, out of line: they are few, and inlined they would set the
 // register budget of the whole loop.
 __device__ __noinline__ double ad_border_row(const StencilGrid<double>& g, const double* __restrict__ x, int64_t c,
@@ -299,7 +365,7 @@ __device__ __noinline__ double ad_border_row(const StencilGrid<double>& g, const
   return boundary_row<double, false>(g, x, i, j, k, (int)c, row);
 }
 
-__global__ void __launch_bounds__(AD_THREADS, 4) k_ad_fast(MatvecArgs<double> a) {
+__global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<double> a) {
   __shared__ double sh[32];
   __shared__ bool last;
   if (a.ctl != CTL_NONE && (a.S->iscalars[I_DONE] || (a.gate && !a.S->iscalars[I_NEEDREP]))) return;
@@ -308,36 +374,25 @@ __global__ void __launch_bounds__(AD_THREADS, 4) k_ad_fast(MatvecArgs<double> a)
   const double* __restrict__ x = a.x;
   DotAcc<double> dw, ds;
   for (int64_t c = blockIdx.x * (int64_t)AD_THREADS + threadIdx.x; c < n; c += (int64_t)gridDim.x * AD_THREADS) {
-    const int row = row_of(g.kind[c]);
-    if (row == ROW_NONE) {
+    const uint32_t u = a.use[c];
+    if (u == 0) {
       if (a.zero_inactive) {
         if (a.y) a.y[c] = 0.0;
         if (a.y32) a.y32[c] = 0.f;
       }
       continue;
     }
-    double v;
     const double* __restrict__ q = g.adc + c;
-    const double q0 = q[0];
-    if (row == ROW_ACTUAL) {   // interior: all six neighbours are inside the box
-      v = q0 * x[c];
-      v = fma(q[nn], x[c - s1], v);
-      v = fma(q[2 * nn], x[c + s1], v);
-      v = fma(q[3 * nn], x[c - s2], v);
-      v = fma(q[4 * nn], x[c + s2], v);
-      v = fma(q[5 * nn], x[c - 1], v);
-      v = fma(q[6 * nn], x[c + 1], v);
-    } else if (q0 == q0) {   // a border row from the table: it reads only its nonzero neighbours
-      const int64_t off[6] = {-s1, s1, -s2, s2, -1, 1};
-      v = q0 * x[c];
-#pragma unroll
-      for (int t = 0; t < 6; t++) {
-        const double qt = q[(t + 1) * nn];
-        if (qt != 0) v = fma(qt, x[c + off[t]], v);
-      }
-    } else {   // an oblique normal difference
-      v = ad_border_row(g, x, c, row);
-    }
+    const double x1 = u & 1 ? x[c - s1] : 0.0, x2 = u & 2 ? x[c + s1] : 0.0, x3 = u & 4 ? x[c - s2] : 0.0;
+    const double x4 = u & 8 ? x[c + s2] : 0.0, x5 = u & 16 ? x[c - 1] : 0.0, x6 = u & 32 ? x[c + 1] : 0.0;
+    double v = q[0] * x[c];
+    v = fma(q[nn], x1, v);
+    v = fma(q[2 * nn], x2, v);
+    v = fma(q[3 * nn], x3, v);
+    v = fma(q[4 * nn], x4, v);
+    v = fma(q[5 * nn], x5, v);
+    v = fma(q[6 * nn], x6, v);
+    if (u & AD_OBLIQUE) v = ad_border_row(g, x, c, row_of(g.kind[c]));
     if (a.sign > 0) v = v + a.s[c];
     else if (a.sign < 0) v = v - a.s[c];
     if (a.neg) v = -v;
@@ -358,30 +413,6 @@ __global__ void __launch_bounds__(AD_THREADS, 4) k_ad_fast(MatvecArgs<double> a)
         control_step(a.S, a.ctl);
       }
     }
-  }
-}
-
-// A unit probe at the row's own cell: a border row evaluated on it is the
-// row's diagonal coefficient.
-struct UnitProbe {
-  __device__ __forceinline__ double operator()(int a, int b, int d) const { return (a | b | d) == 0 ? 1.0 : 0.0; }
-};
-
-// Inverse row diagonals of the fast rows (Actual: the table's centre; border
-// rows: the row on a unit probe), 0 off the active set and where a diagonal
-// is 0.
-__global__ void k_ad_jacobi(StencilGrid<double> g, int64_t n, const double* __restrict__ table,
-                            double* __restrict__ dinv) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    const int row = row_of(g.kind[c]);
-    double d = 0;
-    if (row == ROW_ACTUAL) {
-      d = table[c];
-    } else if (row != ROW_NONE) {
-      const int i = (int)(c / g.s1), j = (int)((c - (int64_t)i * g.s1) / g.s2), k = (int)(c % g.s2);
-      d = boundary_row_acc<double, false>(g, UnitProbe{}, i, j, k, (int)c, row);
-    }
-    dinv[c] = d != 0 ? 1.0 / d : 0.0;
   }
 }
 
@@ -427,10 +458,27 @@ int xf_op_jacobi(const xf_op* op, const double** dinv) {
   return XF_OK;
 }
 
+__global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) b[c] = (float)a[c];
+}
+
+// The FP32 copies of the advection fields, made when the first FP32 row after
+// a setter asks for them (a time step's solves are FP64).
+void xf_op_ready32(const xf_op* op) {
+  if (op->kind != XF_OP_ADVDIFF || op->adv32_valid) return;
+  xf_ctx* ctx = op->g->ctx;
+  const int64_t n = op->g->ncell;
+  const int bl = grid_blocks(ctx, n, 256);
+  for (int d = 0; d < 3; d++) k_d2f<<<bl, 256, 0, ctx->stream>>>(op->adv64[d], op->adv32[d], n);
+  if (op->adD_set) k_d2f<<<bl, 256, 0, ctx->stream>>>(op->adD64, op->adD32, n);
+  op->adv32_valid = 1;
+}
+
 template <typename T>
 static void launch_matvec(const xf_op* op, const T* rho, const MvReq<T>& q) {
   const xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
+  if (std::is_same<T, float>::value) xf_op_ready32(op);
   MatvecArgs<T> a;
   a.g = make_stencil_grid<T>(g, rho);
   a.x = q.x; a.y = q.y; a.y32 = q.y32; a.s = q.s; a.w = q.w; a.diag = g->diag;
@@ -451,7 +499,8 @@ static void launch_matvec(const xf_op* op, const T* rho, const MvReq<T>& q) {
     set_ad_fields<T>(a.g, op);
     if constexpr (std::is_same<T, double>::value) {
       if (!q.exact && a.g.adc) {
-        k_ad_fast<<<grid_blocks(ctx, g->ncell, AD_THREADS), AD_THREADS, 0, ctx->stream>>>(a);
+        a.use = op->adk;
+        k_ad_fast<<<grid_blocks(ctx, g->ncell, AD_THREADS, AD_RESIDENT), AD_THREADS, 0, ctx->stream>>>(a);
         return;
       }
     }
@@ -540,15 +589,12 @@ extern "C" int xf_op_destroy(xf_op* op) {
   if (op->adD32) cudaFree(op->adD32);
   if (op->adc64) cudaFree(op->adc64);
   if (op->adj64) cudaFree(op->adj64);
+  if (op->adk) cudaFree(op->adk);
   if (op->pack) xf_pack_free(op->pack);
   if (op->host_x) xf_vec_destroy(op->host_x);
   if (op->host_b) xf_vec_destroy(op->host_b);
   delete op;
   return XF_OK;
-}
-
-__global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) b[c] = (float)a[c];
 }
 
 extern "C" int xf_op_set_density(xf_op* op, const double* host_rho) {
@@ -580,6 +626,7 @@ extern "C" int xf_op_set_advection(xf_op* op, const xf_vec* u, const xf_vec* v, 
   op->adc_valid = 0;
   const int64_t nax = 5 * ((int64_t)op->g->n1 + op->g->n2 + op->g->n3);   // per-axis factors after the table
   if ((!op->adc64 && cudaMalloc(&op->adc64, (7 * n + nax) * 8) != cudaSuccess) ||
+      (!op->adk && cudaMalloc(&op->adk, n) != cudaSuccess) ||
       (!op->adj64 && cudaMalloc(&op->adj64, n * 8) != cudaSuccess)) {
     cudaGetLastError();
     return xf_fail(ctx, XF_ERR_NOMEM, "xf_op_set_advection: allocation");
@@ -592,9 +639,8 @@ extern "C" int xf_op_set_advection(xf_op* op, const xf_vec* u, const xf_vec* v, 
     }
     if (vel[d]) XF_CUDA(ctx, cudaMemcpyAsync(op->adv64[d], vel[d]->data, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     else XF_CUDA(ctx, cudaMemsetAsync(op->adv64[d], 0, n * 8, ctx->stream));
-    k_d2f<<<grid_blocks(ctx, n, 256), 256, 0, ctx->stream>>>(op->adv64[d], op->adv32[d], n);
   }
-  XF_CUDA(ctx, cudaGetLastError());
+  op->adv32_valid = 0;
   op->ad_tau = tau;
   op->ad_D = diff_coef;
   op->ad_flags = flags;
@@ -621,8 +667,7 @@ extern "C" int xf_op_set_diffusion_field(xf_op* op, const xf_vec* d) {
     return xf_fail(ctx, XF_ERR_NOMEM, "xf_op_set_diffusion_field: allocation");
   }
   XF_CUDA(ctx, cudaMemcpyAsync(op->adD64, d->data, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-  k_d2f<<<grid_blocks(ctx, n, 256), 256, 0, ctx->stream>>>(op->adD64, op->adD32, n);
-  XF_CUDA(ctx, cudaGetLastError());
+  op->adv32_valid = 0;
   op->adD_set = 1;
   return XF_OK;
 }
@@ -641,11 +686,13 @@ int xf_op_ready(const xf_op* op) {
     double* tx = op->adc64 + 7 * n;   // the axis factors sit after the table
     double* ty = tx + 5 * g->n1;
     double* tz = ty + 5 * g->n2;
-    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hx, g->n1, tx);
-    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hy, g->n2, ty);
-    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hz, g->n3, tz);
-    k_ad_coeffs<<<grid_blocks(ctx, n, 256), 256, 0, ctx->stream>>>(s, n, tx, ty, tz, op->adc64);
-    k_ad_jacobi<<<grid_blocks(ctx, n, 256), 256, 0, ctx->stream>>>(s, n, op->adc64, op->adj64);
+    const double conv = s.ad_conv, diff = s.ad_diff;
+    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hx, g->n1, conv, diff, tx);
+    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hy, g->n2, conv, diff, ty);
+    k_ad_axis<<<1, 256, 0, ctx->stream>>>(g->hz, g->n3, conv, diff, tz);
+    const dim3 grid((unsigned)((g->s1 + ADC_THREADS - 1) / ADC_THREADS), (g->n1 + ADC_CHUNK - 1) / ADC_CHUNK);
+    if (s.ad_upwind) k_ad_coeffs<true><<<grid, ADC_THREADS, 0, ctx->stream>>>(s, n, tx, ty, tz, op->adc64, op->adk, op->adj64);
+    else k_ad_coeffs<false><<<grid, ADC_THREADS, 0, ctx->stream>>>(s, n, tx, ty, tz, op->adc64, op->adk, op->adj64);
     XF_CUDA(ctx, cudaGetLastError());
     op->adc_valid = 1;
   }

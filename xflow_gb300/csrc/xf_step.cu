@@ -335,6 +335,22 @@ __global__ void k_mom_transfer(MomArgs a) {
 }
 
 // Pass 3 (XProblem.cpp:5352-5419): rp += dVis . (dVel + dU) on Actual cells.
+// Where the face viscosity is the same on both sides along every axis, the
+// three gradients are +0 and so is their part of rp, whatever the velocities,
+// unless one of those is not finite or a quotient could overflow.  These are
+// compared as bits: the nine quotients of a cell take 50 instructions of the
+// FP64 pipe (1.6 ms for 512 x 128 x 128 cells, where the bytes take 0.07), and
+// in a fluid of one viscosity only the cells beside a border need them.
+__device__ __forceinline__ bool mom_flat(const double* __restrict__ v, int64_t c, int64_t s) {
+  const long long a = __double_as_longlong(v[c - s]), b = __double_as_longlong(v[c + s]);
+  return a == b && (a & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
+}
+// Below 2^500 in magnitude: the difference of two such over a spacing above 2^-500 is finite.
+__device__ __forceinline__ bool mom_tame(double v) { return (__double2hiint(v) & 0x7fffffff) < (1523 << 20); }
+__device__ __forceinline__ bool mom_tame2(const double* __restrict__ v, int64_t c, int64_t s) {
+  return mom_tame(v[c - s]) && mom_tame(v[c + s]);
+}
+
 template <bool SMALL>
 __global__ void k_mom_viscous(MomArgs a) {
   const int64_t n = (int64_t)a.b1 * a.b2 * a.b3;
@@ -345,6 +361,11 @@ __global__ void k_mom_viscous(MomArgs a) {
     if (a.code[c] != PC_ACTUAL) continue;
     int i, j, k;
       split3<SMALL>(c, s1, s2, i, j, k);
+    if (mom_flat(a.visTr, c, s1) && mom_flat(a.visTr, c, s2) && mom_flat(a.visTr, c, 1) && mom_tame2(velTr, c, s1) &&
+        mom_tame2(velTr, c, s2) && mom_tame2(velTr, c, 1) && mom_tame2(a.uTr, c, st) && mom_tame2(a.vTr, c, st) &&
+        mom_tame2(a.wTr, c, st) && mom_tame(a.rhhx[i]) && mom_tame(a.rhhy[j]) && mom_tame(a.rhhz[k]) &&
+        __double_as_longlong(a.rp[c]) != (long long)0x8000000000000000ull)   // -0 + 0 is +0
+      continue;
     const double ddx = a.hx[i] + a.hx[i - 1], ddy = a.hy[j] + a.hy[j - 1], ddz = a.hz[k] + a.hz[k - 1];
     // RN(1/(h[i-1] + h[i])) = RN(1/hh) / 2 exactly, hh = (h[i-1] + h[i]) / 2
     const double rdx = 0.5 * a.rhhx[i], rdy = 0.5 * a.rhhy[j], rdz = 0.5 * a.rhhz[k];
