@@ -306,26 +306,52 @@ __global__ void __launch_bounds__(RED_THREADS) k_bcgs_end(double* __restrict__ U
   const double an = S->scalars[D_AN], wn = S->scalars[D_WN];
   unsigned long long best = 0;
   DotAcc<double> dot;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (!m[i]) continue;
-    double r;
+  // one cell; un and the others are read off the active set too (valid memory, without effect)
+  auto cell = [&](bool on, double& un, double& rn, double sn, double tn, double xp, double xs, double sr) {
+    if (!on) return;
     if (update && EXACT) {
-      double tmp1 = an * (Xp ? Xp[i] : Pn1[i]);
-      double tmp2 = tmp1 + wn * (Xs ? Xs[i] : Sn[i]);
-      Un[i] = Un[i] + tmp2;
-      double t = wn * Tn[i];
-      r = Sn[i] - t;
-      Rn[i] = r;
+      double tmp1 = an * xp;
+      double tmp2 = tmp1 + wn * xs;
+      un = un + tmp2;
+      double t = wn * tn;
+      rn = sn - t;
     } else if (update) {
-      const double sn = Sn[i];
-      Un[i] = fma(an, Xp ? Xp[i] : Pn1[i], fma(wn, Xs ? Xs[i] : sn, Un[i]));
-      r = fma(-wn, Tn[i], sn);
-      Rn[i] = r;
-    } else {
-      r = Rn[i];
+      un = fma(an, xp, fma(wn, xs, un));
+      rn = fma(-wn, tn, sn);
     }
-    best = absmax_bits(best, r);
-    dot.add(sRn[i], r);
+    best = absmax_bits(best, rn);
+    dot.add(sr, rn);
+  };
+  const double* __restrict__ xp = Xp ? Xp : Pn1;
+  const double* __restrict__ xs = Xs ? Xs : Sn;
+  // two cells a thread, every load before the mask decides: with a load behind
+  // the mask the pass ran at half of the memory's rate
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  for (int64_t v = tid; v < n / 2; v += stride) {
+    const uchar2 mv = reinterpret_cast<const uchar2*>(m)[v];
+    double2 rn = reinterpret_cast<const double2*>(Rn)[v];
+    const double2 sr = reinterpret_cast<const double2*>(sRn)[v];
+    if (update) {
+      double2 un = reinterpret_cast<const double2*>(Un)[v];
+      const double2 sn = reinterpret_cast<const double2*>(Sn)[v], tn = reinterpret_cast<const double2*>(Tn)[v];
+      const double2 p2 = reinterpret_cast<const double2*>(xp)[v], s2 = reinterpret_cast<const double2*>(xs)[v];
+      cell(mv.x, un.x, rn.x, sn.x, tn.x, p2.x, s2.x, sr.x);
+      cell(mv.y, un.y, rn.y, sn.y, tn.y, p2.y, s2.y, sr.y);
+      reinterpret_cast<double2*>(Un)[v] = un;
+      reinterpret_cast<double2*>(Rn)[v] = rn;
+    } else {
+      double none = 0;
+      cell(mv.x, none, rn.x, 0, 0, 0, 0, sr.x);
+      cell(mv.y, none, rn.y, 0, 0, 0, 0, sr.y);
+    }
+  }
+  for (int64_t i = n / 2 * 2 + tid; i < n; i += stride) {
+    double un = Un[i], rn = Rn[i];
+    cell(m[i], un, rn, Sn[i], Tn[i], xp[i], xs[i], sRn[i]);
+    if (update) {
+      Un[i] = un;
+      Rn[i] = rn;
+    }
   }
   best = block_max_bits(best, shm);
   if (threadIdx.x == 0) S->partials[SL_D][blockIdx.x] = __longlong_as_double((long long)best);
@@ -434,10 +460,23 @@ struct Bufs {
   template <typename T>
   T* get(int64_t n, bool zero = true) {
     void* p = nullptr;
-    if (cudaMallocAsync(&p, n * sizeof(T), ctx->stream) != cudaSuccess) return nullptr;
+    if (cudaMallocAsync(&p, n * sizeof(T), ctx->stream) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
     if (zero) cudaMemsetAsync(p, 0, n * sizeof(T), ctx->stream);
     ptrs.push_back(p);
     return (T*)p;
+  }
+  // `count` zeroed boxes of n values as one allocation and one fill, 256-byte aligned; false when it cannot be had
+  template <typename T, class... P>
+  bool boxes(int64_t n, P&... out) {
+    const int64_t pitch = (n * (int64_t)sizeof(T) + 255) / 256 * 256;
+    char* p = get<char>(pitch * (int64_t)sizeof...(out));
+    if (!p) return false;
+    int q = 0;
+    ((out = (T*)(p + pitch * q++)), ...);
+    return true;
   }
   ~Bufs() {
     for (void* p : ptrs) cudaFreeAsync(p, ctx->stream);
@@ -513,6 +552,7 @@ static int run_loop(xf_ctx* ctx, const std::function<void(int)>& iter, int chunk
 // iterations, and past the last one only `ahead` iterations' kernels are left
 // to find the solve done (a graph of 16 iterations, two of them in flight, ran
 // 20 iterations too many of the 12 of a momentum solve).
+// The state is left on the device (read_all).
 static int run_stream(xf_ctx* ctx, const std::function<void(int)>& iter, int launches, int ahead, long long maxit,
                       HostState* hs) {
   volatile long long* progress = (volatile long long*)(ctx->host_scalars + 255);
@@ -538,24 +578,31 @@ static int run_stream(xf_ctx* ctx, const std::function<void(int)>& iter, int lau
     queued++;
   }
   XF_CUDA(ctx, cudaGetLastError());
-  const long long kernels = hs->kernels + queued * launches;
-  const int rs = read_state(ctx, hs);
-  hs->kernels = kernels;
-  return rs;
+  hs->kernels += queued * launches;
+  return XF_OK;
 }
 // Before the first launch of a solve that run_stream drives.
 static void reset_progress(xf_ctx* ctx) { *(volatile long long*)(ctx->host_scalars + 255) = 0; }
 constexpr int STREAM_AHEAD = 3;
 
-static int read_scalars(xf_ctx* ctx) {   // all of them, into the pinned buffer
+// The solver's scalars (to the pinned buffer) and its state, by one wait.
+static int read_all(xf_ctx* ctx, HostState* hs) {
   XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, ctx->scratch->scalars, 128 * sizeof(double), cudaMemcpyDeviceToHost,
                                ctx->stream));
+  XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars + 128, ctx->scratch->iscalars, 4 * sizeof(long long),
+                               cudaMemcpyDeviceToHost, ctx->stream));
   XF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (hs) {
+    long long I[4];
+    memcpy(I, ctx->host_scalars + 128, sizeof(I));
+    hs->done = I[0]; hs->status = I[1]; hs->it = I[2]; hs->repl = I[3];
+  }
   return XF_OK;
 }
 
 // True relative residual ||b - A x||_2 / ||b||_2 in FP64 (fast rows).
-static int true_residual(const xf_op* op, const double* x, const double* b, double* tmp, double* rel, double* bbout) {
+static int true_residual(const xf_op* op, const double* x, const double* b, double* tmp, double* rel,
+                         HostState* hs = nullptr) {
   xf_ctx* ctx = op->g->ctx;
   DevScratch* S = ctx->scratch;
   k_dot_ctl<double><<<red_blocks(ctx, op->g->ncell), RED_THREADS, 0, ctx->stream>>>(b, b, op->g->smask, op->g->ncell, S, SL_B, CTL_NONE, 0);
@@ -563,11 +610,10 @@ static int true_residual(const xf_op* op, const double* x, const double* b, doub
   q.x = x; q.y = tmp; q.s = b; q.sign = -1; q.neg = 1; q.zero_inactive = 1; q.dot_self = 1; q.slot = SL_C;
   xf_mv64(op, q);
   XF_CUDA(ctx, cudaGetLastError());
-  int rc = read_scalars(ctx);
+  int rc = read_all(ctx, hs);
   if (rc) return rc;
   const double bb = ctx->host_scalars[SL_B], rr = ctx->host_scalars[SL_C + 1];
   *rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
-  if (bbout) *bbout = bb;
   return XF_OK;
 }
 
@@ -604,7 +650,7 @@ static int solve_cg_coop(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf
   if (st->status == XF_NAN || st->status == XF_BREAKDOWN) {
     double* tmp = B.get<double>(n, false);
     if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate residual");
-    if ((rc = true_residual(op, x, b, tmp, &rel, nullptr))) return rc;
+    if ((rc = true_residual(op, x, b, tmp, &rel))) return rc;
   }
   if (st->status == XF_OK && rel > o.rtol) st->status = I[I_IT] >= o.maxit ? XF_MAXIT : XF_STALL;
   st->iterations = (int)I[I_IT];
@@ -818,15 +864,15 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
     int rc = mixed ? run_loop(ctx, iter, chunk, o.maxit - total_it, &hs)
                    : run_stream(ctx, iter, 3, STREAM_AHEAD, o.maxit - total_it, &hs);
     if (rc) return rc;
-    total_it += (int)hs.it;
-    total_repl += (int)hs.repl;
     hs.kernels += 3 + (mixed ? 1 : 0) + 2;
     if (mixed) {
       // fold any correction left behind by an early stop (no-op otherwise)
       k_fold<<<eb, 256, 0, ctx->stream>>>(x, e32, n, S, 0);
     }
-    int r2 = true_residual(op, x, b, tmp, &rel, nullptr);
+    int r2 = true_residual(op, x, b, tmp, &rel, &hs);
     if (r2) return r2;
+    total_it += (int)hs.it;
+    total_repl += (int)hs.repl;
     // The recursive residual can drift from the true one: restart from the
     // current iterate until the true residual meets the tolerance.
     if (hs.status != XF_OK || rel <= o.rtol || total_it >= o.maxit) break;
@@ -891,9 +937,11 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
   } else if (o.method == XF_BICGSTAB) {
     if (eps <= 0) eps = 1e-5;   // XSLAE.cpp:669
     k_reset_state<<<1, 1, 0, ctx->stream>>>(S, 0.0, eps, o.maxit, 1, 0, 1);
-    double *Rn = B.get<double>(n), *sRn = B.get<double>(n), *Pn = B.get<double>(n), *Pn1 = B.get<double>(n);
-    double *Vn = B.get<double>(n), *Sn = B.get<double>(n), *Tn = B.get<double>(n);
-    if (!Rn || !sRn || !Pn || !Pn1 || !Vn || !Sn || !Tn) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
+    const bool jacobi = o.precond == XF_PRECOND_JACOBI;
+    double *Rn, *sRn, *Pn, *Pn1, *Vn, *Sn, *Tn, *Ph = nullptr, *Sh = nullptr;
+    if (!(jacobi ? B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn, Ph, Sh)
+                 : B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn)))
+      return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
     // Rn = b - A(Un)
     MvReq<double> q0;
     q0.x = x; q0.y = Rn; q0.s = b; q0.sign = -1; q0.neg = 1; q0.exact = exact;
@@ -906,13 +954,9 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     // out rows of very different scales (semi-sums of 1/2, normal differences
     // of 1/h, Actual rows of 1/tau and more).
     const double* dinv = nullptr;
-    double *Ph = nullptr, *Sh = nullptr;
-    if (o.precond == XF_PRECOND_JACOBI) {
+    if (jacobi) {
       int js = xf_op_jacobi(op, &dinv);
       if (js) return js;
-      Ph = B.get<double>(n);
-      Sh = B.get<double>(n);
-      if (!Ph || !Sh) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
     } else if (o.precond != XF_PRECOND_NONE) {
       return xf_fail(ctx, XF_ERR_UNSUPPORTED, "xf_solve: BiCGStab takes XF_PRECOND_JACOBI or none");
     }
@@ -988,7 +1032,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
   double* tmp = B.get<double>(n, false);
   if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
   double rel = 0;
-  int r2 = true_residual(op, x, b, tmp, &rel, nullptr);   // leaves the scalars in the pinned buffer
+  int r2 = true_residual(op, x, b, tmp, &rel, &hs);   // leaves the scalars in the pinned buffer
   if (r2) return r2;
   const double own = ctx->host_scalars[o.method == XF_BICGSTAB ? D_NORM : D_EPSCUR];
   st->status = (int)hs.status;

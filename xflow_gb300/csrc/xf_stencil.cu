@@ -241,37 +241,31 @@ enum { AD_ROW = 64, AD_OBLIQUE = 128 };
 // its 4-point face averages collapsing to single cells.  A normal-difference
 // row with an oblique normal reaches beyond the seven points: NaN in the
 // centre sends it to the general row.
-__device__ void ad_border_coeffs(const StencilGrid<double>& g, int64_t c, int row, double q[7]) {
-  for (int t = 0; t < 7; t++) q[t] = 0.0;
-  const int b = g.brow_of[c];
-  const double nrm[3] = {g.brow_nrm[3 * b], g.brow_nrm[3 * b + 1], g.brow_nrm[3 * b + 2]};
+__device__ __forceinline__ bool ad_nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+struct AdBorder { int axis, nb; double q0, qn; };   // nb: the neighbour read (0 x- .. 5 z+), qn its coefficient
+__device__ __forceinline__ AdBorder ad_border_coeffs(const StencilGrid<double>& g, int64_t c, int row, int i, int j,
+                                                     int k) {
+  const double* nrm = g.brow_nrm + 3 * g.brow_of[c];
+  const double nx = nrm[0], ny = nrm[1], nz = nrm[2];
+  const bool ux = ad_nonzero(nx), uy = ad_nonzero(ny), uz = ad_nonzero(nz);
+  const int ax = uz ? 2 : uy ? 1 : ux ? 0 : -1;
+  const double na = uz ? nz : uy ? ny : nx;
+  AdBorder r = {ax, 0, 0.0, 0.0};
+  if (ax < 0) return r;   // no normal: the row is 0
+  const bool pos = __double_as_longlong(na) >= 0;
+  r.nb = 2 * ax + (pos ? 0 : 1);
   if (row == ROW_PREDEF) {
-    int ax = -1;
-    for (int a = 0; a < 3; a++)
-      if (nrm[a] != 0) ax = a;
-    if (ax < 0) return;   // no normal: the row is 0
-    q[0] = 0.5;
-    q[1 + 2 * ax + (nrm[ax] > 0 ? 0 : 1)] = 0.5;
-    return;
-  }
-  int ax = -1, cnt = 0;
-  for (int a = 0; a < 3; a++)
-    if (nrm[a] != 0) { ax = a; cnt++; }
-  if (cnt == 0) return;   // the row is 0
-  if (cnt > 1) { q[0] = __longlong_as_double(0x7ff8000000000000ll); return; }
-  const int i = (int)(c / g.s1), j = (int)((c - (int64_t)i * g.s1) / g.s2), k = (int)(c % g.s2);
-  const int m = ax == 0 ? i : ax == 1 ? j : k;
-  const double* h = ax == 0 ? g.hx : ax == 1 ? g.hy : g.hz;
-  const double na = nrm[ax];
-  if (na > 0) {
-    const double r = na / h[m - 1];
-    q[0] = r;
-    q[1 + 2 * ax] = -r;
+    r.q0 = r.qn = 0.5;
+  } else if (ux + uy + uz > 1) {
+    r.q0 = __longlong_as_double(0x7ff8000000000000ll);
   } else {
-    const double r = na / h[m];
-    q[0] = -r;
-    q[2 + 2 * ax] = r;
+    const int m = (ax == 0 ? i : ax == 1 ? j : k) - (pos ? 1 : 0);
+    const double* h = ax == 0 ? g.hx : ax == 1 ? g.hy : g.hz;
+    const double d = na / h[m];
+    r.q0 = pos ? d : -d;
+    r.qn = pos ? -d : d;
   }
+  return r;
 }
 
 // A unit probe at the row's own cell: a border row evaluated on it is the
@@ -280,21 +274,24 @@ struct UnitProbe {
   __device__ __forceinline__ double operator()(int a, int b, int d) const { return (a | b | d) == 0 ? 1.0 : 0.0; }
 };
 
-// A border row's part of the table: its coefficients, the neighbours it reads and its inverse diagonal.
-__device__ __noinline__ void ad_border_cell(const StencilGrid<double>& g, int64_t n, int64_t c, int row, int i, int j,
-                                            int k, double* __restrict__ out, uint8_t* __restrict__ use,
-                                            double* __restrict__ dinv) {
-  double q[7];
-  ad_border_coeffs(g, c, row, q);
-  uint8_t u = AD_ROW;
-  if (q[0] != q[0]) u |= AD_OBLIQUE;
-  for (int t = 0; t < 7; t++) {
-    out[t * n + c] = q[t];
-    if (t > 0 && q[t] != 0) u |= 1 << (t - 1);
-  }
-  use[c] = u;
+// The inverse diagonal of an oblique normal difference.
+__device__ __noinline__ double ad_oblique_inverse(const StencilGrid<double>& g, int64_t c, int row, int i, int j, int k) {
   const double d = boundary_row_acc<double, false>(g, UnitProbe{}, i, j, k, (int)c, row);
-  dinv[c] = d != 0 ? 1.0 / d : 0.0;
+  return d != 0 ? 1.0 / d : 0.0;
+}
+
+// A border row's part of the table: its coefficients, the neighbour it reads and its inverse diagonal.
+__device__ __forceinline__ void ad_border_cell(const StencilGrid<double>& g, int64_t n, int64_t c, int row, int i, int j,
+                                               int k, double* __restrict__ out, uint8_t* __restrict__ use,
+                                               double* __restrict__ dinv) {
+  const AdBorder b = ad_border_coeffs(g, c, row, i, j, k);
+  const bool oblique = b.q0 != b.q0;
+  const bool reads = !oblique && ad_nonzero(b.qn);
+  out[c] = b.q0;
+#pragma unroll
+  for (int t = 0; t < 6; t++) out[(t + 1) * n + c] = t == b.nb && !oblique ? b.qn : 0.0;
+  use[c] = AD_ROW | (oblique ? AD_OBLIQUE : 0) | (reads ? 1 << b.nb : 0);
+  dinv[c] = oblique ? ad_oblique_inverse(g, c, row, i, j, k) : ad_reciprocal(b.q0);
 }
 
 // The FP64 coefficient table of the fast rows: for Actual rows a centre
@@ -373,8 +370,12 @@ __global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<
   const int64_t s1 = g.s1, s2 = g.s2, n = (int64_t)g.n1 * s1, nn = g.adc_n;
   const double* __restrict__ x = a.x;
   DotAcc<double> dw, ds;
-  for (int64_t c = blockIdx.x * (int64_t)AD_THREADS + threadIdx.x; c < n; c += (int64_t)gridDim.x * AD_THREADS) {
-    const uint32_t u = a.use[c];
+  const int64_t step = (int64_t)gridDim.x * AD_THREADS;
+  int64_t c = blockIdx.x * (int64_t)AD_THREADS + threadIdx.x;
+  uint32_t next = c < n ? a.use[c] : 0;   // a cell's byte is loaded a cell ahead: the neighbours' loads wait for it
+  for (; c < n; c += step) {
+    const uint32_t u = next;
+    if (c + step < n) next = a.use[c + step];
     if (u == 0) {
       if (a.zero_inactive) {
         if (a.y) a.y[c] = 0.0;

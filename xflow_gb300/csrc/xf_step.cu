@@ -335,12 +335,12 @@ __global__ void k_mom_transfer(MomArgs a) {
 }
 
 // Pass 3 (XProblem.cpp:5352-5419): rp += dVis . (dVel + dU) on Actual cells.
-// Where the face viscosity is the same on both sides along every axis, the
-// three gradients are +0 and so is their part of rp, whatever the velocities,
-// unless one of those is not finite or a quotient could overflow.  These are
-// compared as bits: the nine quotients of a cell take 50 instructions of the
-// FP64 pipe (1.6 ms for 512 x 128 x 128 cells, where the bytes take 0.07), and
-// in a fluid of one viscosity only the cells beside a border need them.
+// Where the face viscosity is the same on both sides along an axis, its
+// gradient is +0 and so, whatever the sign, is that axis's part of rp, unless
+// a velocity is not finite or a quotient could overflow.  These are compared
+// as bits: a cell's nine quotients take 50 instructions of the FP64 pipe (1.6
+// ms for 512 x 128 x 128 cells, where the bytes take 0.07), and in a fluid of
+// one viscosity only the cells beside a border need any, of the axis across it.
 __device__ __forceinline__ bool mom_flat(const double* __restrict__ v, int64_t c, int64_t s) {
   const long long a = __double_as_longlong(v[c - s]), b = __double_as_longlong(v[c + s]);
   return a == b && (a & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
@@ -361,26 +361,32 @@ __global__ void k_mom_viscous(MomArgs a) {
     if (a.code[c] != PC_ACTUAL) continue;
     int i, j, k;
       split3<SMALL>(c, s1, s2, i, j, k);
-    if (mom_flat(a.visTr, c, s1) && mom_flat(a.visTr, c, s2) && mom_flat(a.visTr, c, 1) && mom_tame2(velTr, c, s1) &&
-        mom_tame2(velTr, c, s2) && mom_tame2(velTr, c, 1) && mom_tame2(a.uTr, c, st) && mom_tame2(a.vTr, c, st) &&
-        mom_tame2(a.wTr, c, st) && mom_tame(a.rhhx[i]) && mom_tame(a.rhhy[j]) && mom_tame(a.rhhz[k]) &&
-        __double_as_longlong(a.rp[c]) != (long long)0x8000000000000000ull)   // -0 + 0 is +0
-      continue;
-    const double ddx = a.hx[i] + a.hx[i - 1], ddy = a.hy[j] + a.hy[j - 1], ddz = a.hz[k] + a.hz[k - 1];
+    // a zero part keeps any sum of the others, and rp but for -0 + 0 = +0
+    const double rp = a.rp[c];
+    const bool tame = mom_tame2(velTr, c, s1) && mom_tame2(velTr, c, s2) && mom_tame2(velTr, c, 1) &&
+                      mom_tame2(a.uTr, c, st) && mom_tame2(a.vTr, c, st) && mom_tame2(a.wTr, c, st) &&
+                      mom_tame(a.rhhx[i]) && mom_tame(a.rhhy[j]) && mom_tame(a.rhhz[k]) &&
+                      __double_as_longlong(rp) != (long long)0x8000000000000000ull;
+    const bool skipx = tame && mom_flat(a.visTr, c, s1), skipy = tame && mom_flat(a.visTr, c, s2);
+    const bool skipz = tame && mom_flat(a.visTr, c, 1);
+    if (skipx && skipy && skipz) continue;
     // RN(1/(h[i-1] + h[i])) = RN(1/hh) / 2 exactly, hh = (h[i-1] + h[i]) / 2
-    const double rdx = 0.5 * a.rhhx[i], rdy = 0.5 * a.rhhy[j], rdz = 0.5 * a.rhhz[k];
-    const double dVisX = div_rcp(a.visTr[c + s1] - a.visTr[c - s1], ddx, rdx);
-    const double dVisY = div_rcp(a.visTr[c + s2] - a.visTr[c - s2], ddy, rdy);
-    const double dVisZ = div_rcp(a.visTr[c + 1] - a.visTr[c - 1], ddz, rdz);
+    const double ddx = a.hx[i] + a.hx[i - 1], rdx = 0.5 * a.rhhx[i];
+    const double ddy = a.hy[j] + a.hy[j - 1], rdy = 0.5 * a.rhhy[j];
+    const double ddz = a.hz[k] + a.hz[k - 1], rdz = 0.5 * a.rhhz[k];
     const double dd = a.axis == 1 ? ddx : a.axis == 2 ? ddy : ddz;
     const double rd = a.axis == 1 ? rdx : a.axis == 2 ? rdy : rdz;
-    const double dU = div_rcp(a.uTr[c + st] - a.uTr[c - st], dd, rd);
-    const double dV = div_rcp(a.vTr[c + st] - a.vTr[c - st], dd, rd);
-    const double dW = div_rcp(a.wTr[c + st] - a.wTr[c - st], dd, rd);
-    const double dVelX = div_rcp(velTr[c + s1] - velTr[c - s1], ddx, rdx);
-    const double dVelY = div_rcp(velTr[c + s2] - velTr[c - s2], ddy, rdy);
-    const double dVelZ = div_rcp(velTr[c + 1] - velTr[c - 1], ddz, rdz);
-    a.rp[c] = a.rp[c] + (dVisX * (dVelX + dU) + dVisY * (dVelY + dV) + dVisZ * (dVelZ + dW));
+    // dVis . (dVel + dU) along one axis: across it the velocity of this equation, along this equation's axis the other
+    auto part = [&](bool skip, int64_t s, double dx, double rx, const double* other) {
+      if (skip) return 0.0;
+      const double dVis = div_rcp(a.visTr[c + s] - a.visTr[c - s], dx, rx);
+      const double dMix = div_rcp(other[c + st] - other[c - st], dd, rd);
+      const double dVel = div_rcp(velTr[c + s] - velTr[c - s], dx, rx);
+      return dVis * (dVel + dMix);
+    };
+    const double px = part(skipx, s1, ddx, rdx, a.uTr), py = part(skipy, s2, ddy, rdy, a.vTr);
+    const double pz = part(skipz, 1, ddz, rdz, a.wTr);
+    a.rp[c] = rp + (px + py + pz);
   }
 }
 
