@@ -342,6 +342,27 @@ __device__ inline double finish_partials(DevScratch* S, int slot, double* sh) {
 }
 
 // ---------------------------------------------------------------------------
+// a / b correctly rounded, from y = RN(1/b), itself a normal number (the grid's
+// reciprocal tables, 1/tau from the host, or __drcp_rn).  q = RN(a y) lies within an ulp of a / b, the
+// residual r = a - b q is exact (one FMA), and RN(q + r y) = RN(a / b):
+// Markstein's theorem for FMA-based division (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34(1), 1990; also Muller et al., Handbook of Floating-Point
+// Arithmetic, ch. 5).  Three FP64 operations instead of the IEEE division's
+// reciprocal iteration, which matters at GB300's FP64 rate (1/58 of FP32).
+// The theorem needs a normal, unclamped residual: a numerator or quotient
+// outside [2^-950, 2^1000) in magnitude (zero, tiny, huge, not finite, or a
+// divisor of 0 or infinity) takes the IEEE division itself.  Checked bit for
+// bit against the IEEE division by xf_selftest_division.
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+  const double q = a * y;
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+  if (ea - (1023u - 950u) >= 1950u || eq - (1023u - 950u) >= 1950u) return a / b;
+  const double r = fma(-b, q, a);
+  return fma(r, y, q);
+}
+
+// ---------------------------------------------------------------------------
 // BF16 activations of the learned preconditioner are stored in channel planes
 // of 8: plane q holds channels 8q .. 8q+7 of every cell, 16 bytes per cell,
 // so element (cell c, channel ch) sits at (ch / 8) * plane_stride + c * 8 +

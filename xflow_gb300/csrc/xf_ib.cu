@@ -1,11 +1,12 @@
-// Immersed boundary (TImmersedBoundaryProblem, XProblem.cpp:8436-9046) and
-// batched tridiagonal lines (TSLAE::SolveByScalarRunning, XSLAE.cpp:416-445).
+// Immersed boundary (TImmersedBoundaryProblem, XProblem.cpp:8436-9046).
 //
 // Markers live on the device as the reference's node arrays (positions 3 per
-// node, node kind, next/prev neighbour, rest lengths and curvatures).  One
-// thread per marker; the 7x7x7 cosine-delta weights of a marker are computed
-// once per axis (7 + 7 + 7 values, the reference recomputes them per cell:
-// same values) and the sums run in the reference's i -> j -> k order.
+// node, node kind, next/prev neighbour, rest lengths and curvatures).  A warp
+// a marker interpolates and spreads; the 7x7x7 cosine-delta weights of a
+// marker are computed once per axis (7 + 7 + 7 values, where the reference
+// recomputes them per cell).  2,562 markers, per axis: interpolation and
+// spreading 93 us each with one thread a marker (a thread for the weights),
+// now bound by the launches.
 //
 // Forces are gathered, not scattered: the serial reference loop
 // (XProblem.cpp:8436-8547) adds, node by node, the node's own term to itself
@@ -18,12 +19,6 @@
 // Spreading scatters 343 atomic FP64 adds per marker into the zeroed force
 // box (contributions from different markers to one cell land in any order:
 // last-bit differences against the serial loop).
-//
-// Thomas lines: one thread per line, the reference's recurrences and
-// operation order; the forward coefficients A[m] go to a per-context
-// workspace laid out [m][line] (coalesced across threads), B[m] is kept in
-// u[m] until the back-substitution overwrites it.  Bit-identical to the
-// serial reference (FP64, no contraction, IEEE division).
 #include <math.h>
 
 #include <vector>
@@ -63,51 +58,62 @@ __device__ __forceinline__ int ib_index(double coord, double step, int nend, int
 __device__ __forceinline__ double ib_coord(int index, double step, int type, int axis) {
   return index * step - (type != axis ? 0.5 * step : 0);
 }
-// Cosine delta, XProblem.cpp:9008-9032.
-__device__ __forceinline__ double ib_delta(double distance, double h) {
-  if (distance < 2 * h) return 1.0 / (4 * h) * (1 + cos(M_PI * distance / (2 * h)));
+// Cosine delta, XProblem.cpp:9008-9032.  cospi of distance / (2 h): no
+// argument reduction, and the quotient by a product with the host's 1 / (2 h)
+// (within a rounding or two of the reference's cos(M_PI distance / (2 h))).
+struct IbAxes { double h[3], i2h[3], i4h[3]; };   // h, 1 / (2 h), 1 / (4 h)
+__device__ __forceinline__ double ib_delta(double distance, double h, double i2h, double i4h) {
+  if (distance < 2 * h) return i4h * (1 + cospi(distance * i2h));
   return 0;
 }
 
+// The markers of a block, a warp each: the 21 weights of all of them are one
+// pass over the block's threads (one thread computing a marker's 21 cosines
+// in turn was nine tenths of the spreading).
+constexpr int IB_WARPS = 8, IB_THREADS = 32 * IB_WARPS;
 struct IbWeights {
-  int xi, yi, zi;
-  double wx[7], wy[7], wz[7];
+  int first[IB_WARPS][3];        // first cell of the stencil, per axis
+  double w[IB_WARPS][3][7];
 };
 
-__device__ __forceinline__ void ib_weights(const double* pos, int q, int n1, int n2, int n3, double h0, double h1,
-                                           double h2, int axis, IbWeights& w) {
-  const double px = pos[3 * q], py = pos[3 * q + 1], pz = pos[3 * q + 2];
-  w.xi = ib_index(px, h0, n1 - 1, 1, axis);
-  w.yi = ib_index(py, h1, n2 - 1, 2, axis);
-  w.zi = ib_index(pz, h2, n3 - 1, 3, axis);
-#pragma unroll
-  for (int t = 0; t < 7; t++) {
-    w.wx[t] = ib_delta(fabs(px - ib_coord(w.xi - IB_RANGE + t, h0, 1, axis)), h0);
-    w.wy[t] = ib_delta(fabs(py - ib_coord(w.yi - IB_RANGE + t, h1, 2, axis)), h1);
-    w.wz[t] = ib_delta(fabs(pz - ib_coord(w.zi - IB_RANGE + t, h2, 3, axis)), h2);
+__device__ __forceinline__ void ib_weights(const double* __restrict__ pos, int q0, int nn, int n1, int n2, int n3,
+                                           const IbAxes& ax, int axis, IbWeights& w) {
+  for (int t = threadIdx.x; t < IB_WARPS * 21; t += IB_THREADS) {
+    const int m = t / 21, d = t / 7 % 3, k = t % 7, q = q0 + m;
+    if (q >= nn) continue;
+    const double h = ax.h[d], p = pos[3 * q + d];
+    const int first = ib_index(p, h, (d == 0 ? n1 : d == 1 ? n2 : n3) - 1, d + 1, axis) - IB_RANGE;
+    if (k == 0) w.first[m][d] = first;
+    w.w[m][d][k] = ib_delta(fabs(p - ib_coord(first + k, h, d + 1, axis)), h, ax.i2h[d], ax.i4h[d]);
   }
+  __syncthreads();
 }
 
 // Interpolate, XProblem.cpp:8620-8791: node velocity = sum over the 7^3
-// stencil of (u_ijk * wx * wy * wz) * h^3 (h of the interpolated axis).
-__global__ void k_ib_interpolate(const double* __restrict__ vel, int n1, int n2, int n3, double h0, double h1,
-                                 double h2, int axis, int nn, const double* __restrict__ pos,
-                                 double* __restrict__ node_vel) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+// stencil of (u_ijk * wx * wy * wz) * h^3 (h of the interpolated axis), the
+// stencil's cells shared by the marker's warp and added in a fixed order.
+__global__ void __launch_bounds__(IB_THREADS) k_ib_interpolate(const double* __restrict__ vel, int n1, int n2, int n3,
+                                                               IbAxes ax, int axis, int nn,
+                                                               const double* __restrict__ pos,
+                                                               double* __restrict__ node_vel) {
+  __shared__ IbWeights w;
+  const int q0 = blockIdx.x * IB_WARPS, m = threadIdx.x >> 5, lane = threadIdx.x & 31, q = q0 + m;
+  ib_weights(pos, q0, nn, n1, n2, n3, ax, axis, w);
   if (q >= nn) return;
-  IbWeights w;
-  ib_weights(pos, q, n1, n2, n3, h0, h1, h2, axis, w);
-  const double ha = axis == 1 ? h0 : axis == 2 ? h1 : h2;
-  const double cb = ha * ha * ha;
   const int64_t s1 = (int64_t)n2 * n3, s2 = n3;
+  const double* box = vel + w.first[m][0] * s1 + w.first[m][1] * s2 + w.first[m][2];
   double acc = 0;
-  for (int a = 0; a < 7; a++)
-    for (int b = 0; b < 7; b++) {
-      const double* row = vel + (w.xi - IB_RANGE + a) * s1 + (w.yi - IB_RANGE + b) * s2 + (w.zi - IB_RANGE);
 #pragma unroll
-      for (int c = 0; c < 7; c++) acc += (row[c] * w.wx[a] * w.wy[b] * w.wz[c]) * cb;
+  for (int u = 0; u < 11; u++) {
+    const int t = lane + 32 * u;
+    if (t < 343) {
+      const int a = t / 49, b = t / 7 % 7, c = t % 7;
+      acc = fma(box[a * s1 + b * s2 + c], w.w[m][0][a] * w.w[m][1][b] * w.w[m][2][c], acc);
     }
-  node_vel[q] = acc;
+  }
+  acc = warp_sum(acc);
+  const double ha = ax.h[axis - 1];
+  if (lane == 0) node_vel[q] = acc * (ha * ha * ha);
 }
 
 // UpdateBoundaryPosition, XProblem.cpp:8858-8894.
@@ -166,19 +172,23 @@ __global__ void k_ib_gather(int nn, const int32_t* __restrict__ in_ptr, const in
 
 // SpreadForce, XProblem.cpp:8550-8617 (arithmetic): f_ijk += F * wx * wy * wz
 // over the 7^3 stencil of every marker; fbox is zeroed first (`force |= 0.0`).
-__global__ void k_ib_spread(double* fbox, int n1, int n2, int n3, double h0, double h1, double h2, int axis, int nn,
-                            const double* __restrict__ pos, const double* __restrict__ force) {
-  const int q = blockIdx.x;
-  if (q >= nn) return;
+// The delta's support is 4 or 5 of the 7 cells an axis: a zero weight of a
+// finite force adds nothing and is left out.
+__global__ void __launch_bounds__(IB_THREADS) k_ib_spread(double* fbox, int n1, int n2, int n3, IbAxes ax, int axis,
+                                                          int nn, const double* __restrict__ pos,
+                                                          const double* __restrict__ force) {
   __shared__ IbWeights w;
-  if (threadIdx.x == 0) ib_weights(pos, q, n1, n2, n3, h0, h1, h2, axis, w);
-  __syncthreads();
+  const int q0 = blockIdx.x * IB_WARPS, m = threadIdx.x >> 5, lane = threadIdx.x & 31, q = q0 + m;
+  ib_weights(pos, q0, nn, n1, n2, n3, ax, axis, w);
+  if (q >= nn) return;
   const double F = force[q];
+  const bool all = !isfinite(F);
   const int64_t s1 = (int64_t)n2 * n3, s2 = n3;
-  for (int t = threadIdx.x; t < 343; t += blockDim.x) {
-    const int a = t / 49, b = (t / 7) % 7, c = t % 7;
-    const int64_t cell = (w.xi - IB_RANGE + a) * s1 + (w.yi - IB_RANGE + b) * s2 + (w.zi - IB_RANGE + c);
-    atomicAdd(fbox + cell, F * w.wx[a] * w.wy[b] * w.wz[c]);
+  double* box = fbox + w.first[m][0] * s1 + w.first[m][1] * s2 + w.first[m][2];
+  for (int t = lane; t < 343; t += 32) {
+    const int a = t / 49, b = t / 7 % 7, c = t % 7;
+    const double wx = w.w[m][0][a], wy = w.w[m][1][b], wz = w.w[m][2][c];
+    if (all || (wx != 0 && wy != 0 && wz != 0)) atomicAdd(box + a * s1 + b * s2 + c, F * wx * wy * wz);
   }
 }
 
@@ -317,6 +327,15 @@ extern "C" int xf_ib_upload(xf_ib* ib, int field, const double* host) {
 }
 
 static inline int ib_blocks(int n, int t) { return (n + t - 1) / t; }
+static IbAxes ib_axes(const double* h0) {
+  IbAxes a;
+  for (int d = 0; d < 3; d++) {
+    a.h[d] = h0[d];
+    a.i2h[d] = 1.0 / (2 * h0[d]);
+    a.i4h[d] = 1.0 / (4 * h0[d]);
+  }
+  return a;
+}
 
 extern "C" int xf_ib_interpolate(xf_ib* ib, const xf_vec* vel, const double* h0, int axis) {
   int st = ib_check_box(ib, vel, h0, axis, "xf_ib_interpolate");
@@ -324,8 +343,8 @@ extern "C" int xf_ib_interpolate(xf_ib* ib, const xf_vec* vel, const double* h0,
   xf_ctx* ctx = ib->ctx;
   const xf_grid* g = vel->g;
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
-  k_ib_interpolate<<<ib_blocks(ib->nn, 128), 128, 0, ctx->stream>>>(
-      (const double*)vel->data, g->n1, g->n2, g->n3, h0[0], h0[1], h0[2], axis, ib->nn, ib->pos,
+  k_ib_interpolate<<<ib_blocks(ib->nn, IB_WARPS), IB_THREADS, 0, ctx->stream>>>(
+      (const double*)vel->data, g->n1, g->n2, g->n3, ib_axes(h0), axis, ib->nn, ib->pos,
       ib->vel + (size_t)(axis - 1) * ib->nn);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
@@ -364,8 +383,9 @@ extern "C" int xf_ib_spread(xf_ib* ib, xf_vec* force, const double* h0, int axis
   const xf_grid* g = force->g;
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
   XF_CUDA(ctx, cudaMemsetAsync(force->data, 0, g->ncell * sizeof(double), ctx->stream));
-  k_ib_spread<<<ib->nn, 128, 0, ctx->stream>>>((double*)force->data, g->n1, g->n2, g->n3, h0[0], h0[1], h0[2], axis,
-                                                ib->nn, ib->pos, ib->force + (size_t)(axis - 1) * ib->nn);
+  k_ib_spread<<<ib_blocks(ib->nn, IB_WARPS), IB_THREADS, 0, ctx->stream>>>(
+      (double*)force->data, g->n1, g->n2, g->n3, ib_axes(h0), axis, ib->nn, ib->pos,
+      ib->force + (size_t)(axis - 1) * ib->nn);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }

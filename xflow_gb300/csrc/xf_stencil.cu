@@ -86,10 +86,10 @@ __device__ __forceinline__ T march_lap(const StencilGrid<T>& g, const MatvecArgs
   }
 }
 
-// The fast FP64 advection-diffusion rows stream ten arrays a cell: four
-// blocks an SM (at most 64 registers) keep enough loads in flight.
+// The fast rows are bound by the loads in flight (a plane's are behind the
+// last plane's): four blocks an SM, at most 64 registers.
 template <typename T, int OP, bool EXACT, bool USE_D>
-__global__ void __launch_bounds__(MV_THREADS, (OP == XF_OP_ADVDIFF && !EXACT) ? 4 : 1) k_matvec(MatvecArgs<T> a) {
+__global__ void __launch_bounds__(MV_THREADS, EXACT ? 1 : 4) k_matvec(MatvecArgs<T> a) {
   __shared__ double sh[32];
   __shared__ bool last;
   // Solver kernels turn into no-ops once the solve is done (or, when gated,
@@ -489,9 +489,12 @@ static void launch_matvec(const xf_op* op, const T* rho, const MvReq<T>& q) {
   a.S = ctx->scratch;
   const int P = g->n2 * g->n3;
   const int bx = (P + MV_THREADS - 1) / MV_THREADS;
-  // plane chunk: ~16 planes per block, fewer chunks if the partial-sum table
-  // would overflow
-  int chunk = 16;
+  // plane chunk: 16 planes a block where that leaves four blocks an SM, down to
+  // one plane for small boxes (35 x 31 x 29: 12 blocks of 16 planes took 65 us,
+  // each plane's loads behind the last plane's); longer where the partial-sum
+  // table would overflow
+  int chunk = (int)((int64_t)bx * g->n1 / (4 * ctx->sm_count));
+  chunk = chunk < 1 ? 1 : chunk > 16 ? 16 : chunk;
   while ((int64_t)bx * ((g->n1 + chunk - 1) / chunk) > RED_MAX_BLOCKS) chunk *= 2;
   a.chunk = chunk;
   dim3 grid(bx, (g->n1 + chunk - 1) / chunk);

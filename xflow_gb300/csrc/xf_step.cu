@@ -39,26 +39,6 @@ __device__ __forceinline__ void report(DevScratch* S, int kind, long long cell) 
   atomicMin(&S->iscalars[CHK0 + kind], cell);
 }
 
-// a / b correctly rounded, from y = RN(1/b) (the grid's reciprocal tables,
-// or 1/tau from the host).  q = RN(a y) lies within an ulp of a / b, the
-// residual r = a - b q is exact (one FMA), and RN(q + r y) = RN(a / b):
-// Markstein's theorem for FMA-based division (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34(1), 1990; also Muller et al., Handbook of Floating-Point
-// Arithmetic, ch. 5).  Three FP64 operations instead of the IEEE division's
-// reciprocal iteration, which matters at GB300's FP64 rate (1/58 of FP32).
-// The theorem needs a normal, unclamped residual: a numerator or quotient
-// outside [2^-950, 2^1000) in magnitude (zero, tiny, huge, not finite, or a
-// divisor of 0 or infinity) takes the IEEE division itself.  Checked bit for
-// bit against the IEEE division by xf_selftest_division.
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-  const double q = a * y;
-  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
-  if (ea - (1023u - 950u) >= 1950u || eq - (1023u - 950u) >= 1950u) return a / b;
-  const double r = fma(-b, q, a);
-  return fma(r, y, q);
-}
-
 // (i, j, k) of flat cell c in a box with strides s1 = b2 b3, s2 = b3: 32-bit
 // divisions for boxes below 2^32 cells, 64-bit ones (a software routine of
 // about a hundred instructions each) above.
