@@ -232,7 +232,7 @@ __device__ __forceinline__ double cc_residual(const CoopArgs& a, const double* d
   s = fma((kb & K_MY) ? a.cy : 0.0, __ldcg(x + c - s2), s);
   s = fma((kb & K_PZ) ? a.cz : 0.0, __ldcg(x + c + 1), s);
   s = fma((kb & K_MZ) ? a.cz : 0.0, __ldcg(x + c - 1), s);
-  return a.b[c] - fma(dtab[kb & 63], __ldcg(x + c), -s);
+  return a.b[c] - fma(dtab[kb & 63], __ldcg(x + c), xneg(s));
 }
 
 // The solve's scalars, thread 0's (shared memory; every block holds the same).
@@ -427,16 +427,16 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
           for (int m = 0; m < K; m++) {
             const T pm = pc[m * t1v];
             xs[m * nt + t] = fma(alpha, pm, xs[m * nt + t]);
-            r[m] = fma(-alpha, q[m], r[m]);
+            r[m] = fma(xneg(alpha), q[m], r[m]);
           }
-          rlo = fma(-alpha, qlo, rlo);
-          rhi = fma(-alpha, qhi, rhi);
+          rlo = fma(xneg(alpha), qlo, rlo);
+          rhi = fma(xneg(alpha), qhi, rhi);
           direct(bt, t1v);
         }
 #pragma unroll
         for (int u = 0; u < CC_HALO; u++)
           if (place[u] >= 0) {
-            const T rn = fma(-alpha, v[u], rh[h0 + u * nt]);
+            const T rn = fma(xneg(alpha), v[u], rh[h0 + u * nt]);
             rh[h0 + u * nt] = rn;
             p[place[u]] = fma(bt, p[place[u]], rn);
           }
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
         const T above = pm[t1v];
         const T s = fma(cx, above + below, fma(cy, pm[t2] + pm[-t2], cz * (pm[1] + pm[-1])));
         const int kb = kind(m);
-        q[m] = kb >> K_ROW_SHIFT == ROW_ACTUAL ? fma(dtab[kb & 63], c, -s) : T(0);
+        q[m] = kb >> K_ROW_SHIFT == ROW_ACTUAL ? fma(dtab[kb & 63], c, xneg(s)) : T(0);
         if (m < eim && (edge || m == 0 || m == ei - 1)) qx[c0 + m * s1v] = q[m];
         acc[0].add(c, q[m]);
         acc[1].add(r[m], q[m]);

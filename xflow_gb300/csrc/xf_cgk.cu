@@ -55,7 +55,7 @@ __device__ __forceinline__ T lap_fast(uint8_t kb, T cxm, T cxp, T cym, T cyp, T 
     s = fma(kmy, xjm, s);
     s = fma(kpz, xkp, s);
     s = fma(kmz, xkm, s);
-    return fma(d, xc, -s);
+    return fma(d, xc, xneg(s));
   } else {
     const T tpx = (kb & K_PX) ? cxp * (xp - xc) : T(0);
     const T tmx = (kb & K_MX) ? cxm * (xc - xm) : T(0);

@@ -342,6 +342,14 @@ __device__ inline double finish_partials(DevScratch* S, int slot, double* sh) {
 }
 
 // ---------------------------------------------------------------------------
+// -v by the sign bit: compiled from a minus sign, the negated operand of an
+// FP64 FMA was an instruction of the FP64 pipe of its own (7 of the 18 that a
+// Laplace row took), where this is one integer operation.
+__device__ __forceinline__ double xneg(double v) {
+  return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v));
+}
+__device__ __forceinline__ float xneg(float v) { return -v; }
+
 // a / b correctly rounded, from y = RN(1/b), itself a normal number (the grid's
 // reciprocal tables, 1/tau from the host, or __drcp_rn).  q = RN(a y) lies within an ulp of a / b, the
 // residual r = a - b q is exact (one FMA), and RN(q + r y) = RN(a / b):
@@ -358,7 +366,7 @@ __device__ __forceinline__ double div_rcp(double a, double b, double y) {
   const double q = a * y;
   const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, eq = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
   if (ea - (1023u - 950u) >= 1950u || eq - (1023u - 950u) >= 1950u) return a / b;
-  const double r = fma(-b, q, a);
+  const double r = fma(xneg(b), q, a);
   return fma(r, y, q);
 }
 

@@ -32,10 +32,10 @@ __device__ __forceinline__ void ln_step(double a, double b, double c, double f, 
   const unsigned e = ((unsigned)__double2hiint(den) >> 20) & 0x7ffu;
   if (e - 64u < 1900u) {   // the reciprocal is a normal number
     const double y = __drcp_rn(den);
-    A = div_rcp(-c, den, y);
+    A = div_rcp(xneg(c), den, y);
     B = div_rcp(num, den, y);
   } else {
-    A = (-c) / den;
+    A = xneg(c) / den;
     B = num / den;
   }
 }

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_pack_mv(PackArgs a) {
     for (int q = 0; q < cnt; q++) v = v + a.val[q * a.R + r] * a.x[a.col[q * a.R + r]];
     if (a.sign > 0) v = v + a.s[c];
     else if (a.sign < 0) v = v - a.s[c];
-    if (a.neg) v = -v;
+    if (a.neg) v = xneg(v);
     if (a.dot_w) dw.add(a.w[c], v);
     if (a.dot_self) ds.add(v, v);
     if (a.y) a.y[c] = v;

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_xr(T* __restrict__ x, T* __r
 #pragma unroll
     for (int l = 0; l < L; l++) {
       xa[l] = fma(alpha, pa[l], xa[l]);
-      ra[l] = fma(-alpha, qa[l], ra[l]);
+      ra[l] = fma(xneg(alpha), qa[l], ra[l]);
       acc.add(ra[l], ra[l]);
     }
     reinterpret_cast<VT*>(x)[v] = xv;
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_xr(T* __restrict__ x, T* __r
   }
   for (int64_t c = nv * L + tid; c < n; c += stride) {
     x[c] = fma(alpha, p[c], x[c]);
-    T rv = fma(-alpha, q[c], r[c]);
+    T rv = fma(xneg(alpha), q[c], r[c]);
     r[c] = rv;
     acc.add(rv, rv);
   }
@@ -237,7 +237,7 @@ __global__ void k_bcgs_p(double* __restrict__ Pn1, const double* __restrict__ Rn
       t = bn * t;
       p = Rn[i] + t;
     } else {
-      p = fma(bn, fma(-wn, Vn[i], Pn[i]), Rn[i]);
+      p = fma(bn, fma(xneg(wn), Vn[i], Pn[i]), Rn[i]);
     }
     Pn1[i] = p;
     if (dinv) Ph[i] = dinv[i] * p;
@@ -253,7 +253,7 @@ __global__ void k_bcgs_s(double* __restrict__ Sn, const double* __restrict__ Rn,
   const double an = S->scalars[D_AN];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (!m[i]) continue;
-    const double s = EXACT ? Rn[i] - an * Vn[i] : fma(-an, Vn[i], Rn[i]);
+    const double s = EXACT ? Rn[i] - an * Vn[i] : fma(xneg(an), Vn[i], Rn[i]);
     Sn[i] = s;
     if (dinv) Sh[i] = dinv[i] * s;
   }
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_bcgs_end(double* __restrict__ U
       rn = sn - t;
     } else if (update) {
       un = fma(an, xp, fma(wn, xs, un));
-      rn = fma(-wn, tn, sn);
+      rn = fma(xneg(wn), tn, sn);
     }
     best = absmax_bits(best, rn);
     dot.add(sr, rn);

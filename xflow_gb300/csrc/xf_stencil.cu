@@ -67,12 +67,12 @@ __device__ __forceinline__ T march_lap(const StencilGrid<T>& g, const MatvecArgs
     const T kpy = (kb & K_PY) ? cyp : T(0), kmy = (kb & K_MY) ? cym : T(0);
     const T kpz = (kb & K_PZ) ? czp : T(0), kmz = (kb & K_MZ) ? czm : T(0);
     T acc = (T)a.diag[c] * xc;
-    acc = fma(-kpx, xp, acc);
-    acc = fma(-kmx, xm, acc);
-    acc = fma(-kpy, xjp, acc);
-    acc = fma(-kmy, xjm, acc);
-    acc = fma(-kpz, xkp, acc);
-    acc = fma(-kmz, xkm, acc);
+    acc = fma(xneg(kpx), xp, acc);
+    acc = fma(xneg(kmx), xm, acc);
+    acc = fma(xneg(kpy), xjp, acc);
+    acc = fma(xneg(kmy), xjm, acc);
+    acc = fma(xneg(kpz), xkp, acc);
+    acc = fma(xneg(kmz), xkm, acc);
     return acc;
   } else {
     // FP32: the reference's difference form, c * (x_n - x_c)
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(MV_THREADS, EXACT ? 1 : 4) k_matvec(MatvecArgs
         else v = apply_row<T, OP, EXACT>(g, x, i, j, k, c, kc);
         if (a.sign > 0) v = v + a.s[c];
         else if (a.sign < 0) v = v - a.s[c];
-        if (a.neg) v = -v;
+        if (a.neg) v = xneg(v);
         if (a.dot_w) dw.add(a.w[c], v);
         if (a.dot_self) ds.add(v, v);
         if (a.y) a.y[c] = v;
@@ -203,17 +203,17 @@ __device__ __forceinline__ AdAxis ad_axis(const double* __restrict__ t, int n, i
 // the table's kernel.
 template <bool UP>
 __device__ __forceinline__ void ad_coef_fast(const AdAxis& t, double vd, double D, double& A, double& C, double& centre) {
-  A = -D * t.dA;
-  C = -D * t.dC;
+  A = xneg(D) * t.dA;
+  C = xneg(D) * t.dC;
   centre = fma(D, t.dB, centre);
   if (!UP) {
-    A = fma(-vd, t.r2, A);
+    A = fma(xneg(vd), t.r2, A);
     C = fma(vd, t.r2, C);
   } else if (vd < 0) {
-    centre = fma(-vd, t.rh, centre);
+    centre = fma(xneg(vd), t.rh, centre);
     C = fma(vd, t.rh, C);
   } else {
-    A = fma(-vd, t.rh, A);
+    A = fma(xneg(vd), t.rh, A);
     centre = fma(vd, t.rh, centre);
   }
 }
@@ -227,8 +227,8 @@ __device__ __forceinline__ double ad_reciprocal(double d) {
   if (e < 64 || e > 1982) return d != 0 ? 1.0 / d : 0.0;
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = fma(y, fma(-d, y, 1.0), y);
-  return fma(y, fma(-d, y, 1.0), y);
+  y = fma(y, fma(xneg(d), y, 1.0), y);
+  return fma(y, fma(xneg(d), y, 1.0), y);
 }
 
 enum { AD_ROW = 64, AD_OBLIQUE = 128 };
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<
     if (u & AD_OBLIQUE) v = ad_border_row(g, x, c, row_of(g.kind[c]));
     if (a.sign > 0) v = v + a.s[c];
     else if (a.sign < 0) v = v - a.s[c];
-    if (a.neg) v = -v;
+    if (a.neg) v = xneg(v);
     if (a.dot_w) dw.add(a.w[c], v);
     if (a.dot_self) ds.add(v, v);
     if (a.y) a.y[c] = v;

@@ -95,7 +95,7 @@ __global__ void k_pressure_rhs(const uint8_t* __restrict__ code, int n1, int n2,
       const double d = rho ? rho[c] : 1.0;
       const double div_ = d * d * div_rcp(u_i - u_i_1, hxU[i - 1], rhxU[i - 1]) +
                           div_rcp(v_j - v_j_1, hyV[j - 1], rhyV[j - 1]) + div_rcp(w_k - w_k_1, hzW[k - 1], rhzW[k - 1]);
-      rhs[c] = -div_rcp(div_, tau, rtau);
+      rhs[c] = xneg(div_rcp(div_, tau, rtau));
     } else if (m == PC_PREDEFINED) {
       rhs[c] = border ? border[c] : 0.0;
     } else if (m == PC_PRENORMAL || m == PC_DEFINED || m == PC_NORMAL || m == PC_EQUATION || m == PC_PREEQUATION) {
