@@ -549,9 +549,11 @@ int column_form(int bi) { return (bi + 1) / 2 * 2; }
 
 // The split of an interior of ni x nj x nk cells into at most `blocks`
 // bricks of at most CC_THREADS columns of CC_KMAX cells: the least cells a
-// brick (few cells cost as much as half a block's threads), a halo cell
-// counted by a third (a copy and an FMA against the row's work), a block by
-// half a cell (the polls).
+// brick (few cells cost as much as half a block's threads), a cell of a
+// column's length counted by CC_LENGTH more (the latency of a column's steps;
+// long columns leave few warps to hide it), a halo cell by a third (a copy and
+// an FMA against the row's work), a block by half a cell (the polls).
+constexpr int CC_LENGTH = 48;
 bool make_plan(int ni, int nj, int nk, int blocks, bool mixed, Plan* out) {
   double best = 1e300;
   const int top = blocks < CC_MAX_BLOCKS ? blocks : CC_MAX_BLOCKS;
@@ -569,7 +571,8 @@ bool make_plan(int ni, int nj, int nk, int blocks, bool mixed, Plan* out) {
         const size_t smem = (size_t)K * threads * (mixed ? 4 : 8) + ((box + 1) & ~1ll) * (mixed ? 4 : 8) +
                             2ll * bi * (bj + bk) * (8 + (mixed ? 4 : 8));
         if (smem > (mixed ? 215 : 205) * 1024) continue;   // beside the static part
-        const double cost = (double)(cells > CC_THREADS / 2 ? cells : CC_THREADS / 2) + 0.3 * halo + 0.5 * mi * mj * mk;
+        const double cost = (double)(cells > CC_THREADS / 2 ? cells : CC_THREADS / 2) + CC_LENGTH * K + 0.3 * halo +
+                            0.5 * mi * mj * mk;
         if (cost < best) {
           best = cost;
           *out = {1, bi, bj, bk, mi, mj, mk, threads, smem};
