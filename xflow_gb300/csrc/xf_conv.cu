@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128) k_tc_gemm(const uint16_t* __restrict__ A,
   stage_kmajor(sA, A, TC_M, K, K);
   stage_kmajor(sB, B, N, K, K);
   tc::fence_async_smem();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t ncols = tmem_cols(N);
   if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
   if (threadIdx.x == 0) tc::mbar_init(&mbar, 1);
@@ -178,7 +178,13 @@ __device__ __forceinline__ void conv_store8(const ConvArgs& a, int64_t c, int co
     *reinterpret_cast<uint4*>(a.out16 + (co >> 3) * a.out_ps + c * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   } else {
     const int nq = min(8, a.out_ch - co);
-    for (int q = 0; q < nq; q++) a.out32[c * a.out_ld + co + q] = v[q];
+    float* dst = a.out32 + c * a.out_ld + co;
+    if (nq == 8 && ((uintptr_t)dst & 15) == 0) {   // a cell's 32 bytes by two stores (scalar ones: 8 sectors a lane)
+      reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+      reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+      for (int q = 0; q < nq; q++) dst[q] = v[q];
+    }
   }
 }
 
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(128) k_conv3_tc(ConvArgs a) {
   __shared__ uint32_t tmem_base;
   const int Ci = a.Ci, Co = a.Co, kg = Ci / 8;
   const int stage_a = TC_M * Ci * 2, stage_b = Co * Ci * 2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t ncols = tmem_cols(Co);
   if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
   if (threadIdx.x == 0)
@@ -306,9 +312,10 @@ __global__ void __launch_bounds__(128) k_conv3_tc(ConvArgs a) {
 //       thread issuing all of them was the pipeline's bottleneck), lane 0
 //       keeping the barriers (full: the copies' transaction bytes; empty: the MMAs that
 //       read the stage have completed);
-//   warp 5, one thread: the MMAs into one of two TMEM accumulators (the
-//       epilogue of a tile overlaps the next tile's MMAs), a commit per
-//       stage and one per finished tile;
+//   warp 5: the MMAs into one of two TMEM accumulators (the epilogue of a
+//       tile overlaps the next tile's MMAs), a commit per stage and one per
+//       finished tile.  The whole warp walks the loop and one elected lane
+//       issues, so that the descriptors are uniform;
 //   warps 0-3: the epilogue, TMEM lanes 32 w .. 32 w + 31.
 // Every wait is bounded by the SM clock; a wait that runs out sets the
 // kernel's error flag and an abort flag in shared memory that ends every
@@ -358,6 +365,11 @@ __device__ __forceinline__ bool bk_wait(uint64_t* mbar, uint32_t parity, volatil
       return false;
     }
   }
+}
+// The same by a whole warp, with one answer.
+__device__ __forceinline__ bool bk_wait_warp(uint64_t* mbar, uint32_t parity, volatile int* abort_flag,
+                                             bool honour_abort = true) {
+  return __all_sync(0xffffffffu, bk_wait(mbar, parity, abort_flag, honour_abort));
 }
 // Barrier 1 over the four epilogue warps with an AND of `pred`.
 __device__ __forceinline__ bool epi_sync_and(bool pred) {
@@ -420,7 +432,7 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
   __shared__ __align__(16) float xch[2][4][2][80];   // per tile parity and warp: lane 31's D_-1 row, lane 0's D_+1 row
   const int Ci = a.Ci, Co = a.Co, N3 = 3 * Co, nk = Ci / 16;
   const int S = plan.stages;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t raw = tc::smem_addr(dsm);
   uint8_t* smem = dsm + ((1024u - (raw & 1023u)) & 1023u);
   uint8_t* wsm = smem;                    // resident tiled weights
@@ -499,41 +511,42 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
     }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {   // ---- MMA issuer
+    {   // ---- MMA issuer
+      const bool leader = tc::elect_one();
       const uint32_t idesc = tc::idesc_bf16_f32(128, N3);
       const uint32_t b_lbo = (uint32_t)N3 * 16;
-      bool ok = !plan.resident || my_tiles == 0 || bk_wait(&wfull, 0, abort_p);
+      bool ok = !plan.resident || my_tiles == 0 || bk_wait_warp(&wfull, 0, abort_p);
       int st = 0, pass = 0;
       for (int k = 0; k < my_tiles && ok; k++) {
         const int acc = k & 1;
-        if (k >= 2 && !bk_wait(&tempty[acc], (uint32_t)(((k >> 1) - 1) & 1), abort_p)) break;
+        if (k >= 2 && !bk_wait_warp(&tempty[acc], (uint32_t)(((k >> 1) - 1) & 1), abort_p)) break;
         tc::fence_after_sync();
         const uint32_t dacc = tbase + (uint32_t)(acc * plan.acc_off);
         for (int c = 0; c < nk; c++) {
-          if (!bk_wait(&full[st], (uint32_t)(pass & 1), abort_p)) {
+          if (!bk_wait_warp(&full[st], (uint32_t)(pass & 1), abort_p)) {
             ok = false;
             break;
           }
           tc::fence_after_sync();
           const uint8_t* sa = stg + st * plan.stage_bytes;
           const uint8_t* sb = plan.resident ? wsm + (size_t)c * 9 * N3 * 32 : sa + BK_A;
-#pragma unroll 1
+#pragma unroll
           for (int sl = 0; sl < 9; sl++) {
             const uint64_t ad = tc::smem_desc(tc::smem_addr(sa + sl * BK_SLAB), 2048, 128);
             const uint64_t bd = tc::smem_desc(tc::smem_addr(sb + sl * N3 * 32), b_lbo, 128);
-            tc::mma_bf16(dacc, ad, bd, idesc, c > 0 || sl > 0);
+            if (leader) tc::mma_bf16(dacc, ad, bd, idesc, c > 0 || sl > 0);
           }
-          tc::mma_commit(&empty[st]);
+          if (leader) tc::mma_commit(&empty[st]);
           if (++st == S) {
             st = 0;
             pass++;
           }
         }
-        if (ok) tc::mma_commit(&tfull[acc]);
+        if (ok && leader) tc::mma_commit(&tfull[acc]);
       }
       // every MMA issued has completed before TMEM is freed
-      tc::mma_commit(&mdone);
-      bk_wait(&mdone, 0, abort_p, false);
+      if (leader) tc::mma_commit(&mdone);
+      bk_wait_warp(&mdone, 0, abort_p, false);
     }
     __syncwarp();
   } else {   // ---- epilogue, warps 0-3
@@ -659,7 +672,7 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
   __shared__ uint64_t full[WG_STAGES], empty[WG_STAGES], mdone;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int mt = blockIdx.x % a.mtiles, sp = blockIdx.x / a.mtiles;
   const int cp = a.ci / 8, t0 = mt * a.taps, tn = min(27, t0 + a.taps) - t0;
   const int ga = tn * cp, gb = a.co / 8;   // blocks of A and of B per stage
@@ -721,26 +734,27 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
       }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {   // ---- MMA issuer
+    {   // ---- MMA issuer
+      const bool leader = tc::elect_one();
       const uint32_t idesc = tc::idesc_bf16_f32(128, a.co) | (1u << 15) | (1u << 16);   // A and B MN-major
       int st = 0, pass = 0;
       for (int k = 0; k < my_stages; k++) {
-        if (!bk_wait(&full[st], (uint32_t)(pass & 1), abort_p)) break;
+        if (!bk_wait_warp(&full[st], (uint32_t)(pass & 1), abort_p)) break;
         tc::fence_after_sync();
         const uint8_t* sa = smem + st * a.stage_bytes;
-#pragma unroll 1
+#pragma unroll
         for (int kk = 0; kk < WG_KC / 16; kk++) {
           const uint64_t ad = tc::smem_desc(tc::smem_addr(sa + kk * 256), 128, WG_BLOCK);
           const uint64_t bd = tc::smem_desc(tc::smem_addr(sa + WG_A + kk * 256), 128, WG_BLOCK);
-          tc::mma_bf16(tbase, ad, bd, idesc, k > 0 || kk > 0);
+          if (leader) tc::mma_bf16(tbase, ad, bd, idesc, k > 0 || kk > 0);
         }
-        tc::mma_commit(&empty[st]);
+        if (leader) tc::mma_commit(&empty[st]);
         if (++st == WG_STAGES) {
           st = 0;
           pass++;
         }
       }
-      tc::mma_commit(&mdone);   // every MMA issued
+      if (leader) tc::mma_commit(&mdone);   // every MMA issued
     }
     __syncwarp();
   } else {   // ---- epilogue, warps 0-3: the partial of this tile and range
