@@ -453,9 +453,9 @@ def main(argv=None):
     bpc = {"stencil_f32": 9, "xr_update_f32": 24, "p_update_f32": 12, "residual_f64": 29, "stencil_f64": 25,
            "pq_fused_f32": 17, "pq_march_f32": 17, "poly2_f32": 9, "polyr_f32": 29,
            "cheb_first_fused_f32": 29, "cheb_last_f32": 13, "cheb_middle_f32": 9,
-           # the two-level passes: kind + y, A y; r, A y, kind + w; w, y, r, q_w, kind, mask + z, slot
-           "tl_prolong_ay_f32": 9, "tl_first_f32": 13, "tl_last_f32": 26}
-    # the learned two-level iteration's fine-grid passes: y = P zc with A y,
+           # the two-level passes: r, kind + r'; r', kind + w; w, r, q_w, kind + z
+           "tl_prolong_ay_f32": 9, "tl_first_f32": 9, "tl_last_f32": 17}
+    # the learned two-level iteration's fine-grid passes: r' = r - omega A P zc,
     # the smoother's first and last factor passes (TL_DEGREE / 2 - 2 middle
     # passes between them), and the FP32 stencil with a dot for A p
     per_iter = {"tl_prolong_ay_f32": 1, "tl_first_f32": 1, "tl_last_f32": 1, "cheb_middle_f32": TL_DEGREE // 2 - 2,

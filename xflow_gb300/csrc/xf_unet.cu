@@ -34,17 +34,20 @@ void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mti
 int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps, int co, const void* x, int64_t xps,
                 int ci, float* partial, float* gw);
 void xf_cg_q32_dot(const xf_op* op, const float* p, float* q, int slot);
-bool xf_tl_prolong_ay_supported(const xf_grid* g);
-void xf_tl_prolong_ay(const xf_op* op, const float* zc, int c2, int c3, float* y, float* ay, int slot);
+void xf_tl_faces(const xf_grid* g, const xf_grid* cg, uint32_t* cnt);
+void xf_tl_omega(const xf_grid* g, const xf_grid* cg, const float* zc, const uint32_t* cnt, const double* rc, int slot,
+                 int s_om);
+void xf_tl_sub(const xf_grid* g, const float* r, const float* zc, int c2, int c3, int s_om, float* out);
+void xf_tl_sub_ay(const xf_grid* g, const float* r, const float* ay, int s_yay, int s_yr, int s_om, float* out);
 void xf_cg_res64(const xf_op* op, const double* x, const double* b, float* r32, int slot, int ctl);
 void xf_dot_async(const xf_grid* g, int dtype, const void* a, const void* b, int slot);
 int xf_op_ready(const xf_op* op);
 bool xf_cg_poly_supported(const xf_grid* g);
 bool xf_cheb_factors(double lmax, double ratio, int deg, float (*f)[3]);
 void xf_cheb2_coeffs(double lmax, double ratio, float out[3]);
-void xf_cg_poly_tl_launch(const xf_op* op, bool first, bool last, const float* in, const float* q, float* out,
-                          const float coeffs[3], int s_yay, int s_yr, const float* y, float tsc, float* z2,
-                          const float* r, const float* qw, int s_zr, int s_zq);
+void xf_cg_poly_last_tl_launch(const xf_op* op, const float* in, float* z, const float coeffs[3], int s_om,
+                               const float* zc, int c3, int cs1, int F, float tsc, const float* r, const float* qw,
+                               int s_zr, int s_zq);
 void xf_cg_poly_first_launch(const xf_op* op, const float* r, float* w, const float coeffs[3], const float* q,
                              const float* pa, const float* pb, float* e, float* r_out);
 
@@ -947,36 +950,6 @@ __global__ void k_restrict4(const float* __restrict__ r, int f2, int f3, double*
   }
   rc[((int64_t)I * c2 + J) * c3 + K] = v;
 }
-// Four consecutive cells of a plane per thread: one 4-byte mask load and one
-// 16-byte store.  With F = 4 every fine interior extent is a multiple of 4, so
-// n2 = 4a + 2 and n3 = 4b + 2 and the plane size n2 n3 is a multiple of 4;
-// with the 256-byte aligned allocations of y and the space mask, every
-// thread's group then starts on a 16-byte (y) and 4-byte (mask) boundary.
-__global__ void k_prolong4v(const double* __restrict__ zc, int c2, int c3, const uint8_t* __restrict__ smask, int f1,
-                            int f2, int f3, float* __restrict__ y) {
-  const int P = f2 * f3;
-  const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), i = blockIdx.y;
-  if (p0 >= P) return;
-  const int64_t c0 = (int64_t)i * P + p0;
-  const uchar4 m4 = *reinterpret_cast<const uchar4*>(smask + c0);
-  const unsigned char mk[4] = {m4.x, m4.y, m4.z, m4.w};
-  int j = p0 / f3, k = p0 - j * f3;
-  float v[4];
-  const bool irow = i > 0 && i < f1 - 1;
-  const int64_t ib = (int64_t)(1 + ((i - 1) >> 2)) * c2;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    float t = 0.f;
-    if (mk[q] && irow && j > 0 && j < f2 - 1 && k > 0 && k < f3 - 1)
-      t = (float)__ldg(&zc[(ib + (1 + ((j - 1) >> 2))) * c3 + (1 + ((k - 1) >> 2))]);
-    v[q] = t;
-    if (++k == f3) {
-      k = 0;
-      j++;
-    }
-  }
-  *reinterpret_cast<float4*>(y + c0) = make_float4(v[0], v[1], v[2], v[3]);
-}
 // (a, b) of FP32 boxes that are zero off the active set: exact products
 // accumulated in float-float per thread and per warp, FP64 across warps and
 // blocks; 16-byte loads.  -> scalars[slot]
@@ -1042,8 +1015,8 @@ static double cheb_scale(const float (*f)[3], int nf, double lmax, double ratio)
 }
 
 // scalar slots: 0..7 (z, A p_j); 8 (y, A y), 9 (y, r) of the two-level preconditioner; 10 (z, r); 11 (r, r);
-// 12 (p, r); 14/15 matvec dots
-enum { FS_YAY = 8, FS_YR = 9, FS_ZR = 10, FS_RR = 11, FS_PR = 12, FS_PQ = 14 };
+// 12 (p, r); 13 omega; 14/15 matvec dots
+enum { FS_YAY = 8, FS_YR = 9, FS_ZR = 10, FS_RR = 11, FS_PR = 12, FS_OM = 13, FS_PQ = 14 };
 
 static int read_n(xf_ctx* ctx, int first, int count, double* out) {
   XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, &ctx->scratch->scalars[first], count * 8, cudaMemcpyDeviceToHost,
@@ -1081,9 +1054,9 @@ static int read_n(xf_ctx* ctx, int first, int count, double* out) {
 //
 // The m + 1 iteration blocks are the ring positions of the new direction, so
 // every kernel argument is fixed at capture.  Inside an iteration block:
-//   IF/ELSE (network on): z = M r (restriction, U-Net, prolongation, A y, the
-//                         smoother passes reducing (z, r), (z, q_0)) /
-//                         z = r with its dots
+//   IF/ELSE (network on): z = M r (restriction, U-Net, omega, r - omega A P zc,
+//                         the smoother passes reducing (z, r), (z, q_0)) /
+//                         z = r with its dots; z stands in the direction slot
 //   IF (no descent direction, (z, r) <= 0): z = r with its dots; the third
 //                         time the network is switched off
 //   p = z - sum_j (z, q_j) / (p_j, q_j) p_j, q = A p, (p, q), (p, r), alpha,
@@ -1108,7 +1081,7 @@ struct TlParams {
   double rtol2;
   int maxit, every;
   // kernels per segment, for the launch count
-  int n_ref, n_iter, n_on, n_off, n_fb;
+  int n_init, n_ref, n_iter, n_on, n_off, n_fb;
 };
 struct TlHandles {
   cudaGraphConditionalHandle main, ref, blk[9], pre[9], fb[9];
@@ -1147,7 +1120,7 @@ __global__ void k_tl_init(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles 
   c->rr_true = 0; c->rr_prev_true = 0; c->rr = 0; c->rr_start = 0; c->alpha = 0;
   for (int j = 0; j < 9; j++) c->pq_win[j] = 0;
   for (int j = 0; j < 8; j++) { c->coef[j] = 0.f; c->use_coef[j] = 0; c->win_off[j] = 1; }
-  c->launches = 2;
+  c->launches = p->n_init;
 }
 // x += e after a cycle (none before the first)
 __global__ void k_tl_fold(double* __restrict__ x, const float* __restrict__ e, int64_t n, const TlCtl* c) {
@@ -1372,13 +1345,15 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     t->bufs.push_back(p);
     return p;
   };
-  double *rc = (double*)alloc(nc * 8), *zc = (double*)alloc(nc * 8);
-  float *r = (float*)alloc(n * 4), *e = (float*)alloc(n * 4), *z = (float*)alloc(n * 4), *y = (float*)alloc(n * 4);
-  float *ay = (float*)alloc(n * 4), *w0 = (float*)alloc(n * 4), *w1 = (float*)alloc(n * 4);
+  const bool f4 = F == 4;   // the transfers of xf_tl.cu; else y = P zc and A y are stored
+  double *rc = (double*)alloc(nc * 8), *zc = f4 ? nullptr : (double*)alloc(nc * 8);
+  float *r = (float*)alloc(n * 4), *e = (float*)alloc(n * 4), *ay = f4 ? nullptr : (float*)alloc(n * 4);
+  float *w0 = (float*)alloc(n * 4), *w1 = (float*)alloc(n * 4);
+  uint32_t* faces = f4 ? (uint32_t*)alloc(nc * 4) : nullptr;
   t->ctl = (TlCtl*)alloc(sizeof(TlCtl));
   t->prm = (TlParams*)alloc(sizeof(TlParams));
   float *P[9] = {nullptr}, *Q[9] = {nullptr};   // ring of m + 1: the new direction and the window
-  bool ok = rc && zc && r && e && z && y && ay && w0 && w1 && t->ctl && t->prm;
+  bool ok = rc && (f4 ? faces != nullptr : zc && ay) && r && e && w0 && w1 && t->ctl && t->prm;
   for (int j = 0; j <= m && ok; j++) ok = (P[j] = (float*)alloc(n * 4)) && (Q[j] = (float*)alloc(n * 4));
   if (!ok) return fail(XF_ERR_NOMEM, "allocation");
   if (cudaStreamSynchronize(s) != cudaSuccess) return fail(XF_ERR_CUDA, "workspace");
@@ -1392,10 +1367,10 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
   };
   // the window dots j = j0 .. m-1 of block hd (skipped on the device while j >= nwin)
   auto win_dots = [&](int hd, int j0) {
-    for (int j = j0; j < m; j++) fdot(z, Q[(hd + m - j) % (m + 1)], j, &c->win_off[j]);
+    for (int j = j0; j < m; j++) fdot(P[hd], Q[(hd + m - j) % (m + 1)], j, &c->win_off[j]);
   };
   // warm the network's kernels (attributes, first launches) outside capture
-  int rcode = xf_unet_apply_dev(u, rc, zc);
+  int rcode = f4 ? forward(u, rc) : xf_unet_apply_dev(u, rc, zc);
   if (rcode) {
     delete t;
     return rcode;
@@ -1451,6 +1426,7 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
   // init: (b, b), the state, the block handles; before the loop
   begin(top, nullptr, 0);
   xf_dot_async(g, XF_F64, b, b, FS_RR);
+  if (f4) xf_tl_faces(g, cg, faces);
   k_tl_init<<<1, 32, 0, s>>>(S, c, prm, H, m);
   end_tail(tail);
   if (ce == cudaSuccess) {
@@ -1488,43 +1464,40 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     add_cond(bbody, tail, H.pre[hd], cudaGraphCondTypeIf, 2, ie, &ienode);
     // network on: z = M r with (z, r) and (z, q_newest)
     begin(ie[0], nullptr, 0);
-    if (F == 4)
+    if (f4)
       k_restrict4<<<dim3((cg->n3 + 63) / 64, cg->n2, cg->n1), 64, 0, s>>>(r, g->n2, g->n3, rc, cg->n1, cg->n2, cg->n3);
     else
       k_restrict_blocks<float><<<grid_blocks(ctx, nc, 256), 256, 0, s>>>(r, g->n2, g->n3, F, rc, cg->n1, cg->n2,
                                                                          cg->n3);
-    if (ce == cudaSuccess && (rcode = xf_unet_apply_dev(u, rc, zc))) ce = cudaErrorUnknown;
-    if (F == 4 && xf_tl_prolong_ay_supported(g)) {   // y = P zc, A y and (y, A y) in one pass
-      xf_tl_prolong_ay(op, u->zout, cg->n2, cg->n3, y, ay, FS_YAY);   // the network's FP32 output
-    } else {
-      if (F == 4)   // n2 n3 is a multiple of 4 (see k_prolong4v)
-        k_prolong4v<<<dim3((g->n2 * g->n3 / 4 + 255) / 256, g->n1), 256, 0, s>>>(zc, cg->n2, cg->n3, g->smask,
-                                                                                g->n1, g->n2, g->n3, y);
-      else
-        k_prolong_blocks<float><<<eb, 256, 0, s>>>(zc, cg->n2, cg->n3, F, g->smask, g->n1, g->n2, g->n3, y);
-      xf_cg_q32_dot(op, y, ay, FS_YAY);           // A y, (y, A y)
+    if (f4) {   // omega on the coarse grid, r - omega A P zc in one pass; zc is the network's FP32 output
+      if (ce == cudaSuccess && (rcode = forward(u, rc))) ce = cudaErrorUnknown;
+      xf_tl_omega(g, cg, u->zout, faces, rc, FS_YAY, FS_OM);
+      xf_tl_sub(g, r, u->zout, cg->n2, cg->n3, FS_OM, w1);
+    } else {        // y = P zc, A y with (y, A y), (y, r) = (zc, P^T r)
+      if (ce == cudaSuccess && (rcode = xf_unet_apply_dev(u, rc, zc))) ce = cudaErrorUnknown;
+      k_prolong_blocks<float><<<eb, 256, 0, s>>>(zc, cg->n2, cg->n3, F, g->smask, g->n1, g->n2, g->n3, w0);
+      xf_cg_q32_dot(op, w0, ay, FS_YAY);
+      xf_dot_async(cg, XF_F64, zc, rc, FS_YR);
+      xf_tl_sub_ay(g, r, ay, FS_YAY, FS_YR, FS_OM, w1);
     }
-    xf_dot_async(cg, XF_F64, zc, rc, FS_YR);   // (y, r) = (z_c, P^T r)
     {
-      // the smoother: its first pass takes r - omega A y, its last writes
-      // z = omega y + s p(A)(r - omega A y) (also into the direction slot) and reduces the dots
-      float *src = nullptr, *dst = w0;
-      for (int k = tl_nf - 1; k >= 0; k--) {
-        const bool first = k == tl_nf - 1, last = k == 0;
-        xf_cg_poly_tl_launch(op, first, last, first ? r : src, ay, last ? z : dst, tl_f[k], FS_YAY, FS_YR, y,
-                             (float)tl_scale, pn, r, q_newest, FS_ZR, 0);
-        src = dst;
-        dst = dst == w0 ? w1 : w0;
+      // the smoother on r - omega A y; its last pass writes z = omega y + s p(A)(r - omega A y) and reduces the dots
+      float *src = w1, *dst = w0;
+      for (int k = tl_nf - 1; k > 0; k--) {
+        xf_cg_poly_first_launch(op, src, dst, tl_f[k], nullptr, nullptr, nullptr, nullptr, nullptr);
+        std::swap(src, dst);
       }
+      xf_cg_poly_last_tl_launch(op, src, pn, tl_f[0], FS_OM, u->zout, cg->n3, cg->n2 * cg->n3, F, (float)tl_scale, r,
+                                q_newest, FS_ZR, 0);
     }
     win_dots(hd, 1);
     end_tail(unused);
-    n_on = (F == 4 && xf_tl_prolong_ay_supported(g) ? 3 : 4) + UNET_FORWARD_LAUNCHES + tl_nf + (m - 1);
+    // F = 4: no output conversion of the network
+    n_on = (f4 ? 3 - 1 : 5) + UNET_FORWARD_LAUNCHES + tl_nf + (m - 1);
     // network off: z = r with its dots
     begin(ie[1], nullptr, 0);
-    cudaMemcpyAsync(z, r, n * 4, cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(pn, r, n * 4, cudaMemcpyDeviceToDevice, s);
-    fdot(z, r, FS_ZR, nullptr);
+    fdot(pn, r, FS_ZR, nullptr);
     win_dots(hd, 0);
     end_tail(unused);
     n_off = 1 + m;
@@ -1536,9 +1509,8 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     cudaGraphNode_t fnode = nullptr;
     add_cond(bbody, tail, H.fb[hd], cudaGraphCondTypeIf, 1, &fbody, &fnode);
     begin(fbody, nullptr, 0);
-    cudaMemcpyAsync(z, r, n * 4, cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(pn, r, n * 4, cudaMemcpyDeviceToDevice, s);
-    fdot(z, r, FS_ZR, nullptr);
+    fdot(pn, r, FS_ZR, nullptr);
     win_dots(hd, 0);
     end_tail(unused);
     n_fb = 1 + m;
@@ -1570,7 +1542,7 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     return fail(XF_ERR_CUDA, cudaGetErrorString(ce));
   }
   TlParams hp = {};
-  hp.n_ref = 3; hp.n_iter = n_iter; hp.n_on = n_on; hp.n_off = n_off; hp.n_fb = n_fb;
+  hp.n_init = f4 ? 3 : 2; hp.n_ref = 3; hp.n_iter = n_iter; hp.n_on = n_on; hp.n_off = n_off; hp.n_fb = n_fb;
   if (cudaMemcpy(t->prm, &hp, sizeof(hp), cudaMemcpyHostToDevice) != cudaSuccess) return fail(XF_ERR_CUDA, "params");
   t->op_serial = op->serial; t->x = xv->data; t->b = bv->data; t->m = m; t->F = F; t->nf = tl_nf;
   memcpy(t->f, tl_f, sizeof(float) * 3 * tl_nf);
