@@ -30,6 +30,7 @@
 #include "xf_bulk.cuh"
 #include "xf_control.cuh"
 #include "xf_stencil.cuh"
+#include "xf_tl.cuh"
 
 namespace {
 
@@ -49,10 +50,13 @@ struct PqbArgs {
   int HA, RL;                 // halo width (multiple of 4, >= n3 + 1), region length TILE + 2 HA
   int tiles, chunk, nchunk;   // work items: nchunk plane chunks x tiles
   float cx, cy, cz;
-  int ctl;                    // control step of the last block
+  int slot, ctl;              // of (p', q), and the control step of the last block
+  TlStep step;                // the flexible CG's, in its place (step.ctl not null)
 };
 
+// r + b p; b = 0 leaves p out (a buffer that holds no direction yet)
 __device__ __forceinline__ float4 fma4(float b, float4 p, float4 r) {
+  if (b == 0.f) return r;
   return make_float4(fmaf(b, p.x, r.x), fmaf(b, p.y, r.y), fmaf(b, p.z, r.z), fmaf(b, p.w, r.w));
 }
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -270,12 +274,13 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
     __syncthreads();
     return;
   }
-  if (!publish_acc<float>(S, SL_A, SL_A, acc, sh, &last)) return;
-  double tot = finish_partials(S, SL_A, sh);
+  if (!publish_acc<float>(S, a.slot, a.slot, acc, sh, &last)) return;
+  double tot = finish_partials(S, a.slot, sh);
   if (threadIdx.x == 0) {
-    S->scalars[SL_A] = tot;
-    S->tickets[SL_A] = 0;
-    control_step(S, a.ctl);
+    S->scalars[a.slot] = tot;
+    S->tickets[a.slot] = 0;
+    if (a.step.ctl) tl_alpha(S, a.step);
+    else control_step(S, a.ctl);
   }
 }
 
@@ -292,7 +297,8 @@ bool xf_cg_pqb_supported(const xf_grid* g) {
   return pqb_smem(PQB_TILE + 2 * HA, 2) <= 227 * 1024 - 1024;
 }
 
-void xf_cg_pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int ctl) {
+static void pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int slot, int ctl,
+                       const TlStep& step) {
   const xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
   PqbArgs a;
@@ -303,7 +309,7 @@ void xf_cg_pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, f
   a.RL = PQB_TILE + 2 * a.HA;
   a.tiles = (a.P + PQB_TILE - 1) / PQB_TILE;
   a.cx = (float)g->ucx; a.cy = (float)g->ucy; a.cz = (float)g->ucz;
-  a.ctl = ctl;
+  a.slot = slot; a.ctl = ctl; a.step = step;
   // ring depth 2 (3 blocks per SM)
   const int ns = 2;
   const size_t smem = pqb_smem(a.RL, ns);
@@ -337,4 +343,15 @@ void xf_cg_pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, f
     if (cap >= 1 && cap < blocks) blocks = cap;
   }
   k_cg_pqb<2><<<(int)blocks, PQB_THREADS, smem, ctx->stream>>>(a);
+}
+
+void xf_cg_pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int ctl) {
+  pqb_launch(op, r, pb0, pb1, q, SL_A, ctl, TlStep{});
+}
+
+// The flexible CG's: p = z + beta p_old (beta = scalars[D_BETA], I_PBUF = 0),
+// q = A p, (p, q) -> scalars[slot], alpha.
+void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot,
+                         const TlStep& step) {
+  pqb_launch(op, z, p_old, p, q, slot, CTL_NONE, step);
 }

@@ -53,6 +53,7 @@
 #include "xf_bulk.cuh"
 #include "xf_control.cuh"
 #include "xf_stencil.cuh"
+#include "xf_tl.cuh"
 
 namespace {
 
@@ -78,6 +79,7 @@ struct CpArgs {
   const float* qw;            // the last direction image (nullptr: no second dot)
   float tsc;                  // the smoother's scale s
   int s_zr, s_zq;             // slots of (z, r) and (z, q_w)
+  TlStep step;                // the flexible CG's descent test (ctl null: none)
   int n1, n3, P;
   int HA, R0, R1;             // halo unit (multiple of 4), raw region TILE + 4 HA, level-1 region TILE + 2 HA
   int KS;                     // bytes of a row-kind slot: R1 + 32 rounded up to 16
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
     return;
   }
   if (MODE == CP_FIRST) return;   // a later pass reduces
-  if (OUT_TL) {   // (z, r) and (z, q_w), one ticket; no control step (the flexible CG reads them)
+  if (OUT_TL) {   // (z, r) and (z, q_w), one ticket
     const double bzr = block_sum_acc<float>(acc, sh);
     const double bzq = block_sum_acc<float>(acc_rr, sh);
     if (threadIdx.x == 0) {
@@ -535,6 +537,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
       S->scalars[a.s_zr] = zr;
       if (a.qw) S->scalars[a.s_zq] = zq;
       S->tickets[a.s_zr] = 0;
+      if (a.step.ctl) tl_z(S, a.step);
     }
     return;
   }
@@ -814,12 +817,13 @@ void xf_cg_poly_second_launch(const xf_op* op, const float* w, const float* r, f
 
 // The two-level smoother's last factor pass: z = omega y + s w of its output w,
 // y the value of the cell's block of F^3 cells in zc (rows of c3, planes of
-// cs1), omega = scalars[s_om]; (z, r) -> s_zr and, with qw, (z, qw) -> s_zq.
+// cs1), omega = scalars[s_om]; (z, r) -> s_zr and, with qw, (z, qw) -> s_zq;
+// then the descent test of `step`.
 void xf_cg_poly_last_tl_launch(const xf_op* op, const float* in, float* z, const float coeffs[3], int s_om,
                                const float* zc, int c3, int cs1, int F, float tsc, const float* r, const float* qw,
-                               int s_zr, int s_zq) {
+                               int s_zr, int s_zq, const TlStep& step) {
   CpArgs a = {};
   a.r = in; a.z = z; a.s_om = s_om; a.zc = zc; a.c3 = c3; a.cs1 = cs1; a.F = F;
-  a.dr = r; a.qw = qw; a.tsc = tsc; a.s_zr = s_zr; a.s_zq = s_zq;
+  a.dr = r; a.qw = qw; a.tsc = tsc; a.s_zr = s_zr; a.s_zq = s_zq; a.step = step;
   poly_launch<CP_TL_LAST>(op, a, coeffs);
 }

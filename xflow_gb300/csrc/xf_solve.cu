@@ -20,6 +20,7 @@
 
 #include "xf_control.cuh"
 #include "xf_stencil.cuh"
+#include "xf_tl.cuh"
 
 void xf_mv64(const xf_op* op, const MvReq<double>& q);
 void xf_mv32(const xf_op* op, const MvReq<float>& q);
@@ -40,7 +41,7 @@ bool xf_cheb_factors(double lmax, double ratio, int deg, float (*f)[3]);
 void xf_tl_sub(const xf_grid* g, const float* r, const float* zc, int c2, int c3, int s_om, float* out);
 void xf_cg_poly_last_tl_launch(const xf_op* op, const float* in, float* z, const float coeffs[3], int s_om,
                                const float* zc, int c3, int cs1, int F, float tsc, const float* r, const float* qw,
-                               int s_zr, int s_zq);
+                               int s_zr, int s_zq, const TlStep& step);
 void xf_cg_poly_first_launch(const xf_op* op, const float* r, float* w, const float coeffs[3], const float* q,
                              const float* pa, const float* pb, float* e, float* r_out);
 void xf_cg_poly_second_launch(const xf_op* op, const float* w, const float* r, float* z, const float coeffs[3]);
@@ -1118,7 +1119,7 @@ extern "C" int xf_profile_cg_kernels(xf_op* op, int reps, double* ms_out) {
       ms_out[12] = time([&] { xf_tl_sub(g, r, zc, c2, c3, SL_C, p); });
       ms_out[13] = time([&] { xf_cg_poly_first_launch(op, p, w, f2, nullptr, nullptr, nullptr, nullptr, nullptr); });
       ms_out[14] = time([&] {
-        xf_cg_poly_last_tl_launch(op, w, e, f1, SL_C, zc, c3, c2 * c3, 4, 1.f, r, q, SL_C + 2, SL_C + 3);
+        xf_cg_poly_last_tl_launch(op, w, e, f1, SL_C, zc, c3, c2 * c3, 4, 1.f, r, q, SL_C + 2, SL_C + 3, TlStep{});
       });
     }
   }

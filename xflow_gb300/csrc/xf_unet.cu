@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "xf_control.cuh"
+#include "xf_tl.cuh"
 
 int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* weights,
                    const void* tiled, const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch,
@@ -47,7 +48,9 @@ bool xf_cheb_factors(double lmax, double ratio, int deg, float (*f)[3]);
 void xf_cheb2_coeffs(double lmax, double ratio, float out[3]);
 void xf_cg_poly_last_tl_launch(const xf_op* op, const float* in, float* z, const float coeffs[3], int s_om,
                                const float* zc, int c3, int cs1, int F, float tsc, const float* r, const float* qw,
-                               int s_zr, int s_zq);
+                               int s_zr, int s_zq, const TlStep& step);
+void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot,
+                         const TlStep& step);
 void xf_cg_poly_first_launch(const xf_op* op, const float* r, float* w, const float coeffs[3], const float* q,
                              const float* pa, const float* pb, float* e, float* r_out);
 
@@ -848,7 +851,7 @@ extern "C" int xf_unet_train_step(xf_unet* u, const xf_op* op, const xf_vec* r, 
 // preconditioner off for the rest of the solve (all counted in
 // stats->fallbacks).  The stop rule is the true relative
 // residual ||b - A x|| <= rtol ||b||.  m = opts->reserved[0] (1..8, default 8).
-constexpr int FCG_STRIKES = 3;   // non-descent preconditioned directions before the network is switched off
+
 __global__ void k_fcg_update(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
                              const double* __restrict__ q, double alpha, int64_t n) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
@@ -1014,9 +1017,6 @@ static double cheb_scale(const float (*f)[3], int nf, double lmax, double ratio)
   return 2.0 / (gmin + gmax);
 }
 
-// scalar slots: 0..7 (z, A p_j); 8 (y, A y), 9 (y, r) of the two-level preconditioner; 10 (z, r); 11 (r, r);
-// 12 (p, r); 13 omega; 14/15 matvec dots
-enum { FS_YAY = 8, FS_YR = 9, FS_ZR = 10, FS_RR = 11, FS_PR = 12, FS_OM = 13, FS_PQ = 14 };
 
 static int read_n(xf_ctx* ctx, int first, int count, double* out) {
   XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, &ctx->scratch->scalars[first], count * 8, cudaMemcpyDeviceToHost,
@@ -1038,7 +1038,8 @@ static int read_n(xf_ctx* ctx, int first, int count, double* out) {
 // across a refresh.  The solve ends only on the true FP64 residual.
 //
 // Every scalar decision (alpha, the window coefficients, the fallback to
-// z = r, the refresh and stop tests) is taken by one-thread control kernels
+// z = r, the refresh and stop tests) is taken by the last block of the pass
+// whose sum it needs (xf_tl.cuh), or by a one-thread kernel off the usual path,
 // on the device, and the whole solve is one CUDA graph with conditional
 // nodes, so it needs no host round trip:
 //
@@ -1047,46 +1048,28 @@ static int read_n(xf_ctx* ctx, int first, int count, double* out) {
 //     IF (refresh):   x += e (after a cycle), e = 0, r = float(b - A x) in
 //                     FP64 with (r, r); the stop, iteration-cap and stall
 //                     tests
-//     IF (head == 0): one iteration with direction slot 0
+//     SWITCH (head == 0): one iteration with direction slot 0, with or without
+//                     the network
 //     ...
-//     IF (head == m): one iteration with direction slot m
+//     SWITCH (head == m): one iteration with direction slot m
 //     the loop guard
 //
 // The m + 1 iteration blocks are the ring positions of the new direction, so
 // every kernel argument is fixed at capture.  Inside an iteration block:
-//   IF/ELSE (network on): z = M r (restriction, U-Net, omega, r - omega A P zc,
-//                         the smoother passes reducing (z, r), (z, q_0)) /
-//                         z = r with its dots; z stands in the direction slot
-//   IF (no descent direction, (z, r) <= 0): z = r with its dots; the third
-//                         time the network is switched off
-//   p = z - sum_j (z, q_j) / (p_j, q_j) p_j, q = A p, (p, q), (p, r), alpha,
-//   e += alpha p, r -= alpha q, (r, r), the cycle-end test.
+//   network on: z = M r (restriction, U-Net, omega, r - omega A P zc, the
+//       smoother passes, the last with (z, r), (z, q_0) and the descent test),
+//       the other window dots; IF (no descent direction, (z, r) <= 0): z = r
+//       with its dots; the third time the network is switched off;
+//   network off: z = r with its dots;
+//   p = z - sum_j (z, q_j) / (p_j, q_j) p_j, the last term with q = A p, (p, q)
+//   and alpha in one pass; e += alpha p, r -= alpha q, (r, r), the cycle-end
+//   test.
 // The loop guard ends the loop when the solve is done, and with an error
 // status if a pass made no iteration (the control always runs one per pass
 // until it ends the solve) or the passes exceed the iteration cap, so the
 // device loop ends whatever the handles hold.  The graph, the workspace and
 // the state are built once per operator, vectors and settings, and kept with
 // the network.
-struct TlCtl {
-  double bb, thr, rr_true, rr_prev_true, rr, rr_start, alpha;
-  double pq_win[9];
-  float coef[8];
-  int use_coef[8];
-  int win_off[8];   // window dot j skipped (j >= nwin)
-  int it, it_start, maxit, every, repl, prev_cycle, fallbacks, precond_on, head, nwin, done, status, brk, cycle_ran;
-  int passes, it_seen;   // the loop guard
-  long long launches;
-};
-struct TlParams {
-  double rtol2;
-  int maxit, every;
-  // kernels per segment, for the launch count
-  int n_init, n_ref, n_iter, n_on, n_off, n_fb;
-};
-struct TlHandles {
-  cudaGraphConditionalHandle main, ref, blk[9], pre[9], fb[9];
-};
-
 struct TlGraph {
   unsigned long long op_serial = 0;
   const void *x = nullptr, *b = nullptr;
@@ -1110,8 +1093,9 @@ void xf_tl_graph_free(TlGraph* t) { delete t; }
 __global__ void k_tl_init(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles h, int m) {
   if (threadIdx.x | blockIdx.x) return;
   cudaGraphSetConditional(h.ref, 1u);   // the loop starts with a refresh
-  for (int k = 0; k <= m; k++) cudaGraphSetConditional(h.blk[k], 0u);
-  c->passes = 0; c->it_seen = 0;
+  for (int k = 0; k <= m; k++) cudaGraphSetConditional(h.blk[k], TL_SKIP);
+  S->iscalars[I_PBUF] = 0;   // the direction pass takes its buffers as given
+  c->passes = 0; c->steps = 0; c->steps_seen = 0;
   c->bb = S->scalars[FS_RR];
   c->thr = p->rtol2 * c->bb;
   c->maxit = p->maxit; c->every = p->every;
@@ -1132,6 +1116,7 @@ __global__ void k_tl_fold(double* __restrict__ x, const float* __restrict__ e, i
 __global__ void k_tl_top(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles h, int m) {
   if (threadIdx.x | blockIdx.x) return;
   c->cycle_ran = 0;
+  c->steps++;
   c->launches += p->n_ref;
   const double rr = S->scalars[FS_PQ + 1];
   c->rr_true = rr;
@@ -1156,76 +1141,13 @@ __global__ void k_tl_top(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles h
   }
   cudaGraphSetConditional(h.main, c->done ? 0u : 1u);
   cudaGraphSetConditional(h.ref, 0u);
-  for (int k = 0; k <= m; k++) cudaGraphSetConditional(h.blk[k], (!c->done && k == c->head) ? 1u : 0u);
+  for (int k = 0; k <= m; k++) cudaGraphSetConditional(h.blk[k], TL_SKIP);
+  if (!c->done) tl_next(c, p, h, c->head, m);
 }
-__global__ void k_tl_it(TlCtl* c, const TlParams* p, cudaGraphConditionalHandle pre, int m) {
+// the window coefficients of the block with direction slot hd
+__global__ void k_tl_coef(DevScratch* S, TlCtl* c, int hd, int m) {
   if (threadIdx.x | blockIdx.x) return;
-  c->it++;
-  for (int j = 0; j < m; j++) c->win_off[j] = j >= c->nwin;
-  c->launches += p->n_iter + (c->precond_on ? p->n_on : p->n_off);
-  cudaGraphSetConditional(pre, c->precond_on ? 1u : 0u);
-}
-__global__ void k_tl_z(DevScratch* S, TlCtl* c, const TlParams* p, cudaGraphConditionalHandle fb) {
-  if (threadIdx.x | blockIdx.x) return;
-  const bool bad = !(S->scalars[FS_ZR] > 0) && c->precond_on;   // no descent direction: use r this time
-  if (bad) {
-    if (++c->fallbacks >= FCG_STRIKES) c->precond_on = 0;   // and from the third on, for good
-    c->launches += p->n_fb;
-  }
-  cudaGraphSetConditional(fb, bad ? 1u : 0u);
-}
-// the window coefficients -(z, q_j) / (p_j, q_j) of the block with direction slot hd
-// The window's last term of the new direction with (p, r): p += coef_j p_j
-// (when the control kept term j) and (p, r) into scalars[slot] in one pass;
-// k_dot_f4's grid, mapping and order, so (p, r) is bit for bit the separate dot's.
-__global__ void __launch_bounds__(RED_THREADS) k_tl_axpy_pr(float* __restrict__ y, const float* __restrict__ x,
-                                                            const float* __restrict__ r, const TlCtl* c, int j,
-                                                            int64_t n, DevScratch* S, int slot) {
-  __shared__ double sh[32];
-  __shared__ bool last;
-  const bool use = c->use_coef[j] != 0;
-  const float a = c->coef[j];
-  DotAcc<float> acc;
-  const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * blockDim.x;
-  float4* y4 = reinterpret_cast<float4*>(y);
-  const float4* x4 = reinterpret_cast<const float4*>(x);
-  const float4* r4 = reinterpret_cast<const float4*>(r);
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n4; k += stride) {
-    float4 v = y4[k];
-    if (use) {
-      const float4 xv = __ldg(x4 + k);
-      v.x = fmaf(a, xv.x, v.x); v.y = fmaf(a, xv.y, v.y); v.z = fmaf(a, xv.z, v.z); v.w = fmaf(a, xv.w, v.w);
-      y4[k] = v;
-    }
-    const float4 rv = __ldg(r4 + k);
-    acc.add(v.x, rv.x);
-    acc.add(v.y, rv.y);
-    acc.add(v.z, rv.z);
-    acc.add(v.w, rv.w);
-  }
-  for (int64_t k = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += stride) {
-    float v = y[k];
-    if (use) {
-      v = fmaf(a, x[k], v);
-      y[k] = v;
-    }
-    acc.add(v, r[k]);
-  }
-  if (!publish_acc<float>(S, slot, slot, acc, sh, &last)) return;
-  const double t = finish_partials(S, slot, sh);
-  if (threadIdx.x == 0) {
-    S->scalars[slot] = t;
-    S->tickets[slot] = 0;
-  }
-}
-__global__ void k_tl_coef(const DevScratch* S, TlCtl* c, int hd, int m) {
-  if (threadIdx.x | blockIdx.x) return;
-  for (int j = 0; j < m; j++) {
-    const int sl = (hd + m - j) % (m + 1);
-    const bool use = j < c->nwin && c->pq_win[sl] > 0;
-    c->use_coef[j] = use;
-    c->coef[j] = use ? (float)(-S->scalars[j] / c->pq_win[sl]) : 0.f;
-  }
+  tl_coef(S, c, hd, m);
 }
 __global__ void k_tl_axpy(float* __restrict__ y, const float* __restrict__ x, const TlCtl* c, int j, int64_t n) {
   if (!c->use_coef[j]) return;
@@ -1233,29 +1155,19 @@ __global__ void k_tl_axpy(float* __restrict__ y, const float* __restrict__ x, co
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     y[q] = fmaf(a, x[q], y[q]);
 }
-__global__ void k_tl_alpha(const DevScratch* S, TlCtl* c, int hd, int m) {
-  if (threadIdx.x | blockIdx.x) return;
-  const double pr = S->scalars[FS_PR], pq = S->scalars[FS_PQ];
-  if (!(pq > 0)) {
-    c->status = isnan(pq) ? XF_NAN : XF_BREAKDOWN;
-    c->brk = 1;
-    return;
-  }
-  c->alpha = pr / pq;
-  c->pq_win[hd] = pq;
-  c->head = (hd + 1) % (m + 1);
-  if (c->nwin < m) c->nwin++;
-}
-// e += alpha p, r -= alpha q and (r, r) into scalars[slot] in the same pass;
+// e += alpha p, r -= alpha q, (r, r) into scalars[slot] and the cycle-end test in the same pass;
 // the grid, the thread mapping and the accumulation order are k_dot_f4's, so
 // (r, r) is bit for bit the separate dot's.
 __global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e, float* __restrict__ r,
                                                            const float* __restrict__ p, const float* __restrict__ q,
-                                                           const TlCtl* c, int64_t n, DevScratch* S, int slot) {
+                                                           TlStep step, int64_t n, DevScratch* S, int slot) {
   __shared__ double sh[32];
   __shared__ bool last;
-  if (c->brk) return;
-  const float alpha = (float)c->alpha;
+  if (step.ctl->brk) {   // set by the pass before: every block sees it
+    if ((threadIdx.x | blockIdx.x) == 0) tl_rr(S, step);
+    return;
+  }
+  const float alpha = (float)step.ctl->alpha;
   DotAcc<float> acc;
   const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * blockDim.x;
   float4* e4 = reinterpret_cast<float4*>(e);
@@ -1287,38 +1199,19 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e
   if (threadIdx.x == 0) {
     S->scalars[slot] = t;
     S->tickets[slot] = 0;
+    tl_rr(S, step);
   }
 }
 // The last node of the loop body: see the loop guard above.
 __global__ void k_tl_guard(TlCtl* c, TlHandles h) {
   if (threadIdx.x | blockIdx.x) return;
   c->passes++;
-  if (!c->done && (c->it == c->it_seen || c->passes > c->maxit + 16)) {
+  if (!c->done && (c->steps == c->steps_seen || c->passes > c->maxit + 16)) {
     c->done = 1;
     c->status = XF_ERR_CUDA;
   }
-  c->it_seen = c->it;
+  c->steps_seen = c->steps;
   cudaGraphSetConditional(h.main, c->done ? 0u : 1u);
-}
-// the cycle-end test after the iteration in block hd; sets the next block
-__global__ void k_tl_rr(const DevScratch* S, TlCtl* c, TlHandles h, int hd, int m) {
-  if (threadIdx.x | blockIdx.x) return;
-  bool end = c->brk != 0;
-  if (!end) {
-    const double rr = S->scalars[FS_RR];
-    c->rr = rr;
-    end = isnan(rr) || rr <= c->thr || rr <= 1e-6 * c->rr_start || c->it - c->it_start >= c->every ||
-          c->it >= c->maxit;
-  }
-  if (end) {
-    c->cycle_ran = 1;
-    c->repl++;
-    c->prev_cycle = c->it - c->it_start;
-    cudaGraphSetConditional(h.ref, 1u);
-    for (int k = hd + 1; k <= m; k++) cudaGraphSetConditional(h.blk[k], 0u);
-  } else {
-    cudaGraphSetConditional(h.blk[hd < m ? hd + 1 : 0], 1u);
-  }
 }
 
 static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_f)[3], int tl_nf, double tl_scale,
@@ -1365,9 +1258,10 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
   auto fdot = [&](const float* a, const float* b2, int slot, const int* skip) {
     k_dot_f4<<<db, RED_THREADS, 0, s>>>(a, b2, n, S, slot, skip);
   };
+  float* z = tl_nf % 2 ? w0 : w1;   // where the smoother's last pass writes
   // the window dots j = j0 .. m-1 of block hd (skipped on the device while j >= nwin)
   auto win_dots = [&](int hd, int j0) {
-    for (int j = j0; j < m; j++) fdot(P[hd], Q[(hd + m - j) % (m + 1)], j, &c->win_off[j]);
+    for (int j = j0; j < m; j++) fdot(z, Q[(hd + m - j) % (m + 1)], j, &c->win_off[j]);
   };
   // warm the network's kernels (attributes, first launches) outside capture
   int rcode = f4 ? forward(u, rc) : xf_unet_apply_dev(u, rc, zc);
@@ -1446,24 +1340,29 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
   // iteration blocks
   int n_on = 0, n_off = 0, n_fb = 0, n_iter = 0;
   for (int hd = 0; hd <= m; hd++) {
-    cudaGraph_t bbody = nullptr;
+    cudaGraph_t body[2] = {nullptr, nullptr};   // TL_ON, TL_OFF
     cudaGraphNode_t bnode = nullptr;
-    add_cond(wbody, {prev}, H.blk[hd], cudaGraphCondTypeIf, 1, &bbody, &bnode);
+    add_cond(wbody, {prev}, H.blk[hd], cudaGraphCondTypeSwitch, 2, body, &bnode);
     prev = bnode;
-    handle(bbody, &H.pre[hd], 0, 0);
-    handle(bbody, &H.fb[hd], 0, 0);
-    float* pn = P[hd];
+    handle(body[TL_ON], &H.fb[hd], 0, 0);
+    const TlStep step = {c, prm, H, hd, m};
     float* qn = Q[hd];
     const float* q_newest = Q[(hd + m) % (m + 1)];
-    // it++, the network-on test
-    begin(bbody, nullptr, 0);
-    k_tl_it<<<1, 32, 0, s>>>(c, prm, H.pre[hd], m);
-    end_tail(tail);
-    cudaGraph_t ie[2] = {nullptr, nullptr};
-    cudaGraphNode_t ienode = nullptr;
-    add_cond(bbody, tail, H.pre[hd], cudaGraphCondTypeIf, 2, ie, &ienode);
+    // z = r with its dots and coefficients
+    auto z_is_r = [&]() {
+      cudaMemcpyAsync(z, r, n * 4, cudaMemcpyDeviceToDevice, s);
+      fdot(r, r, FS_ZR, nullptr);
+      win_dots(hd, 0);
+      k_tl_coef<<<1, 32, 0, s>>>(S, c, hd, m);
+    };
+    // the new direction (its last term and image in one pass), alpha, the update, the cycle-end test
+    auto advance = [&]() {
+      for (int j = 0; j < m - 1; j++) k_tl_axpy<<<eb, 256, 0, s>>>(z, P[(hd + m - j) % (m + 1)], c, j, n);
+      xf_cg_pqb_tl_launch(op, z, P[(hd + 1) % (m + 1)], P[hd], qn, FS_PQ, step);
+      k_tl_update<<<db, RED_THREADS, 0, s>>>(e, r, P[hd], qn, step, n, S, FS_RR);
+    };
     // network on: z = M r with (z, r) and (z, q_newest)
-    begin(ie[0], nullptr, 0);
+    begin(body[TL_ON], nullptr, 0);
     if (f4)
       k_restrict4<<<dim3((cg->n3 + 63) / 64, cg->n2, cg->n1), 64, 0, s>>>(r, g->n2, g->n3, rc, cg->n1, cg->n2, cg->n3);
     else
@@ -1487,46 +1386,33 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
         xf_cg_poly_first_launch(op, src, dst, tl_f[k], nullptr, nullptr, nullptr, nullptr, nullptr);
         std::swap(src, dst);
       }
-      xf_cg_poly_last_tl_launch(op, src, pn, tl_f[0], FS_OM, u->zout, cg->n3, cg->n2 * cg->n3, F, (float)tl_scale, r,
-                                q_newest, FS_ZR, 0);
+      // also the descent test and, with one direction, its coefficient
+      xf_cg_poly_last_tl_launch(op, src, dst, tl_f[0], FS_OM, u->zout, cg->n3, cg->n2 * cg->n3, F, (float)tl_scale, r,
+                                q_newest, FS_ZR, 0, step);
     }
     win_dots(hd, 1);
-    end_tail(unused);
-    // F = 4: no output conversion of the network
-    n_on = (f4 ? 3 - 1 : 5) + UNET_FORWARD_LAUNCHES + tl_nf + (m - 1);
-    // network off: z = r with its dots
-    begin(ie[1], nullptr, 0);
-    cudaMemcpyAsync(pn, r, n * 4, cudaMemcpyDeviceToDevice, s);
-    fdot(pn, r, FS_ZR, nullptr);
-    win_dots(hd, 0);
-    end_tail(unused);
-    n_off = 1 + m;
-    // the descent test
-    begin(bbody, &ienode, 1);
-    k_tl_z<<<1, 32, 0, s>>>(S, c, prm, H.fb[hd]);
+    if (m > 1) k_tl_coef<<<1, 32, 0, s>>>(S, c, hd, m);
     end_tail(tail);
+    // F = 4: no output conversion of the network
+    n_on = (f4 ? 3 - 1 : 5) + UNET_FORWARD_LAUNCHES + tl_nf + (m > 1 ? m : 0);
     cudaGraph_t fbody = nullptr;
     cudaGraphNode_t fnode = nullptr;
-    add_cond(bbody, tail, H.fb[hd], cudaGraphCondTypeIf, 1, &fbody, &fnode);
+    add_cond(body[TL_ON], tail, H.fb[hd], cudaGraphCondTypeIf, 1, &fbody, &fnode);
     begin(fbody, nullptr, 0);
-    cudaMemcpyAsync(pn, r, n * 4, cudaMemcpyDeviceToDevice, s);
-    fdot(pn, r, FS_ZR, nullptr);
-    win_dots(hd, 0);
+    z_is_r();
     end_tail(unused);
-    n_fb = 1 + m;
-    // the new direction, its image, alpha, the update, the cycle-end test
-    begin(bbody, &fnode, 1);
-    k_tl_coef<<<1, 32, 0, s>>>(S, c, hd, m);
-    for (int j = 0; j < m - 1; j++) k_tl_axpy<<<eb, 256, 0, s>>>(pn, P[(hd + m - j) % (m + 1)], c, j, n);
-    k_tl_axpy_pr<<<db, RED_THREADS, 0, s>>>(pn, P[(hd + 1) % (m + 1)], r, c, m - 1, n, S, FS_PR);   // with (p, r)
-    xf_cg_q32_dot(op, pn, qn, FS_PQ);   // q = A p, (p, q)
-    k_tl_alpha<<<1, 32, 0, s>>>(S, c, hd, m);
-    k_tl_update<<<db, RED_THREADS, 0, s>>>(e, r, pn, qn, c, n, S, FS_RR);   // with (r, r)
-    k_tl_rr<<<1, 32, 0, s>>>(S, c, H, hd, m);
+    n_fb = 2 + m;
+    begin(body[TL_ON], &fnode, 1);
+    advance();
     end_tail(unused);
-    // it, z-test, coef, m axpys (the last with (p, r)), stencil + dot, alpha, update with (r, r), test, and
-    // the loop guard
-    n_iter = 3 + m + 1 + 1 + 1 + 1 + 1;
+    // network off
+    begin(body[TL_OFF], nullptr, 0);
+    z_is_r();
+    advance();
+    end_tail(unused);
+    n_off = 2 + m;
+    // m - 1 axpys, the direction pass, the update, the loop guard
+    n_iter = (m - 1) + 2 + 1;
   }
   // the loop guard, last in the body
   begin(wbody, &prev, 1);
