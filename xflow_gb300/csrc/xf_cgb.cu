@@ -14,8 +14,8 @@
 // Per plane i the block turns the raw plane i+1, as soon as it has landed,
 // into p'(i+1) over the whole region in a three-plane p' ring (and writes the
 // own cells' p' to global memory), releases the raw slot, synchronises once,
-// and computes q for its own cells of plane i: i+-1 and j+-1 from the p'
-// ring (i-1 from registers), k+-1 from the neighbouring lanes.  Each thread owns two groups of
+// and computes q for its own cells of plane i: the neighbours from the p'
+// ring (i-1 from registers).  Each thread owns two groups of
 // four cells, at 4 t and at PQB_TILE / 2 + 4 t, so that consecutive lanes
 // touch consecutive 16-byte words of shared memory.  The dot (p', q) keeps
 // each product's rounding error (an FMA) and sums a thread's products and
@@ -80,7 +80,6 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
   const int n1 = a.n1, n3 = a.n3, P = a.P, HA = a.HA, RL = a.RL;
   const int64_t total = (int64_t)n1 * P;
   const int items = a.nchunk * a.tiles;
-  const int lane = threadIdx.x & 31;
   if (threadIdx.x < 64) {
     const int b = threadIdx.x;
     dtab[b] = a.cx * (float)(((b >> 0) & 1) + ((b >> 1) & 1)) + a.cy * (float)(((b >> 2) & 1) + ((b >> 3) & 1)) +
@@ -160,10 +159,10 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
     const int xa = base + 4 * threadIdx.x, xb = xa + PQB_HALF;   // this thread's two groups
     const bool va = xa < P, vb = xb < P;                         // P % 4 == 0: whole groups
     const int sa = HA + 4 * threadIdx.x, sb = sa + PQB_HALF;     // their region index
-    uchar4 ka = make_uchar4(0, 0, 0, 0), kb = ka;   // row kinds of the first plane computed
+    uint32_t ka = 0, kb = 0;   // row kinds of the first plane computed
     const int kfirst = dir > 0 ? i0 : i1 - 1;
-    if (va) ka = *reinterpret_cast<const uchar4*>(a.kind + (int64_t)kfirst * P + xa);
-    if (vb) kb = *reinterpret_cast<const uchar4*>(a.kind + (int64_t)kfirst * P + xb);
+    if (va) ka = *reinterpret_cast<const uint32_t*>(a.kind + (int64_t)kfirst * P + xa);
+    if (vb) kb = *reinterpret_cast<const uint32_t*>(a.kind + (int64_t)kfirst * P + xb);
     bool wok = true;
     // own p'(i-1) in registers: the ring slot of plane i-1 is rewritten during
     // step i+1, possibly while a slower warp is still in step i
@@ -198,10 +197,10 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
         }
       }
       // next plane's row kinds, in flight during this plane
-      uchar4 kna = ka, knb = kb;
+      uint32_t kna = ka, knb = kb;
       if (i >= i0 && i < i1 && j >= i0 && j < i1) {
-        if (va) kna = *reinterpret_cast<const uchar4*>(a.kind + (int64_t)j * P + xa);
-        if (vb) knb = *reinterpret_cast<const uchar4*>(a.kind + (int64_t)j * P + xb);
+        if (va) kna = *reinterpret_cast<const uint32_t*>(a.kind + (int64_t)j * P + xa);
+        if (vb) knb = *reinterpret_cast<const uint32_t*>(a.kind + (int64_t)j * P + xb);
       }
       if (__syncthreads_or(!wok)) { ok = false; break; }
       if (load) release();   // plane j's slot is consumed
@@ -214,43 +213,23 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
         const float* pc = pring + (size_t)((i + PQB_NP) % PQB_NP) * RL;
         const float* pp = pring + (size_t)((j + PQB_NP) % PQB_NP) * RL;
         const float4 xca = lds4(pc + sa), xcb = lds4(pc + sb);
-        // k-1 / k+1 of the group ends from the neighbouring lanes (lane 0 / 31 from shared memory)
-        const float la = __shfl_up_sync(0xffffffffu, xca.w, 1), lb = __shfl_up_sync(0xffffffffu, xcb.w, 1);
-        const float ra = __shfl_down_sync(0xffffffffu, xca.x, 1), rb = __shfl_down_sync(0xffffffffu, xcb.x, 1);
         const int64_t pl = (int64_t)i * P;
         float psum = 0.f, esum = 0.f;   // this thread's (p', q) over the plane: FP32 sum + exact-product errors
-        auto group = [&](bool v, int s0, float4 xc, float4 xm, uchar4 k4, float left, float right, int x) {
+        auto group = [&](bool v, int s0, float4 xc, float4 xm, uint32_t k4, int x) {
           if (!v) return;
-          const float4 xp = lds4(pp + s0);
-          const float km0 = lane == 0 ? pc[s0 - 1] : left;
-          const float kp3 = lane == 31 ? pc[s0 + 4] : right;
-          const float2 jm01 = *reinterpret_cast<const float2*>(pc + s0 - n3);
-          const float2 jm23 = *reinterpret_cast<const float2*>(pc + s0 - n3 + 2);
-          const float2 jp01 = *reinterpret_cast<const float2*>(pc + s0 + n3);
-          const float2 jp23 = *reinterpret_cast<const float2*>(pc + s0 + n3 + 2);
-          const float c[4] = {xc.x, xc.y, xc.z, xc.w};
-          const float m[4] = {xm.x, xm.y, xm.z, xm.w};
-          const float pq[4] = {xp.x, xp.y, xp.z, xp.w};
-          const float jm[4] = {jm01.x, jm01.y, jm23.x, jm23.y};
-          const float jp[4] = {jp01.x, jp01.y, jp23.x, jp23.y};
-          const float km[4] = {km0, c[0], c[1], c[2]};
-          const float kp[4] = {c[1], c[2], c[3], kp3};
-          const uint8_t kk[4] = {k4.x, k4.y, k4.z, k4.w};
           float out[4];
+          lap4w(dtab, k4, xc, xm, lds4(pp + s0), pc + s0, n3, a.cx, a.cy, a.cz, out);
+          const float c[4] = {xc.x, xc.y, xc.z, xc.w};
 #pragma unroll
           for (int v2 = 0; v2 < 4; v2++) {
-            float o = fmaf(dtab[kk[v2] & 63], c[v2],
-                           -fmaf(a.cx, pq[v2] + m[v2], fmaf(a.cy, jp[v2] + jm[v2], a.cz * (kp[v2] + km[v2]))));
-            if ((kk[v2] >> K_ROW_SHIFT) == ROW_NONE) o = 0.f;
-            out[v2] = o;
-            const float pr = c[v2] * o;
-            esum += fmaf(c[v2], o, -pr);
+            const float pr = c[v2] * out[v2];
+            esum += fmaf(c[v2], out[v2], -pr);
             psum += pr;
           }
           *reinterpret_cast<float4*>(a.q + pl + x) = make_float4(out[0], out[1], out[2], out[3]);
         };
-        group(va, sa, xca, xma, ka, la, ra, xa);
-        group(vb, sb, xcb, xmb, kb, lb, rb, xb);
+        group(va, sa, xca, xma, ka, xa);
+        group(vb, sb, xcb, xmb, kb, xb);
         acc.add(psum, 1.f);
         acc.add(esum, 1.f);
         xma = xca;

@@ -13,19 +13,19 @@
 // CP_TILE consecutive cells of the flattened (j, k) plane and marches a chunk
 // of i-planes.  The raw r of each plane (tile plus a halo of 2 HA cells,
 // HA >= n3 + 1, on either side) arrives by bulk asynchronous copy
-// (cp.async.bulk) into a CP_NS-deep ring; at step t the block
-//   - computes level 1 for plane t-1 over the tile plus one halo (y1 into a
-//     four-plane ring),
-//   - computes level 2 for plane t-3 on its own cells (z to global memory,
-//     the (r, z) partial),
-//   - waits for raw plane t+1 (its row kinds over the level-1 region come
-//     with it, by a second bulk copy on the same barrier),
-// and synchronises once.  The stencil is the fast Laplace row of the CG
+// (cp.async.bulk) into a ring, with its row kinds over the level-1 region by a
+// second copy on the same barrier; a step of the block computes level 1 for one
+// plane over the tile plus one halo (y1 into a ring of planes), level 2 for an
+// earlier plane on its own cells (z to global memory, the (r, z) partial),
+// waits for the next raw plane and synchronises once.  The stencil is the fast Laplace row of the CG
 // kernels (open-face diagonal, uniform coefficients); rows without an
 // equation give 0, so inactive cells keep z = 0.  Halo cells outside the box
 // hold stale values that only rows without an equation read.
 //
-// The fused form (FUSE) also carries the previous iteration's update: when
+// Two kernels: k_cg_polym, and k_cg_poly2 for the fused form (whose update
+// needs the registers that k_cg_polym marches in).
+//
+// The fused form also carries the previous iteration's update: when
 // raw plane t+1 lands, the block applies r -= alpha q to it in shared memory
 // (q of the same region arrives by bulk copy into a one-plane buffer),
 // writes the updated residual of its own cells to the other residual buffer,
@@ -90,35 +90,6 @@ struct CpArgs {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// Fast Laplace row (uniform grid) of four consecutive cells whose centres are
-// c[0..3]: i-neighbours m, p; j-neighbours at -+n3 from s (shared memory,
-// 8-byte aligned); k-neighbours from the neighbouring lanes' groups (the
-// caller's consecutive lanes hold consecutive groups), s[-1] / s[4] at the
-// warp's ends.
-__device__ __forceinline__ void lap4(const float* dtab, uchar4 k4, float4 c, float4 m, float4 p, const float* s, int n3,
-                                     float cx, float cy, float cz, float out[4], bool last_group = false) {
-  const int lane = threadIdx.x & 31;
-  float left = __shfl_up_sync(0xffffffffu, c.w, 1), right = __shfl_down_sync(0xffffffffu, c.x, 1);
-  if (lane == 0) left = s[-1];
-  if (lane == 31 || last_group) right = s[4];   // the next lane holds no following group
-  const float2 jm01 = *reinterpret_cast<const float2*>(s - n3), jm23 = *reinterpret_cast<const float2*>(s - n3 + 2);
-  const float2 jp01 = *reinterpret_cast<const float2*>(s + n3), jp23 = *reinterpret_cast<const float2*>(s + n3 + 2);
-  const float cc[4] = {c.x, c.y, c.z, c.w};
-  const float mm[4] = {m.x, m.y, m.z, m.w};
-  const float pp[4] = {p.x, p.y, p.z, p.w};
-  const float jm[4] = {jm01.x, jm01.y, jm23.x, jm23.y};
-  const float jp[4] = {jp01.x, jp01.y, jp23.x, jp23.y};
-  const float km[4] = {left, cc[0], cc[1], cc[2]};
-  const float kp[4] = {cc[1], cc[2], cc[3], right};
-  const uint8_t kk[4] = {k4.x, k4.y, k4.z, k4.w};
-#pragma unroll
-  for (int v = 0; v < 4; v++) {
-    float o = fmaf(dtab[kk[v] & 63], cc[v], -fmaf(cx, pp[v] + mm[v], fmaf(cy, jp[v] + jm[v], cz * (kp[v] + km[v]))));
-    if ((kk[v] >> K_ROW_SHIFT) == ROW_NONE) o = 0.f;
-    out[v] = o;
-  }
-}
-
 // Launch modes.  A degree-2 preconditioner is one pass (CP_POLY, or
 // CP_POLY_FUSED carrying the residual update); a degree-4 one is the product
 // of two quadratic factors, z = p1(A) p2(A) r, in two passes: w = p2(A) r
@@ -128,12 +99,9 @@ __device__ __forceinline__ void lap4(const float* dtab, uchar4 k4, float4 c, flo
 // file).
 enum { CP_POLY = 0, CP_POLY_FUSED = 1, CP_FIRST = 2, CP_FIRST_FUSED = 3, CP_SECOND = 4, CP_TL_LAST = 5 };
 
-template <int MODE>
+template <int MODE>   // CP_POLY_FUSED, CP_FIRST_FUSED
 __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constant__ CpArgs a) {
-  constexpr bool FUSE = MODE == CP_POLY_FUSED || MODE == CP_FIRST_FUSED;
-  constexpr bool OUT_TL = MODE == CP_TL_LAST;    // output omega y + s w, two dots
-  constexpr bool DOTZ = MODE == CP_POLY || MODE == CP_POLY_FUSED || MODE == CP_SECOND || OUT_TL;   // (r, z)
-  constexpr bool DOTSEP = MODE == CP_SECOND || OUT_TL;   // r of the dot is not the input
+  constexpr bool DOTZ = MODE == CP_POLY_FUSED;   // (r, z)
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ double sh[32];
   __shared__ bool last;
@@ -145,28 +113,21 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
   uint64_t* qbar = mbar + CP_NS;
   float* ring = reinterpret_cast<float*>(smem + 128);          // CP_NS x R0 raw r
   float* yring = ring + (size_t)CP_NS * R0;                     // CP_NY x R1 level-1 planes
-  float* qbuf = yring + (size_t)CP_NY * R1;                     // FUSE: R0 cells of q
-  uint8_t* kring = reinterpret_cast<uint8_t*>(qbuf + (FUSE ? (size_t)R0 : 0));   // CP_NS x KS row kinds
+  float* qbuf = yring + (size_t)CP_NY * R1;                     // R0 cells of q
+  uint8_t* kring = reinterpret_cast<uint8_t*>(qbuf + R0);   // CP_NS x KS row kinds
   const int KS = a.KS;
   const int64_t total = (int64_t)n1 * P;
   const int64_t total16 = (total + 15) & ~(int64_t)15;   // the kind array holds zero bytes up to here
   const int items = a.nchunk * a.tiles;
-  float alpha = 0.f;   // FUSE: the update's step
-  const float* pdir = a.pa;
-  if (FUSE) {
-    alpha = (float)S->scalars[D_ALPHA];
-    if (S->iscalars[I_PBUF]) pdir = a.pb;
-  }
-  float om = 0.f;
-  if (OUT_TL) om = (float)S->scalars[a.s_om];
-  const float* r2src = FUSE ? a.rout : a.r;   // own-cell residual of level 2
+  const float alpha = (float)S->scalars[D_ALPHA];   // the update's step
+  const float* pdir = S->iscalars[I_PBUF] ? a.pb : a.pa;
   if (threadIdx.x < 64) {
     const int b = threadIdx.x;
     dtab[b] = a.cx * (float)(((b >> 0) & 1) + ((b >> 1) & 1)) + a.cy * (float)(((b >> 2) & 1) + ((b >> 3) & 1)) +
               a.cz * (float)(((b >> 4) & 1) + ((b >> 5) & 1));
   }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < CP_NS + (FUSE ? 1 : 0); s++) mbar_init(&mbar[s], 1);
+    for (int s = 0; s < CP_NS + 1; s++) mbar_init(&mbar[s], 1);
     fence_barrier_init();
   }
   __syncthreads();
@@ -231,7 +192,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
       }
     }
   };
-  // FUSE: q of one raw plane into the one-plane buffer (thread 0; the previous
+  // q of one raw plane into the one-plane buffer (thread 0; the previous
   // reader of the buffer has passed a block barrier)
   long long q_issued = 0, q_waited = 0;
   auto issue_q = [&](int plane, int base) {
@@ -261,54 +222,17 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
     const int xa = base + 4 * threadIdx.x, xb = xa + CP_TILE / 2;
     const bool va = xa < P, vb = xb < P;
     const int ya = HA + 4 * threadIdx.x, yb = ya + CP_TILE / 2;   // their index in the level-1 region
-    // level-2 inputs of the next plane, prefetched one step ahead (FUSE: the
-    // updated residual this thread wrote three steps earlier, read through L2)
-    float4 rpa = make_float4(0.f, 0.f, 0.f, 0.f), rpb = rpa, dpa = rpa, dpb = rpa;
-    float4 ypa = rpa, ypb = rpa, wpa = rpa, wpb = rpa;   // OUT_TL: y, q_w
-    uchar4 kpa = make_uchar4(0, 0, 0, 0), kpb = kpa;
-    int ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};   // OUT_TL: the cells' blocks in a coarse plane
-    if (OUT_TL) {
-      auto blocks = [&](int x, int (&o)[4]) {
-        int j = x / n3, k = x - j * n3;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          o[q] = (1 + (j - 1) / a.F) * a.c3 + 1 + (k - 1) / a.F;   // ghost cells: some block, not used
-          if (++k == n3) {
-            k = 0;
-            j++;
-          }
-        }
-      };
-      if (va) blocks(xa, ca);
-      if (vb) blocks(xb, cb);
-    }
+    // level-2 inputs of the next plane, prefetched one step ahead (the updated
+    // residual this thread wrote three steps earlier, read through L2)
+    float4 rpa = make_float4(0.f, 0.f, 0.f, 0.f), rpb = rpa;
+    uint32_t kpa = 0, kpb = 0;   // row kinds of four cells
     auto prefetch2 = [&](int pl) {
       if (pl < i0 || pl >= i1) return;
       const int64_t o = (int64_t)pl * P;
-      if (DOTSEP) {
-        if (va) dpa = __ldg(reinterpret_cast<const float4*>(a.dr + o + xa));
-        if (vb) dpb = __ldg(reinterpret_cast<const float4*>(a.dr + o + xb));
-      }
-      if (OUT_TL) {
-        const float* zp = a.zc + (int64_t)(1 + (pl - 1) / a.F) * a.cs1;
-        if (va) {
-          ypa = make_float4(__ldg(zp + ca[0]), __ldg(zp + ca[1]), __ldg(zp + ca[2]), __ldg(zp + ca[3]));
-          if (a.qw) wpa = __ldg(reinterpret_cast<const float4*>(a.qw + o + xa));
-        }
-        if (vb) {
-          ypb = make_float4(__ldg(zp + cb[0]), __ldg(zp + cb[1]), __ldg(zp + cb[2]), __ldg(zp + cb[3]));
-          if (a.qw) wpb = __ldg(reinterpret_cast<const float4*>(a.qw + o + xb));
-        }
-      }
-      if (FUSE) {
-        if (va) rpa = __ldcg(reinterpret_cast<const float4*>(r2src + o + xa));
-        if (vb) rpb = __ldcg(reinterpret_cast<const float4*>(r2src + o + xb));
-      } else {
-        if (va) rpa = __ldg(reinterpret_cast<const float4*>(r2src + o + xa));
-        if (vb) rpb = __ldg(reinterpret_cast<const float4*>(r2src + o + xb));
-      }
-      if (va) kpa = *reinterpret_cast<const uchar4*>(a.kind + o + xa);
-      if (vb) kpb = *reinterpret_cast<const uchar4*>(a.kind + o + xb);
+      if (va) rpa = __ldcg(reinterpret_cast<const float4*>(a.rout + o + xa));
+      if (vb) rpb = __ldcg(reinterpret_cast<const float4*>(a.rout + o + xb));
+      if (va) kpa = *reinterpret_cast<const uint32_t*>(a.kind + o + xa);
+      if (vb) kpb = *reinterpret_cast<const uint32_t*>(a.kind + o + xb);
     };
     // row kinds of a loaded plane over its level-1 region (stale outside the
     // box, where only rows without an equation read the level-1 values)
@@ -316,18 +240,18 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
       const int64_t x0 = (int64_t)pl * P + base - HA;
       return kring + (size_t)((item_first + (pl - lo)) % CP_NS) * KS + (int)(x0 & 15);
     };
-    // raw plane pl has landed (and, FUSE, its q)
+    // raw plane pl has landed, and its q
     auto wait_plane = [&](int pl) -> bool {
       const long long L = item_first + (pl - lo);
       bool w = mbar_wait_bounded(&mbar[L % CP_NS], (uint32_t)((L / CP_NS) & 1));
       if (w) waited = L + 1;
-      if (FUSE && w) {
+      if (w) {
         w = mbar_wait_bounded(qbar, (uint32_t)(q_waited & 1));
         if (w) q_waited++;
       }
       return w;
     };
-    // FUSE: e and p' of the own cells of the plane the step's update reaches,
+    // e and p' of the own cells of the plane the step's update reaches,
     // loaded at the top of the step so that their latency hides under the
     // stencil levels
     const int own_n = min(CP_TILE, P - base);   // own cells of the tile in a plane
@@ -344,7 +268,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
         }
       }
     };
-    // FUSE: r -= alpha q over the box cells of raw plane pl; own cells of own
+    // r -= alpha q over the box cells of raw plane pl; own cells of own
     // planes also go to rout with e += alpha p' and (r, r)
     auto update = [&](int pl) {
       float* R = rslot(pl);
@@ -371,7 +295,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
         const int s = 2 * HA + c;
         if (s >= s_hi) continue;
         const float4 rv = upd(s);
-        if (FUSE && own_plane && c < own_n) {
+        if (own_plane && c < own_n) {
           *reinterpret_cast<float4*>(rown + c) = rv;
           float4 ev = ep[h];
           const float4 pv = pp[h];
@@ -389,7 +313,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
           }
         }
       }
-      if (FUSE && own_plane) {
+      if (own_plane) {
         acc_rr.add(psum, 1.f);
         acc_rr.add(esum, 1.f);
       }
@@ -400,17 +324,17 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
     };
     long long rel_next = lo;   // next plane whose raw slot is released
     // the item's first raw plane
-    if (FUSE && threadIdx.x == 0) issue_q(lo, base);
-    if (FUSE) prefetch_e(lo);
+    if (threadIdx.x == 0) issue_q(lo, base);
+    prefetch_e(lo);
     bool wok = wait_plane(lo);
-    if (FUSE && wok) update(lo);
+    if (wok) update(lo);
     if (__syncthreads_or(!wok)) { ok = false; break; }
     for (int t = i0 - 2; t <= i1 + 2; t++) {
       const int pn = t + 1;   // the raw plane that lands during this step
       const bool has_next = pn > lo && pn <= hi;
-      if (FUSE && has_next) {
+      if (has_next) {
         if (threadIdx.x == 0) issue_q(pn, base);
-        if (FUSE) prefetch_e(pn);
+        prefetch_e(pn);
       }
       // (B) level 1 for plane t-1: y1 = a1 r + a2 (A r) over the level-1 region
       const int p1 = t - 1;
@@ -420,20 +344,15 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
         const float* Rp = rslot(p1 + 1);
         const uint8_t* kb = kslot(p1);
         float* Y = yslot(p1);
-        // warp-uniform trip count (the shuffles need every lane); groups past
-        // the region end compute on in-bounds cells and are not stored
-        for (int g0 = 0; g0 < R1 / 4; g0 += CP_THREADS) {
-          const int g = g0 + (int)threadIdx.x;
-          const int gg = g < R1 / 4 ? g : R1 / 4 - 1;
-          const int s = HA + 4 * gg;   // raw index of the group's first cell
+        for (int g = threadIdx.x; g < R1 / 4; g += CP_THREADS) {
+          const int s = HA + 4 * g;   // raw index of the group's first cell
           const float4 c = ld4(Rc + s);
           float ar[4];
-          lap4(dtab, *reinterpret_cast<const uchar4*>(kb + 4 * gg), c, ld4(Rm + s), ld4(Rp + s), Rc + s, n3, a.cx,
-               a.cy, a.cz, ar, g + 1 >= R1 / 4);
-          if (g < R1 / 4)
-            *reinterpret_cast<float4*>(Y + 4 * g) =
-                make_float4(fmaf(a.a2, ar[0], a.a1 * c.x), fmaf(a.a2, ar[1], a.a1 * c.y),
-                            fmaf(a.a2, ar[2], a.a1 * c.z), fmaf(a.a2, ar[3], a.a1 * c.w));
+          lap4w(dtab, *reinterpret_cast<const uint32_t*>(kb + 4 * g), c, ld4(Rm + s), ld4(Rp + s), Rc + s, n3, a.cx,
+                a.cy, a.cz, ar);
+          *reinterpret_cast<float4*>(Y + 4 * g) =
+              make_float4(fmaf(a.a2, ar[0], a.a1 * c.x), fmaf(a.a2, ar[1], a.a1 * c.y),
+                          fmaf(a.a2, ar[2], a.a1 * c.z), fmaf(a.a2, ar[3], a.a1 * c.w));
         }
       }
       // (C) level 2 for plane t-3: z = a0 r + A y1 on the own cells, (r, z)
@@ -445,23 +364,15 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
         const int64_t o = (int64_t)p2 * P;
         // (r, z) of this thread's cells: FP32 sum of the products plus the sum of
         // their exact rounding errors, into the float-float accumulator per plane
-        float psum = 0.f, esum = 0.f, psum2 = 0.f, esum2 = 0.f;
-        auto group = [&](bool v, int s, float4 rr, float4 dd, uchar4 k4, int x, float4 yy, float4 ww) {
+        float psum = 0.f, esum = 0.f;
+        auto group = [&](bool v, int s, float4 rr, uint32_t k4, int x) {
           float ay[4];
-          lap4(dtab, k4, ld4(Yc + s), ld4(Ym + s), ld4(Yp + s), Yc + s, n3, a.cx, a.cy, a.cz, ay);
+          lap4w(dtab, k4, ld4(Yc + s), ld4(Ym + s), ld4(Yp + s), Yc + s, n3, a.cx, a.cy, a.cz, ay);
           if (!v) return;
-          float zz[4] = {fmaf(a.a0, rr.x, ay[0]), fmaf(a.a0, rr.y, ay[1]), fmaf(a.a0, rr.z, ay[2]),
+          const float zz[4] = {fmaf(a.a0, rr.x, ay[0]), fmaf(a.a0, rr.y, ay[1]), fmaf(a.a0, rr.z, ay[2]),
                          fmaf(a.a0, rr.w, ay[3])};
-          if (OUT_TL) {   // z = omega y + s w on the active set, 0 elsewhere
-            const float yv[4] = {yy.x, yy.y, yy.z, yy.w};
-            const uint8_t kv[4] = {k4.x, k4.y, k4.z, k4.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-              zz[q] = (kv[q] >> K_ROW_SHIFT) != ROW_NONE ? fmaf(om, yv[q], a.tsc * zz[q]) : 0.f;
-          }
           *reinterpret_cast<float4*>(a.z + o + x) = make_float4(zz[0], zz[1], zz[2], zz[3]);
           if (!DOTZ) return;
-          if (DOTSEP) rr = dd;
           const float rv[4] = {rr.x, rr.y, rr.z, rr.w};
 #pragma unroll
           for (int q = 0; q < 4; q++) {
@@ -469,25 +380,12 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
             esum += fmaf(rv[q], zz[q], -pr);
             psum += pr;
           }
-          if (OUT_TL) {
-            const float wv[4] = {ww.x, ww.y, ww.z, ww.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              const float pr = wv[q] * zz[q];
-              esum2 += fmaf(wv[q], zz[q], -pr);
-              psum2 += pr;
-            }
-          }
         };
-        group(va, ya, rpa, dpa, kpa, xa, ypa, wpa);
-        group(vb, yb, rpb, dpb, kpb, xb, ypb, wpb);
+        group(va, ya, rpa, kpa, xa);
+        group(vb, yb, rpb, kpb, xb);
         if (DOTZ) {
           acc.add(psum, 1.f);
           acc.add(esum, 1.f);
-        }
-        if (OUT_TL) {
-          acc_rr.add(psum2, 1.f);
-          acc_rr.add(esum2, 1.f);
         }
       }
       // (D) level-2 inputs of the next step
@@ -495,7 +393,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
       // (E) raw plane t+1 for the next step's level 1
       if (has_next) {
         wok = wait_plane(pn);
-        if (FUSE && wok) update(pn);
+        if (wok) update(pn);
       }
       // (F) one barrier per step; a timed-out wait anywhere stops the block
       if (__syncthreads_or(!wok)) { ok = false; break; }
@@ -511,34 +409,11 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
     if (threadIdx.x == 0) {
       atomicExch((unsigned long long*)&S->iscalars[I_ERR], 1ull);
       for (long long L = waited; L < issued; L++) mbar_wait_bounded(&mbar[L % CP_NS], (uint32_t)((L / CP_NS) & 1));
-      if (FUSE && q_issued > q_waited) mbar_wait_bounded(qbar, (uint32_t)(q_waited & 1));
+      if (q_issued > q_waited) mbar_wait_bounded(qbar, (uint32_t)(q_waited & 1));
       S->iscalars[I_DONE] = 1;
       S->iscalars[I_STATUS] = XF_ERR_CUDA;
     }
     __syncthreads();
-    return;
-  }
-  if (MODE == CP_FIRST) return;   // a later pass reduces
-  if (OUT_TL) {   // (z, r) and (z, q_w), one ticket
-    const double bzr = block_sum_acc<float>(acc, sh);
-    const double bzq = block_sum_acc<float>(acc_rr, sh);
-    if (threadIdx.x == 0) {
-      S->partials[a.s_zr][lin_block()] = bzr;
-      S->partials[a.s_zq][lin_block()] = bzq;
-      __threadfence();
-      const unsigned int tk = atomicAdd(&S->tickets[a.s_zr], 1u);
-      last = (tk == (unsigned)num_blocks() - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    const double zr = finish_partials(S, a.s_zr, sh);
-    const double zq = finish_partials(S, a.s_zq, sh);
-    if (threadIdx.x == 0) {
-      S->scalars[a.s_zr] = zr;
-      if (a.qw) S->scalars[a.s_zq] = zq;
-      S->tickets[a.s_zr] = 0;
-      if (a.step.ctl) tl_z(S, a.step);
-    }
     return;
   }
   if (MODE == CP_FIRST_FUSED) {   // (r, r) of the updated residual: the stop test
@@ -551,17 +426,7 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
     }
     return;
   }
-  if (!FUSE) {
-    if (!publish_acc<float>(S, SL_D, SL_D, acc, sh, &last)) return;
-    double tot = finish_partials(S, SL_D, sh);
-    if (threadIdx.x == 0) {
-      S->scalars[SL_D] = tot;
-      S->tickets[SL_D] = 0;
-      control_step(S, CTL_PCG_BETA);
-    }
-    return;
-  }
-  // FUSE: (r, r) of the updated residual and (r, z), one ticket
+  // (r, r) of the updated residual and (r, z), one ticket
   const double brr = block_sum_acc<float>(acc_rr, sh);
   const double brz = block_sum_acc<float>(acc, sh);
   if (threadIdx.x == 0) {
@@ -583,11 +448,320 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_poly2(const __grid_constan
   }
 }
 
+// ---------------------------------------------------------------------------
+// The forms without the residual update (CP_POLY, CP_FIRST, CP_SECOND,
+// CP_TL_LAST), marched in registers.  Bound by instruction issue: the form
+// that kept everything in shared memory ran 94 instructions a cell for 22 us
+// of memory traffic at 256^3.  A thread's own columns stay in registers over
+// the planes (raw t-2, t-1, t and level-1 t-3 .. t-1: the i-neighbours, the
+// second level's input and its centre are no loads), only the j-neighbours and
+// the halo come from shared memory; level 2 follows level 1 by one plane, so
+// that two level-1 planes are held; slots, parities and row-kind offsets step
+// along instead of being divided out of plane numbers; the producer's state is
+// in shared memory; a cell's diagonal is found by its row-kind byte with one
+// shift and one mask.  256^3: CP_FIRST 73.7 -> 55 us, CP_POLY 79 -> 61,
+// CP_SECOND 80 -> 65, CP_TL_LAST 127 -> 87 (with y from zc); the memory's own
+// time is 22 to 43 us.
+constexpr int CM_NS = 5;   // raw ring: planes t-2, t-1, t and two in flight
+
+struct CmProducer { int item, plane, base, hi, slot, issued; };
+
+template <int MODE>
+__global__ void __launch_bounds__(CP_THREADS, 2) k_cg_polym(const __grid_constant__ CpArgs a) {
+  constexpr bool TL = MODE == CP_TL_LAST;                  // output omega y + s w, two dots
+  constexpr bool DOTZ = MODE != CP_FIRST;                  // (r, z)
+  constexpr bool DOTSEP = MODE == CP_SECOND || TL;         // r of the dot is not the input
+  static_assert(ROW_NONE == 0 && K_ROW_SHIFT == 6, "row kinds");
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ double sh[32];
+  __shared__ bool last;
+  __shared__ float dtab[64];
+  __shared__ CmProducer pr;
+  DevScratch* S = a.S;
+  if (S->iscalars[I_DONE] || S->iscalars[I_PAUSE]) return;
+  const int n1 = a.n1, n3 = a.n3, P = a.P, HA = a.HA, R0 = a.R0, R1 = a.R1, KS = a.KS;
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem);
+  float* ring = reinterpret_cast<float*>(smem + 128);           // CM_NS x R0 raw r
+  float* yring = ring + (size_t)CM_NS * R0;                      // 2 x R1 level-1 planes
+  int4* cz4 = reinterpret_cast<int4*>(yring + 2 * (size_t)R1);   // TL: the own cells' blocks in a coarse plane
+  uint8_t* kring = reinterpret_cast<uint8_t*>(cz4 + (TL ? CP_TILE / 4 : 0));   // CM_NS x KS row kinds
+  const int64_t total = (int64_t)n1 * P;
+  const int items = a.nchunk * a.tiles;
+  const int tid = threadIdx.x;
+  const float om = TL ? (float)S->scalars[a.s_om] : 0.f;
+  if (tid < 64)
+    dtab[tid] = a.cx * (float)(((tid >> 0) & 1) + ((tid >> 1) & 1)) + a.cy * (float)(((tid >> 2) & 1) + ((tid >> 3) & 1)) +
+                a.cz * (float)(((tid >> 4) & 1) + ((tid >> 5) & 1));
+  if (tid == 0) {
+    for (int s = 0; s < CM_NS; s++) mbar_init(&mbar[s], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  // an item: planes [i0, i1) of a tile; its raw planes are max(i0 - 2, 0) .. min(i1 + 1, n1 - 1)
+  auto item_range = [&](int item, int& base, int& i0, int& i1) {
+    const int ic = item / a.tiles;
+    base = (item - ic * a.tiles) * CP_TILE;
+    i0 = ic * a.chunk;
+    i1 = min(n1, i0 + a.chunk);
+  };
+  // producer (thread 0): the stream of raw planes over this block's items, with the row kinds of their level-1
+  // region widened to 16-byte boundaries (the kind array holds zero bytes up to a multiple of 16)
+  auto start_item = [&]() {
+    if (pr.item < items) {
+      int i0, i1;
+      item_range(pr.item, pr.base, i0, i1);
+      pr.plane = max(i0 - 2, 0);
+      pr.hi = min(i1 + 1, n1 - 1);
+    }
+  };
+  auto issue_one = [&]() {
+    if (pr.item >= items) return;
+    const int s = pr.slot;
+    const int64_t reg_lo = (int64_t)pr.plane * P + pr.base - 2 * HA, reg_hi = reg_lo + R0;
+    const int64_t c_lo = reg_lo < 0 ? 0 : reg_lo, c_hi = reg_hi > total ? total : reg_hi;
+    const int64_t x0 = reg_lo + HA, total16 = (total + 15) & ~(int64_t)15;
+    const int64_t k_lo = x0 & ~(int64_t)15, k_hi = (x0 + R1 + 15) & ~(int64_t)15;
+    const int64_t kc_lo = k_lo < 0 ? 0 : k_lo, kc_hi = k_hi > total16 ? total16 : k_hi;
+    const uint32_t bytes = (uint32_t)(c_hi - c_lo) * 4u, kbytes = (uint32_t)(kc_hi - kc_lo);
+    mbar_expect_tx(&mbar[s], bytes + kbytes);
+    bulk_g2s(ring + (size_t)s * R0 + (c_lo - reg_lo), a.r + c_lo, bytes, &mbar[s]);
+    bulk_g2s(kring + (size_t)s * KS + (kc_lo - k_lo), a.kind + kc_lo, kbytes, &mbar[s]);
+    pr.issued++;
+    pr.slot = s + 1 == CM_NS ? 0 : s + 1;
+    if (++pr.plane > pr.hi) {
+      pr.item += gridDim.x;
+      start_item();
+    }
+  };
+  if (tid == 0) {
+    pr.item = blockIdx.x;
+    pr.slot = pr.issued = 0;
+    start_item();
+    for (int s = 0; s < CM_NS; s++) issue_one();
+  }
+  auto release = [&](int n) {   // n slots have had their last reader (a block barrier has passed)
+    if (tid == 0) {
+      fence_proxy_async();
+      for (int q = 0; q < n; q++) issue_one();
+    }
+  };
+
+  DotAcc<float> acc, acc2;
+  bool ok = true;
+  int slot = 0, waited = 0;   // the next plane's slot; planes that have landed
+  uint32_t par = 0;           // and its barrier's parity
+  for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    int base, i0, i1;
+    item_range(item, base, i0, i1);
+    const int lo = max(i0 - 2, 0), hi = min(i1 + 1, n1 - 1);
+    const int l1lo = max(i0 - 1, 0), l1hi = min(i1, n1 - 1);   // planes of level 1
+    // own cells: two groups of four at 4 t and TILE/2 + 4 t, from HA on in the
+    // level-1 region and 2 HA in the raw one
+    const int y0 = HA + 4 * tid;
+    if (TL) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int x = min(base + 4 * tid + h * (CP_TILE / 2), P - 4);
+        int j = x / n3, k = x - j * n3, o[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          o[q] = (1 + (j - 1) / a.F) * a.c3 + 1 + (k - 1) / a.F;   // ghost cells: some block, not used
+          if (++k == n3) {
+            k = 0;
+            j++;
+          }
+        }
+        cz4[tid + h * CP_THREADS] = make_int4(o[0], o[1], o[2], o[3]);   // read by this thread only
+      }
+    }
+    int ib = 1 + (max(i0, 1) - 1) / max(a.F, 1), im = (i0 - 1) - (ib - 1) * a.F;   // TL: plane p2's block and place
+    int k16 = (int)(((int64_t)lo * P + base - HA) & 15);   // of plane t: row kinds' offset in their slot
+    int sM = 0, sC = 0, kC = 0;                             // slots of planes t-2, t-1, and the row kinds' offset
+    // registers along i; before the first planes zeros, which only rows of the box faces read
+    float4 rm[2], rc[2], ym[2], yc[2];
+    uint32_t kc[2] = {0, 0};
+    rm[0] = rm[1] = rc[0] = rc[1] = ym[0] = ym[1] = yc[0] = yc[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = lo; t <= i1 + 1; t++) {
+      const int p1 = t - 1, p2 = t - 2;
+      const bool two = p2 >= i0 && p2 < i1;
+      const int64_t o2 = (int64_t)p2 * P + base + 4 * tid;
+      float4 dd[2], ww[2];   // level 2's own inputs, in flight during level 1
+      if (DOTSEP && two) {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          if (base + 4 * tid + h * (CP_TILE / 2) < P) {
+            dd[h] = __ldg(reinterpret_cast<const float4*>(a.dr + o2 + h * (CP_TILE / 2)));
+            if (TL && a.qw) ww[h] = __ldg(reinterpret_cast<const float4*>(a.qw + o2 + h * (CP_TILE / 2)));
+          }
+      }
+      bool wok = true;
+      int sP = sC;   // past the box's last plane: any values, for its face rows
+      if (t <= hi) {
+        sP = slot;
+        wok = mbar_wait_bounded(&mbar[slot], par);
+        waited += wok;
+        if (++slot == CM_NS) {
+          slot = 0;
+          par ^= 1u;
+        }
+      }
+      const float* Rp = ring + sP * R0;
+      float4 rp[2] = {ld4(Rp + HA + y0), ld4(Rp + HA + y0 + CP_TILE / 2)}, yn[2] = {yc[0], yc[1]};
+      uint32_t kn[2] = {kc[0], kc[1]};
+      // (A) level 1 for plane t-1: y1 = a1 r + a2 (A r) over the level-1 region
+      if (wok && p1 >= l1lo && p1 <= l1hi) {
+        const float* Rc = ring + sC * R0 + HA;
+        const uint8_t* kb = kring + sC * KS + kC;
+        float* Y = yring + (p1 & 1) * R1;
+        auto level1 = [&](int y, uint32_t w, float4 m, float4 c, float4 p) {
+          float ar[4];
+          lap4w(dtab, w, c, m, p, Rc + y, n3, a.cx, a.cy, a.cz, ar);
+          return make_float4(fmaf(a.a2, ar[0], a.a1 * c.x), fmaf(a.a2, ar[1], a.a1 * c.y),
+                             fmaf(a.a2, ar[2], a.a1 * c.z), fmaf(a.a2, ar[3], a.a1 * c.w));
+        };
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int y = y0 + h * (CP_TILE / 2);
+          kn[h] = *reinterpret_cast<const uint32_t*>(kb + y);
+          yn[h] = level1(y, kn[h], rm[h], rc[h], rp[h]);
+          *reinterpret_cast<float4*>(Y + y) = yn[h];
+        }
+        const float* Rm = ring + sM * R0 + HA;
+#pragma unroll 1
+        for (int hg = tid; hg < HA / 2; hg += CP_THREADS) {   // halo groups, left then right
+          const int y = 4 * hg + (hg < HA / 4 ? 0 : CP_TILE);
+          *reinterpret_cast<float4*>(Y + y) = level1(y, *reinterpret_cast<const uint32_t*>(kb + y), ld4(Rm + y),
+                                                     ld4(Rc + y), ld4(Rp + HA + y));
+        }
+      }
+      // (B) level 2 for plane t-2: z = a0 r + A y1 on the own cells, and the dots
+      if (wok && two) {
+        const float* Y = yring + (p2 & 1) * R1;
+        const float* zp = TL ? a.zc + (int64_t)ib * a.cs1 : nullptr;
+        // FP32 sums of a thread's products over the plane and of their exact
+        // rounding errors, into the float-float accumulators per plane
+        float psum = 0.f, esum = 0.f, psum2 = 0.f, esum2 = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float ay[4];
+          lap4w(dtab, kc[h], yc[h], ym[h], yn[h], Y + y0 + h * (CP_TILE / 2), n3, a.cx, a.cy, a.cz, ay);
+          if (base + 4 * tid + h * (CP_TILE / 2) >= P) continue;
+          float zz[4] = {fmaf(a.a0, rm[h].x, ay[0]), fmaf(a.a0, rm[h].y, ay[1]), fmaf(a.a0, rm[h].z, ay[2]),
+                         fmaf(a.a0, rm[h].w, ay[3])};
+          if (TL) {   // z = omega y + s w on the active set, 0 elsewhere
+            const int4 o = cz4[tid + h * CP_THREADS];
+            const float yv[4] = {__ldg(zp + o.x), __ldg(zp + o.y), __ldg(zp + o.z), __ldg(zp + o.w)};
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+              zz[q] = kc[h] & (0xc0u << (8 * q)) ? fmaf(om, yv[q], a.tsc * zz[q]) : 0.f;
+          }
+          *reinterpret_cast<float4*>(a.z + o2 + h * (CP_TILE / 2)) = make_float4(zz[0], zz[1], zz[2], zz[3]);
+          if (DOTZ) {
+            const float4 rr = DOTSEP ? dd[h] : rm[h];
+            const float rv[4] = {rr.x, rr.y, rr.z, rr.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const float p = rv[q] * zz[q];
+              esum += fmaf(rv[q], zz[q], -p);
+              psum += p;
+            }
+          }
+          if (TL && a.qw) {
+            const float wv[4] = {ww[h].x, ww[h].y, ww[h].z, ww[h].w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              const float p = wv[q] * zz[q];
+              esum2 += fmaf(wv[q], zz[q], -p);
+              psum2 += p;
+            }
+          }
+        }
+        if (DOTZ) {
+          acc.add(psum, 1.f);
+          acc.add(esum, 1.f);
+        }
+        if (TL) {
+          acc2.add(psum2, 1.f);
+          acc2.add(esum2, 1.f);
+          if (++im == a.F) {
+            im = 0;
+            ib++;
+          }
+        }
+      }
+      // (C) one barrier per step; a timed-out wait anywhere stops the block
+      if (__syncthreads_or(!wok)) {
+        ok = false;
+        break;
+      }
+      if (p2 >= lo) release(1);   // raw plane t-2 has had its last reader
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        rm[h] = rc[h];
+        rc[h] = rp[h];
+        ym[h] = yc[h];
+        yc[h] = yn[h];
+        kc[h] = kn[h];
+      }
+      sM = sC;
+      sC = sP;
+      kC = k16;
+      k16 = (k16 + P) & 15;
+    }
+    if (!ok) break;
+    release(hi - i1 + 1);   // planes i1 .. hi (the last step released i1 - 1)
+  }
+  if (!ok) {
+    if (tid == 0) {   // let the copies in flight land (bounded), end the solve and leave
+      atomicExch((unsigned long long*)&S->iscalars[I_ERR], 1ull);
+      for (int L = waited; L < pr.issued; L++) mbar_wait_bounded(&mbar[L % CM_NS], (uint32_t)((L / CM_NS) & 1));
+      S->iscalars[I_DONE] = 1;
+      S->iscalars[I_STATUS] = XF_ERR_CUDA;
+    }
+    __syncthreads();
+    return;
+  }
+  if (MODE == CP_FIRST) return;   // a later pass reduces
+  if (TL) {   // (z, r) and (z, q_w), one ticket
+    const double bzr = block_sum_acc<float>(acc, sh);
+    const double bzq = block_sum_acc<float>(acc2, sh);
+    if (tid == 0) {
+      S->partials[a.s_zr][lin_block()] = bzr;
+      S->partials[a.s_zq][lin_block()] = bzq;
+      __threadfence();
+      const unsigned int tk = atomicAdd(&S->tickets[a.s_zr], 1u);
+      last = (tk == (unsigned)num_blocks() - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    const double zr = finish_partials(S, a.s_zr, sh);
+    const double zq = finish_partials(S, a.s_zq, sh);
+    if (tid == 0) {
+      S->scalars[a.s_zr] = zr;
+      if (a.qw) S->scalars[a.s_zq] = zq;
+      S->tickets[a.s_zr] = 0;
+      if (a.step.ctl) tl_z(S, a.step);
+    }
+    return;
+  }
+  if (!publish_acc<float>(S, SL_D, SL_D, acc, sh, &last)) return;
+  const double tot = finish_partials(S, SL_D, sh);
+  if (tid == 0) {
+    S->scalars[SL_D] = tot;
+    S->tickets[SL_D] = 0;
+    control_step(S, CTL_PCG_BETA);
+  }
+}
+
 int cp_kslot(int R1) { return (R1 + 32 + 15) & ~15; }
 
-size_t cp_smem(int R0, int R1, bool fuse) {
-  return 128 + (size_t)CP_NS * R0 * 4 + (size_t)CP_NY * R1 * 4 + (fuse ? (size_t)R0 * 4 : 0) +
-         (size_t)CP_NS * cp_kslot(R1);
+size_t cp_smem(int R0, int R1) {
+  return 128 + (size_t)CP_NS * R0 * 4 + (size_t)CP_NY * R1 * 4 + (size_t)R0 * 4 + (size_t)CP_NS * cp_kslot(R1);
+}
+
+size_t cm_smem(int R0, int R1, bool tl) {
+  return 128 + (size_t)CM_NS * R0 * 4 + 2 * (size_t)R1 * 4 + (tl ? (size_t)CP_TILE * 4 : 0) +
+         (size_t)CM_NS * cp_kslot(R1);
 }
 
 int cp_halo(int n3) { return (n3 + 1 + 3) & ~3; }
@@ -729,15 +903,19 @@ bool xf_cg_poly_supported(const xf_grid* g) {
   const int64_t P = (int64_t)g->n2 * g->n3;
   if (!g->uniform || g->nbrow != 0 || P % 4 != 0 || g->n3 % 2 != 0 || g->n3 < 2 || g->n2 < 2) return false;
   const int HA = cp_halo(g->n3);
-  return cp_smem(CP_TILE + 4 * HA, CP_TILE + 2 * HA, true) <= 226 * 1024;
+  return cp_smem(CP_TILE + 4 * HA, CP_TILE + 2 * HA) <= 226 * 1024;   // the larger of the two kernels' rings
 }
 
 namespace {
 
 template <int MODE>
 void poly_launch(const xf_op* op, CpArgs& a, const float coeffs[3]) {
-  // a one-plane q buffer in shared memory: the fused update
   constexpr bool FUSE = MODE == CP_POLY_FUSED || MODE == CP_FIRST_FUSED;
+  constexpr int LEAD = FUSE ? 5 : 4;   // pipeline steps of an item beyond its planes
+  const auto kern = [] {
+    if constexpr (FUSE) return k_cg_poly2<MODE>;
+    else return k_cg_polym<MODE>;
+  }();
   const xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
   a.kind = g->kind; a.S = ctx->scratch;
@@ -749,11 +927,11 @@ void poly_launch(const xf_op* op, CpArgs& a, const float coeffs[3]) {
   a.tiles = (a.P + CP_TILE - 1) / CP_TILE;
   a.cx = (float)g->ucx; a.cy = (float)g->ucy; a.cz = (float)g->ucz;
   a.a0 = coeffs[0]; a.a1 = coeffs[1]; a.a2 = coeffs[2];
-  const size_t smem = cp_smem(a.R0, a.R1, FUSE);
+  const size_t smem = FUSE ? cp_smem(a.R0, a.R1) : cm_smem(a.R0, a.R1, MODE == CP_TL_LAST);
   static size_t attr[64] = {};   // per device: the attribute belongs to the device's copy of the kernel
   size_t& at = attr[ctx->device & 63];
   if (at < smem) {
-    cudaFuncSetAttribute(k_cg_poly2<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     at = smem;
   }
   int resident = (int)((228 * 1024) / (smem + 2048));
@@ -762,9 +940,9 @@ void poly_launch(const xf_op* op, CpArgs& a, const float coeffs[3]) {
   const int64_t B = (int64_t)ctx->sm_count * resident;
   int best = 8;
   double best_cost = 1e30;
-  for (int L = 4; L <= 64; L++) {   // one wave where possible; cost ~ waves x (chunk + 5 pipeline steps)
+  for (int L = 4; L <= 64; L++) {   // one wave where possible; cost ~ waves x (chunk + LEAD)
     const int64_t items = (int64_t)a.tiles * ((g->n1 + L - 1) / L);
-    const double cost = (double)((items + B - 1) / B) * (L + 5);
+    const double cost = (double)((items + B - 1) / B) * (L + LEAD);
     if (cost < best_cost) { best_cost = cost; best = L; }
   }
   a.chunk = best;
@@ -776,7 +954,7 @@ void poly_launch(const xf_op* op, CpArgs& a, const float coeffs[3]) {
     const long cap = strtol(env, nullptr, 10);
     if (cap >= 1 && cap < blocks) blocks = cap;
   }
-  k_cg_poly2<MODE><<<(int)blocks, CP_THREADS, smem, ctx->stream>>>(a);
+  kern<<<(int)blocks, CP_THREADS, smem, ctx->stream>>>(a);
 }
 
 }  // namespace

@@ -290,3 +290,26 @@ __device__ __forceinline__ T apply_row(const StencilGrid<T>& g, const T* __restr
 
 template <typename T>
 StencilGrid<T> make_stencil_grid(const xf_grid* g, const T* rho);
+
+// Fast Laplace row (uniform grid) of four consecutive cells with centres c and
+// i-neighbours m, p; w holds their row kinds (0: no equation, the row gives 0),
+// dtab the open-face diagonal by face bits.  The j- and k-neighbours come from
+// shared memory around s (8-byte aligned, n3 even): for k, shuffles with the
+// warp's ends patched took more instructions and a branch each.
+__device__ __forceinline__ void lap4w(const float* dtab, uint32_t w, float4 c, float4 m, float4 p, const float* s, int n3,
+                                      float cx, float cy, float cz, float out[4]) {
+  const float left = s[-1], right = s[4];
+  const float2 jm01 = *reinterpret_cast<const float2*>(s - n3), jm23 = *reinterpret_cast<const float2*>(s - n3 + 2);
+  const float2 jp01 = *reinterpret_cast<const float2*>(s + n3), jp23 = *reinterpret_cast<const float2*>(s + n3 + 2);
+  const float cc[4] = {c.x, c.y, c.z, c.w};
+  const float ms[4] = {p.x + m.x, p.y + m.y, p.z + m.z, p.w + m.w};
+  const float js[4] = {jp01.x + jm01.x, jp01.y + jm01.y, jp23.x + jm23.x, jp23.y + jm23.y};
+  const float ks[4] = {cc[1] + left, cc[2] + cc[0], cc[3] + cc[1], right + cc[2]};
+  const char* tab = reinterpret_cast<const char*>(dtab);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t at = (q ? w >> (8 * q - 2) : w << 2) & 0xfcu;
+    const float o = fmaf(*reinterpret_cast<const float*>(tab + at), cc[q], -fmaf(cx, ms[q], fmaf(cy, js[q], cz * ks[q])));
+    out[q] = w & (0xc0u << (8 * q)) ? o : 0.f;   // 0: ROW_NONE
+  }
+}

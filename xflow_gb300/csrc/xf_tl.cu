@@ -83,8 +83,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_omega(const float* __restric
 // rows and blocks start at odd k, so a pair lies in one row, and a difference
 // between its two blocks is the pair's only one along k) and marches over the
 // planes: of the six neighbours only the one across the block's j side and
-// the next block along i are loaded, once per four planes.  256^3: 151 MB.
-__global__ void __launch_bounds__(256) k_tl_sub(const uint8_t* __restrict__ kind, const float* __restrict__ r,
+// the next block along i are loaded, once per four planes.  256^3: 151 MB, 22 us
+// of memory time, 37 us measured (41 with two blocks an SM at 90 registers).
+__global__ void __launch_bounds__(256, 3) k_tl_sub(const uint8_t* __restrict__ kind, const float* __restrict__ r,
                                                 const float* __restrict__ zc, int n1, int n3, int P, int c2, int c3,
                                                 int chunk, float cx, float cy, float cz, const DevScratch* S, int s_om,
                                                 float* __restrict__ out) {
