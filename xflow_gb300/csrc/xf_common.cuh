@@ -382,7 +382,20 @@ __device__ __forceinline__ double div_rcp(double a, double b, double y) {
 // chunk c, slab s = 3 (di+1) + (dj+1), 8-channel half q, stacked output row
 // n = dk_index * Co + o, 8 channels): the 9 slabs of one chunk are contiguous,
 // and each (c, s) block is the canonical K-major B operand of one MMA.
+// Outputs wider than 80 channels (3 Co columns of an MMA are at most 256) go
+// tap by tap: per (tap, 8-channel plane, output row, 8 channels).
+__host__ __device__ inline bool conv_wide(int co) { return 3 * co > 256; }
 __host__ __device__ inline int64_t conv_tiled_index(int t, int o, int i, int co, int ci) {
+  if (conv_wide(co)) return (((int64_t)t * (ci / 8) + (i >> 3)) * co + o) * 8 + (i & 7);
   const int s = t / 3, n = (t % 3) * co + o, c = i >> 4, q = (i >> 3) & 1, e = i & 7;
   return ((((int64_t)c * 9 + s) * 2 + q) * (3 * co) + n) * 8 + e;
 }
+
+// The partial sums of one layer's gradients and where their totals go.
+constexpr int WG_LAYERS = 11;
+struct WgSeg {
+  const float *wpart, *bpart;   // [row tile][cell range][128][co]; [chunk][co]
+  float *gw, *gb;               // [27][co][ci]; [co]
+  int mtiles, splits, taps, ci, co, nchunk, block0;
+};
+struct WgSegs { WgSeg s[WG_LAYERS]; };

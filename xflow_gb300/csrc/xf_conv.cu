@@ -141,8 +141,7 @@ struct ConvArgs {
   const uint16_t* in;   // plane 0, cell 0 of the input slice
   int64_t in_ps;        // plane stride (elements)
   int Ci;
-  const uint16_t* W;    // [27][Co][Ci]
-  const uint16_t* Wt;   // the same tiled (conv_tiled_index)
+  const uint16_t* Wt;   // weights tiled (conv_tiled_index)
   const float* bias;    // [Co] or null
   int Co;
   const uint8_t* mask;  // [ncell]
@@ -186,101 +185,6 @@ __device__ __forceinline__ void conv_store8(const ConvArgs& a, int64_t c, int co
       for (int q = 0; q < nq; q++) dst[q] = v[q];
     }
   }
-}
-
-// ---------------------------------------------------------------------------
-// Per-tap form, for wide outputs (3 Co > 256).  A tile is 128 consecutive
-// cells.  For tap t at offset o_t the A operand is the block of rows
-// c0 + o_t .. c0 + o_t + 127 (128 x Ci), the B operand W[t] (Co x Ci); the
-// 27 taps x Ci/16 MMAs accumulate in tensor memory (128 lanes x Co FP32
-// columns).  Operands are staged by the threads in the canonical no-swizzle
-// K-major layout; stages rotate through CONV_STAGES buffers, a stage being
-// refilled only after the tensor core has signalled (mbarrier) that the MMAs
-// reading it are done.
-constexpr int CONV_STAGES = 3;
-
-__global__ void __launch_bounds__(128) k_conv3_tc(ConvArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ uint64_t mbar[CONV_STAGES];
-  __shared__ uint32_t tmem_base;
-  const int Ci = a.Ci, Co = a.Co, kg = Ci / 8;
-  const int stage_a = TC_M * Ci * 2, stage_b = Co * Ci * 2;
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const uint32_t ncols = tmem_cols(Co);
-  if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
-  if (threadIdx.x == 0)
-    for (int s = 0; s < CONV_STAGES; s++) tc::mbar_init(&mbar[s], 1);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t tbase = tmem_base;
-  const uint32_t idesc = tc::idesc_bf16_f32(TC_M, Co);
-  const uint32_t lbo = 128, sbo = (uint32_t)kg * 128;
-  const int64_t P = (int64_t)a.n2 * a.n3;
-  uint32_t issued[CONV_STAGES] = {0, 0, 0}, waited[CONV_STAGES] = {0, 0, 0};
-  bool ok = true;
-  auto drain = [&](int s) {   // wait for the stage's outstanding commit (at most one)
-    if (waited[s] < issued[s]) {
-      const bool w = tc::mbar_wait(&mbar[s], (issued[s] - 1) & 1);
-      if (!w) ok = false;
-      waited[s] = issued[s];
-    }
-  };
-  const int64_t ntiles = (a.ncell + TC_M - 1) / TC_M;
-  for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const int64_t c0 = tile * TC_M;
-    for (int t = 0; t < 27; t++) {
-      const int s = t % CONV_STAGES;
-      drain(s);
-      const int di = t / 9 - 1, dj = (t / 3) % 3 - 1, dk = t % 3 - 1;
-      const int64_t off = di * P + dj * (int64_t)a.n3 + dk;
-      uint8_t* sA = smem + s * (stage_a + stage_b);
-      uint8_t* sB = sA + stage_a;
-      for (int u = threadIdx.x; u < TC_M * kg; u += blockDim.x) {   // A from the channel planes
-        const int r = u / kg, q = u - r * kg;
-        const uint4 v = *reinterpret_cast<const uint4*>(a.in + q * a.in_ps + (c0 + off + r) * 8);
-        *reinterpret_cast<uint4*>(sA + (r >> 3) * kg * 128 + q * 128 + (r & 7) * 16) = v;
-      }
-      stage_kmajor(sB, a.W + (int64_t)t * Co * Ci, Co, Ci, Ci);
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        tc::fence_after_sync();
-        for (int k = 0; k < Ci / 16; k++) {
-          const uint64_t ad = tc::smem_desc(tc::smem_addr(sA + k * 256), lbo, sbo);
-          const uint64_t bd = tc::smem_desc(tc::smem_addr(sB + k * 256), lbo, sbo);
-          tc::mma_bf16(tbase, ad, bd, idesc, t > 0 || k > 0);
-        }
-        tc::mma_commit(&mbar[s]);
-      }
-      issued[s]++;
-    }
-    for (int s = 0; s < CONV_STAGES; s++) drain(s);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    tc::fence_after_sync();
-    // epilogue: warp w owns rows 32w .. 32w+31 (TMEM lanes)
-    const int64_t c = c0 + warp * 32 + lane;
-    const bool live = c < a.ncell;
-    const float m = live ? (float)a.mask[c] : 0.f;
-    for (int co = 0; co < Co; co += 8) {
-      float v[8];
-      tc::tmem_ld8(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)co, v);
-      if (!live || co >= a.out_ch) continue;
-      conv_store8(a, c, co, m, v);
-    }
-    tc::fence_before_sync();
-    __syncthreads();   // TMEM is read before the next tile's first MMA overwrites it
-  }
-  if (!ok) {
-    if (threadIdx.x == 0) atomicExch(a.err, 1);
-    for (int s = 0; s < CONV_STAGES; s++)
-      if (waited[s] < issued[s]) tc::mbar_wait(&mbar[s], (issued[s] - 1) & 1);
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, ncols);
 }
 
 // ---------------------------------------------------------------------------
@@ -614,6 +518,154 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
   if (warp == 0) tc::tmem_dealloc(tbase, (uint32_t)plan.tmem_cols);
 }
 
+// Wide outputs (3 Co > 256), tap by tap: a tile is 128 consecutive cells, the
+// A operand of tap t the rows c0 + o_t .. c0 + o_t + 127, the B operand W[t]; the
+// 27 taps x Ci / 16 MMAs of N = Co accumulate in order.  A stage is one tap: its
+// planes' rows and its weights by bulk copies, already in operand layout, with
+// the roles, waits and two accumulators of the kernel above.  The tensor core
+// is idle most of the time here too (27 x 2 MMAs a tile at Ci = 32); what
+// counts is how many taps are in flight.  32 -> 96 at 34^3: 29.5 us, with the
+// operands staged by the threads and one barrier a tap 81.
+constexpr int WD_MAX_STAGES = 8;
+struct WdPlan { int stages, acc_off, tmem_cols, smem_bytes, per_sm; uint32_t a_bytes, b_bytes, stage_bytes; };
+static WdPlan wd_plan(int ci, int co) {
+  WdPlan p = {};
+  p.acc_off = (co + 31) / 32 * 32;
+  p.tmem_cols = (int)tmem_cols(p.acc_off + co);   // at most 256: two CTAs an SM
+  p.a_bytes = (uint32_t)(ci / 8) * 2048;
+  p.b_bytes = (uint32_t)(co * ci * 2);
+  p.stage_bytes = (p.a_bytes + p.b_bytes + 1023) / 1024 * 1024;
+  for (p.per_sm = 2; p.per_sm >= 1; p.per_sm--) {
+    const int avail = 228 * 1024 / p.per_sm - 1024 - 2048;   // less the part reserved, the static and the slack
+    p.stages = std::min(WD_MAX_STAGES, avail / (int)p.stage_bytes);
+    if (p.stages >= 3 || p.per_sm == 1) break;
+  }
+  p.smem_bytes = p.stages * (int)p.stage_bytes + 1024;
+  return p;
+}
+__global__ void __launch_bounds__(BK_THREADS) k_conv3_wide(ConvArgs a, WdPlan plan) {
+  extern __shared__ uint8_t dsm[];
+  __shared__ uint64_t full[WD_MAX_STAGES], empty[WD_MAX_STAGES], tfull[2], tempty[2], mdone;
+  __shared__ uint32_t tmem_base;
+  __shared__ int abort_flag;
+  const int Ci = a.Ci, Co = a.Co, S = plan.stages;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t raw = tc::smem_addr(dsm);
+  uint8_t* stg = dsm + ((1024u - (raw & 1023u)) & 1023u);
+  if (warp == 0) tc::tmem_alloc(&tmem_base, (uint32_t)plan.tmem_cols);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; s++) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int q = 0; q < 2; q++) {
+      tc::mbar_init(&tfull[q], 1);
+      tc::mbar_init(&tempty[q], 4);
+    }
+    tc::mbar_init(&mdone, 1);
+    abort_flag = 0;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tbase = tmem_base;
+  volatile int* abort_p = &abort_flag;
+  const int64_t P = (int64_t)a.n2 * a.n3;
+  const int64_t ntiles = (a.ncell + TC_M - 1) / TC_M;
+  const int my_tiles = ntiles > blockIdx.x ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+  if (warp == 4) {   // ---- producer: a plane of A per lane (at most 16), the weights by lane 16
+    int st = 0, pass = 0, issued = 0;
+    bool ok = true;
+    for (int k = 0; k < my_tiles && ok; k++) {
+      const int64_t c0 = ((int64_t)blockIdx.x + (int64_t)k * gridDim.x) * TC_M;
+      for (int t = 0; t < 27; t++) {
+        if (pass > 0) {
+          bool w = true;
+          if (lane == 0) w = bk_wait(&empty[st], (uint32_t)((pass - 1) & 1), abort_p);
+          if (!__shfl_sync(0xffffffffu, w, 0)) {
+            ok = false;
+            break;
+          }
+        }
+        uint8_t* sa = stg + (size_t)st * plan.stage_bytes;
+        if (lane == 0) mbar_expect_tx(&full[st], plan.a_bytes + plan.b_bytes);
+        __syncwarp();
+        const int64_t off = (t / 9 - 1) * P + ((t / 3) % 3 - 1) * (int64_t)a.n3 + (t % 3 - 1);
+        if (lane < Ci / 8) bulk_load(sa + lane * 2048, a.in + lane * a.in_ps + (c0 + off) * 8, 2048, &full[st]);
+        else if (lane == 16) bulk_load(sa + plan.a_bytes, a.Wt + (int64_t)t * Co * Ci, plan.b_bytes, &full[st]);
+        issued++;
+        if (++st == S) {
+          st = 0;
+          pass++;
+        }
+      }
+    }
+    if (lane == 0)   // every copy issued has landed before the CTA may leave
+      for (int s = 0; s < S; s++) {
+        const int n = issued / S + (s < issued % S ? 1 : 0);
+        if (n > 0) bk_wait(&full[s], (uint32_t)((n - 1) & 1), abort_p, false);
+      }
+    __syncwarp();
+  } else if (warp == 5) {   // ---- MMA issuer
+    const bool leader = tc::elect_one();
+    const uint32_t idesc = tc::idesc_bf16_f32(TC_M, Co);
+    int st = 0, pass = 0;
+    bool ok = true;
+    for (int k = 0; k < my_tiles && ok; k++) {
+      const int acc = k & 1;
+      if (k >= 2 && !bk_wait_warp(&tempty[acc], (uint32_t)(((k >> 1) - 1) & 1), abort_p)) break;
+      tc::fence_after_sync();
+      const uint32_t dacc = tbase + (uint32_t)(acc * plan.acc_off);
+      for (int t = 0; t < 27; t++) {
+        if (!bk_wait_warp(&full[st], (uint32_t)(pass & 1), abort_p)) {
+          ok = false;
+          break;
+        }
+        tc::fence_after_sync();
+        const uint32_t sa = tc::smem_addr(stg + (size_t)st * plan.stage_bytes), sb = sa + plan.a_bytes;
+        for (int q = 0; q < Ci / 16; q++) {
+          const uint64_t ad = tc::smem_desc(sa + (uint32_t)q * 4096, 2048, 128);
+          const uint64_t bd = tc::smem_desc(sb + (uint32_t)(q * Co * 32), (uint32_t)Co * 16, 128);
+          if (leader) tc::mma_bf16(dacc, ad, bd, idesc, t > 0 || q > 0);
+        }
+        if (leader) tc::mma_commit(&empty[st]);
+        if (++st == S) {
+          st = 0;
+          pass++;
+        }
+      }
+      if (ok && leader) tc::mma_commit(&tfull[acc]);
+    }
+    // every MMA issued has completed before TMEM is freed
+    if (leader) tc::mma_commit(&mdone);
+    bk_wait_warp(&mdone, 0, abort_p, false);
+    __syncwarp();
+  } else {   // ---- epilogue, warps 0-3: TMEM lanes 32 w .. 32 w + 31
+    for (int k = 0; k < my_tiles; k++) {
+      const int acc = k & 1;
+      const bool got = bk_wait(&tfull[acc], (uint32_t)((k >> 1) & 1), abort_p);
+      if (!epi_sync_and(got)) break;
+      tc::fence_after_sync();
+      const int64_t c = ((int64_t)blockIdx.x + (int64_t)k * gridDim.x) * TC_M + warp * 32 + lane;
+      const bool live = c < a.ncell;
+      const float m = live ? (float)a.mask[c] : 0.f;
+      const uint32_t trow = tbase + (uint32_t)(acc * plan.acc_off) + ((uint32_t)(warp * 32) << 16);
+      for (int co = 0; co < Co; co += 8) {
+        float v[8];
+        tc::tmem_ld8(trow + (uint32_t)co, v);
+        if (live && co < a.out_ch) conv_store8(a, c, co, m, v);
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[acc]);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) atomicExch(a.err, 1);
+  tc::fence_after_sync();
+  if (warp == 0) tc::tmem_dealloc(tbase, (uint32_t)plan.tmem_cols);
+}
+
 // Error flag of the convolutions: a slot of the context scratch, cleared by
 // xf_conv_status.
 constexpr int I_CONV_ERR = 60;
@@ -777,22 +829,90 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
   if (warp == 0) tc::tmem_dealloc(tbase, ncols);
 }
 
-// gw[t][co][ci] += the ranges' partials in range order.
-__global__ void k_wgrad_tc_sum(const float* __restrict__ partial, int mtiles, int splits, int taps, int ci, int co,
-                               float* __restrict__ gw) {
-  const int64_t n = (int64_t)27 * co * ci;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int t = (int)(u / ((int64_t)co * ci));
-    const int o = (int)((u / ci) % co), i = (int)(u % ci);
-    const int mt = t / taps, row = (t - mt * taps) * ci + i;
-    float s = 0.f;
-    for (int sp = 0; sp < splits; sp++) s += partial[(((int64_t)mt * splits + sp) * 128 + row) * co + o];
-    gw[u] += s;
+// Bias gradient: partial sums over chunks of cells, a block per chunk and
+// 8-channel plane of g.  Bound by latency (142 blocks at 64^3): a thread's 16
+// loads of a 4,096-cell chunk are in flight together, then a fixed tree over
+// the threads.
+__global__ void __launch_bounds__(256) k_bgrad(const uint16_t* __restrict__ g, int64_t gps, int64_t ncell, int chunk,
+                                               int co, float* __restrict__ bpart) {
+  __shared__ float part[8][256];
+  const int q = blockIdx.y, u = threadIdx.x;
+  const int64_t beg = (int64_t)blockIdx.x * chunk, end = min(ncell, beg + chunk);
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int64_t c0 = beg + u; c0 < end; c0 += 16 * 256) {
+    uint4 v[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      v[k] = make_uint4(0, 0, 0, 0);
+      if (c0 + k * 256 < end) v[k] = __ldg(reinterpret_cast<const uint4*>(g + q * gps + (c0 + k * 256) * 8));
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      if (c0 + k * 256 >= end) break;
+      const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        s[2 * e] += __uint_as_float(w[e] << 16);
+        s[2 * e + 1] += __uint_as_float(w[e] & 0xFFFF0000u);
+      }
+    }
   }
+#pragma unroll
+  for (int e = 0; e < 8; e++) part[e][u] = s[e];
+  __syncthreads();
+  // warp e takes channel e: 128, 64, 32 by shared memory, the rest by shuffles, t += t + h at every level
+  const int e = u >> 5, l = u & 31;
+  float a[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) a[k] = part[e][l + 32 * k];
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int k = 0; k < h; k++) a[k] += a[k + h];
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) a[0] += __shfl_down_sync(0xffffffffu, a[0], h);
+  if (l == 0) bpart[(int64_t)blockIdx.x * co + q * 8 + e] = a[0];
 }
+
+// The layers' partials summed in order: every layer's weights and biases in
+// one launch (11 took 9.9 us each at 64^3, their loads strided by co).  Threads
+// run along co, as the partials lie; a layer's last block sums its bias
+// chunks.
+__global__ void __launch_bounds__(256) k_grad_sum(const __grid_constant__ WgSegs segs) {
+  int k = 0;
+  while (k + 1 < WG_LAYERS && (int)blockIdx.x >= segs.s[k + 1].block0) k++;
+  const WgSeg& g = segs.s[k];
+  const int nw = 27 * g.co * g.ci, u = ((int)blockIdx.x - g.block0) * 256 + threadIdx.x;
+  if (u < nw) {   // nw is a multiple of 256
+    const int o = u % g.co, ti = u / g.co, t = ti / g.ci, i = ti - t * g.ci;
+    const int mt = t / g.taps, row = (t - mt * g.taps) * g.ci + i;
+    const float* p = g.wpart + ((int64_t)mt * g.splits * 128 + row) * g.co + o;
+    const int64_t step = (int64_t)128 * g.co;
+    float s = 0.f;
+#pragma unroll 16
+    for (int sp = 0; sp < g.splits; sp++) s += __ldg(p + sp * step);
+    g.gw[(t * g.co + o) * g.ci + i] = s;
+    return;
+  }
+  const int o = threadIdx.x;   // the chunks in order
+  if (o >= g.co) return;
+  float s = 0.f;
+#pragma unroll 16
+  for (int c = 0; c < g.nchunk; c++) s += __ldg(g.bpart + (int64_t)c * g.co + o);
+  g.gb[o] = s;
+}
+int xf_grad_sum_blocks(int ci, int co) { return 27 * co * ci / 256 + 1; }
+void xf_grad_sum(xf_ctx* ctx, const WgSegs& segs, int blocks) { k_grad_sum<<<blocks, 256, 0, ctx->stream>>>(segs); }
 
 // The row tiles and cell ranges of a layer's weight gradient, and the FP32
 // partial buffer it needs (floats).
+// Chunks of the bias gradient: 4,096 cells, or more in steps of 256 so that there are at most 128.
+void xf_bgrad_plan(int64_t ncell, int* nchunk, int* chunk) {
+  int64_t c = ((ncell + 127) / 128 + 255) / 256 * 256;
+  if (c < 4096) c = 4096;
+  *chunk = (int)c;
+  *nchunk = (int)((ncell + c - 1) / c);
+}
 void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mtiles, int* splits, int* stages,
                       int64_t* partial_floats) {
   const int taps = 128 / ci;
@@ -810,7 +930,7 @@ void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mti
 // (ci channels), both BF16 planes with their zero margins; partial holds
 // xf_wgrad_tc_plan's floats.  ci and co multiples of 16, ci <= 128, co <= 64.
 int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps, int co, const void* x, int64_t xps,
-                int ci, float* partial, float* gw) {
+                int ci, float* partial, float* bpart) {
   if (ci % 16 || co % 16 || ci < 16 || ci > 128 || co < 16 || co > 64)
     return xf_fail(ctx, XF_ERR_ARG, "weight gradient: channel counts out of range");
   WgArgs a;
@@ -825,63 +945,55 @@ int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps,
   a.partial = partial;
   a.err = conv_err_flag(ctx);
   const size_t smem = (size_t)WG_STAGES * a.stage_bytes + 1024;
-  XF_CUDA(ctx, set_max_smem((const void*)k_wgrad_tc, 2, ctx->device, smem));
+  XF_CUDA(ctx, set_max_smem((const void*)k_wgrad_tc, 1, ctx->device, smem));
   k_wgrad_tc<<<a.mtiles * a.splits, BK_THREADS, smem, ctx->stream>>>(a);
-  const int64_t nw = (int64_t)27 * co * ci;
-  k_wgrad_tc_sum<<<(unsigned)((nw + 255) / 256), 256, 0, ctx->stream>>>(partial, a.mtiles, a.splits, a.taps, ci, co,
-                                                                        gw);
+  int nchunk, chunk;
+  xf_bgrad_plan((int64_t)n1 * n2 * n3, &nchunk, &chunk);
+  k_bgrad<<<dim3((unsigned)nchunk, (unsigned)(co / 8)), 256, 0, ctx->stream>>>(a.g, gps, (int64_t)n1 * n2 * n3, chunk, co,
+                                                                              bpart);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }
 
 // Launch on the context stream (arguments checked by the caller).  `weights`
 // is [27][co][ci]; `tiled` the same in the tiled order (needed when 3 co <= 256).
-int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* weights,
-                   const void* tiled, const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch,
-                   int out_ch, int out_fp32, int relu, const void* gate, int64_t gate_ps) {
-  int* err = conv_err_flag(ctx);
+// `tiled`: the weights in conv_tiled_index order.
+int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* tiled,
+                   const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch, int out_ch,
+                   int out_fp32, int relu, const void* gate, int64_t gate_ps) {
   ConvArgs a;
   a.gate = (const uint16_t*)gate; a.gate_ps = gate_ps;
   a.in = (const uint16_t*)in; a.in_ps = in_ps; a.Ci = ci;
-  a.W = (const uint16_t*)weights; a.Wt = (const uint16_t*)tiled; a.bias = bias; a.Co = co;
+  a.Wt = (const uint16_t*)tiled; a.bias = bias; a.Co = co;
   a.mask = mask; a.n2 = n2; a.n3 = n3; a.ncell = (int64_t)n1 * n2 * n3;
   a.out16 = out_fp32 ? nullptr : (uint16_t*)out;
   a.out32 = out_fp32 ? (float*)out : nullptr;
   a.out_ps = out_fp32 ? 0 : out_pitch;
   a.out_ld = out_fp32 ? (int)out_pitch : 0;
-  a.out_ch = out_ch; a.relu = relu; a.err = err;
-  if (3 * co <= 256) {
-    // k-taps stacked along N, operands by bulk copies (the per-tap kernel
-    // below takes wider outputs)
-    static int static_smem = -1;
-    if (static_smem < 0) {
-      cudaFuncAttributes fa;
-      XF_CUDA(ctx, cudaFuncGetAttributes(&fa, k_conv3_bulk));
-      static_smem = (int)fa.sharedSizeBytes;
-    }
-    const BkPlan plan = bk_plan(ci, co, static_smem);
-    if (plan.stages < 2 || !tiled) return xf_fail(ctx, XF_ERR_ARG, "convolution: no stacked-tap plan");
-    XF_CUDA(ctx, set_max_smem((const void*)k_conv3_bulk, 0, ctx->device, (size_t)plan.smem_bytes));
-    const int64_t tiles = (a.ncell + 125) / 126;
-    int64_t blocks = (int64_t)ctx->sm_count * plan.per_sm;
-    if (blocks > tiles) blocks = tiles;
-    k_conv3_bulk<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
+  a.out_ch = out_ch; a.relu = relu; a.err = conv_err_flag(ctx);
+  if (conv_wide(co)) {
+    const WdPlan plan = wd_plan(ci, co);
+    XF_CUDA(ctx, set_max_smem((const void*)k_conv3_wide, 2, ctx->device, (size_t)plan.smem_bytes));
+    const int64_t tiles = (a.ncell + TC_M - 1) / TC_M;
+    const int64_t blocks = std::min(tiles, (int64_t)ctx->sm_count * plan.per_sm);
+    k_conv3_wide<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
     XF_CUDA(ctx, cudaGetLastError());
     return XF_OK;
   }
-  const size_t smem = (size_t)CONV_STAGES * (TC_M * ci * 2 + co * ci * 2);
-  XF_CUDA(ctx, set_max_smem((const void*)k_conv3_tc, 1, ctx->device, smem));
-  // Residency from the kernel's real limits: shared memory (227 KB per SM, with
-  // ~1 KB static and reserved per CTA), tensor-memory columns (512 per SM) and
-  // threads (2048 per SM).
-  int per_sm = (int)((227 * 1024) / (smem + 2048));
-  per_sm = min(per_sm, (int)(512 / tmem_cols(co)));
-  per_sm = min(per_sm, 16);
-  if (per_sm < 1) per_sm = 1;
-  const int64_t ntiles = (a.ncell + TC_M - 1) / TC_M;
-  int64_t blocks = (int64_t)ctx->sm_count * per_sm;
-  if (blocks > ntiles) blocks = ntiles;
-  k_conv3_tc<<<(int)blocks, 128, smem, ctx->stream>>>(a);
+  // k-taps stacked along N
+  static int static_smem = -1;
+  if (static_smem < 0) {
+    cudaFuncAttributes fa;
+    XF_CUDA(ctx, cudaFuncGetAttributes(&fa, k_conv3_bulk));
+    static_smem = (int)fa.sharedSizeBytes;
+  }
+  const BkPlan plan = bk_plan(ci, co, static_smem);
+  if (plan.stages < 2) return xf_fail(ctx, XF_ERR_ARG, "convolution: no stacked-tap plan");
+  XF_CUDA(ctx, set_max_smem((const void*)k_conv3_bulk, 0, ctx->device, (size_t)plan.smem_bytes));
+  const int64_t tiles = (a.ncell + 125) / 126;
+  int64_t blocks = (int64_t)ctx->sm_count * plan.per_sm;
+  if (blocks > tiles) blocks = tiles;
+  k_conv3_bulk<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }
@@ -911,14 +1023,12 @@ extern "C" int xf_conv3d_bf16(xf_ctx* ctx, int n1, int n2, int n3, const void* i
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
   void* tiled = nullptr;
   const int64_t nw = (int64_t)27 * co * ci;
-  if (3 * co <= 256) {
-    XF_CUDA(ctx, cudaMallocAsync(&tiled, nw * 2, ctx->stream));
-    k_tile_weights<<<(unsigned)((nw + 255) / 256), 256, 0, ctx->stream>>>((const uint16_t*)weights, co, ci,
-                                                                          (uint16_t*)tiled);
-  }
-  const int st = xf_conv_launch(ctx, n1, n2, n3, in, in_ps, ci, weights, tiled, bias, co, mask, out, out_pitch,
+  XF_CUDA(ctx, cudaMallocAsync(&tiled, nw * 2, ctx->stream));
+  k_tile_weights<<<(unsigned)((nw + 255) / 256), 256, 0, ctx->stream>>>((const uint16_t*)weights, co, ci,
+                                                                        (uint16_t*)tiled);
+  const int st = xf_conv_launch(ctx, n1, n2, n3, in, in_ps, ci, tiled, bias, co, mask, out, out_pitch,
                                 out_ch, out_fp32, relu, nullptr, 0);
-  if (tiled) cudaFreeAsync(tiled, ctx->stream);
+  cudaFreeAsync(tiled, ctx->stream);
   return st;
 }
 

@@ -21,19 +21,23 @@
 // preconditioned direction (its scale is irrelevant to the flexible CG).
 #include <math.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "xf_control.cuh"
 #include "xf_tl.cuh"
 
-int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* weights,
-                   const void* tiled, const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch,
-                   int out_ch, int out_fp32, int relu, const void* gate, int64_t gate_ps);
+int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* tiled,
+                   const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch, int out_ch,
+                   int out_fp32, int relu, const void* gate, int64_t gate_ps);
 void xf_mv64(const xf_op* op, const MvReq<double>& q);
 void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mtiles, int* splits, int* stages,
                       int64_t* partial_floats);
 int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps, int co, const void* x, int64_t xps,
-                int ci, float* partial, float* gw);
+                int ci, float* partial, float* bpart);
+void xf_bgrad_plan(int64_t ncell, int* nchunk, int* chunk);
+int xf_grad_sum_blocks(int ci, int co);
+void xf_grad_sum(xf_ctx* ctx, const WgSegs& segs, int blocks);
 void xf_cg_q32_dot(const xf_op* op, const float* p, float* q, int slot);
 void xf_tl_faces(const xf_grid* g, const xf_grid* cg, uint32_t* cnt);
 void xf_tl_omega(const xf_grid* g, const xf_grid* cg, const float* zc, const uint32_t* cnt, const double* rc, int slot,
@@ -85,9 +89,8 @@ struct Layer {
   int64_t nw;                 // 27 * co * ci
   float* w = nullptr;         // FP32 master [27][co][ci]
   float* b = nullptr;         // [co]
-  uint16_t* w16 = nullptr;    // BF16 [27][co][ci]
-  uint16_t* wt16 = nullptr;   // BF16 flipped transpose [27][ci][co]: w16[26-t][co][ci]
-  uint16_t *w16t = nullptr, *wt16t = nullptr;   // the same two in the tensor cores' tiled order
+  // BF16 in the tensor cores' tiled order: the weights, and their flipped transpose [26 - t][ci][co]
+  uint16_t *w16t = nullptr, *wt16t = nullptr;
   float *gw = nullptr, *gb = nullptr;                  // gradients
   float *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;   // Adam moments
 };
@@ -110,15 +113,17 @@ struct xf_unet {
   float* zout = nullptr;            // level-0 box, FP32, 1 channel
   // backward buffers (gradients w.r.t. pre-activations, BF16)
   Act G0_16a, G0_16b, G0_48, G1_32a, G1_32b, G1_96, G2_64a, G2_64b, G1_16, G2_32;
-  float* gsum = nullptr;            // FP32 [level-0 cells x 16]: S0 gradient accumulator
-  float* gsum1 = nullptr;           // FP32 [level-1 cells x 32]: S1 gradient accumulator
-  double* red = nullptr;            // device reductions: [0] sum r^2, [1] sum e^2, [2] loss
+  double* red = nullptr;            // device reductions: [0] sum r^2, [1] sum e^2, [2] loss, [6], [7] 1 / rms of r, e
   double* rpart = nullptr;          // per-block partials of the sums of squares, 2 x RP_MAX
   unsigned* rtick = nullptr;        // their last-block tickets
-  float* wpart = nullptr;           // tensor-core weight-gradient partials [row tile][cell range][128][co]
-  float* bpart = nullptr;           // per-chunk bias-gradient partials [chunk][co]
+  float* gpart = nullptr;           // the layers' weight- and bias-gradient partials
+  WgSegs segs;                      // where each layer's lie and sum
+  int sum_blocks = 0;
   double* zd = nullptr;             // level-0 box, FP64: the output (A-norm loss)
   double* az = nullptr;             // A zd
+  // the layers' parameters, gradients and moments, each in one slab in params_io's order
+  float* slab[4] = {nullptr, nullptr, nullptr, nullptr};
+  int64_t nparam = 0;
   int step = 0;
 };
 
@@ -164,150 +169,149 @@ __device__ __forceinline__ uint4 bf8_pack(const float (&s)[8], float scale) {
   for (int q = 0; q < 4; q++) w[q] = (uint32_t)f2bf(s[2 * q] * scale) | ((uint32_t)f2bf(s[2 * q + 1] * scale) << 16);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-__global__ void k_pool(const uint16_t* __restrict__ src, int64_t sps, int f2, int f3, uint16_t* __restrict__ dst,
-                       int64_t dps, const uint8_t* __restrict__ cmask, int c1, int c2, int c3, int C) {
-  const int C8 = C / 8;
-  const int64_t n = (int64_t)c1 * c2 * c3 * C8;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = u / C8;
-    const int g = (int)(u - c * C8);
-    const int I = (int)(c / ((int64_t)c2 * c3)), J = (int)((c / c3) % c2), K = (int)(c % c3);
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (cmask[c])
-      for (int a = 0; a < 2; a++)
-        for (int b = 0; b < 2; b++)
-          for (int d = 0; d < 2; d++)
-            bf8_acc(s, *reinterpret_cast<const uint4*>(
-                           src + g * sps + (((int64_t)(2 * I - 1 + a) * f2 + (2 * J - 1 + b)) * f3 + (2 * K - 1 + d)) * 8));
-    *reinterpret_cast<uint4*>(dst + g * dps + c * 8) = bf8_pack(s, 0.125f);
+// Zeroes the channels whose gate value (BF16) is not positive.
+__device__ __forceinline__ void relu_gate(float (&s)[8], uint4 v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (!(bf2f((uint16_t)(w[q] & 0xFFFFu)) > 0.f)) s[2 * q] = 0.f;
+    if (!(bf2f((uint16_t)(w[q] >> 16)) > 0.f)) s[2 * q + 1] = 0.f;
   }
 }
-
-// Pooling backward: every active fine child receives 1/8 of its parent's
-// gradient, added to an FP32 accumulator (pitch ald).
-__global__ void k_pool_bwd(const uint16_t* __restrict__ gcoarse, int64_t gps, int c2, int c3,
-                           const uint8_t* __restrict__ fmask, int f1, int f2, int f3, float* __restrict__ acc,
-                           int ald, int C) {
-  const int64_t n = (int64_t)f1 * f2 * f3 * C;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = u / C;
-    const int ch = (int)(u - c * C);
-    if (!fmask[c]) continue;
-    const int i = (int)(c / ((int64_t)f2 * f3)), j = (int)((c / f3) % f2), k = (int)(c % f3);
-    const int64_t pc = ((int64_t)(1 + (i - 1) / 2) * c2 + (1 + (j - 1) / 2)) * c3 + (1 + (k - 1) / 2);
-    acc[c * ald + ch] += 0.125f * bf2f(gcoarse[(ch >> 3) * gps + pc * 8 + (ch & 7)]);
+// The elementwise kernels below take one cell and one plane (16 bytes) a
+// thread, the plane by blockIdx.y, and 32-bit cell indices (a network's boxes
+// stay far below 2^31 cells): by channel and with 64-bit divisions they were
+// bound by their index arithmetic.
+__global__ void k_pool(const uint16_t* __restrict__ src, int64_t sps, int f2, int f3, uint16_t* __restrict__ dst,
+                       int64_t dps, const uint8_t* __restrict__ cmask, unsigned n, int c2, int c3) {
+  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int g = blockIdx.y;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (cmask[c]) {
+    const unsigned t = c / (unsigned)c3, K = c - t * c3, I = t / (unsigned)c2, J = t - I * c2;
+    const uint16_t* p = src + g * sps + (((int64_t)(2 * I - 1) * f2 + (2 * J - 1)) * f3 + (2 * K - 1)) * 8;
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int d = 0; d < 2; d++) bf8_acc(s, *reinterpret_cast<const uint4*>(p + (((int64_t)a * f2 + b) * f3 + d) * 8));
   }
+  *reinterpret_cast<uint4*>(dst + g * dps + (int64_t)c * 8) = bf8_pack(s, 0.125f);
+}
+
+// The coarse cell over fine cell c of an f2 x f3 plane box (interior cells).
+__device__ __forceinline__ int64_t parent(unsigned c, int f2, int f3, int c2, int c3) {
+  const unsigned t = c / (unsigned)f3, k = c - t * f3, i = t / (unsigned)f2, j = t - i * f2;
+  return ((int64_t)((i + 1) >> 1) * c2 + ((j + 1) >> 1)) * c3 + ((k + 1) >> 1);
 }
 
 // Nearest upsampling of a coarse slice into a fine slice, times the fine mask;
-// one plane (8 channels, 16 bytes) per thread.
+// four planes a thread.
 __global__ void k_upsample(const uint16_t* __restrict__ src, int64_t sps, int c2, int c3, uint16_t* __restrict__ dst,
-                           int64_t dps, const uint8_t* __restrict__ fmask, int f1, int f2, int f3, int C) {
-  const int C8 = C / 8;
-  const int64_t n = (int64_t)f1 * f2 * f3 * C8;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = u / C8;
-    const int g = (int)(u - c * C8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (fmask[c]) {
-      const int i = (int)(c / ((int64_t)f2 * f3)), j = (int)((c / f3) % f2), k = (int)(c % f3);
-      const int64_t pc = ((int64_t)(1 + (i - 1) / 2) * c2 + (1 + (j - 1) / 2)) * c3 + (1 + (k - 1) / 2);
-      v = *reinterpret_cast<const uint4*>(src + g * sps + pc * 8);
-    }
-    *reinterpret_cast<uint4*>(dst + g * dps + c * 8) = v;
+                           int64_t dps, const uint8_t* __restrict__ fmask, unsigned n, int f2, int f3) {
+  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  uint4 v[4] = {};
+  if (fmask[c]) {
+    const uint16_t* p = src + (int64_t)blockIdx.y * 4 * sps + parent(c, f2, f3, c2, c3) * 8;
+#pragma unroll
+    for (int g = 0; g < 4; g++) v[g] = __ldg(reinterpret_cast<const uint4*>(p + g * sps));
   }
+  uint16_t* q = dst + (int64_t)blockIdx.y * 4 * dps + (int64_t)c * 8;
+#pragma unroll
+  for (int g = 0; g < 4; g++) *reinterpret_cast<uint4*>(q + g * dps) = v[g];
 }
 
 // Upsampling backward: a coarse cell's gradient is the sum over its 8
 // children; then x coarse mask and the coarse activation's ReLU gate.
 __global__ void k_upsample_bwd(const uint16_t* __restrict__ gfine, int64_t gps, int f2, int f3,
                                const uint16_t* __restrict__ gate, int64_t gtps, const uint8_t* __restrict__ cmask,
-                               int c1, int c2, int c3, uint16_t* __restrict__ dst, int64_t dps, int C) {
-  const int64_t n = (int64_t)c1 * c2 * c3 * C;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = u / C;
-    const int ch = (int)(u - c * C);
-    float s = 0.f;
-    const int64_t pl = (int64_t)(ch >> 3), e = ch & 7;
-    if (cmask[c] && bf2f(gate[pl * gtps + c * 8 + e]) > 0.f) {
-      const int I = (int)(c / ((int64_t)c2 * c3)), J = (int)((c / c3) % c2), K = (int)(c % c3);
-      for (int a = 0; a < 2; a++)
-        for (int b = 0; b < 2; b++)
-          for (int d = 0; d < 2; d++)
-            s += bf2f(gfine[pl * gps + (((int64_t)(2 * I - 1 + a) * f2 + (2 * J - 1 + b)) * f3 + (2 * K - 1 + d)) * 8 + e]);
-    }
-    dst[pl * dps + c * 8 + e] = f2bf(s);
+                               unsigned n, int c2, int c3, uint16_t* __restrict__ dst, int64_t dps) {
+  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int g = blockIdx.y;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (cmask[c]) {
+    const unsigned t = c / (unsigned)c3, K = c - t * c3, I = t / (unsigned)c2, J = t - I * c2;
+    const uint16_t* p = gfine + g * gps + (((int64_t)(2 * I - 1) * f2 + (2 * J - 1)) * f3 + (2 * K - 1)) * 8;
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int d = 0; d < 2; d++) bf8_acc(s, *reinterpret_cast<const uint4*>(p + (((int64_t)a * f2 + b) * f3 + d) * 8));
+    relu_gate(s, *reinterpret_cast<const uint4*>(gate + g * gtps + (int64_t)c * 8));
   }
+  *reinterpret_cast<uint4*>(dst + g * dps + (int64_t)c * 8) = bf8_pack(s, 1.f);
 }
 
-// Skip gradient: dPre = (skip part of the decoder's input gradient + pooled
-// path's accumulator) x mask x ReLU gate; the accumulator is cleared.
-__global__ void k_skip_grad(const uint16_t* __restrict__ gskip, int64_t gps, float* __restrict__ acc, int ald,
-                            const uint16_t* __restrict__ gate, int64_t gtps, const uint8_t* __restrict__ mask,
-                            int64_t ncell, uint16_t* __restrict__ dst, int64_t dps, int C) {
-  const int64_t n = ncell * C;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = u / C;
-    const int ch = (int)(u - c * C);
-    const int64_t o = c * 8 + (ch & 7), pl = ch >> 3;
-    float v = bf2f(gskip[pl * gps + o]) + acc[c * ald + ch];
-    acc[c * ald + ch] = 0.f;
-    if (!mask[c] || !(bf2f(gate[pl * gtps + o]) > 0.f)) v = 0.f;
-    dst[pl * dps + o] = f2bf(v);
+// Skip gradient: dPre = (skip part of the decoder's input gradient + 1/8 of
+// the pooled parent's gradient) x mask x ReLU gate.
+__global__ void k_skip_grad(const uint16_t* __restrict__ gskip, int64_t gps, const uint16_t* __restrict__ gpool,
+                            int64_t pps, int c2, int c3, const uint16_t* __restrict__ gate, int64_t gtps,
+                            const uint8_t* __restrict__ mask, unsigned n, int f2, int f3, uint16_t* __restrict__ dst,
+                            int64_t dps) {
+  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int g = blockIdx.y;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (mask[c]) {
+    const int64_t o = (int64_t)c * 8;
+    const uint4 up = *reinterpret_cast<const uint4*>(gpool + g * pps + parent(c, f2, f3, c2, c3) * 8);
+    bf8_acc(s, up);   // exact: 0 + g
+#pragma unroll
+    for (int q = 0; q < 8; q++) s[q] *= 0.125f;
+    bf8_acc(s, *reinterpret_cast<const uint4*>(gskip + g * gps + o));
+    relu_gate(s, *reinterpret_cast<const uint4*>(gate + g * gtps + o));
   }
+  *reinterpret_cast<uint4*>(dst + g * dps + (int64_t)c * 8) = bf8_pack(s, 1.f);
 }
 
-// Sum of squares over the active cells into red[slot].  Per-block partials,
-// summed in a fixed order by the last block to finish, so the result does
-// not depend on scheduling (256 threads, at most RP_MAX blocks).
+// Sum of squares over the active cells into red[slot], and 1 / rms (0 of a zero
+// sum) into red[6 + slot]; slot 0 also clears the loss.  Per-block partials,
+// summed in a fixed order by the last block to finish, so the result does not
+// depend on scheduling (256 threads, at most RP_MAX blocks).
 constexpr int RP_MAX = 4096;
-__global__ void __launch_bounds__(256) k_sumsq(const double* __restrict__ x, const uint8_t* __restrict__ m, int64_t n,
-                                               double* red, int slot, double* part, unsigned* tick) {
-  __shared__ double sw[8];
+__device__ __forceinline__ void sumsq_finish(double s, double* red, int slot, double count, double* part,
+                                             unsigned* tick) {
+  __shared__ double sh[1];
   __shared__ bool last;
-  double s = 0;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
-    if (m[c]) s += x[c] * x[c];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = s;
-  __syncthreads();
+  const double b = block_sum(s, sh);
   if (threadIdx.x == 0) {
-    double b = 0;
-    for (int w = 0; w < 8; w++) b += sw[w];
     part[slot * RP_MAX + blockIdx.x] = b;
     __threadfence();
     last = atomicAdd(&tick[slot], 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
-  // the last block sums the partials: thread t takes t, t + 256, ... in
-  // order, then a fixed tree over the threads (the same order every run)
   __threadfence();
   double t = 0;
   for (unsigned k = threadIdx.x; k < gridDim.x; k += 256) t += __ldcg(&part[slot * RP_MAX + k]);
-  __shared__ double st[256];
-  st[threadIdx.x] = t;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) st[threadIdx.x] += st[threadIdx.x + h];
-    __syncthreads();
-  }
+  t = block_sum(t, sh);
   if (threadIdx.x == 0) {
-    red[slot] = st[0];
+    red[slot] = t;
+    red[6 + slot] = t > 0 ? 1.0 / sqrt(t / count) : 0.0;
+    if (slot == 0) red[2] = 0.0;
     tick[slot] = 0;
   }
 }
+__global__ void __launch_bounds__(256) k_sumsq(const double* __restrict__ x, const uint8_t* __restrict__ m, int64_t n,
+                                               double count, double* red, int slot, double* part, unsigned* tick) {
+  double s = 0;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+    if (m[c]) s = fma(x[c], x[c], s);
+  sumsq_finish(s, red, slot, count, part, tick);
+}
 
-// Level-0 input: channel 0 = r / rms(r) on active cells, channels 1..15 = 0.
+// r / rms(r) into channel 0 of the first layer's input (its other channels stay 0).
 __global__ void k_unet_input(const double* __restrict__ r, const uint8_t* __restrict__ m, int64_t n,
-                             const double* __restrict__ red, double count, uint16_t* __restrict__ x0, int64_t ps) {
-  const double ss = red[0];
-  const float inv = ss > 0 ? (float)(1.0 / sqrt(ss / count)) : 0.f;
+                             const double* __restrict__ red, uint16_t* __restrict__ x0) {
+  const float inv = (float)red[6];
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    uint16_t v[16] = {0};
-    if (m[c]) v[0] = f2bf((float)r[c] * inv);
-    *reinterpret_cast<uint4*>(x0 + c * 8) = *reinterpret_cast<uint4*>(&v[0]);
-    *reinterpret_cast<uint4*>(x0 + ps + c * 8) = *reinterpret_cast<uint4*>(&v[8]);
+    const uint32_t v = m[c] ? f2bf((float)r[c] * inv) : 0u;
+    *reinterpret_cast<uint4*>(x0 + c * 8) = make_uint4(v, 0, 0, 0);
   }
 }
 
@@ -315,15 +319,14 @@ __global__ void k_unet_input(const double* __restrict__ r, const uint8_t* __rest
 // gradient as the output layer's 16-channel dPre (channel 0).
 __global__ void k_unet_loss(const float* __restrict__ z, const double* __restrict__ e, const uint8_t* __restrict__ m,
                             int64_t n, double count, double* red, uint16_t* __restrict__ g16, int64_t ps) {
-  const double ss = red[1];
-  const double inv = ss > 0 ? 1.0 / sqrt(ss / count) : 0.0;
+  const double inv = red[7], dcount = 2.0 / count;
   double l = 0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
     uint16_t v[16] = {0};
     if (m[c]) {
       const double d = (double)z[c] - e[c] * inv;
       l += d * d;
-      v[0] = f2bf((float)(2.0 * d / count));
+      v[0] = f2bf((float)(dcount * d));
     }
     *reinterpret_cast<uint4*>(g16 + c * 8) = *reinterpret_cast<uint4*>(&v[0]);
     *reinterpret_cast<uint4*>(g16 + ps + c * 8) = *reinterpret_cast<uint4*>(&v[8]);
@@ -332,88 +335,89 @@ __global__ void k_unet_loss(const float* __restrict__ z, const double* __restric
   if ((threadIdx.x & 31) == 0) atomicAdd(&red[2], l / count);
 }
 
-// Bias gradient gb[co] += sum over cells of g[c][co] (the weight gradients run
-// on the tensor cores, xf_wgrad_tc).  Block = (8-channel plane, chunk of
-// cells); each thread sums 8 channels over its cells, the block in a fixed
-// tree, and k_bgrad_sum adds the chunks in order (deterministic).
-// Cells per block: 4096, or more so that a level has at most WG_MAX_CHUNKS
-// chunks (the partial buffer's size).
-constexpr int WG_MAX_CHUNKS = 128;
-static int64_t wg_chunk(int64_t n) {
-  int64_t c = (n + WG_MAX_CHUNKS - 1) / WG_MAX_CHUNKS;
-  c = (c + 255) / 256 * 256;
-  return c < 4096 ? 4096 : c;
+// Adam step (bias-corrected, step counts from 1) of every layer's weights and
+// biases, then the BF16 copies of the weights and of their flipped transpose
+// in the tiled order, in one launch (33 of 3.5 us each did this layer by
+// layer).  A layer's last block takes its biases.
+struct AdamSeg {
+  float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb;
+  uint16_t *w16t, *wt16t;
+  int ci, co, block0;
+};
+struct AdamSegs { AdamSeg s[NLAYER]; };
+__device__ __forceinline__ float adam(float* w, const float* g, float* m, float* v, int u, float lr, float b1, float b2,
+                                      float eps, float c1, float c2) {
+  const float gr = g[u];
+  const float mm = b1 * m[u] + (1 - b1) * gr;
+  const float vv = b2 * v[u] + (1 - b2) * gr * gr;
+  m[u] = mm;
+  v[u] = vv;
+  const float x = w[u] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+  w[u] = x;
+  return x;
 }
-__global__ void __launch_bounds__(256) k_bgrad(const uint16_t* __restrict__ g, int64_t gps, int64_t ncell, int chunk,
-                                               int co, float* __restrict__ bpart) {
-  __shared__ float red[8][256];
-  const int q = blockIdx.y;
-  const int64_t c_beg = (int64_t)blockIdx.x * chunk, c_end = min(ncell, c_beg + chunk);
-  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int64_t c = c_beg + threadIdx.x; c < c_end; c += 256) bf8_acc(s, *reinterpret_cast<const uint4*>(g + q * gps + c * 8));
-  for (int e = 0; e < 8; e++) red[e][threadIdx.x] = s[e];
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h)
-      for (int e = 0; e < 8; e++) red[e][threadIdx.x] += red[e][threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x < 8) bpart[(int64_t)blockIdx.x * co + q * 8 + threadIdx.x] = red[threadIdx.x][0];
+__device__ __forceinline__ void weight_bf16(float x, int u, int co, int ci, uint16_t* w16t, uint16_t* wt16t) {
+  const int t = u / (co * ci), o = (u / ci) % co, i = u % ci;
+  const uint16_t h = f2bf(x);
+  w16t[conv_tiled_index(t, o, i, co, ci)] = h;
+  wt16t[conv_tiled_index(26 - t, i, o, ci, co)] = h;
 }
-__global__ void k_bgrad_sum(const float* __restrict__ bpart, int nchunk, int co, float* __restrict__ gb) {
-  const int u = threadIdx.x;
-  if (u >= co) return;
-  float s = 0.f;
-  for (int c = 0; c < nchunk; c++) s += bpart[(int64_t)c * co + u];
-  gb[u] += s;
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamSegs segs, float lr, float b1, float b2,
+                                              float eps, float c1, float c2) {
+  int k = 0;
+  while (k + 1 < NLAYER && (int)blockIdx.x >= segs.s[k + 1].block0) k++;
+  const AdamSeg& a = segs.s[k];
+  const int u = ((int)blockIdx.x - a.block0) * 256 + threadIdx.x, nw = 27 * a.co * a.ci;
+  if (u < nw) weight_bf16(adam(a.w, a.gw, a.mw, a.vw, u, lr, b1, b2, eps, c1, c2), u, a.co, a.ci, a.w16t, a.wt16t);
+  else if (u - nw < a.co) adam(a.b, a.gb, a.mb, a.vb, u - nw, lr, b1, b2, eps, c1, c2);
 }
-
-// Adam step on one layer (bias-corrected, step counts from 1), then the BF16
-// copies: w16[t][co][ci] and the flipped transpose wt16[26-t][ci][co], each
-// also in the tiled order.
-__global__ void k_adam(float* w, float* gwt, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,
-                       float c1, float c2, int clear) {
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const float gr = gwt[u];
-    const float mm = b1 * m[u] + (1 - b1) * gr;
-    const float vv = b2 * v[u] + (1 - b2) * gr * gr;
-    m[u] = mm;
-    v[u] = vv;
-    w[u] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-    if (clear) gwt[u] = 0.f;
-  }
-}
-
-__global__ void k_weights_bf16(const float* __restrict__ w, int co, int ci, uint16_t* __restrict__ w16,
-                               uint16_t* __restrict__ wt16, uint16_t* __restrict__ w16t, uint16_t* __restrict__ wt16t) {
-  const int64_t n = (int64_t)27 * co * ci;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-    const int t = (int)(u / ((int64_t)co * ci));
-    const int o = (int)((u / ci) % co), i = (int)(u % ci);
-    const uint16_t h = f2bf(w[u]);
-    w16[u] = h;
-    wt16[((int64_t)(26 - t) * ci + i) * co + o] = h;
-    w16t[conv_tiled_index(t, o, i, co, ci)] = h;
-    wt16t[conv_tiled_index(26 - t, i, o, ci, co)] = h;
-  }
+__global__ void k_weights_bf16(const float* __restrict__ w, int co, int ci, uint16_t* __restrict__ w16t,
+                               uint16_t* __restrict__ wt16t) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u < 27 * co * ci) weight_bf16(w[u], u, co, ci, w16t, wt16t);
 }
 
 // A-norm loss 1 - (z,r) / sqrt((z,Az)(e,r)) (one minus the A-norm cosine of
-// the output and the error; dots in scalars[10..12]) and its gradient
-// -(r - (z,r)/(z,Az) A z) / sqrt((z,Az)(e,r)) as the output layer's
+// the output and the error) into red[2], and the factors of its gradient
+// -(r - (z,r)/(z,Az) A z) / sqrt((z,Az)(e,r)) into scalars[10], [11]: the three
+// dots over the active cells in one pass (three took 12 us each at 64^3), the
+// divisions and roots in its last block (by every thread of the gradient they
+// took 15 us).
+__global__ void __launch_bounds__(256) k_anorm_dots(const float* __restrict__ z, const double* __restrict__ az,
+                                                            const double* __restrict__ r, const double* __restrict__ e,
+                                                            const uint8_t* __restrict__ m, int64_t n, DevScratch* S,
+                                                            double* red) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  double v[3] = {0.0, 0.0, 0.0};
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+    if (m[c]) {
+      const double zc = (double)z[c], rc = r[c];
+      v[0] = fma(zc, rc, v[0]);
+      v[1] = fma(zc, az[c], v[1]);
+      v[2] = fma(e[c], rc, v[2]);
+    }
+  if (!publish_partials<3>(S, 10, v, sh, &last)) return;
+  const double zr = finish_partials(S, 10, sh), zaz = finish_partials(S, 11, sh), er = finish_partials(S, 12, sh);
+  if (threadIdx.x == 0) {
+    const bool ok = zaz > 0 && er > 0;
+    S->scalars[10] = ok ? -1 / sqrt(zaz * er) : 0.0;
+    S->scalars[11] = ok ? zr / zaz : 0.0;
+    red[2] = ok ? 1 - zr / sqrt(zaz * er) : 1.0;
+    S->tickets[10] = 0;
+  }
+}
+
+// Gradient c1 (r - c2 A z) of the A-norm loss as the output layer's
 // 16-channel dPre (channel 0).
 __global__ void k_anorm_grad(const double* __restrict__ r, const double* __restrict__ az,
-                             const uint8_t* __restrict__ m, int64_t n, const DevScratch* __restrict__ S, double* red,
+                             const uint8_t* __restrict__ m, int64_t n, const DevScratch* __restrict__ S,
                              uint16_t* __restrict__ g16, int64_t ps) {
-  const double zr = S->scalars[10], zaz = S->scalars[11], er = S->scalars[12];
-  const bool ok = zaz > 0 && er > 0;
-  const double c1 = ok ? -1 / sqrt(zaz * er) : 0.0, c2 = ok ? zr / zaz : 0.0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) red[2] = ok ? 1 - zr / sqrt(zaz * er) : 1.0;
+  const double c1 = S->scalars[10], c2 = S->scalars[11];
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    uint16_t v[16] = {0};
-    if (m[c]) v[0] = f2bf((float)(c1 * (r[c] - c2 * az[c])));
-    *reinterpret_cast<uint4*>(g16 + c * 8) = *reinterpret_cast<uint4*>(&v[0]);
-    *reinterpret_cast<uint4*>(g16 + ps + c * 8) = *reinterpret_cast<uint4*>(&v[8]);
+    const uint32_t v = m[c] ? f2bf((float)(c1 * (r[c] - c2 * az[c]))) : 0u;
+    *reinterpret_cast<uint4*>(g16 + c * 8) = make_uint4(v, 0, 0, 0);
+    *reinterpret_cast<uint4*>(g16 + ps + c * 8) = make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -426,8 +430,10 @@ __global__ void k_f2d_mask(const float* __restrict__ z, const uint8_t* __restric
 // ---------------------------------------------------------------------------
 // Host side
 static int ublocks(xf_ctx* ctx, int64_t n) { return grid_blocks(ctx, n, 256); }
-// k_sumsq's grid: its partial buffer holds RP_MAX blocks (the loop is grid-stride)
-static int sumsq_blocks(xf_ctx* ctx, int64_t n) { return std::min(ublocks(ctx, n), RP_MAX); }
+// Grid of the FP64 sums over a level: two blocks an SM, each with a handful of
+// cells a thread, as a block's own sum, its ticket and the last block's pass over
+// the partials are what they cost (64^3: 1,124 blocks 11.6 us, 304 10.4)
+static int sumsq_blocks(xf_ctx* ctx, int64_t n) { return std::min({ublocks(ctx, n), 2 * ctx->sm_count, RP_MAX}); }
 
 static int act_alloc(xf_unet* u, Act& a, int level, int C) {
   a.level = level;
@@ -450,18 +456,17 @@ static void unet_free(xf_unet* u) {
   for (int l = 1; l < 3; l++)
     if (u->L[l].mask) cudaFree(u->L[l].mask);
   for (Layer& y : u->ly) {
-    void* ps[] = {y.w, y.b, y.w16, y.wt16, y.w16t, y.wt16t, y.gw, y.gb, y.mw, y.vw, y.mb, y.vb};
+    void* ps[] = {y.w16t, y.wt16t};
     for (void* p : ps)
       if (p) cudaFree(p);
   }
+  for (float* p : u->slab)
+    if (p) cudaFree(p);
   if (u->zout) cudaFree(u->zout);
-  if (u->gsum) cudaFree(u->gsum);
-  if (u->gsum1) cudaFree(u->gsum1);
   if (u->red) cudaFree(u->red);
   if (u->rpart) cudaFree(u->rpart);
   if (u->rtick) cudaFree(u->rtick);
-  if (u->wpart) cudaFree(u->wpart);
-  if (u->bpart) cudaFree(u->bpart);
+  if (u->gpart) cudaFree(u->gpart);
   if (u->zd) cudaFree(u->zd);
   if (u->az) cudaFree(u->az);
   if (u->tlg) xf_tl_graph_free(u->tlg);
@@ -518,51 +523,66 @@ extern "C" int xf_unet_create(const xf_grid* g, xf_unet** out) {
       {&u->G1_96, 1, 96}, {&u->G2_64a, 2, 64}, {&u->G2_64b, 2, 64}, {&u->G1_16, 1, 16}, {&u->G2_32, 2, 32}};
   for (auto& e : acts)
     if (!st) st = act_alloc(u, *e.a, e.level, e.C);
-  for (int k = 0; k < NLAYER && !st; k++) {
+  for (int k = 0; k < NLAYER; k++) {
     Layer& y = u->ly[k];
     y.ci = LCI[k]; y.co = LCO[k];
     y.nw = (int64_t)27 * y.co * y.ci;
-    float** f32[] = {&y.w, &y.gw, &y.mw, &y.vw};
-    for (float** p : f32)
-      if (!st && cudaMalloc(p, y.nw * 4) != cudaSuccess) st = XF_ERR_NOMEM;
-    float** fb[] = {&y.b, &y.gb, &y.mb, &y.vb};
-    for (float** p : fb)
-      if (!st && cudaMalloc(p, y.co * 4) != cudaSuccess) st = XF_ERR_NOMEM;
-    if (!st && (cudaMalloc(&y.w16, y.nw * 2) != cudaSuccess || cudaMalloc(&y.wt16, y.nw * 2) != cudaSuccess ||
-                cudaMalloc(&y.w16t, y.nw * 2) != cudaSuccess || cudaMalloc(&y.wt16t, y.nw * 2) != cudaSuccess))
+    u->nparam += y.nw + y.co;
+  }
+  for (float*& p : u->slab) {
+    if (!st && cudaMalloc(&p, u->nparam * 4) != cudaSuccess) st = XF_ERR_NOMEM;
+    if (!st) cudaMemsetAsync(p, 0, u->nparam * 4, ctx->stream);
+  }
+  int64_t at = 0;
+  for (int k = 0; k < NLAYER && !st; k++) {
+    Layer& y = u->ly[k];
+    float** pw[] = {&y.w, &y.gw, &y.mw, &y.vw};
+    float** pb[] = {&y.b, &y.gb, &y.mb, &y.vb};
+    for (int q = 0; q < 4; q++) {
+      *pw[q] = u->slab[q] + at;
+      *pb[q] = u->slab[q] + at + y.nw;
+    }
+    at += y.nw + y.co;
+    if (!st && (cudaMalloc(&y.w16t, y.nw * 2) != cudaSuccess || cudaMalloc(&y.wt16t, y.nw * 2) != cudaSuccess))
       st = XF_ERR_NOMEM;
     if (!st) {
-      cudaMemsetAsync(y.w, 0, y.nw * 4, ctx->stream); cudaMemsetAsync(y.gw, 0, y.nw * 4, ctx->stream);
-      cudaMemsetAsync(y.mw, 0, y.nw * 4, ctx->stream); cudaMemsetAsync(y.vw, 0, y.nw * 4, ctx->stream);
-      cudaMemsetAsync(y.b, 0, y.co * 4, ctx->stream); cudaMemsetAsync(y.gb, 0, y.co * 4, ctx->stream);
-      cudaMemsetAsync(y.mb, 0, y.co * 4, ctx->stream); cudaMemsetAsync(y.vb, 0, y.co * 4, ctx->stream);
-      cudaMemsetAsync(y.w16, 0, y.nw * 2, ctx->stream); cudaMemsetAsync(y.wt16, 0, y.nw * 2, ctx->stream);
       cudaMemsetAsync(y.w16t, 0, y.nw * 2, ctx->stream); cudaMemsetAsync(y.wt16t, 0, y.nw * 2, ctx->stream);
     }
   }
-  if (!st && (cudaMalloc(&u->zout, u->L[0].n * 4) != cudaSuccess ||
-              cudaMalloc(&u->gsum, u->L[0].n * 16 * 4) != cudaSuccess ||
-              cudaMalloc(&u->gsum1, u->L[1].n * 32 * 4) != cudaSuccess || cudaMalloc(&u->red, 8 * 8) != cudaSuccess ||
+  if (!st && (cudaMalloc(&u->zout, u->L[0].n * 4) != cudaSuccess || cudaMalloc(&u->red, 8 * 8) != cudaSuccess ||
               cudaMalloc(&u->zd, u->L[0].n * 8) != cudaSuccess || cudaMalloc(&u->az, u->L[0].n * 8) != cudaSuccess))
     st = XF_ERR_NOMEM;
   if (!st) {   // partial buffers of the deterministic reductions
-    int64_t wneed = 1;
+    int64_t need = 0, at[NLAYER][2];
     for (int k = 0; k < NLAYER; k++) {
-      int mt, sp, stg;
-      int64_t need;
-      xf_wgrad_tc_plan(ctx, u->L[LLEV[k]].n, u->ly[k].ci, u->ly[k].co, &mt, &sp, &stg, &need);
-      if (need > wneed) wneed = need;
+      Layer& y = u->ly[k];
+      WgSeg& g = u->segs.s[k];
+      const int64_t n = u->L[LLEV[k]].n;
+      int stages, chunk;
+      int64_t wf;
+      xf_wgrad_tc_plan(ctx, n, y.ci, y.co, &g.mtiles, &g.splits, &stages, &wf);
+      xf_bgrad_plan(n, &g.nchunk, &chunk);
+      g.taps = 128 / y.ci; g.ci = y.ci; g.co = y.co; g.gw = y.gw; g.gb = y.gb;
+      g.block0 = u->sum_blocks;
+      u->sum_blocks += xf_grad_sum_blocks(y.ci, y.co);
+      at[k][0] = need;
+      at[k][1] = need + wf;
+      need += wf + (int64_t)g.nchunk * y.co;   // wf is a multiple of 4: the rows stay 16-byte aligned
+      need = (need + 3) & ~(int64_t)3;
     }
     if (cudaMalloc(&u->rpart, 2 * RP_MAX * 8) != cudaSuccess || cudaMalloc(&u->rtick, 4 * 4) != cudaSuccess ||
-        cudaMalloc(&u->wpart, wneed * 4) != cudaSuccess || cudaMalloc(&u->bpart, WG_MAX_CHUNKS * 64 * 4) != cudaSuccess)
+        cudaMalloc(&u->gpart, need * 4) != cudaSuccess)
       st = XF_ERR_NOMEM;
-    else
+    else {
       cudaMemsetAsync(u->rtick, 0, 4 * 4, ctx->stream);
+      for (int k = 0; k < NLAYER; k++) {
+        u->segs.s[k].wpart = u->gpart + at[k][0];
+        u->segs.s[k].bpart = u->gpart + at[k][1];
+      }
+    }
   }
   if (!st) {
     cudaMemsetAsync(u->zout, 0, u->L[0].n * 4, ctx->stream);
-    cudaMemsetAsync(u->gsum, 0, u->L[0].n * 16 * 4, ctx->stream);
-    cudaMemsetAsync(u->gsum1, 0, u->L[1].n * 32 * 4, ctx->stream);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) st = XF_ERR_CUDA;
   }
   for (int l = 0; l < 3 && !st; l++) {
@@ -581,9 +601,7 @@ extern "C" int xf_unet_create(const xf_grid* g, xf_unet** out) {
 
 extern "C" int xf_unet_param_count(const xf_unet* u, int64_t* n) {
   if (!u || !n) return XF_ERR_ARG;
-  int64_t s = 0;
-  for (const Layer& y : u->ly) s += y.nw + y.co;
-  *n = s;
+  *n = u->nparam;
   return XF_OK;
 }
 
@@ -594,29 +612,27 @@ static int params_io(xf_unet* u, float* host, int which, bool upload) {
   xf_ctx* ctx = u->ctx;
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
   XF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  float* dev = u->slab[which == 0 ? 0 : 1];
+  if (!upload) {   // one copy (22 by layer took 200 us)
+    XF_CUDA(ctx, cudaMemcpy(host, dev, u->nparam * 4, cudaMemcpyDeviceToHost));
+    return XF_OK;
+  }
+  std::vector<float> h(host, host + u->nparam);
   int64_t o = 0;
   for (int k = 0; k < NLAYER; k++) {
-    Layer& y = u->ly[k];
-    float* w = which == 0 ? y.w : y.gw;
-    float* b = which == 0 ? y.b : y.gb;
-    if (upload) {
-      std::vector<float> hw(host + o, host + o + y.nw), hb(host + o + y.nw, host + o + y.nw + y.co);
-      for (int t = 0; t < 27; t++)
-        for (int co = 0; co < y.co; co++)
-          for (int ci = 0; ci < y.ci; ci++)
-            if ((k == ENC0A && ci > 0) || (k == OUTL && co > 0)) hw[((size_t)t * y.co + co) * y.ci + ci] = 0.f;
-      if (k == OUTL)
-        for (int co = 1; co < y.co; co++) hb[co] = 0.f;
-      XF_CUDA(ctx, cudaMemcpy(w, hw.data(), y.nw * 4, cudaMemcpyHostToDevice));
-      XF_CUDA(ctx, cudaMemcpy(b, hb.data(), y.co * 4, cudaMemcpyHostToDevice));
-      if (which == 0)
-        k_weights_bf16<<<ublocks(ctx, y.nw), 256, 0, ctx->stream>>>(y.w, y.co, y.ci, y.w16, y.wt16, y.w16t, y.wt16t);
-    } else {
-      XF_CUDA(ctx, cudaMemcpy(host + o, w, y.nw * 4, cudaMemcpyDeviceToHost));
-      XF_CUDA(ctx, cudaMemcpy(host + o + y.nw, b, y.co * 4, cudaMemcpyDeviceToHost));
-    }
+    const Layer& y = u->ly[k];
+    for (int t = 0; t < 27; t++)
+      for (int co = 0; co < y.co; co++)
+        for (int ci = 0; ci < y.ci; ci++)
+          if ((k == ENC0A && ci > 0) || (k == OUTL && co > 0)) h[o + ((int64_t)t * y.co + co) * y.ci + ci] = 0.f;
+    if (k == OUTL)
+      for (int co = 1; co < y.co; co++) h[o + y.nw + co] = 0.f;
     o += y.nw + y.co;
   }
+  XF_CUDA(ctx, cudaMemcpy(dev, h.data(), u->nparam * 4, cudaMemcpyHostToDevice));
+  if (which == 0)
+    for (const Layer& y : u->ly)
+      k_weights_bf16<<<(unsigned)((y.nw + 255) / 256), 256, 0, ctx->stream>>>(y.w, y.co, y.ci, y.w16t, y.wt16t);
   XF_CUDA(ctx, cudaGetLastError());
   XF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return XF_OK;
@@ -625,10 +641,7 @@ static int params_io(xf_unet* u, float* host, int which, bool upload) {
 extern "C" int xf_unet_set_params(xf_unet* u, const float* host) {
   if (!u || !host) return XF_ERR_ARG;
   u->step = 0;
-  for (Layer& y : u->ly) {   // a new parameter set restarts Adam
-    cudaMemsetAsync(y.mw, 0, y.nw * 4, u->ctx->stream); cudaMemsetAsync(y.vw, 0, y.nw * 4, u->ctx->stream);
-    cudaMemsetAsync(y.mb, 0, y.co * 4, u->ctx->stream); cudaMemsetAsync(y.vb, 0, y.co * 4, u->ctx->stream);
-  }
+  for (int q = 2; q < 4; q++) cudaMemsetAsync(u->slab[q], 0, u->nparam * 4, u->ctx->stream);   // Adam restarts
   return params_io(u, const_cast<float*>(host), 0, true);
 }
 extern "C" int xf_unet_get_params(xf_unet* u, float* host) {
@@ -648,7 +661,7 @@ extern "C" int xf_unet_get_grads(xf_unet* u, float* host) {
 static int conv(xf_unet* u, int k, const Act& in, int in_c0, void* out, int64_t out_pitch, int out_ch, int out_fp32) {
   const Layer& y = u->ly[k];
   const Level& L = u->L[LLEV[k]];
-  return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, in.ch(u->L, in_c0), in.ps(), y.ci, y.w16, y.w16t, y.b, y.co, L.mask,
+  return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, in.ch(u->L, in_c0), in.ps(), y.ci, y.w16t, y.b, y.co, L.mask,
                         out, out_pitch, out_ch, out_fp32, LRELU[k], nullptr, 0);
 }
 // Input gradient of layer k from its pre-activation gradient g: the convolution
@@ -657,53 +670,50 @@ static int conv(xf_unet* u, int k, const Act& in, int in_c0, void* out, int64_t 
 static int dgrad(xf_unet* u, int k, const Act& g, const Act& out, int out_c0, const Act* gate, int gate_c0) {
   const Layer& y = u->ly[k];
   const Level& L = u->L[LLEV[k]];
-  return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, g.p0(u->L), g.ps(), y.co, y.wt16, y.wt16t, nullptr, y.ci, L.mask,
+  return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, g.p0(u->L), g.ps(), y.co, y.wt16t, nullptr, y.ci, L.mask,
                         out.ch(u->L, out_c0), out.ps(), y.ci, 0, 0,
                         gate ? (const void*)gate->ch(u->L, gate_c0) : nullptr, gate ? gate->ps() : 0);
 }
-// Weight and bias gradients of layer k from its pre-activation gradient g and
-// its input x (from channel x_c0 on): the weights on the tensor cores.
+// Weight- and bias-gradient partials of layer k from its pre-activation
+// gradient g and its input x (from channel x_c0 on): the weights on the tensor
+// cores.
 static int wgrad(xf_unet* u, int k, const Act& g, const Act& x, int x_c0) {
   const Layer& y = u->ly[k];
   const Level& L = u->L[LLEV[k]];
-  const int st = xf_wgrad_tc(u->ctx, L.n1, L.n2, L.n3, g.p0(u->L), g.ps(), y.co, x.ch(u->L, x_c0), x.ps(), y.ci,
-                             u->wpart, y.gw);
-  if (st) return st;
-  const int64_t chunk = wg_chunk(L.n);
-  const int nchunk = (int)((L.n + chunk - 1) / chunk);
-  k_bgrad<<<dim3((unsigned)nchunk, (unsigned)(y.co / 8)), 256, 0, u->ctx->stream>>>(g.p0(u->L), g.ps(), L.n,
-                                                                                    (int)chunk, y.co, u->bpart);
-  k_bgrad_sum<<<1, 64, 0, u->ctx->stream>>>(u->bpart, nchunk, y.co, y.gb);
-  return XF_OK;
+  const WgSeg& sg = u->segs.s[k];
+  return xf_wgrad_tc(u->ctx, L.n1, L.n2, L.n3, g.p0(u->L), g.ps(), y.co, x.ch(u->L, x_c0), x.ps(), y.ci,
+                     const_cast<float*>(sg.wpart), const_cast<float*>(sg.bpart));
 }
+// The elementwise kernels' grid: a cell a thread, `planes` rows of blocks.
+static dim3 cell_grid(int64_t n, int planes) { return dim3((unsigned)((n + 255) / 256), (unsigned)planes); }
 
 // Kernels one forward pass launches, with xf_unet_apply_dev's output conversion.
 constexpr int UNET_FORWARD_LAUNCHES = 18;
-static int forward(xf_unet* u, const double* r) {
+static int forward(xf_unet* u, const double* r, bool have_rms = false) {
   xf_ctx* ctx = u->ctx;
   cudaStream_t s = ctx->stream;
   const Level* L = u->L;
   int st;
-  XF_CUDA(ctx, cudaMemsetAsync(u->red, 0, 8 * 8, s));
-  k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, u->red, 0, u->rpart, u->rtick);
-  k_unet_input<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, u->red, (double)L[0].active,
-                                                    u->X0.p0(L), u->X0.ps());
+  if (!have_rms)
+    k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, (double)L[0].active, u->red, 0, u->rpart,
+                                                      u->rtick);
+  k_unet_input<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, u->red, u->X0.p0(L));
   if ((st = conv(u, ENC0A, u->X0, 0, u->A0.p0(L), u->A0.ps(), 16, 0))) return st;
   if ((st = conv(u, ENC0B, u->A0, 0, u->CAT0.ch(L, 32), u->CAT0.ps(), 16, 0))) return st;   // S0
-  k_pool<<<ublocks(ctx, L[1].n * 2), 256, 0, s>>>(u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].n2, L[0].n3, u->P1.p0(L),
-                                                  u->P1.ps(), L[1].mask, L[1].n1, L[1].n2, L[1].n3, 16);
+  k_pool<<<cell_grid(L[1].n, 2), 256, 0, s>>>(u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].n2, L[0].n3, u->P1.p0(L),
+                                                  u->P1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
   if ((st = conv(u, ENC1A, u->P1, 0, u->A1.p0(L), u->A1.ps(), 32, 0))) return st;
   if ((st = conv(u, ENC1B, u->A1, 0, u->CAT1.ch(L, 64), u->CAT1.ps(), 32, 0))) return st;   // S1
-  k_pool<<<ublocks(ctx, L[2].n * 4), 256, 0, s>>>(u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].n2, L[1].n3, u->P2.p0(L),
-                                                  u->P2.ps(), L[2].mask, L[2].n1, L[2].n2, L[2].n3, 32);
+  k_pool<<<cell_grid(L[2].n, 4), 256, 0, s>>>(u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].n2, L[1].n3, u->P2.p0(L),
+                                                  u->P2.ps(), L[2].mask, (unsigned)L[2].n, L[2].n2, L[2].n3);
   if ((st = conv(u, MIDA, u->P2, 0, u->M2a.p0(L), u->M2a.ps(), 64, 0))) return st;
   if ((st = conv(u, MIDB, u->M2a, 0, u->M2b.p0(L), u->M2b.ps(), 64, 0))) return st;
-  k_upsample<<<ublocks(ctx, L[1].n * 8), 256, 0, s>>>(u->M2b.p0(L), u->M2b.ps(), L[2].n2, L[2].n3, u->CAT1.p0(L),
-                                                       u->CAT1.ps(), L[1].mask, L[1].n1, L[1].n2, L[1].n3, 64);
+  k_upsample<<<cell_grid(L[1].n, 2), 256, 0, s>>>(u->M2b.p0(L), u->M2b.ps(), L[2].n2, L[2].n3, u->CAT1.p0(L),
+                                                       u->CAT1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
   if ((st = conv(u, DEC1A, u->CAT1, 0, u->D1a.p0(L), u->D1a.ps(), 32, 0))) return st;
   if ((st = conv(u, DEC1B, u->D1a, 0, u->D1b.p0(L), u->D1b.ps(), 32, 0))) return st;
-  k_upsample<<<ublocks(ctx, L[0].n * 4), 256, 0, s>>>(u->D1b.p0(L), u->D1b.ps(), L[1].n2, L[1].n3, u->CAT0.p0(L),
-                                                       u->CAT0.ps(), L[0].mask, L[0].n1, L[0].n2, L[0].n3, 32);
+  k_upsample<<<cell_grid(L[0].n, 1), 256, 0, s>>>(u->D1b.p0(L), u->D1b.ps(), L[1].n2, L[1].n3, u->CAT0.p0(L),
+                                                       u->CAT0.ps(), L[0].mask, (unsigned)L[0].n, L[0].n2, L[0].n3);
   if ((st = conv(u, DEC0A, u->CAT0, 0, u->D0a.p0(L), u->D0a.ps(), 16, 0))) return st;
   if ((st = conv(u, DEC0B, u->D0a, 0, u->D0b.p0(L), u->D0b.ps(), 16, 0))) return st;
   if ((st = conv(u, OUTL, u->D0b, 0, u->zout, 1, 1, 1))) return st;
@@ -712,7 +722,7 @@ static int forward(xf_unet* u, const double* r) {
 }
 
 // Backward pass from the loss against the target e (FP64 box): weight and
-// bias gradients accumulate into gw / gb.
+// bias gradients into gw / gb.
 static int backward(xf_unet* u, const double* r, const double* e, const xf_op* op) {
   xf_ctx* ctx = u->ctx;
   cudaStream_t s = ctx->stream;
@@ -723,13 +733,13 @@ static int backward(xf_unet* u, const double* r, const double* e, const xf_op* o
     MvReq<double> m;
     m.x = u->zd; m.y = u->az; m.zero_inactive = 1;
     xf_mv64(op, m);
-    xf_dot_async(u->g, XF_F64, u->zd, r, 10);
-    xf_dot_async(u->g, XF_F64, u->zd, u->az, 11);
-    xf_dot_async(u->g, XF_F64, e, r, 12);
-    k_anorm_grad<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, u->az, L[0].mask, L[0].n, ctx->scratch, u->red,
-                                                      u->G0_16a.p0(L), u->G0_16a.ps());
+    k_anorm_dots<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(u->zout, u->az, r, e, L[0].mask, L[0].n, ctx->scratch,
+                                                           u->red);
+    k_anorm_grad<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, u->az, L[0].mask, L[0].n, ctx->scratch, u->G0_16a.p0(L),
+                                                      u->G0_16a.ps());
   } else {
-    k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(e, L[0].mask, L[0].n, u->red, 1, u->rpart, u->rtick);
+    k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(e, L[0].mask, L[0].n, (double)L[0].active, u->red, 1, u->rpart,
+                                                      u->rtick);
     k_unet_loss<<<ublocks(ctx, L[0].n), 256, 0, s>>>(u->zout, e, L[0].mask, L[0].n, (double)L[0].active, u->red,
                                                      u->G0_16a.p0(L), u->G0_16a.ps());
   }
@@ -741,39 +751,36 @@ static int backward(xf_unet* u, const double* r, const double* e, const xf_op* o
   if ((st = wgrad(u, DEC0A, u->G0_16a, u->CAT0, 0))) return st;
   if ((st = dgrad(u, DEC0A, u->G0_16a, u->G0_48, 0, nullptr, 0))) return st;
   // up(D1b) part -> dec1b's pre-activation gradient
-  k_upsample_bwd<<<ublocks(ctx, L[1].n * 32), 256, 0, s>>>(u->G0_48.p0(L), u->G0_48.ps(), L[0].n2, L[0].n3,
-                                                           u->D1b.p0(L), u->D1b.ps(), L[1].mask, L[1].n1, L[1].n2,
-                                                           L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps(), 32);
+  k_upsample_bwd<<<cell_grid(L[1].n, 4), 256, 0, s>>>(u->G0_48.p0(L), u->G0_48.ps(), L[0].n2, L[0].n3,
+                                                           u->D1b.p0(L), u->D1b.ps(), L[1].mask, (unsigned)L[1].n,
+                                                       L[1].n2, L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps());
   if ((st = wgrad(u, DEC1B, u->G1_32a, u->D1a, 0))) return st;
   if ((st = dgrad(u, DEC1B, u->G1_32a, u->G1_32b, 0, &u->D1a, 0))) return st;
   if ((st = wgrad(u, DEC1A, u->G1_32b, u->CAT1, 0))) return st;
   if ((st = dgrad(u, DEC1A, u->G1_32b, u->G1_96, 0, nullptr, 0))) return st;
   // up(M2b) part -> mid_b
-  k_upsample_bwd<<<ublocks(ctx, L[2].n * 64), 256, 0, s>>>(u->G1_96.p0(L), u->G1_96.ps(), L[1].n2, L[1].n3,
-                                                           u->M2b.p0(L), u->M2b.ps(), L[2].mask, L[2].n1, L[2].n2,
-                                                           L[2].n3, u->G2_64a.p0(L), u->G2_64a.ps(), 64);
+  k_upsample_bwd<<<cell_grid(L[2].n, 8), 256, 0, s>>>(u->G1_96.p0(L), u->G1_96.ps(), L[1].n2, L[1].n3,
+                                                           u->M2b.p0(L), u->M2b.ps(), L[2].mask, (unsigned)L[2].n,
+                                                       L[2].n2, L[2].n3, u->G2_64a.p0(L), u->G2_64a.ps());
   if ((st = wgrad(u, MIDB, u->G2_64a, u->M2a, 0))) return st;
   if ((st = dgrad(u, MIDB, u->G2_64a, u->G2_64b, 0, &u->M2a, 0))) return st;
   if ((st = wgrad(u, MIDA, u->G2_64b, u->P2, 0))) return st;
   if ((st = dgrad(u, MIDA, u->G2_64b, u->G2_32, 0, nullptr, 0))) return st;
-  k_pool_bwd<<<ublocks(ctx, L[1].n * 32), 256, 0, s>>>(u->G2_32.p0(L), u->G2_32.ps(), L[2].n2, L[2].n3, L[1].mask,
-                                                       L[1].n1, L[1].n2, L[1].n3, u->gsum1, 32, 32);
   // S1 = enc1b output: skip gradient + pooled path
-  k_skip_grad<<<ublocks(ctx, L[1].n * 32), 256, 0, s>>>(u->G1_96.ch(L, 64), u->G1_96.ps(), u->gsum1, 32,
-                                                        u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].mask, L[1].n,
-                                                        u->G1_32a.p0(L), u->G1_32a.ps(), 32);
+  k_skip_grad<<<cell_grid(L[1].n, 4), 256, 0, s>>>(u->G1_96.ch(L, 64), u->G1_96.ps(), u->G2_32.p0(L), u->G2_32.ps(),
+                                                    L[2].n2, L[2].n3, u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].mask,
+                                                    (unsigned)L[1].n, L[1].n2, L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps());
   if ((st = wgrad(u, ENC1B, u->G1_32a, u->A1, 0))) return st;
   if ((st = dgrad(u, ENC1B, u->G1_32a, u->G1_32b, 0, &u->A1, 0))) return st;
   if ((st = wgrad(u, ENC1A, u->G1_32b, u->P1, 0))) return st;
   if ((st = dgrad(u, ENC1A, u->G1_32b, u->G1_16, 0, nullptr, 0))) return st;
-  k_pool_bwd<<<ublocks(ctx, L[0].n * 16), 256, 0, s>>>(u->G1_16.p0(L), u->G1_16.ps(), L[1].n2, L[1].n3, L[0].mask,
-                                                       L[0].n1, L[0].n2, L[0].n3, u->gsum, 16, 16);
-  k_skip_grad<<<ublocks(ctx, L[0].n * 16), 256, 0, s>>>(u->G0_48.ch(L, 32), u->G0_48.ps(), u->gsum, 16,
-                                                        u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].mask, L[0].n,
-                                                        u->G0_16a.p0(L), u->G0_16a.ps(), 16);
+  k_skip_grad<<<cell_grid(L[0].n, 2), 256, 0, s>>>(u->G0_48.ch(L, 32), u->G0_48.ps(), u->G1_16.p0(L), u->G1_16.ps(),
+                                                    L[1].n2, L[1].n3, u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].mask,
+                                                    (unsigned)L[0].n, L[0].n2, L[0].n3, u->G0_16a.p0(L), u->G0_16a.ps());
   if ((st = wgrad(u, ENC0B, u->G0_16a, u->A0, 0))) return st;
   if ((st = dgrad(u, ENC0B, u->G0_16a, u->G0_16b, 0, &u->A0, 0))) return st;
   if ((st = wgrad(u, ENC0A, u->G0_16b, u->X0, 0))) return st;
+  xf_grad_sum(ctx, u->segs, u->sum_blocks);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }
@@ -813,21 +820,20 @@ extern "C" int xf_unet_train_step(xf_unet* u, const xf_op* op, const xf_vec* r, 
   xf_ctx* ctx = u->ctx;
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  for (Layer& y : u->ly) {
-    XF_CUDA(ctx, cudaMemsetAsync(y.gw, 0, y.nw * 4, s));
-    XF_CUDA(ctx, cudaMemsetAsync(y.gb, 0, y.co * 4, s));
-  }
   if ((st = forward(u, (const double*)r->data))) return st;
   if ((st = backward(u, (const double*)r->data, (const double*)e->data, op))) return st;
   if (apply_update) {
     u->step++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)u->step), c2 = 1.f - powf(b2, (float)u->step);
-    for (Layer& y : u->ly) {
-      k_adam<<<ublocks(ctx, y.nw), 256, 0, s>>>(y.w, y.gw, y.mw, y.vw, y.nw, (float)lr, b1, b2, 1e-8f, c1, c2, 0);
-      k_adam<<<1, 256, 0, s>>>(y.b, y.gb, y.mb, y.vb, y.co, (float)lr, b1, b2, 1e-8f, c1, c2, 0);
-      k_weights_bf16<<<ublocks(ctx, y.nw), 256, 0, s>>>(y.w, y.co, y.ci, y.w16, y.wt16, y.w16t, y.wt16t);
+    AdamSegs segs;
+    int blocks = 0;
+    for (int k = 0; k < NLAYER; k++) {
+      const Layer& y = u->ly[k];
+      segs.s[k] = {y.w, y.gw, y.mw, y.vw, y.b, y.gb, y.mb, y.vb, y.w16t, y.wt16t, y.ci, y.co, blocks};
+      blocks += (int)(y.nw / 256) + 1;   // nw is a multiple of 256
     }
+    k_adam<<<blocks, 256, 0, s>>>(segs, (float)lr, b1, b2, 1e-8f, c1, c2);
   }
   XF_CUDA(ctx, cudaGetLastError());
   if (loss) {
@@ -927,31 +933,39 @@ __global__ void k_twolevel_z(const T* __restrict__ y, const float* __restrict__ 
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
     z[c] = smask[c] ? (T)(om * (double)y[c] + sc * (double)w[c]) : (T)0;
 }
-// The F = 4 transfers of the mixed path.  Restriction: one thread per coarse
-// cell, its 64 loads unrolled (a warp reads 32 consecutive runs of 4 floats).
-// Prolongation: 2-D grid over (j, k) plane positions and i planes, 32-bit
-// index arithmetic.
-__global__ void k_restrict4(const float* __restrict__ r, int f2, int f3, double* __restrict__ rc, int c1, int c2,
-                            int c3) {
-  const int K = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y, I = blockIdx.z;
-  if (K >= c3) return;
-  double v = 0.0;
-  if (I > 0 && I < c1 - 1 && J > 0 && J < c2 - 1 && K > 0 && K < c3 - 1) {
-    const int64_t base = ((int64_t)(1 + 4 * (I - 1)) * f2 + (1 + 4 * (J - 1))) * f3 + (1 + 4 * (K - 1));
-    float part[4];
+// The restriction of the mixed path, F = 4, with the network's 1 / rms of its
+// result (sumsq_finish): one thread a coarse cell, its 16 runs of 4 floats by
+// a float2 and two floats (rows have an even length and blocks start at an odd
+// cell).
+__global__ void __launch_bounds__(256) k_restrict4(const float* __restrict__ r, int f2, int f3, double* __restrict__ rc,
+                                                   int c1, int c2, int c3, const uint8_t* __restrict__ m, double count,
+                                                   double* red, double* part, unsigned* tick) {
+  const unsigned n = (unsigned)c1 * c2 * c3;
+  double s = 0;
+  for (unsigned c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
+    const unsigned t = c / (unsigned)c3, I = t / (unsigned)c2;
+    const int K = (int)(c - t * c3), J = (int)(t - I * c2);
+    double v = 0.0;
+    if (I > 0 && (int)I < c1 - 1 && J > 0 && J < c2 - 1 && K > 0 && K < c3 - 1) {
+      const int64_t base = ((int64_t)(1 + 4 * ((int)I - 1)) * f2 + (1 + 4 * (J - 1))) * f3 + (1 + 4 * (K - 1));
+      float p[4];
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      float sa = 0.f;
+      for (int a = 0; a < 4; a++) {
+        float sa = 0.f;
 #pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const float* row = r + base + ((int64_t)a * f2 + b) * f3;
-        sa += (__ldg(row) + __ldg(row + 1)) + (__ldg(row + 2) + __ldg(row + 3));
+        for (int b = 0; b < 4; b++) {
+          const float* row = r + base + ((int64_t)a * f2 + b) * f3;
+          const float2 mid = __ldg(reinterpret_cast<const float2*>(row + 1));
+          sa += (__ldg(row) + mid.x) + (mid.y + __ldg(row + 3));
+        }
+        p[a] = sa;
       }
-      part[a] = sa;
+      v = ((double)p[0] + (double)p[1]) + ((double)p[2] + (double)p[3]);
     }
-    v = ((double)part[0] + (double)part[1]) + ((double)part[2] + (double)part[3]);
+    rc[c] = v;
+    if (m[c]) s = fma(v, v, s);
   }
-  rc[((int64_t)I * c2 + J) * c3 + K] = v;
+  sumsq_finish(s, red, 0, count, part, tick);
 }
 // (a, b) of FP32 boxes that are zero off the active set: exact products
 // accumulated in float-float per thread and per warp, FP64 across warps and
@@ -1364,12 +1378,13 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     // network on: z = M r with (z, r) and (z, q_newest)
     begin(body[TL_ON], nullptr, 0);
     if (f4)
-      k_restrict4<<<dim3((cg->n3 + 63) / 64, cg->n2, cg->n1), 64, 0, s>>>(r, g->n2, g->n3, rc, cg->n1, cg->n2, cg->n3);
+      k_restrict4<<<sumsq_blocks(ctx, nc), 256, 0, s>>>(r, g->n2, g->n3, rc, cg->n1, cg->n2, cg->n3, u->L[0].mask,
+                                                        (double)u->L[0].active, u->red, u->rpart, u->rtick);
     else
       k_restrict_blocks<float><<<grid_blocks(ctx, nc, 256), 256, 0, s>>>(r, g->n2, g->n3, F, rc, cg->n1, cg->n2,
                                                                          cg->n3);
     if (f4) {   // omega on the coarse grid, r - omega A P zc in one pass; zc is the network's FP32 output
-      if (ce == cudaSuccess && (rcode = forward(u, rc))) ce = cudaErrorUnknown;
+      if (ce == cudaSuccess && (rcode = forward(u, rc, true))) ce = cudaErrorUnknown;
       xf_tl_omega(g, cg, u->zout, faces, rc, FS_YAY, FS_OM);
       xf_tl_sub(g, r, u->zout, cg->n2, cg->n3, FS_OM, w1);
     } else {        // y = P zc, A y with (y, A y), (y, r) = (zc, P^T r)
@@ -1393,8 +1408,8 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     win_dots(hd, 1);
     if (m > 1) k_tl_coef<<<1, 32, 0, s>>>(S, c, hd, m);
     end_tail(tail);
-    // F = 4: no output conversion of the network
-    n_on = (f4 ? 3 - 1 : 5) + UNET_FORWARD_LAUNCHES + tl_nf + (m > 1 ? m : 0);
+    // F = 4: no sum of squares and no output conversion of the network's own
+    n_on = (f4 ? 3 - 2 : 5) + UNET_FORWARD_LAUNCHES + tl_nf + (m > 1 ? m : 0);
     cudaGraph_t fbody = nullptr;
     cudaGraphNode_t fnode = nullptr;
     add_cond(body[TL_ON], tail, H.fb[hd], cudaGraphCondTypeIf, 1, &fbody, &fnode);
