@@ -137,6 +137,24 @@ int xf_fail(xf_ctx* ctx, int status, const char* fmt, ...);
                                           cudaGetErrorString(e_), __FILE__, __LINE__);   \
   } while (0)
 
+// Programmatic dependent launch: a kernel launched by launch_dep may start while
+// the kernel before it on the stream drains (once all its blocks have left or
+// called dep_trigger); dep_wait returns when that kernel has completed and its
+// writes are visible, and before it only data that no kernel of the chain
+// writes may be touched.  A plain launch makes both calls empty.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_dep(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);   // an error shows in cudaGetLastError
+}
+
 inline int grid_blocks(const xf_ctx* ctx, int64_t n, int threads, int per_sm = 8) {
   int64_t b = (n + threads - 1) / threads;
   int64_t cap = (int64_t)ctx->sm_count * per_sm;

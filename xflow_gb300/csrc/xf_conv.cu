@@ -368,11 +368,13 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
     return st + 126 > a.ncell ? (a.ncell > 126 ? a.ncell - 126 : (int64_t)0) : st;
   };
 
+  dep_trigger();
   if (warp == 4) {   // ---- producer: lane 0 takes the barriers, lanes 0..17 one A copy each
-    if (plan.resident && my_tiles > 0 && lane == 0) {
+    if (plan.resident && my_tiles > 0 && lane == 0) {   // weights: not written by the kernels before
       mbar_expect_tx(&wfull, plan.w_bytes);
       bulk_load(wsm, a.Wt, plan.w_bytes, &wfull);
     }
+    dep_wait();
     // this lane's copy: slab sl = lane / 2, plane q = lane % 2 (lane 18: the
     // streamed weights)
     const int sl = lane >> 1, q = lane & 1;
@@ -454,6 +456,7 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
     }
     __syncwarp();
   } else {   // ---- epilogue, warps 0-3
+    dep_wait();
     for (int k = 0; k < my_tiles; k++) {
       const int acc = k & 1;
       const bool got = bk_wait(&tfull[acc], (uint32_t)((k >> 1) & 1), abort_p);
@@ -573,7 +576,9 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_wide(ConvArgs a, WdPlan pl
   const int64_t P = (int64_t)a.n2 * a.n3;
   const int64_t ntiles = (a.ncell + TC_M - 1) / TC_M;
   const int my_tiles = ntiles > blockIdx.x ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+  dep_trigger();
   if (warp == 4) {   // ---- producer: a plane of A per lane (at most 16), the weights by lane 16
+    dep_wait();
     int st = 0, pass = 0, issued = 0;
     bool ok = true;
     for (int k = 0; k < my_tiles && ok; k++) {
@@ -641,6 +646,7 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_wide(ConvArgs a, WdPlan pl
     bk_wait_warp(&mdone, 0, abort_p, false);
     __syncwarp();
   } else {   // ---- epilogue, warps 0-3: TMEM lanes 32 w .. 32 w + 31
+    dep_wait();
     for (int k = 0; k < my_tiles; k++) {
       const int acc = k & 1;
       const bool got = bk_wait(&tfull[acc], (uint32_t)((k >> 1) & 1), abort_p);
@@ -957,10 +963,11 @@ int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps,
 
 // Launch on the context stream (arguments checked by the caller).  `weights`
 // is [27][co][ci]; `tiled` the same in the tiled order (needed when 3 co <= 256).
-// `tiled`: the weights in conv_tiled_index order.
+// `tiled`: the weights in conv_tiled_index order.  dep: launched by launch_dep,
+// the weights not written by the kernel before.
 int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* tiled,
                    const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch, int out_ch,
-                   int out_fp32, int relu, const void* gate, int64_t gate_ps) {
+                   int out_fp32, int relu, const void* gate, int64_t gate_ps, bool dep) {
   ConvArgs a;
   a.gate = (const uint16_t*)gate; a.gate_ps = gate_ps;
   a.in = (const uint16_t*)in; a.in_ps = in_ps; a.Ci = ci;
@@ -976,7 +983,8 @@ int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t 
     XF_CUDA(ctx, set_max_smem((const void*)k_conv3_wide, 2, ctx->device, (size_t)plan.smem_bytes));
     const int64_t tiles = (a.ncell + TC_M - 1) / TC_M;
     const int64_t blocks = std::min(tiles, (int64_t)ctx->sm_count * plan.per_sm);
-    k_conv3_wide<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
+    if (dep) launch_dep(k_conv3_wide, dim3((unsigned)blocks), BK_THREADS, plan.smem_bytes, ctx->stream, a, plan);
+    else k_conv3_wide<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
     XF_CUDA(ctx, cudaGetLastError());
     return XF_OK;
   }
@@ -993,7 +1001,8 @@ int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t 
   const int64_t tiles = (a.ncell + 125) / 126;
   int64_t blocks = (int64_t)ctx->sm_count * plan.per_sm;
   if (blocks > tiles) blocks = tiles;
-  k_conv3_bulk<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
+  if (dep) launch_dep(k_conv3_bulk, dim3((unsigned)blocks), BK_THREADS, plan.smem_bytes, ctx->stream, a, plan);
+  else k_conv3_bulk<<<(int)blocks, BK_THREADS, plan.smem_bytes, ctx->stream>>>(a, plan);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }
@@ -1027,7 +1036,7 @@ extern "C" int xf_conv3d_bf16(xf_ctx* ctx, int n1, int n2, int n3, const void* i
   k_tile_weights<<<(unsigned)((nw + 255) / 256), 256, 0, ctx->stream>>>((const uint16_t*)weights, co, ci,
                                                                         (uint16_t*)tiled);
   const int st = xf_conv_launch(ctx, n1, n2, n3, in, in_ps, ci, tiled, bias, co, mask, out, out_pitch,
-                                out_ch, out_fp32, relu, nullptr, 0);
+                                out_ch, out_fp32, relu, nullptr, 0, false);
   cudaFreeAsync(tiled, ctx->stream);
   return st;
 }

@@ -29,7 +29,7 @@
 
 int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* tiled,
                    const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch, int out_ch,
-                   int out_fp32, int relu, const void* gate, int64_t gate_ps);
+                   int out_fp32, int relu, const void* gate, int64_t gate_ps, bool dep);
 void xf_mv64(const xf_op* op, const MvReq<double>& q);
 void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mtiles, int* splits, int* stages,
                       int64_t* partial_floats);
@@ -184,6 +184,8 @@ __device__ __forceinline__ void relu_gate(float (&s)[8], uint4 v) {
 // bound by their index arithmetic.
 __global__ void k_pool(const uint16_t* __restrict__ src, int64_t sps, int f2, int f3, uint16_t* __restrict__ dst,
                        int64_t dps, const uint8_t* __restrict__ cmask, unsigned n, int c2, int c3) {
+  dep_trigger();
+  dep_wait();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int g = blockIdx.y;
@@ -211,6 +213,8 @@ __device__ __forceinline__ int64_t parent(unsigned c, int f2, int f3, int c2, in
 // four planes a thread.
 __global__ void k_upsample(const uint16_t* __restrict__ src, int64_t sps, int c2, int c3, uint16_t* __restrict__ dst,
                            int64_t dps, const uint8_t* __restrict__ fmask, unsigned n, int f2, int f3) {
+  dep_trigger();
+  dep_wait();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   uint4 v[4] = {};
@@ -229,6 +233,8 @@ __global__ void k_upsample(const uint16_t* __restrict__ src, int64_t sps, int c2
 __global__ void k_upsample_bwd(const uint16_t* __restrict__ gfine, int64_t gps, int f2, int f3,
                                const uint16_t* __restrict__ gate, int64_t gtps, const uint8_t* __restrict__ cmask,
                                unsigned n, int c2, int c3, uint16_t* __restrict__ dst, int64_t dps) {
+  dep_trigger();
+  dep_wait();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int g = blockIdx.y;
@@ -253,6 +259,8 @@ __global__ void k_skip_grad(const uint16_t* __restrict__ gskip, int64_t gps, con
                             int64_t pps, int c2, int c3, const uint16_t* __restrict__ gate, int64_t gtps,
                             const uint8_t* __restrict__ mask, unsigned n, int f2, int f3, uint16_t* __restrict__ dst,
                             int64_t dps) {
+  dep_trigger();
+  dep_wait();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int g = blockIdx.y;
@@ -308,6 +316,8 @@ __global__ void __launch_bounds__(256) k_sumsq(const double* __restrict__ x, con
 // r / rms(r) into channel 0 of the first layer's input (its other channels stay 0).
 __global__ void k_unet_input(const double* __restrict__ r, const uint8_t* __restrict__ m, int64_t n,
                              const double* __restrict__ red, uint16_t* __restrict__ x0) {
+  dep_trigger();
+  dep_wait();
   const float inv = (float)red[6];
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t v = m[c] ? f2bf((float)r[c] * inv) : 0u;
@@ -662,7 +672,7 @@ static int conv(xf_unet* u, int k, const Act& in, int in_c0, void* out, int64_t 
   const Layer& y = u->ly[k];
   const Level& L = u->L[LLEV[k]];
   return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, in.ch(u->L, in_c0), in.ps(), y.ci, y.w16t, y.b, y.co, L.mask,
-                        out, out_pitch, out_ch, out_fp32, LRELU[k], nullptr, 0);
+                        out, out_pitch, out_ch, out_fp32, LRELU[k], nullptr, 0, true);
 }
 // Input gradient of layer k from its pre-activation gradient g: the convolution
 // with the flipped transposed weights, x mask, x the ReLU gate of `gate` (the
@@ -672,7 +682,7 @@ static int dgrad(xf_unet* u, int k, const Act& g, const Act& out, int out_c0, co
   const Level& L = u->L[LLEV[k]];
   return xf_conv_launch(u->ctx, L.n1, L.n2, L.n3, g.p0(u->L), g.ps(), y.co, y.wt16t, nullptr, y.ci, L.mask,
                         out.ch(u->L, out_c0), out.ps(), y.ci, 0, 0,
-                        gate ? (const void*)gate->ch(u->L, gate_c0) : nullptr, gate ? gate->ps() : 0);
+                        gate ? (const void*)gate->ch(u->L, gate_c0) : nullptr, gate ? gate->ps() : 0, true);
 }
 // Weight- and bias-gradient partials of layer k from its pre-activation
 // gradient g and its input x (from channel x_c0 on): the weights on the tensor
@@ -697,23 +707,23 @@ static int forward(xf_unet* u, const double* r, bool have_rms = false) {
   if (!have_rms)
     k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, (double)L[0].active, u->red, 0, u->rpart,
                                                       u->rtick);
-  k_unet_input<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, L[0].mask, L[0].n, u->red, u->X0.p0(L));
+  launch_dep(k_unet_input, dim3(ublocks(ctx, L[0].n)), 256, 0, s, r, L[0].mask, L[0].n, u->red, u->X0.p0(L));
   if ((st = conv(u, ENC0A, u->X0, 0, u->A0.p0(L), u->A0.ps(), 16, 0))) return st;
   if ((st = conv(u, ENC0B, u->A0, 0, u->CAT0.ch(L, 32), u->CAT0.ps(), 16, 0))) return st;   // S0
-  k_pool<<<cell_grid(L[1].n, 2), 256, 0, s>>>(u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].n2, L[0].n3, u->P1.p0(L),
-                                                  u->P1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
+  launch_dep(k_pool, cell_grid(L[1].n, 2), 256, 0, s, u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].n2, L[0].n3, u->P1.p0(L),
+             u->P1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
   if ((st = conv(u, ENC1A, u->P1, 0, u->A1.p0(L), u->A1.ps(), 32, 0))) return st;
   if ((st = conv(u, ENC1B, u->A1, 0, u->CAT1.ch(L, 64), u->CAT1.ps(), 32, 0))) return st;   // S1
-  k_pool<<<cell_grid(L[2].n, 4), 256, 0, s>>>(u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].n2, L[1].n3, u->P2.p0(L),
-                                                  u->P2.ps(), L[2].mask, (unsigned)L[2].n, L[2].n2, L[2].n3);
+  launch_dep(k_pool, cell_grid(L[2].n, 4), 256, 0, s, u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].n2, L[1].n3, u->P2.p0(L),
+             u->P2.ps(), L[2].mask, (unsigned)L[2].n, L[2].n2, L[2].n3);
   if ((st = conv(u, MIDA, u->P2, 0, u->M2a.p0(L), u->M2a.ps(), 64, 0))) return st;
   if ((st = conv(u, MIDB, u->M2a, 0, u->M2b.p0(L), u->M2b.ps(), 64, 0))) return st;
-  k_upsample<<<cell_grid(L[1].n, 2), 256, 0, s>>>(u->M2b.p0(L), u->M2b.ps(), L[2].n2, L[2].n3, u->CAT1.p0(L),
-                                                       u->CAT1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
+  launch_dep(k_upsample, cell_grid(L[1].n, 2), 256, 0, s, u->M2b.p0(L), u->M2b.ps(), L[2].n2, L[2].n3, u->CAT1.p0(L),
+             u->CAT1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3);
   if ((st = conv(u, DEC1A, u->CAT1, 0, u->D1a.p0(L), u->D1a.ps(), 32, 0))) return st;
   if ((st = conv(u, DEC1B, u->D1a, 0, u->D1b.p0(L), u->D1b.ps(), 32, 0))) return st;
-  k_upsample<<<cell_grid(L[0].n, 1), 256, 0, s>>>(u->D1b.p0(L), u->D1b.ps(), L[1].n2, L[1].n3, u->CAT0.p0(L),
-                                                       u->CAT0.ps(), L[0].mask, (unsigned)L[0].n, L[0].n2, L[0].n3);
+  launch_dep(k_upsample, cell_grid(L[0].n, 1), 256, 0, s, u->D1b.p0(L), u->D1b.ps(), L[1].n2, L[1].n3, u->CAT0.p0(L),
+             u->CAT0.ps(), L[0].mask, (unsigned)L[0].n, L[0].n2, L[0].n3);
   if ((st = conv(u, DEC0A, u->CAT0, 0, u->D0a.p0(L), u->D0a.ps(), 16, 0))) return st;
   if ((st = conv(u, DEC0B, u->D0a, 0, u->D0b.p0(L), u->D0b.ps(), 16, 0))) return st;
   if ((st = conv(u, OUTL, u->D0b, 0, u->zout, 1, 1, 1))) return st;
@@ -751,32 +761,32 @@ static int backward(xf_unet* u, const double* r, const double* e, const xf_op* o
   if ((st = wgrad(u, DEC0A, u->G0_16a, u->CAT0, 0))) return st;
   if ((st = dgrad(u, DEC0A, u->G0_16a, u->G0_48, 0, nullptr, 0))) return st;
   // up(D1b) part -> dec1b's pre-activation gradient
-  k_upsample_bwd<<<cell_grid(L[1].n, 4), 256, 0, s>>>(u->G0_48.p0(L), u->G0_48.ps(), L[0].n2, L[0].n3,
-                                                           u->D1b.p0(L), u->D1b.ps(), L[1].mask, (unsigned)L[1].n,
-                                                       L[1].n2, L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps());
+  launch_dep(k_upsample_bwd, cell_grid(L[1].n, 4), 256, 0, s, u->G0_48.p0(L), u->G0_48.ps(), L[0].n2, L[0].n3,
+             u->D1b.p0(L), u->D1b.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2, L[1].n3, u->G1_32a.p0(L),
+             u->G1_32a.ps());
   if ((st = wgrad(u, DEC1B, u->G1_32a, u->D1a, 0))) return st;
   if ((st = dgrad(u, DEC1B, u->G1_32a, u->G1_32b, 0, &u->D1a, 0))) return st;
   if ((st = wgrad(u, DEC1A, u->G1_32b, u->CAT1, 0))) return st;
   if ((st = dgrad(u, DEC1A, u->G1_32b, u->G1_96, 0, nullptr, 0))) return st;
   // up(M2b) part -> mid_b
-  k_upsample_bwd<<<cell_grid(L[2].n, 8), 256, 0, s>>>(u->G1_96.p0(L), u->G1_96.ps(), L[1].n2, L[1].n3,
-                                                           u->M2b.p0(L), u->M2b.ps(), L[2].mask, (unsigned)L[2].n,
-                                                       L[2].n2, L[2].n3, u->G2_64a.p0(L), u->G2_64a.ps());
+  launch_dep(k_upsample_bwd, cell_grid(L[2].n, 8), 256, 0, s, u->G1_96.p0(L), u->G1_96.ps(), L[1].n2, L[1].n3,
+             u->M2b.p0(L), u->M2b.ps(), L[2].mask, (unsigned)L[2].n, L[2].n2, L[2].n3, u->G2_64a.p0(L),
+             u->G2_64a.ps());
   if ((st = wgrad(u, MIDB, u->G2_64a, u->M2a, 0))) return st;
   if ((st = dgrad(u, MIDB, u->G2_64a, u->G2_64b, 0, &u->M2a, 0))) return st;
   if ((st = wgrad(u, MIDA, u->G2_64b, u->P2, 0))) return st;
   if ((st = dgrad(u, MIDA, u->G2_64b, u->G2_32, 0, nullptr, 0))) return st;
   // S1 = enc1b output: skip gradient + pooled path
-  k_skip_grad<<<cell_grid(L[1].n, 4), 256, 0, s>>>(u->G1_96.ch(L, 64), u->G1_96.ps(), u->G2_32.p0(L), u->G2_32.ps(),
-                                                    L[2].n2, L[2].n3, u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].mask,
-                                                    (unsigned)L[1].n, L[1].n2, L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps());
+  launch_dep(k_skip_grad, cell_grid(L[1].n, 4), 256, 0, s, u->G1_96.ch(L, 64), u->G1_96.ps(), u->G2_32.p0(L),
+             u->G2_32.ps(), L[2].n2, L[2].n3, u->CAT1.ch(L, 64), u->CAT1.ps(), L[1].mask, (unsigned)L[1].n, L[1].n2,
+             L[1].n3, u->G1_32a.p0(L), u->G1_32a.ps());
   if ((st = wgrad(u, ENC1B, u->G1_32a, u->A1, 0))) return st;
   if ((st = dgrad(u, ENC1B, u->G1_32a, u->G1_32b, 0, &u->A1, 0))) return st;
   if ((st = wgrad(u, ENC1A, u->G1_32b, u->P1, 0))) return st;
   if ((st = dgrad(u, ENC1A, u->G1_32b, u->G1_16, 0, nullptr, 0))) return st;
-  k_skip_grad<<<cell_grid(L[0].n, 2), 256, 0, s>>>(u->G0_48.ch(L, 32), u->G0_48.ps(), u->G1_16.p0(L), u->G1_16.ps(),
-                                                    L[1].n2, L[1].n3, u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].mask,
-                                                    (unsigned)L[0].n, L[0].n2, L[0].n3, u->G0_16a.p0(L), u->G0_16a.ps());
+  launch_dep(k_skip_grad, cell_grid(L[0].n, 2), 256, 0, s, u->G0_48.ch(L, 32), u->G0_48.ps(), u->G1_16.p0(L),
+             u->G1_16.ps(), L[1].n2, L[1].n3, u->CAT0.ch(L, 32), u->CAT0.ps(), L[0].mask, (unsigned)L[0].n, L[0].n2,
+             L[0].n3, u->G0_16a.p0(L), u->G0_16a.ps());
   if ((st = wgrad(u, ENC0B, u->G0_16a, u->A0, 0))) return st;
   if ((st = dgrad(u, ENC0B, u->G0_16a, u->G0_16b, 0, &u->A0, 0))) return st;
   if ((st = wgrad(u, ENC0A, u->G0_16b, u->X0, 0))) return st;
