@@ -477,6 +477,8 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_cg_polym(const __grid_constan
   __shared__ bool last;
   __shared__ float dtab[64];
   __shared__ CmProducer pr;
+  dep_trigger();
+  dep_wait();
   DevScratch* S = a.S;
   if (S->iscalars[I_DONE] || S->iscalars[I_PAUSE]) return;
   const int n1 = a.n1, n3 = a.n3, P = a.P, HA = a.HA, R0 = a.R0, R1 = a.R1, KS = a.KS;
@@ -954,7 +956,8 @@ void poly_launch(const xf_op* op, CpArgs& a, const float coeffs[3]) {
     const long cap = strtol(env, nullptr, 10);
     if (cap >= 1 && cap < blocks) blocks = cap;
   }
-  kern<<<(int)blocks, CP_THREADS, smem, ctx->stream>>>(a);
+  if (FUSE) kern<<<(int)blocks, CP_THREADS, smem, ctx->stream>>>(a);
+  else launch_dep(kern, dim3((unsigned)blocks), CP_THREADS, smem, ctx->stream, a);
 }
 
 }  // namespace

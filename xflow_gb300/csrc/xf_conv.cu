@@ -755,7 +755,9 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
   const int64_t cell0 = (int64_t)sp * a.stages * WG_KC;
   // this range's stages: the last range stops at the box's last 128-cell chunk
   const int my_stages = (int)min((int64_t)a.stages, a.chunks - (int64_t)sp * a.stages);
+  dep_trigger();
   if (warp == 4) {   // ---- producer: one copy per lane
+    dep_wait();
     const bool is_a = lane < ga, is_b = lane >= ga && lane < ga + gb;
     const uint16_t* src = nullptr;
     uint32_t dst_off = 0;
@@ -816,6 +818,7 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
     }
     __syncwarp();
   } else {   // ---- epilogue, warps 0-3: the partial of this tile and range
+    dep_wait();
     const bool got = bk_wait(&mdone, 0, abort_p, false);
     if (__all_sync(0xffffffffu, got) && !*abort_p) {
       tc::fence_after_sync();
@@ -842,6 +845,8 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
 __global__ void __launch_bounds__(256) k_bgrad(const uint16_t* __restrict__ g, int64_t gps, int64_t ncell, int chunk,
                                                int co, float* __restrict__ bpart) {
   __shared__ float part[8][256];
+  dep_trigger();
+  dep_wait();
   const int q = blockIdx.y, u = threadIdx.x;
   const int64_t beg = (int64_t)blockIdx.x * chunk, end = min(ncell, beg + chunk);
   float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -885,6 +890,8 @@ __global__ void __launch_bounds__(256) k_bgrad(const uint16_t* __restrict__ g, i
 // run along co, as the partials lie; a layer's last block sums its bias
 // chunks.
 __global__ void __launch_bounds__(256) k_grad_sum(const __grid_constant__ WgSegs segs) {
+  dep_trigger();
+  dep_wait();
   int k = 0;
   while (k + 1 < WG_LAYERS && (int)blockIdx.x >= segs.s[k + 1].block0) k++;
   const WgSeg& g = segs.s[k];
@@ -908,7 +915,7 @@ __global__ void __launch_bounds__(256) k_grad_sum(const __grid_constant__ WgSegs
   g.gb[o] = s;
 }
 int xf_grad_sum_blocks(int ci, int co) { return 27 * co * ci / 256 + 1; }
-void xf_grad_sum(xf_ctx* ctx, const WgSegs& segs, int blocks) { k_grad_sum<<<blocks, 256, 0, ctx->stream>>>(segs); }
+void xf_grad_sum(xf_ctx* ctx, const WgSegs& segs, int blocks) { launch_dep(k_grad_sum, dim3(blocks), 256, 0, ctx->stream, segs); }
 
 // The row tiles and cell ranges of a layer's weight gradient, and the FP32
 // partial buffer it needs (floats).
@@ -952,11 +959,11 @@ int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps,
   a.err = conv_err_flag(ctx);
   const size_t smem = (size_t)WG_STAGES * a.stage_bytes + 1024;
   XF_CUDA(ctx, set_max_smem((const void*)k_wgrad_tc, 1, ctx->device, smem));
-  k_wgrad_tc<<<a.mtiles * a.splits, BK_THREADS, smem, ctx->stream>>>(a);
+  launch_dep(k_wgrad_tc, dim3((unsigned)(a.mtiles * a.splits)), BK_THREADS, smem, ctx->stream, a);
   int nchunk, chunk;
   xf_bgrad_plan((int64_t)n1 * n2 * n3, &nchunk, &chunk);
-  k_bgrad<<<dim3((unsigned)nchunk, (unsigned)(co / 8)), 256, 0, ctx->stream>>>(a.g, gps, (int64_t)n1 * n2 * n3, chunk, co,
-                                                                              bpart);
+  launch_dep(k_bgrad, dim3((unsigned)nchunk, (unsigned)(co / 8)), 256, 0, ctx->stream, a.g, gps, (int64_t)n1 * n2 * n3,
+             chunk, co, bpart);
   XF_CUDA(ctx, cudaGetLastError());
   return XF_OK;
 }

@@ -55,6 +55,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_omega(const float* __restric
                                                           int s_om) {
   __shared__ double sh[32];
   __shared__ bool last;
+  dep_trigger();
+  dep_wait();
   double v[2] = {0.0, 0.0};
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t m = cnt[c];
@@ -89,6 +91,8 @@ __global__ void __launch_bounds__(256, 3) k_tl_sub(const uint8_t* __restrict__ k
                                                 const float* __restrict__ zc, int n1, int n3, int P, int c2, int c3,
                                                 int chunk, float cx, float cy, float cz, const DevScratch* S, int s_om,
                                                 float* __restrict__ out) {
+  dep_trigger();
+  dep_wait();
   const int p0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (p0 >= P) return;
   const float om = (float)S->scalars[s_om];
@@ -192,8 +196,8 @@ void xf_tl_faces(const xf_grid* g, const xf_grid* cg, uint32_t* cnt) {
 void xf_tl_omega(const xf_grid* g, const xf_grid* cg, const float* zc, const uint32_t* cnt, const double* rc, int slot,
                  int s_om) {
   const int blocks = red_blocks(g->ctx, cg->ncell);
-  k_tl_omega<<<blocks, RED_THREADS, 0, g->ctx->stream>>>(zc, cnt, rc, cg->ncell, cg->n2 * cg->n3, cg->n3, (float)g->ucx,
-                                                         (float)g->ucy, (float)g->ucz, g->ctx->scratch, slot, s_om);
+  launch_dep(k_tl_omega, dim3(blocks), RED_THREADS, 0, g->ctx->stream, zc, cnt, rc, cg->ncell, cg->n2 * cg->n3, cg->n3,
+             (float)g->ucx, (float)g->ucy, (float)g->ucz, g->ctx->scratch, slot, s_om);
 }
 
 // Plane sizes and row lengths of the grid fit four-cell groups of whole pairs:
@@ -203,9 +207,8 @@ void xf_tl_sub(const xf_grid* g, const float* r, const float* zc, int c2, int c3
   const int bx = (P / 4 + 255) / 256;
   int chunk = 16;   // blocks of 4 planes: z and its neighbours are reloaded at a chunk's start
   while (chunk > 4 && (int64_t)bx * ((g->n1 + chunk - 1) / chunk) < 4 * g->ctx->sm_count) chunk >>= 1;
-  k_tl_sub<<<dim3(bx, (g->n1 + chunk - 1) / chunk), 256, 0, g->ctx->stream>>>(
-      g->kind, r, zc, g->n1, g->n3, P, c2, c3, chunk, (float)g->ucx, (float)g->ucy, (float)g->ucz, g->ctx->scratch, s_om,
-      out);
+  launch_dep(k_tl_sub, dim3(bx, (g->n1 + chunk - 1) / chunk), 256, 0, g->ctx->stream, g->kind, r, zc, g->n1, g->n3, P, c2,
+             c3, chunk, (float)g->ucx, (float)g->ucy, (float)g->ucz, g->ctx->scratch, s_om, out);
 }
 
 void xf_tl_sub_ay(const xf_grid* g, const float* r, const float* ay, int s_yay, int s_yr, int s_om, float* out) {

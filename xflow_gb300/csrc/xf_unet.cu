@@ -374,6 +374,8 @@ __device__ __forceinline__ void weight_bf16(float x, int u, int co, int ci, uint
 }
 __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamSegs segs, float lr, float b1, float b2,
                                               float eps, float c1, float c2) {
+  dep_trigger();
+  dep_wait();
   int k = 0;
   while (k + 1 < NLAYER && (int)blockIdx.x >= segs.s[k + 1].block0) k++;
   const AdamSeg& a = segs.s[k];
@@ -399,6 +401,8 @@ __global__ void __launch_bounds__(256) k_anorm_dots(const float* __restrict__ z,
                                                             double* red) {
   __shared__ double sh[32];
   __shared__ bool last;
+  dep_trigger();
+  dep_wait();
   double v[3] = {0.0, 0.0, 0.0};
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
     if (m[c]) {
@@ -423,6 +427,8 @@ __global__ void __launch_bounds__(256) k_anorm_dots(const float* __restrict__ z,
 __global__ void k_anorm_grad(const double* __restrict__ r, const double* __restrict__ az,
                              const uint8_t* __restrict__ m, int64_t n, const DevScratch* __restrict__ S,
                              uint16_t* __restrict__ g16, int64_t ps) {
+  dep_trigger();
+  dep_wait();
   const double c1 = S->scalars[10], c2 = S->scalars[11];
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t v = m[c] ? f2bf((float)(c1 * (r[c] - c2 * az[c]))) : 0u;
@@ -433,6 +439,8 @@ __global__ void k_anorm_grad(const double* __restrict__ r, const double* __restr
 
 __global__ void k_f2d_mask(const float* __restrict__ z, const uint8_t* __restrict__ m, int64_t n,
                            double* __restrict__ out) {
+  dep_trigger();
+  dep_wait();
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
     out[c] = m[c] ? (double)z[c] : 0.0;
 }
@@ -739,14 +747,14 @@ static int backward(xf_unet* u, const double* r, const double* e, const xf_op* o
   const Level* L = u->L;
   int st;
   if (op) {   // A-norm loss
-    k_f2d_mask<<<ublocks(ctx, L[0].n), 256, 0, s>>>(u->zout, L[0].mask, L[0].n, u->zd);
+    launch_dep(k_f2d_mask, dim3(ublocks(ctx, L[0].n)), 256, 0, s, u->zout, L[0].mask, L[0].n, u->zd);
     MvReq<double> m;
     m.x = u->zd; m.y = u->az; m.zero_inactive = 1;
     xf_mv64(op, m);
-    k_anorm_dots<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(u->zout, u->az, r, e, L[0].mask, L[0].n, ctx->scratch,
-                                                           u->red);
-    k_anorm_grad<<<ublocks(ctx, L[0].n), 256, 0, s>>>(r, u->az, L[0].mask, L[0].n, ctx->scratch, u->G0_16a.p0(L),
-                                                      u->G0_16a.ps());
+    launch_dep(k_anorm_dots, dim3(sumsq_blocks(ctx, L[0].n)), 256, 0, s, u->zout, u->az, r, e, L[0].mask, L[0].n,
+               ctx->scratch, u->red);
+    launch_dep(k_anorm_grad, dim3(ublocks(ctx, L[0].n)), 256, 0, s, r, u->az, L[0].mask, L[0].n, ctx->scratch,
+               u->G0_16a.p0(L), u->G0_16a.ps());
   } else {
     k_sumsq<<<sumsq_blocks(ctx, L[0].n), 256, 0, s>>>(e, L[0].mask, L[0].n, (double)L[0].active, u->red, 1, u->rpart,
                                                       u->rtick);
@@ -805,7 +813,7 @@ static int check_box(const xf_unet* u, const xf_vec* v, const char* who) {
 int xf_unet_apply_dev(xf_unet* u, const double* r, double* z) {
   int st = forward(u, r);
   if (st) return st;
-  k_f2d_mask<<<ublocks(u->ctx, u->L[0].n), 256, 0, u->ctx->stream>>>(u->zout, u->L[0].mask, u->L[0].n, z);
+  launch_dep(k_f2d_mask, dim3(ublocks(u->ctx, u->L[0].n)), 256, 0, u->ctx->stream, u->zout, u->L[0].mask, u->L[0].n, z);
   XF_CUDA(u->ctx, cudaGetLastError());
   return XF_OK;
 }
@@ -843,7 +851,7 @@ extern "C" int xf_unet_train_step(xf_unet* u, const xf_op* op, const xf_vec* r, 
       segs.s[k] = {y.w, y.gw, y.mw, y.vw, y.b, y.gb, y.mb, y.vb, y.w16t, y.wt16t, y.ci, y.co, blocks};
       blocks += (int)(y.nw / 256) + 1;   // nw is a multiple of 256
     }
-    k_adam<<<blocks, 256, 0, s>>>(segs, (float)lr, b1, b2, 1e-8f, c1, c2);
+    launch_dep(k_adam, dim3(blocks), 256, 0, s, segs, (float)lr, b1, b2, 1e-8f, c1, c2);
   }
   XF_CUDA(ctx, cudaGetLastError());
   if (loss) {
@@ -1187,6 +1195,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e
                                                            TlStep step, int64_t n, DevScratch* S, int slot) {
   __shared__ double sh[32];
   __shared__ bool last;
+  dep_trigger();
+  dep_wait();
   if (step.ctl->brk) {   // set by the pass before: every block sees it
     if ((threadIdx.x | blockIdx.x) == 0) tl_rr(S, step);
     return;
@@ -1383,7 +1393,7 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     auto advance = [&]() {
       for (int j = 0; j < m - 1; j++) k_tl_axpy<<<eb, 256, 0, s>>>(z, P[(hd + m - j) % (m + 1)], c, j, n);
       xf_cg_pqb_tl_launch(op, z, P[(hd + 1) % (m + 1)], P[hd], qn, FS_PQ, step);
-      k_tl_update<<<db, RED_THREADS, 0, s>>>(e, r, P[hd], qn, step, n, S, FS_RR);
+      launch_dep(k_tl_update, dim3(db), RED_THREADS, 0, s, e, r, P[hd], qn, step, n, S, (int)FS_RR);
     };
     // network on: z = M r with (z, r) and (z, q_newest)
     begin(body[TL_ON], nullptr, 0);
