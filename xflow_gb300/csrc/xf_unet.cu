@@ -284,7 +284,7 @@ __global__ void k_skip_grad(const uint16_t* __restrict__ gskip, int64_t gps, con
 constexpr int RP_MAX = 4096;
 __device__ __forceinline__ void sumsq_finish(double s, double* red, int slot, double count, double* part,
                                              unsigned* tick) {
-  __shared__ double sh[1];
+  __shared__ double sh[32];
   __shared__ bool last;
   const double b = block_sum(s, sh);
   if (threadIdx.x == 0) {
