@@ -30,8 +30,11 @@ enum { PC_FICTIVE = 0, PC_ACTUAL = 1, PC_DEFINED = 3, PC_PREDEFINED = 4, PC_NORM
        PC_EQUATION = 7, PC_PREEQUATION = 8 };
 
 // Error kinds, each the minimum offending cell in iscalars[CHK0 + kind].
-enum { CHK0 = 48, E_RANGE = 0, E_NOTIMPL_P, E_UNKNOWN, E_DEFINED, E_PREDEF_NONE, E_PREDEF_MANY, E_PREDEF_VALUE,
-       E_NOTIMPL_V, E_NOTIMPL_EQ, E_NOTIMPL_C, E_RANGE_C, E_COUNT };
+// E_MOM_*: not errors but what k_mom_viscous wants to know of the transfer
+// pass's cells: the least bits of an Actual cell's viscosity, the least of
+// their complements, and 0 where a value stood that its quick test excludes.
+enum { CHK0 = 44, E_RANGE = 0, E_NOTIMPL_P, E_UNKNOWN, E_DEFINED, E_PREDEF_NONE, E_PREDEF_MANY, E_PREDEF_VALUE,
+       E_NOTIMPL_V, E_NOTIMPL_EQ, E_NOTIMPL_C, E_RANGE_C, E_MOM_VMIN, E_MOM_VMAX, E_MOM_WILD, E_COUNT };
 constexpr long long NO_CELL = 0x7f7f7f7f7f7f7f7fLL;   // cudaMemset byte 0x7f
 constexpr int SL_STEP = 8;                              // reduction slot of xf_divergence_max (and SL_STEP + 1)
 
@@ -256,6 +259,8 @@ struct MomArgs {
   DevScratch* S;
 };
 
+// Below 2^500 in magnitude: the difference of two such over a spacing above 2^-500 is finite.
+__device__ __forceinline__ bool mom_tame(double v) { return (__double2hiint(v) & 0x7fffffff) < (1523 << 20); }
 template <bool SMALL>
 __global__ void k_mom_transfer(MomArgs a) {
   const int64_t n = (int64_t)a.b1 * a.b2 * a.b3;
@@ -265,6 +270,8 @@ __global__ void k_mom_transfer(MomArgs a) {
   const int64_t vs1 = (int64_t)(n2 - 1) * n3, vs2 = n3;
   const int64_t ws1 = (int64_t)n2 * (n3 - 1), ws2 = n3 - 1;
   const int64_t ps1 = (int64_t)n2 * n3, ps2 = n3;
+  long long vmin = NO_CELL, vmax = NO_CELL;
+  bool wild = false;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
     const int m = a.code[c];
     double ut = 0, vt = 0, wt = 0, vist = 0, r = 0;
@@ -298,6 +305,10 @@ __global__ void k_mom_transfer(MomArgs a) {
         if (a.vis) vist = (a.vis[cp] + a.vis[cp + 1]) / 2;
       }
       r = a.force ? a.force[c] : 0.0;   // GetForce replaces the Actual rows' zero
+      const long long b = __double_as_longlong(vist);
+      vmin = min(vmin, b);
+      vmax = min(vmax, ~b);
+      wild |= !(mom_tame(ut) && mom_tame(vt) && mom_tame(wt)) || __double_as_longlong(r) == (long long)0x8000000000000000ull;
     } else if (m == PC_DEFINED || m == PC_PREDEFINED) {
       r = a.border ? a.border[c] : 0.0;
     } else if (m == PC_NORMAL) {
@@ -312,6 +323,19 @@ __global__ void k_mom_transfer(MomArgs a) {
     }
     a.uTr[c] = ut; a.vTr[c] = vt; a.wTr[c] = wt; a.visTr[c] = vist; a.rp[c] = r;
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    vmin = min(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
+    vmax = min(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+  }
+  wild = __any_sync(0xffffffffu, wild);
+  if ((threadIdx.x & 31) == 0) {   // in a fluid of one viscosity only the first warps write
+    volatile long long* at = a.S->iscalars + CHK0;
+    const long long v0 = at[E_MOM_VMIN], v1 = at[E_MOM_VMAX];
+    if (vmin < v0) report(a.S, E_MOM_VMIN, vmin);
+    if (vmax < v1) report(a.S, E_MOM_VMAX, vmax);
+    if (wild) report(a.S, E_MOM_WILD, 0);
+  }
 }
 
 // Pass 3 (XProblem.cpp:5352-5419): rp += dVis . (dVel + dU) on Actual cells.
@@ -321,12 +345,14 @@ __global__ void k_mom_transfer(MomArgs a) {
 // as bits: a cell's nine quotients take 50 instructions of the FP64 pipe (1.6
 // ms for 512 x 128 x 128 cells, where the bytes take 0.07), and in a fluid of
 // one viscosity only the cells beside a border need any, of the axis across it.
+// The transfer pass has seen every value: when its Actual cells all hold one
+// finite viscosity (the others hold 0), tame velocities and no -0, the cells'
+// codes tell where the viscosity differs, 7 bytes a cell instead of 19 doubles
+// (512 x 128 x 128: 460 us with the doubles).
 __device__ __forceinline__ bool mom_flat(const double* __restrict__ v, int64_t c, int64_t s) {
   const long long a = __double_as_longlong(v[c - s]), b = __double_as_longlong(v[c + s]);
   return a == b && (a & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
 }
-// Below 2^500 in magnitude: the difference of two such over a spacing above 2^-500 is finite.
-__device__ __forceinline__ bool mom_tame(double v) { return (__double2hiint(v) & 0x7fffffff) < (1523 << 20); }
 __device__ __forceinline__ bool mom_tame2(const double* __restrict__ v, int64_t c, int64_t s) {
   return mom_tame(v[c - s]) && mom_tame(v[c + s]);
 }
@@ -337,10 +363,17 @@ __global__ void k_mom_viscous(MomArgs a) {
   const int64_t s1 = (int64_t)a.b2 * a.b3, s2 = a.b3;
   const int64_t st = a.axis == 1 ? s1 : a.axis == 2 ? s2 : 1;
   const double* velTr = a.axis == 1 ? a.uTr : a.axis == 2 ? a.vTr : a.wTr;
+  const long long vis = a.S->iscalars[CHK0 + E_MOM_VMIN];
+  const bool quick = vis == ~a.S->iscalars[CHK0 + E_MOM_VMAX] && (vis & 0x7ff0000000000000ll) != 0x7ff0000000000000ll &&
+                     a.S->iscalars[CHK0 + E_MOM_WILD] != 0;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
     if (a.code[c] != PC_ACTUAL) continue;
     int i, j, k;
-      split3<SMALL>(c, s1, s2, i, j, k);
+    split3<SMALL>(c, s1, s2, i, j, k);
+    if (quick && mom_tame(a.rhhx[i]) && mom_tame(a.rhhy[j]) && mom_tame(a.rhhz[k])) {
+      auto same = [&](int64_t s) { return (a.code[c - s] == PC_ACTUAL) == (a.code[c + s] == PC_ACTUAL); };
+      if (same(s1) && same(s2) && same(1)) continue;
+    }
     // a zero part keeps any sum of the others, and rp but for -0 + 0 = +0
     const double rp = a.rp[c];
     const bool tame = mom_tame2(velTr, c, s1) && mom_tame2(velTr, c, s2) && mom_tame2(velTr, c, 1) &&
