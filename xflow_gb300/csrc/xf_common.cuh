@@ -119,6 +119,12 @@ struct xf_op {
   // and the inverse row diagonals (0 off the active set), for the Jacobi
   // preconditioner of BiCGStab, refreshed with the table
   mutable double* adj64 = nullptr;
+  // the six neighbour coefficients times the neighbours' inverse diagonals
+  // (A D^-1 has a unit diagonal) and their use bytes, made by xf_op_scaled
+  // for the solves that want them; invalid whenever the table is
+  mutable double* ads64 = nullptr;
+  mutable uint8_t* adks = nullptr;
+  mutable int ads_valid = 0;
   mutable int lap_jac_valid = 0;   // XF_OP_LAPLACE: adj64 holds its inverse diagonals (built on first use)
   // device staging boxes of xf_solve_host, kept between calls
   xf_vec* host_x = nullptr;

@@ -50,6 +50,7 @@ struct MvReq {
   int slot = SL_A;
   int ctl = CTL_NONE;
   int gate = 0;   // 1: run only while a true-residual replacement is pending
+  int scaled = 0;   // XF_OP_ADVDIFF: A D^-1 (after xf_op_scaled)
   int transpose = 0;   // packed operators: apply the other side (A^T when op applies A)
   int guard = 0;       // packed operators: skip once the solve is done (implied by ctl)
 };

@@ -52,7 +52,8 @@ struct MatvecArgs {
   const double* __restrict__ diag;
   int sign, neg, zero_inactive, dot_w, dot_self;
   int slot_w, ctl, gate, chunk;
-  const uint8_t* __restrict__ use;   // k_ad_fast: xf_op::adk
+  const uint8_t* __restrict__ use;   // k_ad_fast: xf_op::adk, or adks
+  const double* __restrict__ dinv;   // the same, scaled: the inverse diagonals
   DevScratch* S;
 };
 
@@ -362,6 +363,34 @@ __device__ __noinline__ double ad_border_row(const StencilGrid<double>& g, const
   return boundary_row<double, false>(g, x, i, j, k, (int)c, row);
 }
 
+// A D^-1's row of a cell that the scaled table does not hold: an oblique
+// normal difference, or a row whose diagonal is 0 (D^-1 holds 0 there).
+struct ScaledProbe {
+  const double *x, *dinv;
+  int64_t c, s1, s2;
+  __device__ __forceinline__ double operator()(int a, int b, int d) const {
+    const int64_t at = c + a * s1 + b * s2 + d;
+    return dinv[at] * x[at];
+  }
+};
+__device__ __noinline__ double ad_scaled_row(const StencilGrid<double>& g, const double* __restrict__ x,
+                                             const double* __restrict__ dinv, int64_t c, uint32_t u) {
+  const int row = row_of(g.kind[c]);
+  const int64_t s1 = g.s1, s2 = g.s2, nn = g.adc_n;
+  if (row == ROW_ACTUAL) {
+    const int64_t off[6] = {-s1, s1, -s2, s2, -1, 1};
+    double v = 0.0;
+    for (int t = 0; t < 6; t++)
+      if (u >> t & 1) v = fma(g.adc[t * nn + c], x[c + off[t]], v);
+    return v;
+  }
+  const int i = (int)(c / s1), j = (int)((c - (int64_t)i * s1) / s2), k = (int)(c % s2);
+  return boundary_row_acc<double, false>(g, ScaledProbe{x, dinv, c, s1, s2}, i, j, k, (int)c, row);
+}
+
+// SCALED: A D^-1 from the scaled table, its diagonal 1: a product and 8 bytes a
+// cell less, and the solver keeps no preconditioned copies of its vectors.
+template <bool SCALED>
 __global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<double> a) {
   __shared__ double sh[32];
   __shared__ bool last;
@@ -386,14 +415,15 @@ __global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<
     const double* __restrict__ q = g.adc + c;
     const double x1 = u & 1 ? x[c - s1] : 0.0, x2 = u & 2 ? x[c + s1] : 0.0, x3 = u & 4 ? x[c - s2] : 0.0;
     const double x4 = u & 8 ? x[c + s2] : 0.0, x5 = u & 16 ? x[c - 1] : 0.0, x6 = u & 32 ? x[c + 1] : 0.0;
-    double v = q[0] * x[c];
-    v = fma(q[nn], x1, v);
-    v = fma(q[2 * nn], x2, v);
-    v = fma(q[3 * nn], x3, v);
-    v = fma(q[4 * nn], x4, v);
-    v = fma(q[5 * nn], x5, v);
-    v = fma(q[6 * nn], x6, v);
-    if (u & AD_OBLIQUE) v = ad_border_row(g, x, c, row_of(g.kind[c]));
+    double v = SCALED ? x[c] : q[0] * x[c];
+    if (!SCALED) q += nn;
+    v = fma(q[0], x1, v);
+    v = fma(q[nn], x2, v);
+    v = fma(q[2 * nn], x3, v);
+    v = fma(q[3 * nn], x4, v);
+    v = fma(q[4 * nn], x5, v);
+    v = fma(q[5 * nn], x6, v);
+    if (u & AD_OBLIQUE) v = SCALED ? ad_scaled_row(g, x, a.dinv, c, u) : ad_border_row(g, x, c, row_of(g.kind[c]));
     if (a.sign > 0) v = v + a.s[c];
     else if (a.sign < 0) v = v - a.s[c];
     if (a.neg) v = xneg(v);
@@ -424,6 +454,7 @@ __global__ void __launch_bounds__(AD_THREADS, AD_RESIDENT) k_ad_fast(MatvecArgs<
 // 130 x 130: 168 -> 162 us a call (FP64 issue bounds both); the predictors of
 // 64^3 2.48 -> 2.41 ms, the scalar of 256 x 64 x 64 1.60 -> 1.53.
 constexpr int AD2_RESIDENT = 3;
+template <bool SCALED>
 __global__ void __launch_bounds__(AD_THREADS, AD2_RESIDENT) k_ad_fast2(MatvecArgs<double> a) {
   __shared__ double sh[32];
   __shared__ bool last;
@@ -460,10 +491,15 @@ __global__ void __launch_bounds__(AD_THREADS, AD2_RESIDENT) k_ad_fast2(MatvecArg
         if (!(u1 & 16)) x5.y = 0.0;
         if (!(u0 & 32)) x6.x = 0.0;
       }
-      const double2 q0 = ld2(q), q1 = ld2(q + nn), q2 = ld2(q + 2 * nn), q3 = ld2(q + 3 * nn);
-      const double2 q4 = ld2(q + 4 * nn), q5 = ld2(q + 5 * nn), q6 = ld2(q + 6 * nn);
-      v.x = q0.x * xc.x;
-      v.y = q0.y * xc.y;
+      v = xc;
+      if (!SCALED) {
+        const double2 q0 = ld2(q);
+        v.x *= q0.x;
+        v.y *= q0.y;
+        q += nn;
+      }
+      const double2 q1 = ld2(q), q2 = ld2(q + nn), q3 = ld2(q + 2 * nn), q4 = ld2(q + 3 * nn);
+      const double2 q5 = ld2(q + 4 * nn), q6 = ld2(q + 5 * nn);
       v.x = fma(q1.x, x1.x, v.x);
       v.y = fma(q1.y, x1.y, v.y);
       v.x = fma(q2.x, x2.x, v.x);
@@ -477,8 +513,9 @@ __global__ void __launch_bounds__(AD_THREADS, AD2_RESIDENT) k_ad_fast2(MatvecArg
       v.x = fma(q6.x, x6.x, v.x);
       v.y = fma(q6.y, x6.y, v.y);
       if (any & AD_OBLIQUE) {
-        if (u0 & AD_OBLIQUE) v.x = ad_border_row(g, x, c, row_of(g.kind[c]));
-        if (u1 & AD_OBLIQUE) v.y = ad_border_row(g, x, c + 1, row_of(g.kind[c + 1]));
+        if (u0 & AD_OBLIQUE) v.x = SCALED ? ad_scaled_row(g, x, a.dinv, c, u0) : ad_border_row(g, x, c, row_of(g.kind[c]));
+        if (u1 & AD_OBLIQUE)
+          v.y = SCALED ? ad_scaled_row(g, x, a.dinv, c + 1, u1) : ad_border_row(g, x, c + 1, row_of(g.kind[c + 1]));
       }
       if (a.sign) {
         const double2 s = ld2(a.s + c);
@@ -525,6 +562,51 @@ __global__ void __launch_bounds__(AD_THREADS, AD2_RESIDENT) k_ad_fast2(MatvecArg
       }
     }
   }
+}
+
+// The scaled table: each neighbour coefficient times the neighbour's inverse
+// diagonal.  Bound by memory (6 planes in, 6 out: 0.15 ms for 514 x 130 x 130
+// cells, against 69 us that each iteration gains).
+__global__ void __launch_bounds__(AD_THREADS) k_ad_scale(const double* __restrict__ q, const uint8_t* __restrict__ use,
+                                                         const double* __restrict__ dinv, int64_t n, int64_t s1,
+                                                         int64_t s2, double* __restrict__ out,
+                                                         uint8_t* __restrict__ uses) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t u = use[c];
+    uses[c] = (uint8_t)(u && dinv[c] == 0.0 ? u | AD_OBLIQUE : u);
+    if (u == 0) continue;
+    const int64_t off[6] = {-s1, s1, -s2, s2, -1, 1};
+#pragma unroll
+    for (int t = 0; t < 6; t++) out[t * n + c] = u >> t & 1 ? q[(t + 1) * n + c] * dinv[c + off[t]] : 0.0;
+  }
+}
+// x += D^-1 y on the active set.
+__global__ void k_ad_unscale(double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ dinv,
+                             const uint8_t* __restrict__ m, int64_t n) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+    if (m[c]) x[c] = fma(dinv[c], y[c], x[c]);
+}
+
+// The scaled table of a ready operator; false where it has none (no table) or
+// no memory is left for it: the caller keeps to A and preconditioned copies.
+bool xf_op_scaled(const xf_op* op) {
+  if (op->kind != XF_OP_ADVDIFF || !op->adc_valid) return false;
+  if (op->ads_valid) return true;
+  const xf_grid* g = op->g;
+  const int64_t n = g->ncell;
+  if ((!op->ads64 && cudaMalloc(&op->ads64, 6 * n * 8) != cudaSuccess) ||
+      (!op->adks && cudaMalloc(&op->adks, n) != cudaSuccess)) {
+    cudaGetLastError();
+    return false;
+  }
+  k_ad_scale<<<grid_blocks(g->ctx, n, AD_THREADS), AD_THREADS, 0, g->ctx->stream>>>(op->adc64, op->adk, op->adj64, n, g->s1,
+                                                                                   g->s2, op->ads64, op->adks);
+  op->ads_valid = 1;
+  return true;
+}
+void xf_op_unscale(const xf_op* op, double* x, const double* y) {
+  const xf_grid* g = op->g;
+  k_ad_unscale<<<grid_blocks(g->ctx, g->ncell, 256), 256, 0, g->ctx->stream>>>(x, y, op->adj64, g->smask, g->ncell);
 }
 
 // The Laplace operator's inverse row diagonals (Actual: the fast row's
@@ -613,13 +695,17 @@ static void launch_matvec(const xf_op* op, const T* rho, const MvReq<T>& q) {
     set_ad_fields<T>(a.g, op);
     if constexpr (std::is_same<T, double>::value) {
       if (!q.exact && a.g.adc) {
-        a.use = op->adk;
+        a.use = q.scaled ? op->adks : op->adk;
+        a.dinv = op->adj64;
+        if (q.scaled) a.g.adc = op->ads64;
         // pairs where rows are even and every vector is 16-byte aligned, faster at every size there
         const uintptr_t at = (uintptr_t)a.x | (uintptr_t)a.y | (uintptr_t)a.s | (uintptr_t)a.w | (uintptr_t)a.g.adc;
         if (g->n3 % 2 == 0 && at % 16 == 0 && (uintptr_t)a.y32 % 8 == 0)
-          k_ad_fast2<<<grid_blocks(ctx, g->ncell / 2, AD_THREADS, AD2_RESIDENT), AD_THREADS, 0, ctx->stream>>>(a);
+          (q.scaled ? k_ad_fast2<true> : k_ad_fast2<false>)<<<grid_blocks(ctx, g->ncell / 2, AD_THREADS, AD2_RESIDENT),
+                                                              AD_THREADS, 0, ctx->stream>>>(a);
         else
-          k_ad_fast<<<grid_blocks(ctx, g->ncell, AD_THREADS, AD_RESIDENT), AD_THREADS, 0, ctx->stream>>>(a);
+          (q.scaled ? k_ad_fast<true> : k_ad_fast<false>)<<<grid_blocks(ctx, g->ncell, AD_THREADS, AD_RESIDENT),
+                                                            AD_THREADS, 0, ctx->stream>>>(a);
         return;
       }
     }
@@ -708,6 +794,8 @@ extern "C" int xf_op_destroy(xf_op* op) {
   if (op->adD32) cudaFree(op->adD32);
   if (op->adc64) cudaFree(op->adc64);
   if (op->adj64) cudaFree(op->adj64);
+  if (op->ads64) cudaFree(op->ads64);
+  if (op->adks) cudaFree(op->adks);
   if (op->adk) cudaFree(op->adk);
   if (op->pack) xf_pack_free(op->pack);
   if (op->host_x) xf_vec_destroy(op->host_x);
@@ -814,6 +902,7 @@ int xf_op_ready(const xf_op* op) {
     else k_ad_coeffs<false><<<grid, ADC_THREADS, 0, ctx->stream>>>(s, n, tx, ty, tz, op->adc64, op->adk, op->adj64);
     XF_CUDA(ctx, cudaGetLastError());
     op->adc_valid = 1;
+    op->ads_valid = 0;
   }
   if (op->kind == XF_OP_VARDIV && !op->rho_set)
     return xf_fail(op->g->ctx, XF_ERR_STATE, "variable-density operator used before xf_op_set_density");
