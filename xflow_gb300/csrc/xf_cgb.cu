@@ -52,6 +52,8 @@ struct PqbArgs {
   float cx, cy, cz;
   int slot, ctl;              // of (p', q), and the control step of the last block
   TlStep step;                // the flexible CG's, in its place (step.ctl not null)
+  float* e;                   // and its correction's last step: e += alpha pe (pe null: the p of the ring)
+  const float* pe;
 };
 
 // r + b p; b = 0 leaves p out (a buffer that holds no direction yet)
@@ -61,7 +63,7 @@ __device__ __forceinline__ float4 fma4(float b, float4 p, float4 r) {
 }
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-template <int PQB_NS>   // raw ring depth (planes in flight)
+template <int PQB_NS, bool TL>   // raw ring depth (planes in flight); the flexible CG's
 __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3 : 2) k_cg_pqb(const __grid_constant__ PqbArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ double sh[32];
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
   float* ring = reinterpret_cast<float*>(smem + 128);          // PQB_NS x {r, p} x RL
   float* pring = ring + (size_t)PQB_NS * 2 * a.RL;             // PQB_NP x RL
   const float beta = (float)S->scalars[D_BETA];
+  const float step_e = TL ? (float)a.step.ctl->alpha : 0.f;
   const int sel = (int)S->iscalars[I_PBUF];
   const float* __restrict__ po = sel ? a.pb1 : a.pb0;
   float* __restrict__ pn = sel ? a.pb0 : a.pb1;
@@ -172,7 +175,19 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
     const int first = dir > 0 ? i0 - 2 : i1 + 1, stop = dir > 0 ? i1 : i0 - 1;
     for (int i = first; i != stop; i += dir) {
       const int j = i + dir;
-      const bool load = j >= lo && j <= hi;
+      const bool load = j >= lo && j <= hi, own = j >= i0 && j < i1;
+      float4 ea, eb, fa, fb;   // TL: e (and pe) of the own cells of plane j, in flight while it lands
+      if (TL && own) {
+        const int64_t pl = (int64_t)j * P;
+        if (va) {
+          ea = *reinterpret_cast<const float4*>(a.e + pl + xa);
+          if (a.pe) fa = *reinterpret_cast<const float4*>(a.pe + pl + xa);
+        }
+        if (vb) {
+          eb = *reinterpret_cast<const float4*>(a.e + pl + xb);
+          if (a.pe) fb = *reinterpret_cast<const float4*>(a.pe + pl + xb);
+        }
+      }
       if (load) {
         const long long L = item_first + (dir > 0 ? j - lo : hi - j);
         wok = mbar_wait_bounded(&mbar[L % PQB_NS], (uint32_t)((L / PQB_NS) & 1));
@@ -189,10 +204,14 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
             const int t = 4 * (h < HA / 4 ? h : h + PQB_TILE / 4);
             *reinterpret_cast<float4*>(pj + t) = fma4(beta, lds4(Q + t), lds4(R + t));
           }
-          if (j >= i0 && j < i1) {   // p' of the chunk's own cells, written once
+          if (own) {   // p' of the chunk's own cells, written once
             const int64_t pl = (int64_t)j * P;
             if (va) *reinterpret_cast<float4*>(pn + pl + xa) = ga;
             if (vb) *reinterpret_cast<float4*>(pn + pl + xb) = gb;
+            if (TL && step_e != 0.f) {
+              if (va) *reinterpret_cast<float4*>(a.e + pl + xa) = fma4(step_e, a.pe ? fa : lds4(Q + sa), ea);
+              if (vb) *reinterpret_cast<float4*>(a.e + pl + xb) = fma4(step_e, a.pe ? fb : lds4(Q + sb), eb);
+            }
           }
         }
       }
@@ -258,7 +277,7 @@ __global__ void __launch_bounds__(PQB_THREADS, PQB_NS == 1 ? 4 : PQB_NS == 2 ? 3
   if (threadIdx.x == 0) {
     S->scalars[a.slot] = tot;
     S->tickets[a.slot] = 0;
-    if (a.step.ctl) tl_alpha(S, a.step);
+    if (TL) tl_alpha(S, a.step);
     else control_step(S, a.ctl);
   }
 }
@@ -276,8 +295,9 @@ bool xf_cg_pqb_supported(const xf_grid* g) {
   return pqb_smem(PQB_TILE + 2 * HA, 2) <= 227 * 1024 - 1024;
 }
 
+template <bool TL>
 static void pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int slot, int ctl,
-                       const TlStep& step) {
+                       const TlStep& step, float* e, const float* pe) {
   const xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
   PqbArgs a;
@@ -288,14 +308,14 @@ static void pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, 
   a.RL = PQB_TILE + 2 * a.HA;
   a.tiles = (a.P + PQB_TILE - 1) / PQB_TILE;
   a.cx = (float)g->ucx; a.cy = (float)g->ucy; a.cz = (float)g->ucz;
-  a.slot = slot; a.ctl = ctl; a.step = step;
+  a.slot = slot; a.ctl = ctl; a.step = step; a.e = e; a.pe = pe;
   // ring depth 2 (3 blocks per SM)
   const int ns = 2;
   const size_t smem = pqb_smem(a.RL, ns);
   static size_t attr_smem[5][64] = {};   // per ring depth and device
   size_t& at = attr_smem[ns][ctx->device & 63];
   if (at < smem) {
-    cudaFuncSetAttribute(k_cg_pqb<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_cg_pqb<2, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     at = smem;
   }
   // resident blocks per SM from shared memory (1 KB reserved per block) and the launch bounds
@@ -321,16 +341,19 @@ static void pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, 
     const long cap = strtol(env, nullptr, 10);
     if (cap >= 1 && cap < blocks) blocks = cap;
   }
-  k_cg_pqb<2><<<(int)blocks, PQB_THREADS, smem, ctx->stream>>>(a);
+  k_cg_pqb<2, TL><<<(int)blocks, PQB_THREADS, smem, ctx->stream>>>(a);
 }
 
 void xf_cg_pqb_launch(const xf_op* op, const float* r, float* pb0, float* pb1, float* q, int ctl) {
-  pqb_launch(op, r, pb0, pb1, q, SL_A, ctl, TlStep{});
+  pqb_launch<false>(op, r, pb0, pb1, q, SL_A, ctl, TlStep{}, nullptr, nullptr);
 }
 
 // The flexible CG's: p = z + beta p_old (beta = scalars[D_BETA], I_PBUF = 0),
-// q = A p, (p, q) -> scalars[slot], alpha.
-void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot,
-                         const TlStep& step) {
-  pqb_launch(op, z, p_old, p, q, slot, CTL_NONE, step);
+// q = A p, (p, q) -> scalars[slot], alpha; and the step before's part of the
+// correction, e += alpha_old p_new (p_new the newest direction, p_old the
+// window's oldest), here because the pass reads p_old anyway: with r -= alpha q
+// it took two streams more (24 bytes a cell instead of 12 and 8).
+void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot, const TlStep& step,
+                         float* e, const float* p_new) {
+  pqb_launch<true>(op, z, p_old, p, q, slot, CTL_NONE, step, e, p_new == p_old ? nullptr : p_new);
 }

@@ -81,6 +81,7 @@ __device__ __forceinline__ void tl_alpha(DevScratch* S, const TlStep& t) {
   if (!(pq > 0)) {
     c->status = isnan(pq) ? XF_NAN : XF_BREAKDOWN;
     c->brk = 1;
+    c->alpha = 0;   // e has taken the step before
     return;
   }
   c->alpha = pr / pq;

@@ -53,8 +53,8 @@ void xf_cheb2_coeffs(double lmax, double ratio, float out[3]);
 void xf_cg_poly_last_tl_launch(const xf_op* op, const float* in, float* z, const float coeffs[3], int s_om,
                                const float* zc, int c3, int cs1, int F, float tsc, const float* r, const float* qw,
                                int s_zr, int s_zq, const TlStep& step);
-void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot,
-                         const TlStep& step);
+void xf_cg_pqb_tl_launch(const xf_op* op, const float* z, float* p_old, float* p, float* q, int slot, const TlStep& step,
+                         float* e, const float* p_new);
 void xf_cg_poly_first_launch(const xf_op* op, const float* r, float* w, const float coeffs[3], const float* q,
                              const float* pa, const float* pb, float* e, float* r_out);
 
@@ -1138,16 +1138,22 @@ __global__ void k_tl_init(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles 
   for (int j = 0; j < 8; j++) { c->coef[j] = 0.f; c->use_coef[j] = 0; c->win_off[j] = 1; }
   c->launches = p->n_init;
 }
-// x += e after a cycle (none before the first)
-__global__ void k_tl_fold(double* __restrict__ x, const float* __restrict__ e, int64_t n, const TlCtl* c) {
+// x += e after a cycle (none before the first), with the last step's part of e,
+// alpha p of the newest direction
+struct TlDirs { const float* p[9]; };
+__global__ void k_tl_fold(double* __restrict__ x, const float* __restrict__ e, TlDirs dirs, int m, int64_t n,
+                          const TlCtl* c) {
   if (!c->cycle_ran) return;
+  const float* p = dirs.p[(c->head + m) % (m + 1)];
+  const float a = (float)c->alpha;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-    x[q] += (double)e[q];
+    x[q] += (double)(a != 0.f ? fmaf(a, p[q], e[q]) : e[q]);
 }
 // after the refresh: the stop, cap and stall tests; the next block
 __global__ void k_tl_top(DevScratch* S, TlCtl* c, const TlParams* p, TlHandles h, int m) {
   if (threadIdx.x | blockIdx.x) return;
   c->cycle_ran = 0;
+  c->alpha = 0;
   c->steps++;
   c->launches += p->n_ref;
   const double rr = S->scalars[FS_PQ + 1];
@@ -1187,11 +1193,11 @@ __global__ void k_tl_axpy(float* __restrict__ y, const float* __restrict__ x, co
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     y[q] = fmaf(a, x[q], y[q]);
 }
-// e += alpha p, r -= alpha q, (r, r) into scalars[slot] and the cycle-end test in the same pass;
-// the grid, the thread mapping and the accumulation order are k_dot_f4's, so
-// (r, r) is bit for bit the separate dot's.
-__global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e, float* __restrict__ r,
-                                                           const float* __restrict__ p, const float* __restrict__ q,
+// r -= alpha q, (r, r) into scalars[slot] and the cycle-end test in the same
+// pass (e += alpha p goes with the next direction); the grid, the thread mapping
+// and the accumulation order are k_dot_f4's, so (r, r) is bit for bit the
+// separate dot's.
+__global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ r, const float* __restrict__ q,
                                                            TlStep step, int64_t n, DevScratch* S, int slot) {
   __shared__ double sh[32];
   __shared__ bool last;
@@ -1204,18 +1210,14 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e
   const float alpha = (float)step.ctl->alpha;
   DotAcc<float> acc;
   const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * blockDim.x;
-  float4* e4 = reinterpret_cast<float4*>(e);
   float4* r4 = reinterpret_cast<float4*>(r);
-  const float4* p4 = reinterpret_cast<const float4*>(p);
   const float4* q4 = reinterpret_cast<const float4*>(q);
+#pragma unroll 2
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n4; k += stride) {
-    float4 ev = e4[k], rv = r4[k];
-    const float4 pv = __ldg(p4 + k), qv = __ldg(q4 + k);
-    ev.x = fmaf(alpha, pv.x, ev.x); ev.y = fmaf(alpha, pv.y, ev.y);
-    ev.z = fmaf(alpha, pv.z, ev.z); ev.w = fmaf(alpha, pv.w, ev.w);
+    float4 rv = r4[k];
+    const float4 qv = __ldg(q4 + k);
     rv.x = fmaf(-alpha, qv.x, rv.x); rv.y = fmaf(-alpha, qv.y, rv.y);
     rv.z = fmaf(-alpha, qv.z, rv.z); rv.w = fmaf(-alpha, qv.w, rv.w);
-    e4[k] = ev;
     r4[k] = rv;
     acc.add(rv.x, rv.x);
     acc.add(rv.y, rv.y);
@@ -1223,7 +1225,6 @@ __global__ void __launch_bounds__(RED_THREADS) k_tl_update(float* __restrict__ e
     acc.add(rv.w, rv.w);
   }
   for (int64_t k = 4 * n4 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += stride) {
-    e[k] = fmaf(alpha, p[k], e[k]);
     const float rv = fmaf(-alpha, q[k], r[k]);
     r[k] = rv;
     acc.add(rv, rv);
@@ -1366,7 +1367,9 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
   cudaGraphNode_t prev = nullptr;
   add_cond(wbody, {}, H.ref, cudaGraphCondTypeIf, 1, &rbody, &prev);
   begin(rbody, nullptr, 0);
-  k_tl_fold<<<eb, 256, 0, s>>>(x, e, n, c);
+  TlDirs dirs = {};
+  for (int j = 0; j <= m; j++) dirs.p[j] = P[j];
+  k_tl_fold<<<eb, 256, 0, s>>>(x, e, dirs, m, n, c);
   cudaMemsetAsync(e, 0, n * 4, s);
   xf_cg_res64(op, x, b, r, FS_PQ, CTL_NONE);   // r = float(b - A x), (r, r) in FP64 -> FS_PQ + 1
   k_tl_top<<<1, 32, 0, s>>>(S, c, prm, H, m);   // reads H.main, H.ref, H.blk only
@@ -1392,8 +1395,8 @@ static int tl_graph_build(xf_op* op, xf_unet* u, int m, int F, const float (*tl_
     // the new direction (its last term and image in one pass), alpha, the update, the cycle-end test
     auto advance = [&]() {
       for (int j = 0; j < m - 1; j++) k_tl_axpy<<<eb, 256, 0, s>>>(z, P[(hd + m - j) % (m + 1)], c, j, n);
-      xf_cg_pqb_tl_launch(op, z, P[(hd + 1) % (m + 1)], P[hd], qn, FS_PQ, step);
-      launch_dep(k_tl_update, dim3(db), RED_THREADS, 0, s, e, r, P[hd], qn, step, n, S, (int)FS_RR);
+      xf_cg_pqb_tl_launch(op, z, P[(hd + 1) % (m + 1)], P[hd], qn, FS_PQ, step, e, P[(hd + m) % (m + 1)]);
+      launch_dep(k_tl_update, dim3(db), RED_THREADS, 0, s, r, qn, step, n, S, (int)FS_RR);
     };
     // network on: z = M r with (z, r) and (z, q_newest)
     begin(body[TL_ON], nullptr, 0);
