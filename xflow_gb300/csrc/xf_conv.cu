@@ -205,10 +205,14 @@ __device__ __forceinline__ void conv_store8(const ConvArgs& a, int64_t c, int co
 // exchanges cost about three times as long).  A tile therefore yields 126 cells;
 // the last tile starts at ncell - 126 (its overlap rewrites identical values).
 //
-// A pipeline stage is one (tile, 16-channel input chunk): for each of the
-// nine slabs the two 8-channel planes' 128 rows, 2 KB each, one bulk copy
-// (cp.async.bulk) apiece, which is already the canonical K-major operand
-// layout; nine MMAs read it.  The tiled weights stay resident in shared
+// A pipeline stage is one (tile, 16-channel input chunk): for each di and
+// 8-channel plane the rows of its three slabs, which is already the canonical
+// K-major operand layout; nine MMAs read it.  Where a row of the box is
+// shorter than a tile, the slabs of dj = -1, 0, 1 overlap and come as one copy of
+// 128 + 2 n3 rows (cp.async.bulk), the MMAs starting n3 rows apart: 25 KB a
+// stage at n3 = 66 instead of 37, so that three CTAs fit an SM (64^3, 16 -> 16:
+// 14.5 -> 13.1 us; 48 -> 16 27.3 -> 19.6; 96 -> 32 at 34^3 20.3 -> 14.1);
+// otherwise nine copies of 128 rows a plane.  The tiled weights stay resident in shared
 // memory when they fit beside two stages, else each stage also carries its
 // chunk's nine B blocks.  Each control step therefore covers nine MMAs.
 // The CTA is persistent and warp-specialised:
@@ -228,8 +232,6 @@ __device__ __forceinline__ void conv_store8(const ConvArgs& a, int64_t c, int co
 // multiples of 16.
 constexpr int BK_THREADS = 192;
 constexpr int BK_MAX_STAGES = 6;
-constexpr uint32_t BK_SLAB = 128 * 32;            // one slab's A block (two planes x 2 KB)
-constexpr uint32_t BK_A = 9 * BK_SLAB;            // the nine slabs of one chunk
 constexpr long long BK_WAIT_CYCLES = 1ll << 31;   // about a second at the SM clock
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
@@ -294,22 +296,29 @@ __device__ __forceinline__ void epi_sync() { asm volatile("barrier.cta.sync 1, 1
 struct BkPlan {
   int stages, per_sm, resident, acc_off, tmem_cols, smem_bytes;
   uint32_t w_bytes, b_bytes, stage_bytes, w_region;
+  uint32_t a_bytes, plane_bytes;   // A of a stage; one plane's rows of one di
+  int step, merged;                // rows between the slabs of dj = -1, 0, 1; they overlap and come as one copy
 };
-static BkPlan bk_plan(int ci, int co, int static_smem) {
+static BkPlan bk_plan(int ci, int co, int rows, int static_smem) {
   BkPlan p = {};
+  p.merged = rows < 128;
+  p.step = std::min(rows, 128);
+  p.plane_bytes = (uint32_t)(128 + 2 * p.step) * 16;
+  p.a_bytes = (6 * p.plane_bytes + 127) / 128 * 128;   // B behind it keeps its 128-byte rows
   const int n3 = 3 * co;
   p.acc_off = (n3 + 31) / 32 * 32;
   p.tmem_cols = (int)tmem_cols(p.acc_off + n3);
-  const int per_sm_t = std::min(2, 512 / p.tmem_cols);
+  const int per_sm_t = std::min(3, 512 / p.tmem_cols);
   p.w_bytes = (uint32_t)(27 * co * ci * 2);
   p.b_bytes = (uint32_t)(9 * n3 * 32);
   const uint32_t w_region = (p.w_bytes + 1023) / 1024 * 1024;
-  const uint32_t st_res = BK_A, st_str = (BK_A + p.b_bytes + 1023) / 1024 * 1024;
-  // (CTAs per SM, weights resident): two CTAs first, resident weights first
-  for (int k = 0; k < 4; k++) {
-    const int per_sm = k < 2 ? per_sm_t : 1;
-    const bool res = (k % 2) == 0;
-    if (k < 2 && per_sm_t < 2) continue;
+  const uint32_t st_res = (p.a_bytes + 1023) / 1024 * 1024, st_str = (p.a_bytes + p.b_bytes + 1023) / 1024 * 1024;
+  // (CTAs per SM, weights resident): three CTAs with resident weights, then two, resident weights first, then one
+  const int order[5][2] = {{3, 1}, {2, 1}, {2, 0}, {1, 1}, {1, 0}};
+  for (const auto& way : order) {
+    const int per_sm = way[0];
+    const bool res = way[1];
+    if (per_sm > per_sm_t) continue;
     // dynamic shared memory of one CTA: 228 KB per SM less 1 KB reserved per
     // CTA, at most 227 KB per CTA, less the static part and the alignment slack
     const int dyn = std::min(227 * 1024, (228 * 1024) / per_sm - 1024) - static_smem - 1024;
@@ -375,10 +384,13 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
       bulk_load(wsm, a.Wt, plan.w_bytes, &wfull);
     }
     dep_wait();
-    // this lane's copy: slab sl = lane / 2, plane q = lane % 2 (lane 18: the
-    // streamed weights)
-    const int sl = lane >> 1, q = lane & 1;
-    const int64_t slab_off = (sl / 3 - 1) * P + (sl % 3 - 1) * (int64_t)a.n3;
+    // this lane's copy: (di, plane q), and dj where the slabs do not overlap
+    // (the lane after: the streamed weights)
+    const int copies = plan.merged ? 6 : 18, sl = lane >> 1, q = lane & 1;
+    const int di = plan.merged ? sl : sl / 3, dj = plan.merged ? 0 : sl % 3;
+    const int64_t slab_off = (di - 1) * P + (dj - 1) * (int64_t)a.n3;
+    const uint32_t slab_dst = (uint32_t)(2 * di + q) * plan.plane_bytes + (uint32_t)dj * 2048u;
+    const uint32_t slab_bytes = plan.merged ? plan.plane_bytes : 2048u;
     int st = 0, pass = 0, issued = 0;
     bool ok = true;
     for (int k = 0; k < my_tiles && ok; k++) {
@@ -393,12 +405,11 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
           }
         }
         uint8_t* sa = stg + st * plan.stage_bytes;
-        if (lane == 0) mbar_expect_tx(&full[st], BK_A + (plan.resident ? 0u : plan.b_bytes));
-        if (lane < 18)
-          bulk_load(sa + sl * BK_SLAB + q * 2048, a.in + (2 * c + q) * a.in_ps + (row_base + slab_off) * 8, 2048,
-                    &full[st]);
-        else if (lane == 18 && !plan.resident)
-          bulk_load(sa + BK_A, a.Wt + (int64_t)c * 9 * N3 * 16, plan.b_bytes, &full[st]);
+        if (lane == 0) mbar_expect_tx(&full[st], 6u * plan.plane_bytes + (plan.resident ? 0u : plan.b_bytes));
+        if (lane < copies)
+          bulk_load(sa + slab_dst, a.in + (2 * c + q) * a.in_ps + (row_base + slab_off) * 8, slab_bytes, &full[st]);
+        else if (lane == copies && !plan.resident)
+          bulk_load(sa + plan.a_bytes, a.Wt + (int64_t)c * 9 * N3 * 16, plan.b_bytes, &full[st]);
         issued++;
         if (++st == S) {
           st = 0;
@@ -435,10 +446,11 @@ __global__ void __launch_bounds__(BK_THREADS) k_conv3_bulk(ConvArgs a, BkPlan pl
           }
           tc::fence_after_sync();
           const uint8_t* sa = stg + st * plan.stage_bytes;
-          const uint8_t* sb = plan.resident ? wsm + (size_t)c * 9 * N3 * 32 : sa + BK_A;
+          const uint8_t* sb = plan.resident ? wsm + (size_t)c * 9 * N3 * 32 : sa + plan.a_bytes;
 #pragma unroll
           for (int sl = 0; sl < 9; sl++) {
-            const uint64_t ad = tc::smem_desc(tc::smem_addr(sa + sl * BK_SLAB), 2048, 128);
+            const uint64_t ad = tc::smem_desc(tc::smem_addr(sa) + (uint32_t)(sl / 3) * 2u * plan.plane_bytes +
+                                                  (uint32_t)((sl % 3) * plan.step) * 16u, plan.plane_bytes, 128);
             const uint64_t bd = tc::smem_desc(tc::smem_addr(sb + sl * N3 * 32), b_lbo, 128);
             if (leader) tc::mma_bf16(dacc, ad, bd, idesc, c > 0 || sl > 0);
           }
@@ -1002,7 +1014,7 @@ int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t 
     XF_CUDA(ctx, cudaFuncGetAttributes(&fa, k_conv3_bulk));
     static_smem = (int)fa.sharedSizeBytes;
   }
-  const BkPlan plan = bk_plan(ci, co, static_smem);
+  const BkPlan plan = bk_plan(ci, co, n3, static_smem);
   if (plan.stages < 2) return xf_fail(ctx, XF_ERR_ARG, "convolution: no stacked-tap plan");
   XF_CUDA(ctx, set_max_smem((const void*)k_conv3_bulk, 0, ctx->device, (size_t)plan.smem_bytes));
   const int64_t tiles = (a.ncell + 125) / 126;
