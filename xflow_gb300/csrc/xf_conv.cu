@@ -707,21 +707,26 @@ static cudaError_t set_max_smem(const void* kern, int which, int device, size_t 
 // With the activations in channel planes, 8 consecutive cells of one plane
 // are also the canonical MN-major core matrix (8 channels along M or N, one
 // cell per 16-byte row along K), so the sum over cells is the K dimension of
-// an MMA: M = 128 rows of stacked (tap, input channel) pairs (128 / ci taps per
-// row tile), N = co, A = the shifted x blocks, B = g.  A stage is 128 cells:
-// per (tap, plane) of the row tile and per plane of g one 2 KB bulk copy (one
-// per lane of the producer warp), eight MMAs of K = 16 cells.  Each CTA takes
-// one row tile and one range of cells (a multiple of 128: the cells past the
-// box read the zero margins), accumulates in TMEM, and writes its FP32
-// partial; k_wgrad_tc_sum adds the ranges in a fixed order (deterministic).
+// an MMA: M = 128 rows of stacked (di, dj, input channel) groups of 8, N = co, A
+// = the shifted x blocks, B = g.  The three dk of a (di, dj) read the same block
+// of 130 cells a cell (16 bytes) apart, into accumulators of their own: a row
+// tile of single taps copied every block three times, and the copies were what
+// bound it (48 -> 16 at 66^3: 880 MB from L2 in 107 us, now 280 MB in 77; 96 -> 32
+// at 34^3 58 -> 27).  Now the MMAs do, about 60 cycles each.  A stage is 128 cells:
+// per group of the row tile and per plane of g one bulk copy (one per lane of
+// the producer warp), eight K steps of 16 cells, three MMAs each.  Each CTA
+// takes one row tile and one range of cells (a multiple of 128: the cells past
+// the box read the zero margins), accumulates in TMEM, and writes its FP32
+// partials where the sum looks for them: [tile of 128 / ci taps][range][row];
+// k_grad_sum adds the ranges in a fixed order (deterministic).  Groups past
+// the last compute on whatever the stage holds, in rows that nothing reads.
 // Descriptors: no swizzle, MN-major (instruction descriptor bits 15 and 16),
 // LBO = the K-direction core-matrix stride (128 bytes), SBO = the MN-direction
-// stride (2 KB).
+// stride (a block).
 constexpr int WG_KC = 128;                         // cells per stage
 constexpr int WG_STAGES = 3;
-constexpr uint32_t WG_BLOCK = WG_KC * 16;          // one (tap, plane) block of a stage
-constexpr uint32_t WG_A = 16 * WG_BLOCK;           // the row tile's A region (16 blocks)
-
+constexpr uint32_t WG_BLOCK = WG_KC * 16;          // one plane of g of a stage
+constexpr uint32_t WG_GROUP = (WG_KC + 2) * 16;    // one (di, dj, plane) group
 struct WgArgs {
   const uint16_t* g;   // plane 0, cell 0
   int64_t gps;
@@ -730,7 +735,9 @@ struct WgArgs {
   int64_t xps;
   int ci;
   int n2, n3;
-  int taps, mtiles, splits, stages;   // taps per row tile, row tiles, cell ranges, stages per range
+  int taps, splits, stages;      // of the partials: taps a tile, cell ranges; stages a range
+  int tiles, per_tile;           // row tiles here, groups a tile
+  uint32_t a_bytes;              // A's part of a stage
   int64_t chunks;                      // 128-cell stages in all
   uint32_t stage_bytes;
   float* partial;   // [mtile][split][128][co]
@@ -743,12 +750,12 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int mt = blockIdx.x % a.mtiles, sp = blockIdx.x / a.mtiles;
-  const int cp = a.ci / 8, t0 = mt * a.taps, tn = min(27, t0 + a.taps) - t0;
-  const int ga = tn * cp, gb = a.co / 8;   // blocks of A and of B per stage
+  const int mt = blockIdx.x % a.tiles, sp = blockIdx.x / a.tiles;
+  const int cp = a.ci / 8, g0 = mt * a.per_tile;
+  const int ga = min(9 * cp - g0, a.per_tile), gb = a.co / 8;   // blocks of A and of B per stage
   const uint32_t raw = tc::smem_addr(dsm);
   uint8_t* smem = dsm + ((1024u - (raw & 1023u)) & 1023u);
-  const uint32_t ncols = tmem_cols(a.co);
+  const uint32_t ncols = tmem_cols(3 * a.co);
   if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
   if (threadIdx.x == 0) {
     for (int st = 0; st < WG_STAGES; st++) {
@@ -773,16 +780,16 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
     const bool is_a = lane < ga, is_b = lane >= ga && lane < ga + gb;
     const uint16_t* src = nullptr;
     uint32_t dst_off = 0;
-    if (is_a) {
-      const int t = t0 + lane / cp, q = lane % cp;
-      const int64_t off = (t / 9 - 1) * P + ((t / 3) % 3 - 1) * (int64_t)a.n3 + (t % 3 - 1);
-      src = a.x + q * a.xps + off * 8;
-      dst_off = (uint32_t)lane * WG_BLOCK;
+    if (is_a) {   // from the cell before the range's first
+      const int dij = (g0 + lane) / cp, q = (g0 + lane) % cp;
+      src = a.x + q * a.xps + ((dij / 3 - 1) * P + (dij % 3 - 1) * (int64_t)a.n3 - 1) * 8;
+      dst_off = (uint32_t)lane * WG_GROUP;
     } else if (is_b) {
       const int q = lane - ga;
       src = a.g + q * a.gps;
-      dst_off = WG_A + (uint32_t)q * WG_BLOCK;
+      dst_off = a.a_bytes + (uint32_t)q * WG_BLOCK;
     }
+    const uint32_t bytes = is_a ? WG_GROUP : WG_BLOCK;
     int st = 0, pass = 0, issued = 0;
     for (int k = 0; k < my_stages; k++) {
       if (pass > 0) {
@@ -791,8 +798,8 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
         if (!__shfl_sync(0xffffffffu, w, 0)) break;
       }
       uint8_t* sa = smem + st * a.stage_bytes;
-      if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)(ga + gb) * WG_BLOCK);
-      if (is_a || is_b) bulk_load(sa + dst_off, src + (cell0 + (int64_t)k * WG_KC) * 8, WG_BLOCK, &full[st]);
+      if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)ga * WG_GROUP + (uint32_t)gb * WG_BLOCK);
+      if (is_a || is_b) bulk_load(sa + dst_off, src + (cell0 + (int64_t)k * WG_KC) * 8, bytes, &full[st]);
       issued++;
       if (++st == WG_STAGES) {
         st = 0;
@@ -816,9 +823,12 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
         const uint8_t* sa = smem + st * a.stage_bytes;
 #pragma unroll
         for (int kk = 0; kk < WG_KC / 16; kk++) {
-          const uint64_t ad = tc::smem_desc(tc::smem_addr(sa + kk * 256), 128, WG_BLOCK);
-          const uint64_t bd = tc::smem_desc(tc::smem_addr(sa + WG_A + kk * 256), 128, WG_BLOCK);
-          if (leader) tc::mma_bf16(tbase, ad, bd, idesc, k > 0 || kk > 0);
+          const uint64_t bd = tc::smem_desc(tc::smem_addr(sa) + a.a_bytes + (uint32_t)kk * 256u, 128, WG_BLOCK);
+#pragma unroll
+          for (int dk = 0; dk < 3; dk++) {
+            const uint64_t ad = tc::smem_desc(tc::smem_addr(sa) + (uint32_t)kk * 256u + (uint32_t)dk * 16u, 128, WG_GROUP);
+            if (leader) tc::mma_bf16(tbase + (uint32_t)(dk * a.co), ad, bd, idesc, k > 0 || kk > 0);
+          }
         }
         if (leader) tc::mma_commit(&empty[st]);
         if (++st == WG_STAGES) {
@@ -834,13 +844,18 @@ __global__ void __launch_bounds__(BK_THREADS) k_wgrad_tc(WgArgs a) {
     const bool got = bk_wait(&mdone, 0, abort_p, false);
     if (__all_sync(0xffffffffu, got) && !*abort_p) {
       tc::fence_after_sync();
-      const int row = warp * 32 + lane;
-      float* dst = a.partial + (((int64_t)mt * a.splits + sp) * 128 + row) * a.co;
-      for (int co = 0; co < a.co; co += 8) {
-        float v[8];
-        tc::tmem_ld8(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)co, v);
-        *reinterpret_cast<float4*>(dst + co) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4*>(dst + co + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      const int row = warp * 32 + lane, grp = g0 + (row >> 3);
+      const bool live = (row >> 3) < ga;
+      for (int dk = 0; dk < 3; dk++) {
+        const int t = grp / cp * 3 + dk, r = (t % a.taps) * a.ci + grp % cp * 8 + (row & 7);
+        float* dst = a.partial + (((int64_t)(t / a.taps) * a.splits + sp) * 128 + r) * a.co;
+        for (int co = 0; co < a.co; co += 8) {
+          float v[8];
+          tc::tmem_ld8(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dk * a.co + co), v);
+          if (!live) continue;
+          *reinterpret_cast<float4*>(dst + co) = make_float4(v[0], v[1], v[2], v[3]);
+          *reinterpret_cast<float4*>(dst + co + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        }
       }
     }
   }
@@ -963,15 +978,21 @@ int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps,
   a.x = (const uint16_t*)x; a.xps = xps; a.ci = ci;
   a.n2 = n2; a.n3 = n3;
   int64_t pf = 0;
-  xf_wgrad_tc_plan(ctx, (int64_t)n1 * n2 * n3, ci, co, &a.mtiles, &a.splits, &a.stages, &pf);
+  int mtiles;
+  xf_wgrad_tc_plan(ctx, (int64_t)n1 * n2 * n3, ci, co, &mtiles, &a.splits, &a.stages, &pf);
   a.taps = 128 / ci;
+  const int groups = 9 * (ci / 8);
+  a.tiles = (groups + 15) / 16;
+  a.per_tile = (groups + a.tiles - 1) / a.tiles;
+  a.a_bytes = ((uint32_t)a.per_tile * WG_GROUP + 127) / 128 * 128;
   a.chunks = ((int64_t)n1 * n2 * n3 + WG_KC - 1) / WG_KC;
-  a.stage_bytes = (WG_A + (uint32_t)co / 8 * WG_BLOCK + 1023) / 1024 * 1024;
+  a.stage_bytes = (a.a_bytes + (uint32_t)co / 8 * WG_BLOCK + 1023) / 1024 * 1024;
   a.partial = partial;
   a.err = conv_err_flag(ctx);
-  const size_t smem = (size_t)WG_STAGES * a.stage_bytes + 1024;
+  // the last stage's rows of absent groups lie past it, in memory of the block's own
+  const size_t smem = (size_t)WG_STAGES * a.stage_bytes + 1024 + 16 * WG_GROUP;
   XF_CUDA(ctx, set_max_smem((const void*)k_wgrad_tc, 1, ctx->device, smem));
-  launch_dep(k_wgrad_tc, dim3((unsigned)(a.mtiles * a.splits)), BK_THREADS, smem, ctx->stream, a);
+  launch_dep(k_wgrad_tc, dim3((unsigned)(a.tiles * a.splits)), BK_THREADS, smem, ctx->stream, a);
   int nchunk, chunk;
   xf_bgrad_plan((int64_t)n1 * n2 * n3, &nchunk, &chunk);
   launch_dep(k_bgrad, dim3((unsigned)nchunk, (unsigned)(co / 8)), 256, 0, ctx->stream, a.g, gps, (int64_t)n1 * n2 * n3,
