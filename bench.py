@@ -457,9 +457,9 @@ def main(argv=None):
            "tl_prolong_ay_f32": 9, "tl_first_f32": 9, "tl_last_f32": 17}
     # the learned two-level iteration's fine-grid passes: r' = r - omega A P zc,
     # the smoother's first and last factor passes (TL_DEGREE / 2 - 2 middle
-    # passes between them), and the FP32 stencil with a dot for A p
+    # passes between them), and the direction pass with A p
     per_iter = {"tl_prolong_ay_f32": 1, "tl_first_f32": 1, "tl_last_f32": 1, "cheb_middle_f32": TL_DEGREE // 2 - 2,
-                "stencil_f32": 1}
+                "pq_fused_f32": 1}
     peak, peak_kind = peaks()
     kernels = {k: {"ms": kms[k], "bytes_per_cell": bpc[k], "GB_s": ncell * bpc[k] / (kms[k] * 1e-3) / 1e9,
                    "frac": ncell * bpc[k] / (kms[k] * 1e-3) / 1e9 / peak} for k in kms}

@@ -79,29 +79,44 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_xr(T* __restrict__ x, T* __r
   if (p_alt && S->iscalars[I_PBUF]) p = p_alt;
   typedef typename V16<T>::type VT;
   constexpr int L = 16 / sizeof(T);
-  const T alpha = (T)S->scalars[D_ALPHA];
+  const T alpha = (T)S->scalars[D_ALPHA], back = xneg(alpha);
   DotAcc<T> acc;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t nv = n / L;
-  for (int64_t v = tid; v < nv; v += stride) {
-    VT xv = reinterpret_cast<const VT*>(x)[v], rv = reinterpret_cast<const VT*>(r)[v];
-    const VT pv = reinterpret_cast<const VT*>(p)[v], qv = reinterpret_cast<const VT*>(q)[v];
-    T* xa = reinterpret_cast<T*>(&xv);
-    T* ra = reinterpret_cast<T*>(&rv);
-    const T* pa = reinterpret_cast<const T*>(&pv);
-    const T* qa = reinterpret_cast<const T*>(&qv);
+  // FP64 takes four rounds at a time, their sixteen loads issued together (258^3: 125 us, 132 one by one);
+  // FP32 has more warps an SM instead.
+  constexpr int U = sizeof(T) == 8 ? 4 : 1;
+  auto rounds = [&](auto nr, int64_t v) {
+    constexpr int R = decltype(nr)::value;
+    VT xv[R], rv[R], pv[R], qv[R];
 #pragma unroll
-    for (int l = 0; l < L; l++) {
-      xa[l] = fma(alpha, pa[l], xa[l]);
-      ra[l] = fma(xneg(alpha), qa[l], ra[l]);
-      acc.add(ra[l], ra[l]);
+    for (int u = 0; u < R; u++) {
+      xv[u] = reinterpret_cast<const VT*>(x)[v + u * stride], rv[u] = reinterpret_cast<const VT*>(r)[v + u * stride];
+      pv[u] = reinterpret_cast<const VT*>(p)[v + u * stride], qv[u] = reinterpret_cast<const VT*>(q)[v + u * stride];
     }
-    reinterpret_cast<VT*>(x)[v] = xv;
-    reinterpret_cast<VT*>(r)[v] = rv;
-  }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      T* xa = reinterpret_cast<T*>(&xv[u]);
+      T* ra = reinterpret_cast<T*>(&rv[u]);
+      const T* pa = reinterpret_cast<const T*>(&pv[u]);
+      const T* qa = reinterpret_cast<const T*>(&qv[u]);
+#pragma unroll
+      for (int l = 0; l < L; l++) {
+        xa[l] = fma(alpha, pa[l], xa[l]);
+        ra[l] = fma(back, qa[l], ra[l]);
+        acc.add(ra[l], ra[l]);
+      }
+      reinterpret_cast<VT*>(x)[v + u * stride] = xv[u];
+      reinterpret_cast<VT*>(r)[v + u * stride] = rv[u];
+    }
+  };
+  int64_t v = tid;
+  if constexpr (U > 1)
+    for (; v + (U - 1) * stride < nv; v += U * stride) rounds(std::integral_constant<int, U>(), v);
+  for (; v < nv; v += stride) rounds(std::integral_constant<int, 1>(), v);
   for (int64_t c = nv * L + tid; c < n; c += stride) {
     x[c] = fma(alpha, p[c], x[c]);
-    T rv = fma(xneg(alpha), q[c], r[c]);
+    T rv = fma(back, q[c], r[c]);
     r[c] = rv;
     acc.add(rv, rv);
   }
@@ -711,9 +726,7 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
   double* tmp = B.get<double>(n, false);
   if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate residual");
   for (int attempt = 0; attempt < 3; attempt++) {
-    reset_progress(ctx);
-    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit - total_it, o.replace_every, mixed ? 1 : 0,
-                                            mixed ? 0 : 1);
+    k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit - total_it, o.replace_every, mixed ? 1 : 0);
     k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(b, b, g->smask, n, S, SL_B, CTL_NONE, 0);
     std::function<void(int)> iter;
     int chunk = o.replace_every;
@@ -865,8 +878,10 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
     }
     if (mixed) xf_op_ready32(op);   // not inside the captured iterations
     XF_CUDA(ctx, cudaGetLastError());
-    int rc = mixed ? run_loop(ctx, iter, chunk, o.maxit - total_it, &hs)
-                   : run_stream(ctx, iter, 3, STREAM_AHEAD, o.maxit - total_it, &hs);
+    // grids beyond the resident kernel take hundreds of iterations: a graph's
+    // closer launches pay for its making (FP64 CG at 128^3, 822 iterations: 59 ms,
+    // 65 by run_stream)
+    int rc = run_loop(ctx, iter, chunk, o.maxit - total_it, &hs);
     if (rc) return rc;
     hs.kernels += 3 + (mixed ? 1 : 0) + 2;
     if (mixed) {
