@@ -111,8 +111,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_cg_xr(T* __restrict__ x, T* __r
     }
   };
   int64_t v = tid;
-  if constexpr (U > 1)
+  if constexpr (U > 1) {
     for (; v + (U - 1) * stride < nv; v += U * stride) rounds(std::integral_constant<int, U>(), v);
+    if (v + (U / 2 - 1) * stride < nv) rounds(std::integral_constant<int, U / 2>(), v), v += U / 2 * stride;
+  }
   for (; v < nv; v += stride) rounds(std::integral_constant<int, 1>(), v);
   for (int64_t c = nv * L + tid; c < n; c += stride) {
     x[c] = fma(alpha, p[c], x[c]);
@@ -729,7 +731,7 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
     k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit - total_it, o.replace_every, mixed ? 1 : 0);
     k_dot_ctl<double><<<rb, RED_THREADS, 0, ctx->stream>>>(b, b, g->smask, n, S, SL_B, CTL_NONE, 0);
     std::function<void(int)> iter;
-    int chunk = o.replace_every;
+    int chunk = mixed ? o.replace_every : o.check_every > 0 ? o.check_every : 16;
     const bool lap = op->kind == XF_OP_LAPLACE;
     if (!mixed) {
       MvReq<double> m0;
@@ -879,8 +881,8 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
     if (mixed) xf_op_ready32(op);   // not inside the captured iterations
     XF_CUDA(ctx, cudaGetLastError());
     // grids beyond the resident kernel take hundreds of iterations: a graph's
-    // closer launches pay for its making (FP64 CG at 128^3, 822 iterations: 59 ms,
-    // 65 by run_stream)
+    // closer launches pay for its making (FP64 CG at 128^3, 815 iterations: 58 ms,
+    // 65 launched one by one)
     int rc = run_loop(ctx, iter, chunk, o.maxit - total_it, &hs);
     if (rc) return rc;
     hs.kernels += 3 + (mixed ? 1 : 0) + 2;
