@@ -554,6 +554,7 @@ int column_form(int bi) { return (bi + 1) / 2 * 2; }
 // long columns leave few warps to hide it), a halo cell by a third (a copy and
 // an FMA against the row's work), a block by half a cell (the polls).
 constexpr int CC_LENGTH = 48;
+constexpr size_t CC_SMEM[2] = {205 * 1024, 215 * 1024};   // dynamic shared memory at most, beside the static part: FP64, mixed
 bool make_plan(int ni, int nj, int nk, int blocks, bool mixed, Plan* out) {
   double best = 1e300;
   const int top = blocks < CC_MAX_BLOCKS ? blocks : CC_MAX_BLOCKS;
@@ -570,7 +571,7 @@ bool make_plan(int ni, int nj, int nk, int blocks, bool mixed, Plan* out) {
         const int64_t box = (int64_t)(K + 2) * (bj + 2) * (bk + 2);
         const size_t smem = (size_t)K * threads * (mixed ? 4 : 8) + ((box + 1) & ~1ll) * (mixed ? 4 : 8) +
                             2ll * bi * (bj + bk) * (8 + (mixed ? 4 : 8));
-        if (smem > (mixed ? 215 : 205) * 1024) continue;   // beside the static part
+        if (smem > CC_SMEM[mixed]) continue;
         const double cost = (double)(cells > CC_THREADS / 2 ? cells : CC_THREADS / 2) + CC_LENGTH * K + 0.3 * halo +
                             0.5 * mi * mj * mk;
         if (cost < best) {
@@ -632,7 +633,9 @@ int xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const e
   a.cx = g->ucx; a.cy = g->ucy; a.cz = g->ucz; a.rtol = rtol; a.maxit = maxit; a.every = every;
   XF_CUDA(ctx, cudaMemsetAsync(slots, 0, xf_cg_coop_slots() * sizeof(double), ctx->stream));
   const void* f = mixed ? kernel_for<float>(p.bi) : kernel_for<double>(p.bi);
-  XF_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  // The attribute is the kernel's, whatever context sets it, and plans of different sizes share a kernel: always
+  // the same value, so that no thread lowers it under another's launch.
+  XF_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM[mixed]));
   void* args[] = {&a};
   XF_CUDA(ctx, cudaLaunchCooperativeKernel(f, dim3(p.mi * p.mj * p.mk), dim3(p.threads), args, p.smem, ctx->stream));
   return XF_OK;
