@@ -618,25 +618,31 @@ bool xf_cg_coop_supported(const xf_op* op, bool mixed) {
 // The whole solve, for a supported operator.  ex: two boxes of float (mixed)
 // or double; slots: xf_cg_coop_slots() doubles.  The state (status,
 // iterations, replacements, the true residual and (b, b)) is left in the
-// context's scratch.
+// context's scratch.  False where the driver refuses the cooperative launch
+// (nothing of the solve has run then): the grid keeps to the kernel chain from
+// there on.
 size_t xf_cg_coop_slots() { return 2 * CC_VALUES * CC_MAX_BLOCKS + 1; }
 
-int xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
-                      int maxit, int every) {
-  const xf_grid* g = op->g;
+bool xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
+                       int maxit, int every) {
+  xf_grid* g = op->g;
   xf_ctx* ctx = g->ctx;
-  const Plan& p = g->coop[mixed];
+  Plan& p = g->coop[mixed];
   CoopArgs a;
   a.n1 = g->n1; a.n2 = g->n2; a.n3 = g->n3;
   a.bi = p.bi; a.bj = p.bj; a.bk = p.bk; a.mj = p.mj; a.mk = p.mk;
   a.kind = g->kind; a.b = b; a.x = x; a.ex0 = ex[0]; a.ex1 = ex[1]; a.slots = reinterpret_cast<unsigned long long*>(slots); a.S = ctx->scratch;
   a.cx = g->ucx; a.cy = g->ucy; a.cz = g->ucz; a.rtol = rtol; a.maxit = maxit; a.every = every;
-  XF_CUDA(ctx, cudaMemsetAsync(slots, 0, xf_cg_coop_slots() * sizeof(double), ctx->stream));
   const void* f = mixed ? kernel_for<float>(p.bi) : kernel_for<double>(p.bi);
+  void* args[] = {&a};
   // The attribute is the kernel's, whatever context sets it, and plans of different sizes share a kernel: always
   // the same value, so that no thread lowers it under another's launch.
-  XF_CUDA(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM[mixed]));
-  void* args[] = {&a};
-  XF_CUDA(ctx, cudaLaunchCooperativeKernel(f, dim3(p.mi * p.mj * p.mk), dim3(p.threads), args, p.smem, ctx->stream));
-  return XF_OK;
+  cudaError_t e = cudaMemsetAsync(slots, 0, xf_cg_coop_slots() * sizeof(double), ctx->stream);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CC_SMEM[mixed]);
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel(f, dim3(p.mi * p.mj * p.mk), dim3(p.threads), args, p.smem, ctx->stream);
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  p.state = -1;
+  return false;
 }

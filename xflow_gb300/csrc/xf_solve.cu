@@ -49,8 +49,8 @@ void xf_cg_pq32_variant(const xf_op* op, const float* r, float* pb0, float* pb1,
 bool xf_cg_pqt_supported(const xf_grid* g);
 bool xf_cg_coop_supported(const xf_op* op, bool mixed);
 size_t xf_cg_coop_slots();
-int xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
-                      int maxit, int every);
+bool xf_cg_coop_launch(const xf_op* op, double* x, const double* b, void* const ex[2], double* slots, bool mixed, double rtol,
+                       int maxit, int every);
 int xf_op_ready(const xf_op* op);
 void xf_op_ready32(const xf_op* op);
 int xf_op_jacobi(const xf_op* op, const double** dinv);
@@ -641,8 +641,10 @@ static int true_residual(const xf_op* op, const double* x, const double* b, doub
 // ---------------------------------------------------------------------------
 // The whole CG solve as one resident kernel (xf_cgc.cu), for the grids that
 // fit the chip.  The kernel's own last residual is the true one except where
-// the solve broke off between two of them.
-static int solve_cg_coop(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec* bv, xf_solve_stats* st) {
+// the solve broke off between two of them.  refused: the launch could not be
+// had, and nothing has been solved.
+static int solve_cg_coop(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec* bv, xf_solve_stats* st,
+                         bool* refused) {
   xf_ctx* ctx = op->g->ctx;
   DevScratch* S = ctx->scratch;
   const int64_t n = op->g->ncell;
@@ -655,8 +657,9 @@ static int solve_cg_coop(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf
   double* slots = B.get<double>((int64_t)xf_cg_coop_slots(), false);
   if (!ex[0] || !ex[1] || !slots) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: cannot allocate CG vectors");
   k_reset_state<<<1, 1, 0, ctx->stream>>>(S, o.rtol * o.rtol, 0.0, o.maxit, o.replace_every, mixed ? 1 : 0);
-  int rc = xf_cg_coop_launch(op, x, b, ex, slots, mixed, o.rtol, o.maxit, o.replace_every);
-  if (rc) return rc;
+  *refused = !xf_cg_coop_launch(op, x, b, ex, slots, mixed, o.rtol, o.maxit, o.replace_every);
+  if (*refused) return XF_OK;
+  int rc;
   long long I[16];
   double D[32];
   XF_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, S->iscalars, sizeof(I), cudaMemcpyDeviceToHost, ctx->stream));
@@ -692,8 +695,11 @@ static int solve_cg(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const xf_vec*
   const double* b = (const double*)bv->data;
   // XF_PQ_FUSE and XF_PQT name kernels of the launch chain
   if (o.precond != XF_PRECOND_CHEB && x != b && !getenv("XF_PQ_FUSE") && !getenv("XF_PQT") &&
-      xf_cg_coop_supported(op, mixed))
-    return solve_cg_coop(op, o, xv, bv, st);
+      xf_cg_coop_supported(op, mixed)) {
+    bool refused = false;
+    const int rc = solve_cg_coop(op, o, xv, bv, st, &refused);
+    if (!refused) return rc;
+  }
   Bufs B(ctx);
   const int rb = red_blocks(ctx, n), eb = grid_blocks(ctx, n, 256);
   const int xb32 = xr_blocks<float>(ctx, n), xb64 = xr_blocks<double>(ctx, n);
