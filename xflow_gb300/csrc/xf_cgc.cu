@@ -19,7 +19,12 @@
 //
 // One sum an iteration: with alpha = (r, r) / (p, q), the next (r, r) is
 // (r, r) - 2 alpha (r, q) + alpha^2 (q, q), so beta and the stop test need no
-// second one; (r, r) is measured again each time, so nothing drifts.  Only q
+// second one; (r, r) is measured again each time, so nothing drifts.  Where it
+// falls a thousandfold in one FP64 step, as it does when CG has come to the end
+// of its space, too few bits of that difference are left: the true residual is
+// taken there and the direction goes on from it (without it, right-hand sides of
+// 1 to 5 eigenvectors took an iteration more than with a measured (r, r)).  The
+// mixed solve's sums carry more than its FP32 residual does.  Only q
 // travels: a block keeps r and p of its halo and forms them as their owner
 // does, from the same bits.
 //
@@ -39,7 +44,7 @@
 //
 // The mixed solve folds e into the FP64 iterate and takes r = b - A x in FP64
 // every `every` iterations and whenever the FP32 recursion meets the
-// tolerance; the FP64 solve takes its true residual at the end and starts
+// tolerance; the FP64 solve takes its true residual at the end too and starts
 // again from it while that misses the tolerance (three times at most).
 #include <math.h>
 
@@ -53,6 +58,7 @@ constexpr int CC_KMAX = 16;               // cells of a column at most: 128 regi
 constexpr int CC_HALO = 4;                // halo loads a thread keeps in flight
 constexpr int CC_MAX_BLOCKS = 256;
 constexpr uint32_t CC_SPIN_LIMIT = 1u << 22;
+constexpr double CC_CANCEL = 1.0 / 1024;   // FP64: the recurrence of (r, r) is taken down to this part of it
 
 struct CoopArgs {
   int n1, n2, n3;
@@ -241,7 +247,7 @@ template <typename T>
 struct CoopState {
   double rr_prev, rr_true, bb, thr;
   T alpha, beta;
-  int it, repl, since, starts, fail, next, floor32;
+  int it, repl, since, starts, fail, next, floor32, cancel;
   long long status;
 };
 
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
 
   if (t == 0) {
     st.fail = 0;
-    st.it = st.repl = st.since = st.starts = st.floor32 = 0;
+    st.it = st.repl = st.since = st.starts = st.floor32 = st.cancel = 0;
     st.status = XF_OK;
     st.alpha = st.beta = T(0);
   }
@@ -500,7 +506,8 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
       }
       st.rr_prev = rr;
       st.beta = rn > 0.0 ? (T)(rn / rr) : T(0);
-      if (rn <= st.thr || st.it >= a.maxit || (MIXED && st.since >= a.every)) st.next = CC_REPLACE;
+      st.cancel = !MIXED && rn < CC_CANCEL * rr;
+      if (rn <= st.thr || st.cancel || st.it >= a.maxit || (MIXED && st.since >= a.every)) st.next = CC_REPLACE;
     });
     if (!st.fail && st.next == CC_REPLACE) {   // take the step; the true residual of the iterate
       const T al = st.alpha;
@@ -517,11 +524,11 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
         if (isnan(v)) st.status = XF_NAN;
         else if (met(v)) return;
         else if (st.it >= a.maxit) st.status = XF_MAXIT;
-        else if (!MIXED && ++st.starts >= 3) return;
+        else if (!MIXED && !st.cancel && ++st.starts >= 3) return;
         else {
-          // mixed: the direction goes on from the replaced residual; FP64: the recursive
-          // residual has drifted, the solve starts again from the iterate
-          st.beta = MIXED && !st.floor32 ? (T)(v / st.rr_prev) : T(0);
+          // mixed, and after a cancelled recurrence: the direction goes on from the replaced residual; FP64: the
+          // recursive residual has drifted, the solve starts again from the iterate
+          st.beta = (MIXED || st.cancel) && !st.floor32 ? (T)(v / st.rr_prev) : T(0);
           st.next = CC_GO;
         }
       });
