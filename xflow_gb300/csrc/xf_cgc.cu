@@ -20,11 +20,11 @@
 // One sum an iteration: with alpha = (r, r) / (p, q), the next (r, r) is
 // (r, r) - 2 alpha (r, q) + alpha^2 (q, q), so beta and the stop test need no
 // second one; (r, r) is measured again each time, so nothing drifts.  Where it
-// falls a thousandfold in one FP64 step, as it does when CG has come to the end
-// of its space, too few bits of that difference are left: the true residual is
+// falls a thousandfold in one step, as it does when CG has come to the end of
+// its space, too few bits of that difference are left: the true residual is
 // taken there and the direction goes on from it (without it, right-hand sides of
-// 1 to 5 eigenvectors took an iteration more than with a measured (r, r)).  The
-// mixed solve's sums carry more than its FP32 residual does.  Only q
+// 1 to 5 eigenvectors took an iteration more in FP64 than with a measured (r, r)).
+// Only q
 // travels: a block keeps r and p of its halo and forms them as their owner
 // does, from the same bits.
 //
@@ -45,7 +45,15 @@
 // The mixed solve folds e into the FP64 iterate and takes r = b - A x in FP64
 // every `every` iterations and whenever the FP32 recursion meets the
 // tolerance; the FP64 solve takes its true residual at the end too and starts
-// again from it while that misses the tolerance (three times at most).
+// again from it while that misses the tolerance (three times at most).  The
+// mixed solve's direction goes on from a replaced residual, but where the true
+// (r, r) is twice the recursion's, or misses a tolerance that the recursion
+// meets, the recursion was rounding and its direction is worth nothing: it starts
+// again too.  (Kept, the direction took smooth right-hand sides at 1e-12 away
+// from the solution: 18 of 40 solves between 40 x 36 x 44 and 128 x 64 x 64 ran
+// to a cap of 4,000 iterations, now none, 830 on average; right-hand sides of
+// 1 to 7 eigenvectors met 1e-9 in none of 15, now in 76 iterations on average.
+// Right-hand sides of noise take as many iterations as before.)
 #include <math.h>
 
 #include "xf_control.cuh"
@@ -58,7 +66,8 @@ constexpr int CC_KMAX = 16;               // cells of a column at most: 128 regi
 constexpr int CC_HALO = 4;                // halo loads a thread keeps in flight
 constexpr int CC_MAX_BLOCKS = 256;
 constexpr uint32_t CC_SPIN_LIMIT = 1u << 22;
-constexpr double CC_CANCEL = 1.0 / 1024;   // FP64: the recurrence of (r, r) is taken down to this part of it
+constexpr double CC_CANCEL = 1.0 / 1024;   // the recurrence of (r, r) is taken down to this part of it
+constexpr double CC_DRIFT = 2.0;           // mixed: a true (r, r) beyond this many of the recursion's starts the direction again
 
 struct CoopArgs {
   int n1, n2, n3;
@@ -245,7 +254,7 @@ __device__ __forceinline__ double cc_residual(const CoopArgs& a, const double* d
 enum { CC_GO, CC_REPLACE, CC_STOP };
 template <typename T>
 struct CoopState {
-  double rr_prev, rr_true, bb, thr;
+  double rr_prev, rr_next, rr_true, bb, thr;
   T alpha, beta;
   int it, repl, since, starts, fail, next, floor32, cancel;
   long long status;
@@ -506,7 +515,8 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
       }
       st.rr_prev = rr;
       st.beta = rn > 0.0 ? (T)(rn / rr) : T(0);
-      st.cancel = !MIXED && rn < CC_CANCEL * rr;
+      st.rr_next = rn;
+      st.cancel = rn < CC_CANCEL * rr;
       if (rn <= st.thr || st.cancel || st.it >= a.maxit || (MIXED && st.since >= a.every)) st.next = CC_REPLACE;
     });
     if (!st.fail && st.next == CC_REPLACE) {   // take the step; the true residual of the iterate
@@ -526,9 +536,10 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
         else if (st.it >= a.maxit) st.status = XF_MAXIT;
         else if (!MIXED && !st.cancel && ++st.starts >= 3) return;
         else {
-          // mixed, and after a cancelled recurrence: the direction goes on from the replaced residual; FP64: the
-          // recursive residual has drifted, the solve starts again from the iterate
-          st.beta = (MIXED || st.cancel) && !st.floor32 ? (T)(v / st.rr_prev) : T(0);
+          // mixed, and after a cancelled recurrence: the direction goes on from the replaced residual, unless the
+          // recursive one has drifted from it: then the solve starts again from the iterate
+          const bool on = st.cancel || (MIXED && !st.floor32 && st.rr_next > st.thr && v <= CC_DRIFT * st.rr_next);
+          st.beta = on ? (T)(v / st.rr_prev) : T(0);
           st.next = CC_GO;
         }
       });
