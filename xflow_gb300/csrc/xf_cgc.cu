@@ -54,6 +54,13 @@
 // to a cap of 4,000 iterations, now none, 830 on average; right-hand sides of
 // 1 to 7 eigenvectors met 1e-9 in none of 15, now in 76 iterations on average.
 // Right-hand sides of noise take as many iterations as before.)
+//
+// r, p, q and the iterate (mixed: e) are kept times a power of two, exact
+// wherever nothing under- or overflows, that puts the norms of r between the
+// first and the last, rtol |b|, around 1: the sums of squares stay in range, in
+// FP32 for any |b| (without it, a mixed solve of |b| = 1e-14 or below ended in
+// NaN, and an FP64 one of 1e150).  A mixed solve that started further out than
+// that takes a new power, and a new direction, once r is small.
 #include <math.h>
 
 #include "xf_control.cuh"
@@ -67,6 +74,7 @@ constexpr int CC_HALO = 4;                // halo loads a thread keeps in flight
 constexpr int CC_MAX_BLOCKS = 256;
 constexpr uint32_t CC_SPIN_LIMIT = 1u << 22;
 constexpr double CC_CANCEL = 1.0 / 1024;   // the recurrence of (r, r) is taken down to this part of it
+constexpr double CC_LOW = 0x1p-60;         // mixed: a (r, r) in its scale below which the scale is taken anew
 constexpr double CC_DRIFT = 2.0;           // mixed: a true (r, r) beyond this many of the recursion's starts the direction again
 
 struct CoopArgs {
@@ -250,11 +258,19 @@ __device__ __forceinline__ double cc_residual(const CoopArgs& a, const double* d
   return a.b[c] - fma(dtab[kb & 63], __ldcg(x + c), xneg(s));
 }
 
+// The power of two for a solve from (r, r) = v down to `end`: the first norm of r a half of the way above 1, but no more
+// than 2^20, for the sake of (q, q).
+__device__ __forceinline__ double cc_scale(double v, double end) {
+  auto log2 = [](double s) { return (__double2hiint(s) >> 20 & 0x7ff) - 1023; };
+  const int up = end > 0.0 ? max(0, min(20, (log2(v) - log2(end)) >> 2)) : 0;
+  return __hiloint2double((1023 + max(-500, min(500, up - (log2(v) >> 1)))) << 20, 0);
+}
+
 // The solve's scalars, thread 0's (shared memory; every block holds the same).
-enum { CC_GO, CC_REPLACE, CC_STOP };
+enum { CC_GO, CC_REPLACE, CC_AGAIN, CC_STOP };
 template <typename T>
 struct CoopState {
-  double rr_prev, rr_next, rr_true, bb, thr;
+  double rr_prev, rr_next, rr_true, bb, thr, scale;   // rr_prev, rr_next and thr in the scale of r
   T alpha, beta;
   int it, repl, since, starts, fail, next, floor32, cancel;
   long long status;
@@ -262,7 +278,7 @@ struct CoopState {
 
 // T: float the mixed solve, double the FP64 one.  K: cells a column.
 template <typename T, int K>
-__global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
+__global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(const __grid_constant__ CoopArgs a) {
   constexpr bool MIXED = sizeof(T) == 4;
   extern __shared__ double smem[];
   __shared__ double sh[16 * CC_VALUES];
@@ -293,6 +309,7 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
     st.it = st.repl = st.since = st.starts = st.floor32 = st.cancel = 0;
     st.status = XF_OK;
     st.alpha = st.beta = T(0);
+    st.scale = 0.0;
   }
   for (int q = t; q < 64; q += nt) {
     const T cx = (T)a.cx, cy = (T)a.cy, cz = (T)a.cz;
@@ -346,21 +363,33 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
   T r[K], q[K];
   const T cx = (T)a.cx, cy = (T)a.cy, cz = (T)a.cz;
   auto met = [&](double v) { return (st.bb > 0 ? sqrt(v / st.bb) : sqrt(v)) <= a.rtol; };
+  // whether the scale changes for a residual with (r, r) = v, which is then taken again (thread 0)
+  auto rescale = [&](double v) {
+    const double end = a.rtol * a.rtol * st.bb, now = cc_scale(v, end);
+    if (now == st.scale) return false;
+    st.scale = now;
+    st.thr = a.rtol * a.rtol * (st.bb * now * now);
+    st.next = CC_AGAIN;
+    return true;
+  };
   // r = b - A x from the box, (r, r) in FP64; by way of a box, so that this
   // rare step is a rolled loop that leaves the iteration its registers
   auto take_residual = [&](auto control) {
-    DotAcc<double> acc[1];
-    if (mine) {
+    do {
+      DotAcc<double> acc[1];
+      if (mine) {
+        const double scale = st.scale;
 #pragma unroll 1
-      for (int m = 0; m < ei; m++) {
-        const int c = c0 + m * s1, kb = a.kind[c];
-        double v = 0.0;
-        if (kb >> K_ROW_SHIFT == ROW_ACTUAL) v = cc_residual(a, dtab64, c, kb);
-        acc[0].add(v, v);
-        ex0[c] = (T)v;
+        for (int m = 0; m < ei; m++) {
+          const int c = c0 + m * s1, kb = a.kind[c];
+          double v = 0.0;
+          if (kb >> K_ROW_SHIFT == ROW_ACTUAL) v = cc_residual(a, dtab64, c, kb);
+          acc[0].add(v, v);
+          ex0[c] = (T)(scale * v);
+        }
       }
-    }
-    G.run(acc, sh, [&](const double (&v)[1]) { control(v[0]); });
+      G.run(acc, sh, [&](const double (&v)[1]) { control(v[0]); });
+    } while (!st.fail && st.next == CC_AGAIN);
 #pragma unroll
     for (int m = 0; m < K; m++) r[m] = m < eim ? __ldcg(ex0 + c0 + m * s1) : T(0);
     rlo = lo_in ? __ldcg(ex0 + c0 - s1) : T(0);
@@ -370,10 +399,14 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
   // the iterate of the active cells to the box (mixed: x += e)
   auto put_iterate = [&]() {
     if (!mine) return;
+    const double back = 1.0 / st.scale;
 #pragma unroll 1
     for (int m = 0; m < ei; m++) {
       const int c = c0 + m * s1;
-      if (a.kind[c] >> K_ROW_SHIFT == ROW_ACTUAL) a.x[c] = MIXED ? __ldcg(a.x + c) + (double)xs[m * nt + t] : (double)xs[m * nt + t];
+      if (a.kind[c] >> K_ROW_SHIFT == ROW_ACTUAL) {
+        const double v = back * (double)xs[m * nt + t];
+        a.x[c] = MIXED ? __ldcg(a.x + c) + v : v;
+      }
       if (MIXED) xs[m * nt + t] = T(0);
     }
   };
@@ -383,21 +416,26 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
 #pragma unroll 1
       for (int m = 0; m < ei; m++) {
         const int c = c0 + m * s1;
-        if (!MIXED) xs[m * nt + t] = (T)a.x[c];
         const double bv = a.kind[c] >> K_ROW_SHIFT == ROW_ACTUAL ? a.b[c] : 0.0;
         acc[0].add(bv, bv);
       }
     }
     G.run(acc, sh, [&](const double (&v)[1]) {
       st.bb = v[0];
-      st.thr = a.rtol * a.rtol * v[0];
+      rescale(v[0]);
     });
     take_residual([&](double v) {
-      st.rr_prev = st.rr_true = v;
+      st.rr_true = v;
       st.next = CC_GO;
+      if (rescale(v)) return;   // another first residual than b
       if (isnan(v)) { st.status = XF_NAN; st.next = CC_STOP; }
-      else if (v <= st.thr) st.next = CC_STOP;
+      else if (v <= a.rtol * a.rtol * st.bb) st.next = CC_STOP;
     });
+    if (!MIXED && mine) {
+      const double scale = st.scale;
+#pragma unroll 1
+      for (int m = 0; m < ei; m++) xs[m * nt + t] = (T)(scale * a.x[c0 + m * s1]);
+    }
   }
   // p = r + beta p of the column and of the halo (r of both in place)
   auto direct = [&](T bt, int t1v) {
@@ -527,6 +565,12 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
       const DotAcc<T> none[1];
       G.run(none, sh, [](const double (&)[1]) {});   // every block's part of x is in the box
       take_residual([&](double v) {
+        const double w = v * st.scale * st.scale;
+        if (MIXED && w < CC_LOW && rescale(v)) {
+          st.floor32 = 1;   // no direction is kept
+          st.cancel = 0;
+          return;
+        }
         st.rr_true = v;
         st.since = 0;
         if (MIXED) st.repl++;
@@ -538,8 +582,8 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
         else {
           // mixed, and after a cancelled recurrence: the direction goes on from the replaced residual, unless the
           // recursive one has drifted from it: then the solve starts again from the iterate
-          const bool on = st.cancel || (MIXED && !st.floor32 && st.rr_next > st.thr && v <= CC_DRIFT * st.rr_next);
-          st.beta = on ? (T)(v / st.rr_prev) : T(0);
+          const bool on = st.cancel || (MIXED && !st.floor32 && st.rr_next > st.thr && w <= CC_DRIFT * st.rr_next);
+          st.beta = on ? (T)(w / st.rr_prev) : T(0);
           st.next = CC_GO;
         }
       });
@@ -548,7 +592,7 @@ __global__ void __launch_bounds__(CC_THREADS, 1) k_cg_coop(CoopArgs a) {
     }
   }
   // a solve that ended between two replacements still owes the iterate its last steps
-  put_iterate();
+  if (st.it > 0) put_iterate();
   if (st.fail) S->iscalars[I_ERR] = 1;
   if (blockIdx.x == 0 && t == 0) {
     S->iscalars[I_STATUS] = st.status;
