@@ -432,8 +432,7 @@ int xf_npy_write(const char* path, const xf_vec* vec);
  * (l1, l2) of every array is at offset l1*ls1 + l2*ls2 + m*ms.  All arrays are
  * FP64 device memory (e.g. xf_vec_data of boxes).  The reference's recurrences
  * and operation order: bit-identical results.  Asynchronous on the context
- * stream; uses a context workspace of M * nl1 * nl2 doubles (twice that for
- * lines with ms = 1). */
+ * stream; uses a context workspace of M * nl1 * nl2 doubles. */
 int xf_thomas_lines(xf_ctx* ctx, int M, int nl1, int nl2, int64_t ls1, int64_t ls2, int64_t ms, double* u,
                     const double* a, const double* b, const double* c, const double* f);
 

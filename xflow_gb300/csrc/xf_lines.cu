@@ -21,7 +21,9 @@
 // neighbours in memory (ms = 1, the sweep along k) are staged through shared
 // memory in tiles of LN_TILE steps by asynchronous copies, two tiles in
 // flight: the threads of a warp would otherwise touch a sector each for 8
-// bytes of it.
+// bytes of it.  Their B goes back to u by the same tiles, so that the workspace
+// is A's alone on every axis (a box of its own for B was freed for and allocated
+// again between two axes: the first pass over a 66^3 box took 402 us, 283 now).
 #include "xf_common.cuh"
 
 constexpr int LN_THREADS = 64, LN_STEPS = 4, LN_TILE = 16;
@@ -49,7 +51,6 @@ struct LnArgs {
   const double* __restrict__ c;
   const double* __restrict__ f;
   double* __restrict__ Aw;   // [m][line]
-  double* __restrict__ Bw;   // [m][line] (k_thomas_k)
 };
 
 // Lines side by side in memory.  B[m] waits in u[m] until the back-substitution.
@@ -116,9 +117,9 @@ __device__ __forceinline__ void ln_copy8(double* dst, const double* src) {
 
 // Lines along the memory (ms = 1).
 constexpr int LN_PITCH = LN_TILE + 1;                 // doubles of a line in a tile: 16 lanes hit 32 banks
-constexpr int LN_STAGE = 4 * LN_THREADS * LN_PITCH;   // a, b, c, f
+constexpr int LN_BOX = LN_THREADS * LN_PITCH;         // a tile of one array
 __global__ void __launch_bounds__(LN_THREADS) k_thomas_k(LnArgs g) {
-  extern __shared__ double ln_sm[];
+  extern __shared__ double ln_sm[];   // two stages of a, b, c, f
   __shared__ int64_t bases[LN_THREADS];
   const int t = threadIdx.x;
   const int64_t l0 = blockIdx.x * (int64_t)LN_THREADS, l = l0 + t;
@@ -130,19 +131,32 @@ __global__ void __launch_bounds__(LN_THREADS) k_thomas_k(LnArgs g) {
   __syncthreads();
   const int last = g.M - 1;
   // a half warp a line: LN_TILE consecutive elements of each array
+  const int e = t % LN_TILE, q0 = t / LN_TILE;
+  constexpr int LINES = LN_THREADS / LN_TILE;
   auto stage = [&](int tile) {
-    double* s = ln_sm + (tile & 1) * LN_STAGE;
-    const int e = t % LN_TILE, m = 1 + tile * LN_TILE + e;
+    double* s = ln_sm + (tile & 1) * 4 * LN_BOX + e;
+    const int m = 1 + tile * LN_TILE + e;
     if (m <= last)
-      for (int q = t / LN_TILE; q < LN_THREADS; q += LN_THREADS / LN_TILE) {
+      for (int q = q0; q < LN_THREADS; q += LINES) {
         const int64_t src = bases[q] + m;
-        double* dst = s + q * LN_PITCH + e;
+        double* dst = s + q * LN_PITCH;
         ln_copy8(dst, g.a + src);
-        ln_copy8(dst + LN_THREADS * LN_PITCH, g.b + src);
-        ln_copy8(dst + 2 * LN_THREADS * LN_PITCH, g.c + src);
-        ln_copy8(dst + 3 * LN_THREADS * LN_PITCH, g.f + src);
+        ln_copy8(dst + LN_BOX, g.b + src);
+        ln_copy8(dst + 2 * LN_BOX, g.c + src);
+        ln_copy8(dst + 3 * LN_BOX, g.f + src);
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto stage_u = [&](int tile) {
+    const int m = 1 + tile * LN_TILE + e;
+    if (tile >= 0 && m <= last)
+      for (int q = q0; q < LN_THREADS; q += LINES) ln_copy8(ln_sm + (tile & 1) * LN_BOX + q * LN_PITCH + e, g.u + bases[q] + m);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto put_u = [&](int tile, const double* box) {   // between two block barriers
+    const int m = 1 + tile * LN_TILE + e;
+    if (m <= last)
+      for (int q = q0; q < LN_THREADS && l0 + q < g.nl; q += LINES) g.u[bases[q] + m] = box[q * LN_PITCH + e];
   };
   const int tiles = (last + LN_TILE - 1) / LN_TILE;
   double A = 0, B = g.u[base];
@@ -151,46 +165,40 @@ __global__ void __launch_bounds__(LN_THREADS) k_thomas_k(LnArgs g) {
     stage(tile + 1);   // past the end: an empty group
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    const double* s = ln_sm + (tile & 1) * LN_STAGE + t * LN_PITCH;
+    double* s = ln_sm + (tile & 1) * 4 * LN_BOX + t * LN_PITCH;
     const int m0 = 1 + tile * LN_TILE;
 #pragma unroll 4
     for (int q = 0; q < LN_TILE; q++) {
       const int m = m0 + q;
       if (m > last) break;
-      ln_step(s[q], s[LN_THREADS * LN_PITCH + q], s[2 * LN_THREADS * LN_PITCH + q], s[3 * LN_THREADS * LN_PITCH + q], A, B);
-      if (mine) {
-        g.Aw[(int64_t)m * g.nl + l] = A;
-        g.Bw[(int64_t)m * g.nl + l] = B;
-      }
+      ln_step(s[q], s[LN_BOX + q], s[2 * LN_BOX + q], s[3 * LN_BOX + q], A, B);
+      if (mine) g.Aw[(int64_t)m * g.nl + l] = A;
+      s[3 * LN_BOX + q] = B;
     }
+    __syncthreads();
+    put_u(tile, s + 3 * LN_BOX - t * LN_PITCH);
     __syncthreads();   // the tile's place is filled again two stages on
   }
   double un = g.u[base + g.M];
-  constexpr int BS = 2 * LN_STEPS;
+  stage_u(tiles - 1);
   for (int tile = tiles - 1; tile >= 0; tile--) {
     const int m0 = 1 + tile * LN_TILE;
-    double* row = ln_sm + t * LN_PITCH;
+    double a[LN_TILE];
 #pragma unroll
-    for (int half = LN_TILE / BS - 1; half >= 0; half--) {
-      double a[BS], b[BS];
-#pragma unroll
-      for (int q = 0; q < BS; q++) {
-        const int m = min(m0 + half * BS + q, last);
-        a[q] = g.Aw[(int64_t)m * g.nl + lc];
-        b[q] = g.Bw[(int64_t)m * g.nl + lc];
-      }
-#pragma unroll
-      for (int q = BS - 1; q >= 0; q--)
-        if (m0 + half * BS + q <= last) {
-          un = a[q] * un + b[q];
-          row[half * BS + q] = un;
-        }
-    }
+    for (int q = 0; q < LN_TILE; q++) a[q] = g.Aw[(int64_t)min(m0 + q, last) * g.nl + lc];
+    stage_u(tile - 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    const int e = t % LN_TILE, m = m0 + e;
-    if (m <= last)
-      for (int q = t / LN_TILE; q < LN_THREADS && l0 + q < g.nl; q += LN_THREADS / LN_TILE)
-        g.u[bases[q] + m] = ln_sm[q * LN_PITCH + e];
+    double* box = ln_sm + (tile & 1) * LN_BOX;
+    double* row = box + t * LN_PITCH;
+#pragma unroll
+    for (int q = LN_TILE - 1; q >= 0; q--)
+      if (m0 + q <= last) {
+        un = a[q] * un + row[q];
+        row[q] = un;
+      }
+    __syncthreads();
+    put_u(tile, box);
     __syncthreads();
   }
 }
@@ -202,14 +210,12 @@ extern "C" int xf_thomas_lines(xf_ctx* ctx, int M, int nl1, int nl2, int64_t ls1
   const int64_t nl = (int64_t)nl1 * nl2;
   if (nl == 0 || M == 1) return XF_OK;   // nothing between the two boundary values
   XF_CUDA(ctx, cudaSetDevice(ctx->device));
-  // along the memory, where neighbouring lines are not one element apart; B needs a box of its own there
-  const bool along = ms == 1 && !(nl2 > 1 ? ls2 == 1 : ls1 == 1);
-  double* Aw = (double*)xf_ctx_work(ctx, (size_t)M * nl * sizeof(double) * (along ? 2 : 1));
+  double* Aw = (double*)xf_ctx_work(ctx, (size_t)M * nl * sizeof(double));
   if (!Aw) return xf_fail(ctx, XF_ERR_NOMEM, "xf_thomas_lines: workspace of %lld doubles", (long long)(M * nl));
-  LnArgs g = {M, nl2, nl, ls1, ls2, ms, u, a, b, c, f, Aw, along ? Aw + (size_t)M * nl : nullptr};
+  LnArgs g = {M, nl2, nl, ls1, ls2, ms, u, a, b, c, f, Aw};
   const unsigned blocks = (unsigned)((nl + LN_THREADS - 1) / LN_THREADS);
-  if (along) {
-    const int smem = 2 * LN_STAGE * (int)sizeof(double);
+  if (ms == 1 && !(nl2 > 1 ? ls2 == 1 : ls1 == 1)) {   // along the memory, and neighbouring lines not one element apart
+    const int smem = 2 * 4 * LN_BOX * (int)sizeof(double);
     XF_CUDA(ctx, cudaFuncSetAttribute(k_thomas_k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     k_thomas_k<<<blocks, LN_THREADS, smem, ctx->stream>>>(g);
   } else {
