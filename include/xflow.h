@@ -235,7 +235,10 @@ enum { XF_PREC_FP64 = 0, XF_PREC_MIXED = 1 };
  * the border rows' own): the residual and the stop rule stay those of
  * A x = b, and rows of very different scales (semi-sums of 1/2, normal
  * differences of 1/h, Actual rows of 1/h^2 or 1/tau) no longer slow the
- * iteration down. */
+ * iteration down.  A transport operator of half a million cells or more keeps
+ * a scaled copy of its rows for these solves, 49 bytes a cell, from the first
+ * of them until it is destroyed; a solve that has no room beside it gives it
+ * back. */
 enum { XF_PRECOND_NONE = 0, XF_PRECOND_JACOBI = 1, XF_PRECOND_UNET = 2, XF_PRECOND_CHEB = 3, XF_PRECOND_UNET2 = 4 };
 /* Host only (no device work): the XF_PRECOND_CHEB polynomial as the solver
  * builds it, in powers of A.  degree 2 writes its three Horner coefficients

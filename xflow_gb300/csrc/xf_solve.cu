@@ -55,6 +55,7 @@ int xf_op_ready(const xf_op* op);
 void xf_op_ready32(const xf_op* op);
 int xf_op_jacobi(const xf_op* op, const double** dinv);
 bool xf_op_scaled(const xf_op* op);
+void xf_op_scaled_free(const xf_op* op);
 void xf_op_unscale(const xf_op* op, double* x, const double* y);
 
 #define GUARD_DONE(S) \
@@ -487,15 +488,20 @@ struct Bufs {
     ptrs.push_back(p);
     return (T*)p;
   }
-  // `count` zeroed boxes of n values as one allocation and one fill, 256-byte aligned; false when it cannot be had
+  // Zeroed boxes of n values as one allocation and one fill, 256-byte aligned, or one by one where that cannot be had;
+  // false, and none of them kept, when neither can.
   template <typename T, class... P>
   bool boxes(int64_t n, P&... out) {
     const int64_t pitch = (n * (int64_t)sizeof(T) + 255) / 256 * 256;
-    char* p = get<char>(pitch * (int64_t)sizeof...(out));
-    if (!p) return false;
-    int q = 0;
-    ((out = (T*)(p + pitch * q++)), ...);
-    return true;
+    const size_t had = ptrs.size();
+    if (char* p = get<char>(pitch * (int64_t)sizeof...(out))) {
+      int q = 0;
+      ((out = (T*)(p + pitch * q++)), ...);
+      return true;
+    }
+    if ((((out = get<T>(n)) != nullptr) && ...)) return true;
+    for (; ptrs.size() > had; ptrs.pop_back()) cudaFreeAsync(ptrs.back(), ctx->stream);
+    return false;
   }
   ~Bufs() {
     for (void* p : ptrs) cudaFreeAsync(p, ctx->stream);
@@ -928,6 +934,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
   std::function<void(int)> iter;
   bool scaled = false;     // BiCGStab on A D^-1, its x gathered in xs
   double* xs = nullptr;
+  double* spare = nullptr;   // a vector of the iteration, for the true residual after it
   int launches = 0;   // kernels an iteration
   reset_progress(ctx);
   HostState hs = {0, 0, 0, 0, 0};
@@ -973,12 +980,18 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
     // a unit diagonal: the predictors of 512 x 128 x 128 26.3 -> 24.2 ms, the
     // scalar of 256 x 64 x 64 1.53 -> 1.51; at 64^3 (2.45 ms either way) the
     // table costs what it gains, so smaller boxes keep to the copies.
+    // The table is 49 bytes a cell that stay with the operator; where it leaves no
+    // room for the vectors it is given back, and the copies are taken.
     scaled = jacobi && !exact && n >= SCALED_MIN_CELLS && xf_op_scaled(op);
     double *Rn, *sRn, *Pn, *Pn1, *Vn, *Sn, *Tn, *Ph = nullptr, *Sh = nullptr;
-    if (!(scaled ? B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn, xs)
-          : jacobi ? B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn, Ph, Sh)
-                 : B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn)))
+    if (scaled && !B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn, xs)) {
+      xf_op_scaled_free(op);
+      scaled = false;
+    }
+    if (!scaled && !(jacobi ? B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn, Ph, Sh)
+                            : B.boxes<double>(n, Rn, sRn, Pn, Pn1, Vn, Sn, Tn)))
       return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
+    spare = Tn;
     // Rn = b - A(Un)
     MvReq<double> q0;
     q0.x = x; q0.y = Rn; q0.s = b; q0.sign = -1; q0.neg = 1; q0.exact = exact;
@@ -1070,7 +1083,7 @@ static int solve_reference(xf_op* op, const xf_solve_opts& o, xf_vec* xv, const 
   int rc = run_stream(ctx, iter, launches, STREAM_AHEAD, o.maxit, &hs);
   if (rc) return rc;
   if (scaled) xf_op_unscale(op, x, xs);
-  double* tmp = B.get<double>(n, false);
+  double* tmp = spare ? spare : B.get<double>(n, false);
   if (!tmp) return xf_fail(ctx, XF_ERR_NOMEM, "xf_solve: allocation");
   double rel = 0;
   int r2 = true_residual(op, x, b, tmp, &rel, &hs);   // leaves the scalars in the pinned buffer

@@ -604,6 +604,13 @@ bool xf_op_scaled(const xf_op* op) {
   op->ads_valid = 1;
   return true;
 }
+void xf_op_scaled_free(const xf_op* op) {
+  cudaFree(op->ads64);
+  cudaFree(op->adks);
+  op->ads64 = nullptr;
+  op->adks = nullptr;
+  op->ads_valid = 0;
+}
 void xf_op_unscale(const xf_op* op, double* x, const double* y) {
   const xf_grid* g = op->g;
   k_ad_unscale<<<grid_blocks(g->ctx, g->ncell, 256), 256, 0, g->ctx->stream>>>(x, y, op->adj64, g->smask, g->ncell);
