@@ -52,3 +52,23 @@ def test_strides_wider_than_a_line(ctx):
 @pytest.mark.parametrize("M", [2, 17, 50])
 def test_divisors_at_the_ends_of_the_range(ctx, M):
     lines(ctx, M, 40, 20, 20 * (M + 1), M + 1, 800 * (M + 1), extreme=True)
+
+
+@pytest.mark.parametrize("shape", [(20, 5, 37), (34, 18, 16)])
+@pytest.mark.parametrize("axis", [1, 2, 3])
+def test_right_hand_side_in_place(ctx, axis, shape):
+    """f and u the same array: every f[m] is read before u[m] is written."""
+    rng = np.random.default_rng(axis)
+    a, c = rng.uniform(-1, 0, shape), rng.uniform(-1, 0, shape)
+    b, u = 2.5 + rng.uniform(0, 1, shape), rng.standard_normal(shape)
+    dev = [torch.from_numpy(t.copy()).cuda() for t in (u, a, b, c)]
+    torch.cuda.synchronize()
+    M, *where = xf.box_lines(shape, axis)
+    pu, pa, pb, pc = (t.data_ptr() for t in dev)
+    xf.thomas_lines(ctx, M, pu, pa, pb, pc, pu, *where)
+    ctx.synchronize()
+    want = u.copy()
+    W, A, B, C, F = (np.moveaxis(t, axis - 1, -1) for t in (want, a, b, c, u))
+    for at in np.ndindex(W.shape[:-1]):
+        W[at] = O.thomas(M, W[at], A[at], B[at], C[at], F[at])
+    np.testing.assert_array_equal(dev[0].cpu().numpy(), want)
