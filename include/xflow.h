@@ -258,8 +258,11 @@ typedef struct {
   double atol;           /* absolute tolerance of the reference-semantics methods; */
                          /* <= 0 means the reference's hard-coded value            */
   int replace_every;     /* mixed: true-residual replacement period (50)           */
-  int check_every;       /* accepted, without effect: the host watches a word that  */
-                         /* the device writes at the end of every iteration (16)   */
+  int check_every;       /* FP64 CG of grids beyond the resident kernel: the host   */
+                         /* looks for the end every this many iterations (16).     */
+                         /* Without effect elsewhere: mixed CG looks every         */
+                         /* replace_every, the resident CG and the                 */
+                         /* reference-semantics methods at every iteration's end   */
   int exact;             /* reference-semantics methods: use XF_EXACT matvecs      */
   int reserved[7];
 } xf_solve_opts;

@@ -40,7 +40,10 @@
 // All scalar work (the divisions behind alpha and beta, the tests) is one
 // thread's, and the mixed solve's sums travel as float-float: an FP64
 // instruction takes 16 cycles of the SM's FP64 pipe, and 16 warps repeating
-// the scalars were a third of an iteration.
+// the scalars were a third of an iteration.  Float-float across warps and
+// blocks too leaves a sum of a million products off by 2e-15 on average and
+// 5e-15 at most (2e-15 at most with FP64 from the warps on, for 0.5 us an
+// iteration more); alpha and beta are rounded to FP32 right after.
 //
 // The mixed solve folds e into the FP64 iterate and takes r = b - A x in FP64
 // every `every` iterations and whenever the FP32 recursion meets the
@@ -662,14 +665,15 @@ const void* kernel_for(int bi) {
 
 }  // namespace
 
-// Uniform Laplace grids without border rows whose interior fits the chip (up
-// to 1.2 million cells on 152 SMs): there it is the faster form throughout,
-// and past that the vectors no longer fit, so the kernel chain takes over.
-// Measured on GB300, a projection solved to 1e-12 (us an iteration), chain
-// and resident: 64^3 FP64 39.0 and 16.5; 75 x 61 x 83 mixed 23.3 and 7.0;
-// 256 x 64 x 64 mixed 24.3 and 9.4.  What bounds it now: FP64 issue (14
-// operations a cell) in the first, the grid sum (3 us) and the reductions
-// before it in the others.
+// Uniform Laplace grids without border rows whose interior fits the chip (16
+// cells a column, 512 columns a brick, a brick an SM: on 152 SMs 102^3 and
+// 128 x 152 x 64 do, 104 x 108 x 104 does not): there it is the faster form
+// throughout, and past that the vectors no longer fit, so the kernel chain takes
+// over.  Measured on GB300 (us an iteration), chain and resident: 64^3 FP64 39.0
+// and 14.6; 75 x 61 x 83 mixed 23.3 and 6.6; 256 x 64 x 64 mixed 24.3 and 9.25;
+// 128 x 152 x 64 FP64 60.4 and 40.2, mixed 25.1 and 10.7.  What bounds it now:
+// FP64 issue (14 operations a cell) in the first, rows 6.1, update 3.3, grid sum
+// with its reductions and scalars 5.0; the grid sum (3.8 to 4.1) in the mixed ones.
 // The split depends on the grid's extents alone and stays with the grid.
 bool xf_cg_coop_supported(const xf_op* op, bool mixed) {
   xf_grid* g = op->g;

@@ -712,7 +712,8 @@ static cudaError_t set_max_smem(const void* kern, int which, int device, size_t 
 // of 130 cells a cell (16 bytes) apart, into accumulators of their own: a row
 // tile of single taps copied every block three times, and the copies were what
 // bound it (48 -> 16 at 66^3: 880 MB from L2 in 107 us, now 280 MB in 77; 96 -> 32
-// at 34^3 58 -> 27).  Now the MMAs do, about 60 cycles each.  A stage is 128 cells:
+// at 34^3 58 -> 27).  Now shared memory does (58 to 62% of its throughput, the tensor
+// pipe at 7 to 11%): an MMA of N = 16 takes about 60 cycles.  A stage is 128 cells:
 // per group of the row tile and per plane of g one bulk copy (one per lane of
 // the producer warp), eight K steps of 16 cells, three MMAs each.  Each CTA
 // takes one row tile and one range of cells (a multiple of 128: the cells past
@@ -944,8 +945,6 @@ __global__ void __launch_bounds__(256) k_grad_sum(const __grid_constant__ WgSegs
 int xf_grad_sum_blocks(int ci, int co) { return 27 * co * ci / 256 + 1; }
 void xf_grad_sum(xf_ctx* ctx, const WgSegs& segs, int blocks) { launch_dep(k_grad_sum, dim3(blocks), 256, 0, ctx->stream, segs); }
 
-// The row tiles and cell ranges of a layer's weight gradient, and the FP32
-// partial buffer it needs (floats).
 // Chunks of the bias gradient: 4,096 cells, or more in steps of 256 so that there are at most 128.
 void xf_bgrad_plan(int64_t ncell, int* nchunk, int* chunk) {
   int64_t c = ((ncell + 127) / 128 + 255) / 256 * 256;
@@ -953,6 +952,7 @@ void xf_bgrad_plan(int64_t ncell, int* nchunk, int* chunk) {
   *chunk = (int)c;
   *nchunk = (int)((ncell + c - 1) / c);
 }
+// The row tiles and cell ranges of a layer's weight-gradient partials, and the FP32 buffer they need (floats).
 void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mtiles, int* splits, int* stages,
                       int64_t* partial_floats) {
   const int taps = 128 / ci;
@@ -966,9 +966,10 @@ void xf_wgrad_tc_plan(const xf_ctx* ctx, int64_t ncell, int ci, int co, int* mti
   *partial_floats = (int64_t)*mtiles * *splits * 128 * co;
 }
 
-// gw ([27][co][ci] FP32) += the weight gradient of g (co channels) against x
-// (ci channels), both BF16 planes with their zero margins; partial holds
-// xf_wgrad_tc_plan's floats.  ci and co multiples of 16, ci <= 128, co <= 64.
+// The partials of the weight gradient of g (co channels) against x (ci channels),
+// both BF16 planes with their zero margins, into `partial` (xf_wgrad_tc_plan's
+// floats), and of the bias gradient into bpart; xf_grad_sum adds them.  ci and co
+// multiples of 16, ci <= 128, co <= 64.
 int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps, int co, const void* x, int64_t xps,
                 int ci, float* partial, float* bpart) {
   if (ci % 16 || co % 16 || ci < 16 || ci > 128 || co < 16 || co > 64)
@@ -1001,10 +1002,9 @@ int xf_wgrad_tc(xf_ctx* ctx, int n1, int n2, int n3, const void* g, int64_t gps,
   return XF_OK;
 }
 
-// Launch on the context stream (arguments checked by the caller).  `weights`
-// is [27][co][ci]; `tiled` the same in the tiled order (needed when 3 co <= 256).
-// `tiled`: the weights in conv_tiled_index order.  dep: launched by launch_dep,
-// the weights not written by the kernel before.
+// Launch on the context stream (arguments checked by the caller).  `tiled`: the
+// weights in conv_tiled_index order.  dep: launched by launch_dep, the weights not
+// written by the kernel before.
 int xf_conv_launch(xf_ctx* ctx, int n1, int n2, int n3, const void* in, int64_t in_ps, int ci, const void* tiled,
                    const float* bias, int co, const uint8_t* mask, void* out, int64_t out_pitch, int out_ch,
                    int out_fp32, int relu, const void* gate, int64_t gate_ps, bool dep) {

@@ -74,7 +74,10 @@ __device__ __forceinline__ void tl_z(DevScratch* S, const TlStep& t) {
 }
 
 // (p, q) is known.  (p, r) = (z, r): r is orthogonal to every direction of the
-// window after its line search.
+// window after its line search, up to FP32's rounding and what a refresh of r
+// changes.  That makes alpha's error up to 3e-5 late in a cycle (1e-6 with (p, r)
+// measured, which costs the direction pass a stream more); a step's part of the
+// decrease loses its square, and the iterations are as many.
 __device__ __forceinline__ void tl_alpha(DevScratch* S, const TlStep& t) {
   TlCtl* c = t.ctl;
   const double pr = S->scalars[FS_ZR], pq = S->scalars[FS_PQ];
